@@ -215,9 +215,10 @@ B200Q_HD void gemv_load_x(int lane, int s, int nblk, const GemvAct &act, const i
     }
 }
 
-// sw: the staged words of one weight row for the stage X was loaded for. acc[c] += partial.
+// sw: the staged words of one weight row for the stage X was loaded for, off0 bytes into them (rows that begin inside a
+// 16-byte unit: an even number, a multiple of 8 for IQ4_XS; 0 for Q4_K and Q5_K). acc[c] += partial.
 template <int TYPE, int NC>
-B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X, float (&acc)[NC]) {
+B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X, float (&acc)[NC], uint32_t off0 = 0) {
     typedef GemvFmt<TYPE> F;
     const Stage sw(sw_ptr);
     if (TYPE == B200Q_TYPE_Q4_0) {
@@ -227,7 +228,7 @@ B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X
 #ifdef B200Q_RED_DROP
             if (((32 * u + lane) & 7) == 7) continue;
 #endif
-            const uint32_t off = (uint32_t)F::BLK_B * (uint32_t)(32 * u + lane);
+            const uint32_t off = off0 + (uint32_t)F::BLK_B * (uint32_t)(32 * u + lane);
             const float d = hd_half_bits(stage_u16(sw, off));
             uint32_t q[4];
             stage_words<4>(sw, off + 2, q);
@@ -250,7 +251,7 @@ B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             if (!(u ? X.live2 : X.live)) continue;
-            const uint32_t off = (uint32_t)F::BLK_B * (uint32_t)(32 * u + lane);
+            const uint32_t off = off0 + (uint32_t)F::BLK_B * (uint32_t)(32 * u + lane);
             const float d = hd_half_bits(stage_u16(sw, off));
             uint32_t q[4], lo[4], hi[4];
             stage_words<4>(sw, off + 2, q);
@@ -276,7 +277,7 @@ B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X
 #ifdef B200Q_RED_DROP
             if (((32 * u + lane) & 7) == 7) continue;
 #endif
-            const uint32_t off = (uint32_t)F::BLK_B * (uint32_t)(32 * u + lane);
+            const uint32_t off = off0 + (uint32_t)F::BLK_B * (uint32_t)(32 * u + lane);
             const float d = hd_half_bits(stage_u16(sw, off));
             uint32_t w[8];
             stage_words<8>(sw, off + 2, w);
@@ -384,7 +385,7 @@ B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X
     } else if (TYPE == B200Q_TYPE_IQ4_XS) {
         if (!X.live) return;
         const int sb = lane >> 2, pp = lane & 3;
-        const uint32_t bw = sb * (136 / 4);                 // word index; blocks are 8-byte aligned inside the stage
+        const uint32_t bw = (off0 >> 2) + sb * (136 / 4);                 // word index; blocks are 8-byte aligned inside the stage
         const uint32_t hd = sw.w(bw), sl = sw.w(bw + 1);
         const float d = hd_half_bits((uint16_t)hd);
         const int ls0 = iq4xs_ls(hd >> 16, sl, 2 * pp) - 32, ls1 = iq4xs_ls(hd >> 16, sl, 2 * pp + 1) - 32;
@@ -414,7 +415,7 @@ B200Q_HD void gemv_lane_row(const uint32_t *sw_ptr, int lane, const GemvX<NC> &X
     } else if (TYPE == B200Q_TYPE_Q6_K) {
         if (!X.live) return;
         const int sb = lane >> 2, n = (lane >> 1) & 1, hi16 = lane & 1, t0 = 16 * hi16;
-        const uint32_t off = 210u * (uint32_t)sb;
+        const uint32_t off = off0 + 210u * (uint32_t)sb;
         uint32_t qa[4], qb[4], qh[4], scw[2];
         stage_words<4>(sw, off + 64 * n + t0, qa);            // parts 0 (low) and 2 (high)
         stage_words<4>(sw, off + 64 * n + 32 + t0, qb);       // parts 1 and 3

@@ -39,6 +39,20 @@ struct GemvId {
     int64_t        ld1, ld2;        // dst strides of slot i and token t, in floats
 };
 
+// How a product's rows lie: every row a 16-byte multiple from a 16-byte start; rows whose starts are only a multiple of what
+// the lane code needs (gemv_row_align); anything else.
+enum { GEMV_ROWS_BYTES = 0, GEMV_ROWS_ALIGNED = 1, GEMV_ROWS_SHIFTED = 2 };
+// the start alignment with which the lane code takes a row: words at any even byte, 8 bytes (IQ4_XS), 16 (Q4_K, Q5_K)
+__host__ __device__ constexpr int gemv_row_align(int type) {
+    return type == B200Q_TYPE_Q4_K || type == B200Q_TYPE_Q5_K ? 16 : type == B200Q_TYPE_IQ4_XS ? 8 : 2;
+}
+// all_starts: the matrix address and every stride between rows (and experts) or-ed together
+inline int gemv_row_mode(int type, size_t all_starts, size_t row_bytes) {
+    if (all_starts % 16 == 0 && row_bytes % 16 == 0) return GEMV_ROWS_ALIGNED;
+    return all_starts % (size_t)gemv_row_align(type) == 0 ? GEMV_ROWS_SHIFTED : GEMV_ROWS_BYTES;
+}
+template <int TYPE> __host__ __device__ constexpr int gemv_kernel_slot(int rows) { return GemvStage<TYPE>::SLOT + (rows == GEMV_ROWS_SHIFTED ? 16 : 0); }
+
 // One warp owns a batch of B consecutive rows at a time and walks the row in stages of 2048
 // weights. For each stage it holds the activation side (64 codes per lane and column, scales,
 // block sums) in registers and runs the B staged row chunks against it, so the activation
@@ -46,7 +60,10 @@ struct GemvId {
 // arrive through a per-warp ring of NSETS sets of B slots filled with 16-byte asynchronous
 // copies: NSETS-1 sets are in flight while the current one is consumed. More
 // than four columns are taken as two column groups over the same staged set.
-template <int TYPE, int NC, int B, int WARPS, int NSETS, bool ALIGNED, bool ID>
+// ROWS: how the rows lie (gemv_row_mode): 16-byte aligned, shifted (a row's stage starts anywhere in a 16-byte unit: the
+// copies start at the boundary below and the lane code adds the remainder; a copy never leaves the 16-byte units that
+// hold the row's own bytes) or fetched two bytes at a time.
+template <int TYPE, int NC, int B, int WARPS, int NSETS, int ROWS, bool ID>
 __global__ void __launch_bounds__(WARPS * 32)
 gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, GemvAct act,
             float *__restrict__ dst, int ldd, GemvId id) {
@@ -55,10 +72,11 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
     constexpr int NCG = NC <= 4 ? NC : (NC + 1) / 2;      // columns of the first group
     constexpr int NC2 = NC - NCG;                         // columns of the second group (0: none)
     constexpr int N2 = NC2 > 0 ? NC2 : 1;
-    constexpr int PIECES = (S::BYTES + 511) / 512;        // 16-byte copies per lane and chunk
+    constexpr int SLOT = gemv_kernel_slot<TYPE>(ROWS);
+    constexpr int PIECES = (S::BYTES + (ROWS == GEMV_ROWS_SHIFTED ? 15 : 0) + 511) / 512;        // 16-byte copies per lane and chunk
     extern __shared__ __align__(16) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *ring = smem + warp * (NSETS * B * S::SLOT);
+    uint8_t *ring = smem + warp * (NSETS * B * SLOT);
     if (ID) pdl_wait();                  // the route (tile lists, counts) comes from the kernel before
 
     const int row_bytes = nblk * F::BLK_B;
@@ -83,11 +101,18 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
             const int row0 = (ID ? p_u % n_bt : p_u) * B;
             const uint8_t *src = W + (size_t)row0 * row_stride + off;
             if (ID) src += (size_t)(direct ? pair_expert(p_u / n_bt) : __ldg(id.tiles + 4 * (p_u / n_bt))) * id.expert_stride;
-            uint8_t *d = ring + p_set * (B * S::SLOT);
+            uint8_t *d = ring + p_set * (B * SLOT);
 #pragma unroll
             for (int r = 0; r < B; ++r) {
                 if (row0 + r < M) {              // rows past the end keep stale bytes; never stored
-                    if (ALIGNED) {
+                    if (ROWS == GEMV_ROWS_SHIFTED) {
+                        const int sh = (int)((uintptr_t)src & 15);
+#pragma unroll
+                        for (int j = 0; j < PIECES; ++j) {
+                            const int b = lane * 16 + j * 512;
+                            if (b < sh + bytes) cp_async16(d + b, src - sh + b);
+                        }
+                    } else if (ROWS == GEMV_ROWS_ALIGNED) {
 #pragma unroll
                         for (int j = 0; j < PIECES; ++j) {
                             const int b = lane * 16 + j * 512;
@@ -99,7 +124,7 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
                     }
                 }
                 src += row_stride;
-                d += S::SLOT;
+                d += SLOT;
             }
             if (++p_s == nstages) { p_s = 0; p_u += tw; }
         }
@@ -119,10 +144,12 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
         int cols[NC];
         int64_t outs[NC];
         int ncol = NC;
+        uintptr_t wbase = (uintptr_t)W;                    // where the unit's matrix begins (shifted rows)
         if (ID) {
             const int tile = u / n_bt;
             const int first = direct ? tile : __ldg(id.tiles + 4 * tile + 1);
             ncol = direct ? 1 : __ldg(id.tiles + 4 * tile + 2);
+            if (ROWS == GEMV_ROWS_SHIFTED) wbase += (size_t)(direct ? pair_expert(tile) : __ldg(id.tiles + 4 * tile)) * id.expert_stride;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const int p = direct ? tile : __ldg(id.pairs + first + min(c, ncol - 1));   // short tiles repeat their last pair
@@ -143,12 +170,16 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
         for (int r = 0; r < B; ++r)
 #pragma unroll
             for (int c = 0; c < NC; ++c) acc[r][c] = 0.f;
+        const int row0 = (ID ? u % n_bt : u) * B;
+        uint32_t shift[B];                                 // a stage is a multiple of 16 bytes: the same for all of a row's
+#pragma unroll
+        for (int r = 0; r < B; ++r) shift[r] = ROWS == GEMV_ROWS_SHIFTED ? (uint32_t)(wbase + (size_t)(row0 + r) * row_stride) & 15u : 0u;
         for (int s = 0; s < nstages; ++s) {
             __syncwarp();                    // every lane is done with the set about to be refilled
             issue();
             cp_async_wait<NSETS - 1>();      // all but the NSETS-1 newest sets have landed
             __syncwarp();
-            const uint8_t *set = ring + c_set * (B * S::SLOT);
+            const uint8_t *set = ring + c_set * (B * SLOT);
             c_set = c_set + 1 == NSETS ? 0 : c_set + 1;
             {
                 GemvX<NCG> X;
@@ -158,7 +189,7 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
                     float a[NCG];
 #pragma unroll
                     for (int c = 0; c < NCG; ++c) a[c] = acc[r][c];
-                    gemv_lane_row<TYPE, NCG>(reinterpret_cast<const uint32_t *>(set + r * S::SLOT), lane, X, a);
+                    gemv_lane_row<TYPE, NCG>(reinterpret_cast<const uint32_t *>(set + r * SLOT), lane, X, a, shift[r]);
 #pragma unroll
                     for (int c = 0; c < NCG; ++c) acc[r][c] = a[c];
                 }
@@ -171,14 +202,13 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
                     float a[N2];
 #pragma unroll
                     for (int c = 0; c < N2; ++c) a[c] = acc[r][second_group_index<NCG, NC2>(c)];
-                    gemv_lane_row<TYPE, N2>(reinterpret_cast<const uint32_t *>(set + r * S::SLOT), lane, X, a);
+                    gemv_lane_row<TYPE, N2>(reinterpret_cast<const uint32_t *>(set + r * SLOT), lane, X, a, shift[r]);
 #pragma unroll
                     for (int c = 0; c < N2; ++c)
                         if (c < NC2) acc[r][second_group_index<NCG, NC2>(c)] = a[c];
                 }
             }
         }
-        const int row0 = (ID ? u % n_bt : u) * B;
 #pragma unroll
         for (int r = 0; r < B; ++r)
 #pragma unroll

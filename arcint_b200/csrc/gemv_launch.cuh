@@ -1,0 +1,333 @@
+// gemv_launch.cuh -- host side of the decode GEMV, per weight type: which kernel, tile and grid a product gets. The templates
+// are instantiated one weight type to a translation unit (gemv_<type>.cu), so that the types compile side by side.
+#pragma once
+
+#include "gemv_kernel.cuh"
+#include "gemv_stream.cuh"
+#include "gemv_mma.cuh"
+#include "common.cuh"
+
+#include <limits.h>
+
+namespace b200q {
+
+template <int TYPE, int NC, int B, int WARPS, int NSETS, bool ID>
+static b200q_status launch_one(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K,
+                               const GemvAct &act, float *dst, int64_t ldd, int rows, const GemvId &id,
+                               int64_t max_tiles) {
+    const size_t smem = (size_t)WARPS * NSETS * B * gemv_kernel_slot<TYPE>(rows);
+    if (M > INT32_MAX / 2 || K / GemvFmt<TYPE>::BLK_W > INT32_MAX / 256 || ldd > INT32_MAX)
+        return fail(ctx, B200Q_UNSUPPORTED, "gemv: dimensions beyond 32-bit indexing");
+    auto kern = gemv_kernel<TYPE, NC, B, WARPS, NSETS, GEMV_ROWS_BYTES, ID>;
+    if (rows == GEMV_ROWS_ALIGNED) kern = gemv_kernel<TYPE, NC, B, WARPS, NSETS, GEMV_ROWS_ALIGNED, ID>;
+    // (Q4_K and Q5_K rows are never shifted: their blocks are 16-byte multiples and need 16-byte starts)
+    if constexpr (gemv_row_align(TYPE) < 16)
+        if (rows == GEMV_ROWS_SHIFTED) kern = gemv_kernel<TYPE, NC, B, WARPS, NSETS, GEMV_ROWS_SHIFTED, ID>;
+    // resident CTAs per SM of this instantiation, asked once: the grid is one full wave of
+    // persistent CTAs (or fewer when the work is small) and each warp strides over its units
+    static int occ_dev[B200Q_MAX_DEVICES][3] = {};
+    int *occ = occ_dev[ctx->device % B200Q_MAX_DEVICES];
+    if (occ[rows] == 0) {
+        if (smem > 48 * 1024)
+            B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int n = 0;
+        B200Q_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, WARPS * 32, smem));
+        occ[rows] = n > 0 ? n : 1;
+    }
+    const int64_t n_bt = (M + B - 1) / B;
+    const int64_t n_units = ID ? n_bt * max_tiles : n_bt;      // ID: an upper bound, the kernel reads the count
+    int64_t blocks = (n_units + WARPS - 1) / WARPS;
+    const int64_t cap = (int64_t)ctx->sm_count * occ[rows];
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3((unsigned)blocks), dim3(WARPS * 32), smem, ctx->stream,
+                               (const uint8_t *)w, row_stride, (int)M, (int)(K / GemvFmt<TYPE>::BLK_W), act, dst, (int)ldd, id));
+    B200Q_CUDA(ctx, cudaGetLastError());
+    return B200Q_OK;
+}
+
+// One launch of the slice-resident kernel built with the launch bounds (MAXT, MINB); resident blocks per SM for the
+// block shape are asked once per (device, shape).
+template <int TYPE, int NC, int R, int NSETS, bool QX, bool AR, int MAXT, int MINB, bool SH>
+static b200q_status launch_stream_kernel(b200q_ctx *ctx, int threads, size_t smem, int groups, const void *w, size_t row_stride, int64_t M,
+                                         int nblk, const GemvAct &act, float *dst, int64_t ldd, const GemvAr &ar_args) {
+    auto kern = gemv_stream_kernel<TYPE, NC, R, NSETS, QX, AR, MAXT, MINB, SH>;
+    struct Occ { int threads; size_t smem; int blocks; bool attr; };
+    static Occ occ_dev[B200Q_MAX_DEVICES] = {};
+    Occ &o = occ_dev[ctx->device % B200Q_MAX_DEVICES];
+    if (!o.attr) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return fail(ctx, B200Q_CUDA_ERROR, "gemv_stream attribute: %s", cudaGetErrorString(e));
+        o.attr = true;
+    }
+    if (o.threads != threads || o.smem != smem) {
+        int n = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem);
+        if (e != cudaSuccess) return fail(ctx, B200Q_CUDA_ERROR, "gemv_stream occupancy: %s", cudaGetErrorString(e));
+        o.threads = threads;
+        o.smem = smem;
+        o.blocks = n > 0 ? n : 1;
+    }
+    const int64_t n_units = (M + R - 1) / R;
+    int64_t blocks = (n_units + groups - 1) / groups;
+    const int64_t cap = (int64_t)ctx->sm_count * o.blocks;
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    cudaError_t e = launch_pdl(!ctx->no_pdl, kern, dim3((unsigned)blocks), dim3(threads), smem, ctx->stream, (const uint8_t *)w,
+                               row_stride, (int)M, nblk, act, dst, (int)ldd, groups, ctx->error_word, ar_args);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e == cudaSuccess ? B200Q_OK : fail(ctx, B200Q_CUDA_ERROR, "gemv_stream launch: %s", cudaGetErrorString(e));
+}
+
+// The slice-resident kernel (gemv_stream.cuh) for rows that bulk copies can fetch (16-byte aligned
+// start, stride and length). Returns false when the shape does not fit it: more than 16 warps per
+// group (K beyond 16 slices, or 8 for more than four columns) or a ring beyond shared memory.
+template <int TYPE, int NC, int R, bool QX = false, bool AR = false, bool SH = false>
+static bool try_launch_stream(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act,
+                              float *dst, int64_t ldd, b200q_status *st, const GemvAr *ar = nullptr) {
+    typedef GemvFmt<TYPE> F;
+    constexpr int CW = NC > 4 ? 2 : 1, NSETS = 3;      // a four-stage ring at one and two columns measured 5-15 % slower
+    const int nblk = (int)(K / F::BLK_W), nsl = (nblk + F::STAGE_BLOCKS - 1) / F::STAGE_BLOCKS, nw = nsl * CW;
+    if (nw > GEMV_STREAM_MAX_THREADS / 32) return false;
+    const int row_bytes = nblk * F::BLK_B + (SH ? 16 : 0);
+    const size_t gb = (gemv_stream_group_smem(row_bytes, R, NSETS, nw) + 15) / 16 * 16;
+    if (gb > 200 * 1024) return false;
+    int target_warps = 4;                                  // blocks of about four warps measured best
+    if (ctx->gemv_block_warps) {
+        if (ctx->gemv_block_warps >= 1 && ctx->gemv_block_warps <= GEMV_STREAM_MAX_THREADS / 32) target_warps = ctx->gemv_block_warps;
+        else count(ctx, ST_GEMV_KNOB_IGNORED);
+    }
+    int groups = target_warps / nw < 1 ? 1 : target_warps / nw;
+    if (groups * nw > GEMV_STREAM_MAX_THREADS / 32) groups = (GEMV_STREAM_MAX_THREADS / 32) / nw;
+    while (groups > 1 && groups * gb > 200 * 1024) --groups;
+    const size_t smem = groups * gb;
+    const int threads = groups * nw * 32;
+    GemvAr ar_args = {};
+    if (ar) ar_args = *ar;
+    // Q6_K at four and more columns in blocks of one 128-thread group: the build with room for 170 registers
+    constexpr bool has_small = ((TYPE == B200Q_TYPE_Q6_K && NC >= 2) || (TYPE == B200Q_TYPE_Q4_K && NC >= 4)) && !QX && !AR;
+    if constexpr (has_small) {
+        if (threads <= 128 && !ctx->gemv_no_small) {
+            // (two blocks per SM with up to 255 registers measured slower: Q6_K 8 columns 60.4 against 55.5 us)
+            *st = launch_stream_kernel<TYPE, NC, R, NSETS, QX, AR, 128, 3, SH>(ctx, threads, smem, groups, w, row_stride, M, nblk, act, dst, ldd, ar_args);
+            return true;
+        }
+    }
+    *st = launch_stream_kernel<TYPE, NC, R, NSETS, QX, AR, GEMV_STREAM_MAX_THREADS, 0, SH>(ctx, threads, smem, groups, w, row_stride, M, nblk, act, dst,
+                                                                                      ldd, ar_args);
+    return true;
+}
+
+// The warp-MMA kernel (gemv_mma.cuh) for rows that bulk copies can fetch. Returns false when the shape does not fit it:
+// more than twelve warps per group (K beyond 12288) or a ring beyond shared memory.
+template <int TYPE, int NSETS, int SLICE, bool SH>
+static bool try_launch_mma(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act, int ncols,
+                           float *dst, int64_t ldd, b200q_status *st) {
+    typedef GemvFmt<TYPE> F;
+    constexpr int MAX_WARPS = gemv_mma_max_threads(SLICE) / 32;
+    constexpr size_t SMEM_CAP = 227 * 1024;
+    if (K % 256) return false;                                     // the kernel counts in chunks of 256 weights
+    const int nblk = (int)(K / 256), nw = (nblk + SLICE - 1) / SLICE;
+    if (nw > MAX_WARPS) return false;
+    const int row_bytes = nblk * gemv_mma_chunk_bytes<TYPE>() + (SH ? 16 : 0);
+    const size_t gb = (gemv_mma_group_smem(row_bytes, NSETS, nw) + 127) / 128 * 128;
+    if (gb > SMEM_CAP || gemv_mma_xstages((int)K, row_bytes) > NSETS - 1) return false;
+    int groups = MAX_WARPS / nw;
+    while (groups > 1 && groups * gb > SMEM_CAP) --groups;
+    const int per_sm = groups;                                     // groups an SM holds
+    if (ctx->gemv_mma_groups == 1) groups = 1;                     // ... as blocks of one group each
+    const int64_t n_units = (M + GEMV_MMA_ROWS - 1) / GEMV_MMA_ROWS;
+    // few rows: rather more blocks than full ones
+    while (groups > 1 && n_units < (int64_t)groups * ctx->sm_count) --groups;
+    const size_t smem = groups * gb;
+    const int threads = groups * nw * 32;
+    auto kern = gemv_mma_kernel<TYPE, NSETS, SLICE, SH>;
+    static bool attr_dev[B200Q_MAX_DEVICES] = {};
+    bool &attr = attr_dev[ctx->device % B200Q_MAX_DEVICES];
+    if (!attr) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP);
+        if (e != cudaSuccess) { *st = fail(ctx, B200Q_CUDA_ERROR, "gemv_mma attribute: %s", cudaGetErrorString(e)); return true; }
+        attr = true;
+    }
+    int64_t blocks = (n_units + groups - 1) / groups;
+    const int64_t cap = (int64_t)ctx->sm_count * (per_sm / groups);
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    cudaError_t e = launch_pdl(!ctx->no_pdl, kern, dim3((unsigned)blocks), dim3(threads), smem, ctx->stream, (const uint8_t *)w, row_stride,
+                               (int)M, nblk, act, ncols, dst, (int)ldd, groups, ctx->error_word);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    *st = e == cudaSuccess ? B200Q_OK : fail(ctx, B200Q_CUDA_ERROR, "gemv_mma launch: %s", cudaGetErrorString(e));
+    return true;
+}
+
+// Which kernel takes a dense, aligned product of NC columns (measured on B200, CUDA-graph replay over
+// rotating weight copies): the slice-resident kernel everywhere except the 210-byte Q6_K blocks at one
+// column, where the per-warp ring kernel is 10 % faster (23.1 against 25.9 us on the 32000x4096 head). With four
+// rows per ring stage it also wins at two columns (Q4_K 4096x11008: 8.9 against 10.8 us).
+template <int TYPE, int NC>
+static bool stream_preferred() {
+    if (NC == 1 && TYPE == B200Q_TYPE_Q6_K) return false;
+    return true;
+}
+
+// From how many columns the warp-MMA kernel wins (measured): Q6_K 3, Q8_0 7, the others 4. Returns whether it took the product.
+template <int TYPE, int NC, bool SH>
+static bool launch_nc_mma(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act, float *dst, int64_t ldd,
+                          b200q_status *st) {
+    if (NC < (ctx->gemv_mma_min ? ctx->gemv_mma_min : (TYPE == B200Q_TYPE_Q6_K ? 3 : TYPE == B200Q_TYPE_Q8_0 ? 7 : 4))) return false;
+    // the narrowest slice per warp that covers a row with sixteen warps (twelve at four super-blocks)
+    const int nblk = (int)(K / 256);
+    int slice = nblk <= 32 ? 2 : nblk <= 48 ? 3 : 4;
+    if (ctx->gemv_mma_slice >= 2 && ctx->gemv_mma_slice <= 4) slice = ctx->gemv_mma_slice;
+    if (TYPE == B200Q_TYPE_Q6_K && slice == 3) slice = 4;      // Q6_K: even slices only
+    const bool four = !ctx->gemv_mma_sets3;
+    bool took = false;
+    if (slice == 2) took = (four && try_launch_mma<TYPE, 4, 2, SH>(ctx, w, row_stride, M, K, act, NC, dst, ldd, st)) ||
+                           try_launch_mma<TYPE, 3, 2, SH>(ctx, w, row_stride, M, K, act, NC, dst, ldd, st);
+    else if (slice == 3) {
+        if constexpr (TYPE != B200Q_TYPE_Q6_K)
+            took = (four && try_launch_mma<TYPE, 4, 3, SH>(ctx, w, row_stride, M, K, act, NC, dst, ldd, st)) ||
+                   try_launch_mma<TYPE, 3, 3, SH>(ctx, w, row_stride, M, K, act, NC, dst, ldd, st);
+    }
+    else took = (four && try_launch_mma<TYPE, 4, 4, SH>(ctx, w, row_stride, M, K, act, NC, dst, ldd, st)) ||
+                try_launch_mma<TYPE, 3, 4, SH>(ctx, w, row_stride, M, K, act, NC, dst, ldd, st);
+    if (took && *st == B200Q_OK) count(ctx, ST_GEMV_MMA);
+    return took;
+}
+
+// The slice-resident kernel: rows per ring stage four; two at a single column unless the rows are long (measured: Q4_K
+// 11008x4096 at one column 7.4 us with two and 7.6 with four, 4096x11008 7.55 with two and 7.1 with four; at 4 and 8 columns
+// four rows win everywhere, by up to 25 % on the long rows), and two when a ring of four rows does not fit shared memory.
+template <int TYPE, int NC, bool SH>
+static bool launch_nc_stream(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act, float *dst, int64_t ldd,
+                             b200q_status *st) {
+    typedef GemvFmt<TYPE> F;
+    const int row_bytes = (int)(K / F::BLK_W) * F::BLK_B;
+    bool two = NC == 1 && row_bytes <= 4096;
+    if (ctx->gemv_rows == 2 || ctx->gemv_rows == 4) two = ctx->gemv_rows == 2;
+    else if (ctx->gemv_rows) count(ctx, ST_GEMV_KNOB_IGNORED);
+    bool took = !two && try_launch_stream<TYPE, NC, 4, false, false, SH>(ctx, w, row_stride, M, K, act, dst, ldd, st);
+    if (!took) took = try_launch_stream<TYPE, NC, 2, false, false, SH>(ctx, w, row_stride, M, K, act, dst, ldd, st);
+    if (took && *st == B200Q_OK) count(ctx, ST_GEMV_STREAM);
+    return took;
+}
+
+template <int TYPE, int NC>
+static b200q_status launch_nc(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K,
+                              const GemvAct &act, float *dst, int64_t ldd, int rows) {
+    // rows per warp batch of the per-warp ring kernel: four; eight for three or four columns of a small-block type, where
+    // the activation registers are worth sharing further (measured on B200)
+    constexpr bool wide = (NC == 3 || NC == 4) && GemvStage<TYPE>::BYTES <= 1152;
+    const bool want_stream = ctx->gemv_stream_mask >= 0 ? ((ctx->gemv_stream_mask >> NC) & 1) != 0 : stream_preferred<TYPE, NC>();
+    // Super-block rows that begin inside a 16-byte unit take the same kernels as aligned ones (Q6_K unless K % 2048 = 0,
+    // IQ4_XS with an odd super-block count). The per-32 types have such rows only when K % 256 != 0 and stay on the
+    // per-warp ring kernel.
+    constexpr bool can_shift = TYPE == B200Q_TYPE_Q6_K || TYPE == B200Q_TYPE_IQ4_XS;
+    b200q_status st = B200Q_OK;
+    if (!ctx->no_stream && M <= INT32_MAX / 2 && ldd <= INT32_MAX) {
+        if (rows == GEMV_ROWS_ALIGNED) {
+            if (launch_nc_mma<TYPE, NC, false>(ctx, w, row_stride, M, K, act, dst, ldd, &st)) return st;
+            if (want_stream && launch_nc_stream<TYPE, NC, false>(ctx, w, row_stride, M, K, act, dst, ldd, &st)) return st;
+        }
+        if constexpr (can_shift) {
+            if (rows == GEMV_ROWS_SHIFTED) {
+                if (launch_nc_mma<TYPE, NC, true>(ctx, w, row_stride, M, K, act, dst, ldd, &st)) return st;
+                if (want_stream && launch_nc_stream<TYPE, NC, true>(ctx, w, row_stride, M, K, act, dst, ldd, &st)) return st;
+            }
+        }
+    }
+    GemvId none = {};
+    return launch_one<TYPE, NC, wide ? 8 : 4, 4, 2, false>(ctx, w, row_stride, M, K, act, dst, ldd, rows, none, 0);
+}
+
+template <int TYPE>
+b200q_status launch_type(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K,
+                                const GemvAct &act, int nc, float *dst, int64_t ldd, int rows) {
+    switch (nc) {
+    case 1: return launch_nc<TYPE, 1>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 2: return launch_nc<TYPE, 2>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 3: return launch_nc<TYPE, 3>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 4: return launch_nc<TYPE, 4>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 5: return launch_nc<TYPE, 5>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 6: return launch_nc<TYPE, 6>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 7: return launch_nc<TYPE, 7>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    case 8: return launch_nc<TYPE, 8>(ctx, w, row_stride, M, K, act, dst, ldd, rows);
+    }
+    return fail(ctx, B200Q_INVALID, "gemv: %d columns", nc);
+}
+
+// MUL_MAT_ID over route tiles of at most nc pairs (nc = 1, 2, 4 or 8)
+template <int TYPE>
+b200q_status launch_id_type(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K,
+                                   const GemvAct &act, int nc, float *dst, int rows, const GemvId &id,
+                                   int64_t max_tiles) {
+    switch (nc) {
+    case 1: return launch_one<TYPE, 1, 4, 4, 2, true>(ctx, w, row_stride, M, K, act, dst, 0, rows, id, max_tiles);
+    case 2: return launch_one<TYPE, 2, 4, 4, 2, true>(ctx, w, row_stride, M, K, act, dst, 0, rows, id, max_tiles);
+    case 4: return launch_one<TYPE, 4, 4, 4, 2, true>(ctx, w, row_stride, M, K, act, dst, 0, rows, id, max_tiles);
+    case 8: return launch_one<TYPE, 8, 4, 4, 2, true>(ctx, w, row_stride, M, K, act, dst, 0, rows, id, max_tiles);
+    }
+    return fail(ctx, B200Q_INVALID, "gemv_id: tile of %d pairs", nc);
+}
+
+// One or two columns of a small per-32 product with the activation quantized inside the GEMV (no quantizer launch):
+// B200Q_UNSUPPORTED when the shape does not qualify and the caller should take the two-kernel route.
+template <int TYPE>
+b200q_status launch_fused_t(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act, int nc,
+                                   float *dst, int64_t ldd) {
+    b200q_status st = B200Q_OK;
+    bool took = false;
+    if (nc == 1) took = try_launch_stream<TYPE, 1, 2, true>(ctx, w, row_stride, M, K, act, dst, ldd, &st);
+    else if (nc == 2) took = try_launch_stream<TYPE, 2, 4, true>(ctx, w, row_stride, M, K, act, dst, ldd, &st);
+    if (!took) return B200Q_UNSUPPORTED;
+    if (st == B200Q_OK) { count(ctx, ST_GEMV_STREAM); count(ctx, ST_GEMV_FUSED_QUANT); count(ctx, ST_GEMV_COL0 + nc); }
+    return st;
+}
+
+// Product + all-reduce in one kernel (row split over several GPUs): 1, 2, 4 or 8 columns of a shape the slice-resident
+// kernel takes, NC * M results within the all-reduce buffer. src1 != NULL: quantize inside the kernel (per-32 types,
+// 1-2 columns). B200Q_UNSUPPORTED: not that case.
+template <int TYPE, int NC, bool QX>
+static b200q_status launch_ar_t(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act, float *dst,
+                                int64_t ldd, const GemvAr &ar) {
+    typedef GemvFmt<TYPE> F;
+    const int row_bytes = (int)(K / F::BLK_W) * F::BLK_B;
+    const bool two = NC == 1 && row_bytes <= 4096;              // as in launch_nc
+    b200q_status st = B200Q_OK;
+    bool took = !two && try_launch_stream<TYPE, NC, 4, QX, true>(ctx, w, row_stride, M, K, act, dst, ldd, &st, &ar);
+    if (!took) took = try_launch_stream<TYPE, NC, 2, QX, true>(ctx, w, row_stride, M, K, act, dst, ldd, &st, &ar);
+    if (!took) return B200Q_UNSUPPORTED;
+    if (st == B200Q_OK) { count(ctx, ST_GEMV_STREAM); count(ctx, ST_GEMV_ALLREDUCE_FUSED); count(ctx, ST_GEMV_COL0 + NC); if (QX) count(ctx, ST_GEMV_FUSED_QUANT); }
+    return st;
+}
+
+template <int TYPE>
+b200q_status launch_ar_type(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const GemvAct &act, int nc,
+                                   bool qx, float *dst, int64_t ldd, const GemvAr &ar) {
+    constexpr bool per32 = TYPE == B200Q_TYPE_Q4_0 || TYPE == B200Q_TYPE_Q8_0;
+    if constexpr (per32) {
+        if (qx && nc == 1) return launch_ar_t<TYPE, 1, true>(ctx, w, row_stride, M, K, act, dst, ldd, ar);
+        if (qx && nc == 2) return launch_ar_t<TYPE, 2, true>(ctx, w, row_stride, M, K, act, dst, ldd, ar);
+    }
+    if (qx) return B200Q_UNSUPPORTED;
+    switch (nc) {
+    case 1: return launch_ar_t<TYPE, 1, false>(ctx, w, row_stride, M, K, act, dst, ldd, ar);
+    case 2: return launch_ar_t<TYPE, 2, false>(ctx, w, row_stride, M, K, act, dst, ldd, ar);
+    case 4: return launch_ar_t<TYPE, 4, false>(ctx, w, row_stride, M, K, act, dst, ldd, ar);
+    case 8: return launch_ar_t<TYPE, 8, false>(ctx, w, row_stride, M, K, act, dst, ldd, ar);
+    }
+    return B200Q_UNSUPPORTED;
+}
+
+// the four entry points of a type
+#define B200Q_GEMV_TYPE(EXTERN, TYPE)                                                                                          \
+    EXTERN template b200q_status launch_type<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, float *, int64_t, int); \
+    EXTERN template b200q_status launch_id_type<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, float *, int, \
+                                                      const GemvId &, int64_t);
+#define B200Q_GEMV_TYPE_AR(EXTERN, TYPE)                                                                                       \
+    EXTERN template b200q_status launch_ar_type<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, bool, float *, \
+                                                      int64_t, const GemvAr &);
+#define B200Q_GEMV_TYPE_FUSED(EXTERN, TYPE)                                                                                    \
+    EXTERN template b200q_status launch_fused_t<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, float *, int64_t);
+
+}  // namespace b200q

@@ -93,6 +93,12 @@ __device__ __forceinline__ uint32_t gemv_mma_word(const uint8_t *p, bool mis) {
     return __funnelshift_r(w[0], w[1], 16);
 }
 
+// the four bytes at p, any even address
+__device__ __forceinline__ uint32_t gemv_mma_word_any(const uint8_t *p) {
+    const uint32_t *w = reinterpret_cast<const uint32_t *>((uintptr_t)p & ~(uintptr_t)3);
+    return __funnelshift_r(w[0], w[1], ((uint32_t)(uintptr_t)p & 2u) * 8u);
+}
+
 // bulk copy without a cache hint (the activation is read by every block: it should stay in L2)
 __device__ __forceinline__ void gemv_bulk_g2s_plain(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -105,7 +111,9 @@ __device__ __forceinline__ int gemv_dp2a_hi_su(uint32_t a, uint32_t b, int c) {
     return d;
 }
 
-template <int TYPE, int NSETS, int SLICE>
+// SH: rows begin anywhere in a 16-byte unit (Q6_K unless K % 2048 = 0, IQ4_XS with an odd super-block count): a row's copy starts at the
+// boundary below and ends at the one above, and the readers add the remainder.
+template <int TYPE, int NSETS, int SLICE, bool SH>
 __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, const GemvAct &act,
                                               int ncols, float *__restrict__ dst, int ldd, const GemvGroupSmem &sm, int gg, int tg,
                                               int lane, int wi, int nw, int *error_word, int g, uint8_t *ring0, uint32_t bar_x) {
@@ -119,7 +127,7 @@ __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, siz
     typedef GemvFmt<TYPE> F;
     constexpr int R = GEMV_MMA_ROWS;
     const int row_bytes = nblk * gemv_mma_chunk_bytes<TYPE>();
-    const int slot = gemv_mma_slot(row_bytes);
+    const int slot_bytes = row_bytes + (SH ? 16 : 0), slot = gemv_mma_slot(slot_bytes);
     const int n_units = (M + R - 1) / R;
     bool ok = true;
     const uint64_t policy = gemv_policy_evict_first();
@@ -127,7 +135,7 @@ __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, siz
     // Every warp of the group requests its share of the rows of a batch (rows wi, wi + nw, ...): a bulk copy blocks its
     // issuer while the copy engine's queue is full, which at full memory load is most of the time, and one warp
     // issuing all eight rows ran a microsecond and more behind the others, which then waited for its partial sums.
-    const int K = act.K, xstride = gemv_mma_xstride(K), xs = gemv_mma_xstages(K, row_bytes);
+    const int K = act.K, xstride = gemv_mma_xstride(K), xs = gemv_mma_xstages(K, slot_bytes);
     int p_n = 0, p_set = 0;
     auto issue = [&]() {
         const int u = gg + p_n * tg;
@@ -144,11 +152,21 @@ __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, siz
             const uint32_t d = sm.ring + p_set * (R * slot);
             // (16-byte cp.async copies by all lanes instead of the bulk copies measured 7-12 % slower)
             if (lane == 0 && ok) {
-                int mine = 0;
-                for (int r = wi; r < rows; r += nw) ++mine;
-                tc::mbar_expect_tx(sm.bar_full + 8 * p_set, (uint32_t)row_bytes * (uint32_t)mine);     // one arrival per warp
-                for (int r = wi; r < rows; r += nw)
-                    gemv_bulk_g2s(d + r * slot, src + (size_t)r * row_stride, (uint32_t)row_bytes, sm.bar_full + 8 * p_set, policy);
+                if (SH) {
+                    uint32_t total = 0;
+                    for (int r = wi; r < rows; r += nw) total += (uint32_t)(((uintptr_t)(src + (size_t)r * row_stride) & 15) + row_bytes + 15) & ~15u;
+                    tc::mbar_expect_tx(sm.bar_full + 8 * p_set, total);
+                    for (int r = wi; r < rows; r += nw) {
+                        const uintptr_t a = (uintptr_t)(src + (size_t)r * row_stride);
+                        gemv_bulk_g2s(d + r * slot, (const void *)(a & ~(uintptr_t)15), (uint32_t)((a & 15) + row_bytes + 15) & ~15u, sm.bar_full + 8 * p_set, policy);
+                    }
+                } else {
+                    int mine = 0;
+                    for (int r = wi; r < rows; r += nw) ++mine;
+                    tc::mbar_expect_tx(sm.bar_full + 8 * p_set, (uint32_t)row_bytes * (uint32_t)mine);     // one arrival per warp
+                    for (int r = wi; r < rows; r += nw)
+                        gemv_bulk_g2s(d + r * slot, src + (size_t)r * row_stride, (uint32_t)row_bytes, sm.bar_full + 8 * p_set, policy);
+                }
             }
         }
         p_set = p_set + 1 == NSETS ? 0 : p_set + 1;
@@ -254,6 +272,7 @@ __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, siz
         if (n < 6) pt_wait[n] = now();
 #endif
         const uint8_t *rowp = sm.ring_ptr + c_set * (R * slot) + rl * slot;
+        if (SH) rowp += ((uintptr_t)W + (size_t)(u * R + rl) * row_stride) & 15;
         float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
         for (int sb = 0; sb < SLICE; ++sb) {
@@ -351,17 +370,18 @@ __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, siz
                 // Q6_K: ql[128] | qh[64] | scales[16] | d; the 210-byte blocks alternate between 4-byte aligned and not
                 const bool odd = (sb & 1) != 0;                             // blk0 is even: 210 (blk0 + sb) is 2 modulo 4 for odd sb
                 const uint8_t *b = rowp + (blk0 + sb) * 210;
+                auto word = [&](const uint8_t *p) { return SH ? gemv_mma_word_any(p) : gemv_mma_word(p, odd); };
                 uint32_t scw[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) scw[i] = gemv_mma_word(b + 192 + 4 * i, odd);
+                for (int i = 0; i < 4; ++i) scw[i] = word(b + 192 + 4 * i);
                 const float d = hd_half_bits(*reinterpret_cast<const uint16_t *>(b + 208));
                 int i0 = 0, i1 = 0;
 #pragma unroll
                 for (int nh = 0; nh < 4; ++nh) {
                     const int n = nh >> 1, hh = nh & 1;                     // half of the block, half of each 32-weight part
                     const uint32_t o = 64 * n + 16 * hh + 4 * c;
-                    const uint32_t qa = gemv_mma_word(b + o, odd), qb = gemv_mma_word(b + o + 32, odd);
-                    const uint32_t qh = gemv_mma_word(b + 128 + 32 * n + 16 * hh + 4 * c, odd);
+                    const uint32_t qa = word(b + o), qb = word(b + o + 32);
+                    const uint32_t qh = word(b + 128 + 32 * n + 16 * hh + 4 * c);
                     const uint32_t w0 = six_minus32((qa & 0x0F0F0F0Fu) | ((qh << 4) & 0x30303030u));
                     const uint32_t w1 = six_minus32((qb & 0x0F0F0F0Fu) | ((qh << 2) & 0x30303030u));
                     const uint32_t w2 = six_minus32(((qa >> 4) & 0x0F0F0F0Fu) | (qh & 0x30303030u));
@@ -439,14 +459,14 @@ __device__ __forceinline__ void gemv_mma_warp(const uint8_t *__restrict__ W, siz
 
 // dst[m + c*ldd] = sum_k W[m][k] x_c[k] for c < ncols (2..8). A block holds `groups` groups of ceil(nblk / 4) warps;
 // the grid is one wave of persistent blocks and group number gg takes the row batches gg, gg + (all groups), ...
-template <int TYPE, int NSETS, int SLICE>
+template <int TYPE, int NSETS, int SLICE, bool SH>
 __global__ void __launch_bounds__(gemv_mma_max_threads(SLICE), 1)
 gemv_mma_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, GemvAct act, int ncols, float *__restrict__ dst,
                 int ldd, int groups, int *__restrict__ error_word) {
     typedef GemvFmt<TYPE> F;
     extern __shared__ __align__(128) uint8_t smem[];
     const int nw = (nblk + SLICE - 1) / SLICE;
-    const int row_bytes = nblk * gemv_mma_chunk_bytes<TYPE>(), slot = gemv_mma_slot(row_bytes);
+    const int row_bytes = nblk * gemv_mma_chunk_bytes<TYPE>() + (SH ? 16 : 0), slot = gemv_mma_slot(row_bytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp / nw, wi = warp - g * nw;
     const size_t gbytes = (gemv_mma_group_smem(row_bytes, NSETS, nw) + 127) / 128 * 128;
     GemvGroupSmem sm;
@@ -477,7 +497,7 @@ gemv_mma_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nbl
     // group 0's barrier block sits at the same offset as every group's
     const uint32_t bar_x0 = tc::smem_u32(smem) + (sm.bar_free + 16 - sm.ring);
     if (g < groups)
-        gemv_mma_warp<TYPE, NSETS, SLICE>(W, row_stride, M, nblk, act, ncols, dst, ldd, sm, gg, tg, lane, wi, nw, error_word, g, smem, bar_x0);
+        gemv_mma_warp<TYPE, NSETS, SLICE, SH>(W, row_stride, M, nblk, act, ncols, dst, ldd, sm, gg, tg, lane, wi, nw, error_word, g, smem, bar_x0);
     pdl_trigger();
 }
 

@@ -1,0 +1,9 @@
+// gemv_q6_k.cu -- the decode GEMV of Q6_K weights (instantiation only, see gemv_launch.cuh).
+#include "gemv_launch.cuh"
+
+namespace b200q {
+
+B200Q_GEMV_TYPE(, B200Q_TYPE_Q6_K)
+B200Q_GEMV_TYPE_AR(, B200Q_TYPE_Q6_K)
+
+}  // namespace b200q

@@ -86,6 +86,7 @@ struct GemvGroupSmem {
     float   *part_ptr;
 };
 
+// (row_bytes: for rows that begin inside a 16-byte unit, 16 more than a row has)
 __host__ __device__ inline int gemv_stream_slot(int row_bytes) { return ((row_bytes + 15) / 16) * 16 + 16; }
 // bytes of shared memory per group of nw warps
 __host__ __device__ inline size_t gemv_stream_group_smem(int row_bytes, int R, int nsets, int nw) {
@@ -163,7 +164,9 @@ __device__ __forceinline__ void gemv_quant_x(int lane, int slice, int nblk, cons
 
 // What one warp of a group does: slice `slice` of every row, columns [col0, col0 + NCW) of the launch.
 // wi: the warp's index in its group of nw warps; warp 0 of the group also runs the producer side.
-template <int TYPE, int NC, int NCW, int R, int NSETS, bool QX, bool AR>
+// SH: rows begin anywhere in a 16-byte unit (shifted rows): a row's copy starts at the boundary below and ends at the one
+// above, and the lane code adds the remainder.
+template <int TYPE, int NC, int NCW, int R, int NSETS, bool QX, bool AR, bool SH>
 __device__ __forceinline__ void gemv_stream_warp(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk,
                                                  const GemvAct &act, float *__restrict__ dst, int ldd, const GemvGroupSmem &sm,
                                                  int gg, int tg, int lane, int wi, int nw, int slice, int col0,
@@ -172,7 +175,7 @@ __device__ __forceinline__ void gemv_stream_warp(const uint8_t *__restrict__ W, 
     typedef GemvFmt<TYPE> F;
     typedef GemvStage<TYPE> S;
     const int row_bytes = nblk * F::BLK_B;
-    const int slot = gemv_stream_slot(row_bytes);
+    const int slot = gemv_stream_slot(row_bytes + (SH ? 16 : 0));
     const int n_units = (M + R - 1) / R;
     const bool leader = wi == 0;
     bool ok = true;
@@ -189,10 +192,23 @@ __device__ __forceinline__ void gemv_stream_warp(const uint8_t *__restrict__ W, 
                 const int row0 = u * R, rows = min(R, M - row0);
                 const uint8_t *src = W + (size_t)row0 * row_stride;
                 const uint32_t d = sm.ring + p_set * (R * slot);
-                tc::mbar_expect_tx(sm.bar_full + 8 * p_set, (uint32_t)row_bytes * (uint32_t)rows);
+                if (SH) {
+                    uint32_t n[R], total = 0;
 #pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (r < rows) gemv_bulk_g2s(d + r * slot, src + (size_t)r * row_stride, (uint32_t)row_bytes, sm.bar_full + 8 * p_set, policy);
+                    for (int r = 0; r < R; ++r) {
+                        n[r] = r < rows ? (uint32_t)(((uintptr_t)(src + (size_t)r * row_stride) & 15) + row_bytes + 15) & ~15u : 0u;
+                        total += n[r];
+                    }
+                    tc::mbar_expect_tx(sm.bar_full + 8 * p_set, total);
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        if (r < rows) gemv_bulk_g2s(d + r * slot, (const void *)((uintptr_t)(src + (size_t)r * row_stride) & ~(uintptr_t)15), n[r], sm.bar_full + 8 * p_set, policy);
+                } else {
+                    tc::mbar_expect_tx(sm.bar_full + 8 * p_set, (uint32_t)row_bytes * (uint32_t)rows);
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        if (r < rows) gemv_bulk_g2s(d + r * slot, src + (size_t)r * row_stride, (uint32_t)row_bytes, sm.bar_full + 8 * p_set, policy);
+                }
             }
         }
         p_set = p_set + 1 == NSETS ? 0 : p_set + 1;
@@ -232,7 +248,10 @@ __device__ __forceinline__ void gemv_stream_warp(const uint8_t *__restrict__ W, 
         if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
         const uint8_t *set = sm.ring_ptr + c_set * (R * slot) + slice_off;
 #pragma unroll
-        for (int r = 0; r < R; ++r) gemv_lane_row<TYPE, NCW>(reinterpret_cast<const uint32_t *>(set + r * slot), lane, X, acc[r]);
+        for (int r = 0; r < R; ++r) {
+            const uint32_t shift = SH ? (uint32_t)((uintptr_t)W + (size_t)(u * R + r) * row_stride) & 15u : 0u;
+            gemv_lane_row<TYPE, NCW>(reinterpret_cast<const uint32_t *>(set + r * slot), lane, X, acc[r], shift);
+        }
         __syncwarp();                                              // every lane has read the stage
         if (lane == 0) tc::mbar_arrive(sm.bar_empty + 8 * c_set);
         c_set = c_set + 1 == NSETS ? 0 : c_set + 1;
@@ -327,7 +346,7 @@ __device__ __forceinline__ void gemv_stream_warp(const uint8_t *__restrict__ W, 
 // row batches gg, gg + (all groups), ...
 // MAXT, MINB: the launch bounds. The default (512 threads) caps a thread at 128 registers, which the wide Q6_K forms
 // reach: they are also built for blocks of at most 128 threads, three to an SM (170 registers).
-template <int TYPE, int NC, int R, int NSETS, bool QX = false, bool AR = false, int MAXT = GEMV_STREAM_MAX_THREADS, int MINB = 0>
+template <int TYPE, int NC, int R, int NSETS, bool QX = false, bool AR = false, int MAXT = GEMV_STREAM_MAX_THREADS, int MINB = 0, bool SH = false>
 __global__ void __launch_bounds__(MAXT, MINB)
 gemv_stream_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, GemvAct act, float *__restrict__ dst,
                    int ldd, int groups, int *__restrict__ error_word, GemvAr ar) {
@@ -336,7 +355,7 @@ gemv_stream_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int 
     constexpr int NCA = CW == 2 ? (NC + 1) / 2 : NC, NCB = NC - NCA;
     extern __shared__ __align__(128) uint8_t smem[];
     const int nslices = (nblk + F::STAGE_BLOCKS - 1) / F::STAGE_BLOCKS, nw = nslices * CW;
-    const int row_bytes = nblk * F::BLK_B, slot = gemv_stream_slot(row_bytes);
+    const int row_bytes = nblk * F::BLK_B + (SH ? 16 : 0), slot = gemv_stream_slot(row_bytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp / nw, wi = warp - g * nw;
     const int slice = wi / CW, sub = wi - slice * CW;
     const size_t gbytes = (gemv_stream_group_smem(row_bytes, R, NSETS, nw) + 15) / 16 * 16;
@@ -369,13 +388,13 @@ gemv_stream_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int 
         // one copy of the warp code when both column halves are equally wide (8 and 6 columns): the instruction
         // cache is a measured bottleneck of the wide forms
         if (CW == 1 || NCA == NCB)
-            gemv_stream_warp<TYPE, NC, NCA, R, NSETS, QX, AR>(W, row_stride, M, nblk, act, dst, ldd, sm, gg, tg, lane, wi, nw, slice, sub * NCA,
+            gemv_stream_warp<TYPE, NC, NCA, R, NSETS, QX, AR, SH>(W, row_stride, M, nblk, act, dst, ldd, sm, gg, tg, lane, wi, nw, slice, sub * NCA,
                                                               error_word, ar, seq);
         else if (sub == 0)
-            gemv_stream_warp<TYPE, NC, NCA, R, NSETS, QX, AR>(W, row_stride, M, nblk, act, dst, ldd, sm, gg, tg, lane, wi, nw, slice, 0, error_word, ar,
+            gemv_stream_warp<TYPE, NC, NCA, R, NSETS, QX, AR, SH>(W, row_stride, M, nblk, act, dst, ldd, sm, gg, tg, lane, wi, nw, slice, 0, error_word, ar,
                                                               seq);
         else
-            gemv_stream_warp<TYPE, NC, (NCB > 0 ? NCB : 1), R, NSETS, QX, AR>(W, row_stride, M, nblk, act, dst, ldd, sm, gg, tg, lane, wi, nw,
+            gemv_stream_warp<TYPE, NC, (NCB > 0 ? NCB : 1), R, NSETS, QX, AR, SH>(W, row_stride, M, nblk, act, dst, ldd, sm, gg, tg, lane, wi, nw,
                                                                               slice, NCA, error_word, ar, seq);
     }
     if (AR) {
