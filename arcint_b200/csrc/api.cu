@@ -180,10 +180,11 @@ static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor 
         ActEntry &e = ctx->act_cache[pick];
         e.valid = false;
         b200q_status st;
-        if (form == ACT_Q8_0_TILED || form == ACT_Q8_256_TILED) {
-            const bool per32 = form == ACT_Q8_0_TILED;
-            if ((st = ws_reserve(ctx, &e.codes, per32 ? gemm_tc_act_bytes(K, N) : gemm_kq_act_bytes(K, N))) != B200Q_OK) return st;
+        if (form == ACT_Q8_0_TILED || form == ACT_Q8_256_TILED || form == ACT_Q8_256_TILED_F16) {
+            const bool per32 = form == ACT_Q8_0_TILED, f16 = form == ACT_Q8_256_TILED_F16;
+            if ((st = ws_reserve(ctx, &e.codes, per32 ? gemm_tc_act_bytes(K, N) : f16 ? gemm_kf_act_bytes(K, N) : gemm_kq_act_bytes(K, N))) != B200Q_OK) return st;
             st = per32 ? launch_quantize_tiled(ctx, src1, (uint8_t *)e.codes.ptr)
+               : f16   ? launch_quantize_f16(ctx, src1, (uint8_t *)e.codes.ptr)
                        : launch_quantize_tiled256(ctx, src1, (uint8_t *)e.codes.ptr);
             if (st != B200Q_OK) return st;
             e.key = key;
@@ -303,8 +304,6 @@ b200q_status b200q_init(b200q_ctx **out, int device, void *stream) {
     if (mma_slice && mma_slice[0]) ctx->gemv_mma_slice = atoi(mma_slice);
     const char *canary = getenv("B200Q_CANARY");         // debugging: guard words around every scratch block
     ctx->canary = canary && canary[0] == '1';
-    const char *mins_pass = getenv("B200Q_MOE_MINS_PASS");
-    ctx->moe_mins_pass = mins_pass && mins_pass[0] == '1';
     const char *no_stream = getenv("B200Q_NO_STREAM");   // the older GEMV kernel for every shape (comparisons)
     ctx->no_stream = no_stream && no_stream[0] == '1';
     *out = ctx;
@@ -392,6 +391,11 @@ b200q_status b200q_mul_mat(b200q_ctx *ctx, const b200q_tensor *src0, const b200q
         return launch_gemm_kq(ctx, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
                               (float *)dst->data, ldd);
     }
+    if (N > 8 && uniform && !ctx->no_tc && gemm_kf_supported(src0->type, M, K, N, src0->data, src0->nb[1])) {
+        if ((st = get_activation(ctx, ACT_Q8_256_TILED_F16, src1, &act)) != B200Q_OK) return st;
+        return launch_gemm_kf(ctx, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
+                              (float *)dst->data, ldd);
+    }
     if (N > 8) count(ctx, ST_GEMM_FALLBACK_SHAPE);
     // small per-32 products at one or two columns: the GEMV quantizes its own slice of the activation, one launch
     // instead of two (what matters once a tensor-parallel shard is a microsecond of weights)
@@ -436,11 +440,14 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
     // enough pairs per expert on average to beat the per-tile GEMV below)
     const bool per32 = gemm_tc_supported(src0->type, M, K, 1, src0->data, src0->nb[1]);
     const bool per256 = gemm_kq_supported(src0->type, M, K, 1, src0->data, src0->nb[1]);
-    if ((int64_t)n_used * n_tok >= 8 * (int64_t)n_expert && (int64_t)n_used * n_tok >= 256 && !ctx->no_tc && (per32 || per256) &&
+    const bool f16 = gemm_kf_supported(src0->type, M, K, 1, src0->data, src0->nb[1]);
+    if ((int64_t)n_used * n_tok >= 8 * (int64_t)n_expert && (int64_t)n_used * n_tok >= 256 && !ctx->no_tc && (per32 || per256 || f16) &&
         src0->nb[2] % 16 == 0 && src1->nb[1] % 16 == 0 && src1->nb[2] % 16 == 0 && (uintptr_t)src1->data % 16 == 0) {
         RouteView rv;
         if ((st = moe_route(ctx, ids, n_expert, &rv)) != B200Q_OK) return st;
-        const size_t bytes = per32 ? gemm_tc_id_act_bytes(K, rv.max_tiles128) : gemm_kq_id_act_bytes(K, rv.max_tiles128);
+        const int form = per32 ? ACT_Q8_0_TILED : f16 ? ACT_Q8_256_TILED_F16 : ACT_Q8_256_TILED;
+        const size_t bytes = per32 ? gemm_tc_id_act_bytes(K, rv.max_tiles128) : f16 ? gemm_kf_id_act_bytes(K, rv.max_tiles128)
+                                                                                : gemm_kq_id_act_bytes(K, rv.max_tiles128);
         const void *before = ctx->moe_ws[7].ptr;
         if ((st = ws_reserve(ctx, &ctx->moe_ws[7], bytes)) != B200Q_OK) return st;
         const bool grew = ctx->moe_ws[7].ptr != before;
@@ -448,7 +455,7 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
         count(ctx, ST_MOE_GEMM);
         // the scratch may already hold this very activation, gathered for these ids in this graph
         auto &ma = ctx->moe_act;
-        bool ready = !grew && ma.src1 == src1->data && ma.ids == ids->data && ma.src1_id == src1->id && ma.ids_id == ids->id && ma.gen == ctx->generation && ma.per32 == (int)per32 &&
+        bool ready = !grew && ma.src1 == src1->data && ma.ids == ids->data && ma.src1_id == src1->id && ma.ids_id == ids->id && ma.gen == ctx->generation && ma.form == form &&
                      ma.n_expert == n_expert;
         for (int i = 0; i < 4 && ready; ++i) ready = ma.ne[i] == src1->ne[i] && ma.nb[i] == src1->nb[i];
         if (ready) count(ctx, ST_ACT_CACHE_HIT);
@@ -457,10 +464,11 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
         ma.src1_id = src1->id;
         ma.ids_id = ids->id;
         ma.gen = ctx->generation;
-        ma.per32 = (int)per32;
+        ma.form = form;
         ma.n_expert = n_expert;
         for (int i = 0; i < 4; ++i) { ma.ne[i] = src1->ne[i]; ma.nb[i] = src1->nb[i]; }
         return per32 ? launch_gemm_tc_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
+             : f16   ? launch_gemm_kf_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
                      : launch_gemm_kq_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready);
     }
     ActView act;

@@ -39,7 +39,7 @@ __host__ __device__ inline bool type_info(int type, TypeInfo *ti) {
     }
 }
 
-enum { ACT_Q8_0 = 0, ACT_Q8_256 = 1, ACT_Q8_0_TILED = 2, ACT_Q8_256_TILED = 3 };   // TILED: the tensor-core GEMM's chunk layout
+enum { ACT_Q8_0 = 0, ACT_Q8_256 = 1, ACT_Q8_0_TILED = 2, ACT_Q8_256_TILED = 3, ACT_Q8_256_TILED_F16 = 4 };   // TILED: the tensor-core GEMM's chunk layout (F16: codes as halves)
 
 // Quantized activation as the kernels read it: column c of K values at
 //   codes  + c*K            int8
@@ -118,7 +118,7 @@ struct b200q_ctx {
     uint64_t     generation = 1;
     // what the gathered, tiled activation scratch of the tensor-core MUL_MAT_ID holds (gate and up of a layer
     // read the same src1 through the same ids: the second call finds it ready)
-    struct { const void *src1 = nullptr, *ids = nullptr, *src1_id = nullptr, *ids_id = nullptr; int64_t ne[4] = {0, 0, 0, 0}; size_t nb[4] = {0, 0, 0, 0}; uint64_t gen = 0; int per32 = -1, n_expert = 0; } moe_act;
+    struct { const void *src1 = nullptr, *ids = nullptr, *src1_id = nullptr, *ids_id = nullptr; int64_t ne[4] = {0, 0, 0, 0}; size_t nb[4] = {0, 0, 0, 0}; uint64_t gen = 0; int form = -1, n_expert = 0; } moe_act;
     bool         route_skip_negative = false;   // expert-parallel local product: negative ids are empty slots
     int          route_pinned = -1;       // a route entry in use across a nested call: not a victim
     uint64_t     private_generation = 0;  // expert-parallel calls: generations of their internal products
@@ -141,7 +141,6 @@ struct b200q_ctx {
     int          gemv_mma_slice = 0;      // B200Q_GEMV_MMA_SLICE=2|3|4: super-blocks per warp of the warp-MMA GEMV (0: by row length)
     int          gemv_mma_min = 0;        // B200Q_GEMV_MMA_MIN: fewest columns at which a product takes the warp-MMA GEMV (99: never; 0: Q6_K 3, Q8_0 7, the others 4, measured)
     bool         gemv_no_small = false;   // B200Q_GEMV_NO_SMALL=1: never the 128-thread, 170-register build of the wide Q6_K GEMV
-    bool         moe_mins_pass = false;   // B200Q_MOE_MINS_PASS=1: Q4_K route tiles take the mins term in a separate pass
     bool         no_stream = false;       // B200Q_NO_STREAM=1: every GEMV through the per-warp ring kernel (comparisons)
     std::string  last_error;
     std::string  stats_text;
@@ -253,7 +252,15 @@ b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
 b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd);
 
-// gemm_kq.cu: tensor-core prefill GEMM for the super-block types IQ4_XS, Q4_K and Q6_K (integer sub-scales folded into two int8 limbs)
+// the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
+b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
+
+// K parts of a product whose tiles fill the SMs badly; the times of a 256-weight step on a full tile that it counts with
+int          choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_t outputs);
+constexpr int TC_SB_NS = 2000, KQ_SB_NS = 2000, KF_SB_NS = 900;
+
+// gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types
+// (integer sub-scales folded into the weight operand)
 bool         gemm_kq_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride);
 size_t       gemm_kq_act_bytes(int64_t K, int64_t N);
 b200q_status launch_quantize_tiled256(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out);
@@ -261,6 +268,14 @@ size_t       gemm_kq_id_act_bytes(int64_t K, int64_t max_tiles);
 b200q_status launch_gemm_kq_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
                                int64_t max_tiles, uint8_t *act, float *dst, bool act_ready);
 b200q_status launch_gemm_kq(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd);
+bool         gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride);
+size_t       gemm_kf_act_bytes(int64_t K, int64_t N);
+b200q_status launch_quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out);
+size_t       gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles);
+b200q_status launch_gemm_kf_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
+                               int64_t max_tiles, uint8_t *act, float *dst, bool act_ready);
+b200q_status launch_gemm_kf(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd);
 
 }  // namespace b200q

@@ -1,0 +1,678 @@
+// gemm_kf.cu -- prefill GEMM for the super-block types Q4_K and Q5_K on the tensor cores (tcgen05 kind::f16).
+//
+//   dst[M, N] = W[M, K] (144-byte Q4_K / 176-byte Q5_K super-blocks) x X[K, N] (f32), N > 8 tokens
+//
+// ggml's form for these types is integer inside a 256-weight super-block and float once per super-block:
+// out += d * d_x * sum_sb sc_sb I_sb - dmin * d_x * sum_sb m_sb bsum_sb, with I_sb the exact dot of the weight codes with the
+// int8 activation (per-256 activation scale) and bsum_sb the sum of the activation codes. The integer sub-scale is folded
+// into the weight operand: p = sc * q <= 63 * 31 = 1953 is an integer that a half holds exactly, the activation code too, so
+// one chain of kind::f16 MMAs over the super-block gives sum(p x) in an f32 accumulator: every partial sum below 2^24 is
+// exact, larger ones carry f32 rounding as ggml's own float(sumi) does. The mins term is one more K = 16 MMA per
+// super-block into an accumulator of its own: a row of A is [m_0..m_7, m_0..m_7], a column of B is
+// [bl_0..bl_7, 256 bh_0..256 bh_7] with bsum_j = 256 bh_j + bl_j (all exact in f16).
+//
+// The weight operand goes through TENSOR MEMORY: an unpack thread decodes a row's blocks in registers and stores them with
+// tcgen05.st into the lane of its row, and the MMAs take A from there: no operand stores, proxy fences and operand reads
+// in shared memory, whose port (128 bytes per clock) the B reads of the MMAs alone fill by half.
+//
+// Tensor memory, 512 columns: two main accumulators of 128 columns, one for the mins term, and the ring of A blocks (two
+// groups of four 32-weight blocks, 16 columns of packed half pairs a block). Warp roles: producer, MMA issuer, two idle,
+// eight unpack warps (a thread = a row and half of the blocks of a group), eight scale-accumulate warps (four per half of
+// the columns, a lane quarter each). Persistent blocks walk the units (row tile, column tile, part of K). Every mbarrier
+// wait is bounded.
+//
+// B200, quantizer and GEMM together, against two int8 limbs through shared memory and a second kernel for the mins: Q4_K
+// 11008x4096 x 512 tokens 149.3 -> 80.9 us, x 24 tokens 53.6 -> 23.4 us, a 512-expert block over 2048 tokens 842 -> 581 us. The
+// tensor pipe is active 32 % of the time; what is left is the chain unpack -> MMA -> scaling, whose one mins accumulator and
+// two-group operand ring (all of tensor memory) let it overlap only in part. Reading the accumulators in the 32x32b shape, sixteen columns at a
+// time, measured the same on dense products and 2 % slower on the 512-expert block.
+//
+// The reference's mins correction is a DPAS of its own, too (marfrit/arcint contrib/llama.cpp/patches/
+// 0000-01-kquant-integer-dpas.patch:3740-3801); the fold of the sub-scales is this build's own.
+#include <cuda.h>
+
+#include "formats.cuh"
+#include "common.cuh"
+#include "pdl.cuh"
+#include "tc_common.cuh"
+
+namespace b200q {
+
+namespace kf {
+
+using namespace tc;
+
+constexpr int BM = 128, BN = 128, SB = 8;
+constexpr int GB = 4;                                     // blocks per A group and per stage of activation codes
+constexpr int NG = 2;                                     // groups in the A ring
+constexpr int A_COLS = 16;                                // tensor-memory columns of one A block
+constexpr int Y_BASE = 2 * BN, A_BASE = 3 * BN;           // tensor memory: X0, X1, Y, A ring
+static_assert(A_BASE + NG * GB * A_COLS <= 512, "tensor memory");
+constexpr int NCODE = 4;                                  // stages of activation codes (half a super-block each) in flight
+constexpr int NX = 3;                                     // super-blocks of activation scales, mins operands and row scales in flight
+constexpr int THREADS = 32 * 20;                          // warp groups: {producer, MMA, 2 idle}, 2 x unpack, 2 x scale-accumulate
+// Registers per thread by role (setmaxnreg): a warp group that asks for more waits until others have
+// given theirs back, so the sum must fit the pool the launch allocated (THREADS x LAUNCH_REGS).
+constexpr int LAUNCH_REGS = (65536 / THREADS) / 8 * 8;
+static_assert(128 * 48 + 256 * 56 + 256 * 160 <= THREADS * LAUNCH_REGS, "register pool: 48 control, 56 unpack, 160 scale-accumulate");
+
+// The activation of a (column tile, super-block), by groups of eight columns, so that what a tile with few columns needs
+// (a route tile of a small expert) is a short prefix of each part:
+//   codes, twice (blocks 0..3, 4..7): [group g < 16][block j < 4][piece c < 4][column r < 8][8 codes as halves, each run of four
+//          in the order 0 2 1 3, in which the unpack threads mask nibbles out of a word]
+//   extra: 128 f32 scales, then the mins operand [group g < 16][piece c < 2][column r < 8][8 halves: bl_0..7 or 256 bh_0..7]
+constexpr int CODE_BLOCK = 512, CODE_GROUP = GB * CODE_BLOCK, CODE_STAGE = (BN / 8) * CODE_GROUP;
+constexpr int MINS_GROUP = 256, EXTRA_MINS = BN * 4, EXTRA = EXTRA_MINS + (BN / 8) * MINS_GROUP;
+constexpr int CHUNK = 2 * CODE_STAGE + EXTRA;
+
+template <int TYPE> struct Fmt;
+template <> struct Fmt<B200Q_TYPE_Q4_K> { enum { SBB = 144, NRAW = 3 }; };
+template <> struct Fmt<B200Q_TYPE_Q5_K> { enum { SBB = 176, NRAW = 2 }; };
+
+template <int TYPE> struct Smem {
+    enum {
+        NRAW = Fmt<TYPE>::NRAW, RAW_STAGE = BM * Fmt<TYPE>::SBB,
+        RAW_OFF = 0,
+        CODE_OFF = RAW_OFF + NRAW * RAW_STAGE,
+        EXTRA_OFF = CODE_OFF + NCODE * CODE_STAGE,
+        MINS_OFF = EXTRA_OFF + NX * EXTRA,               // the rows' mins as an A operand, two super-blocks
+        DW_OFF = MINS_OFF + 2 * 4096,                    // the rows' (d, -dmin), NX super-blocks
+        BAR_OFF = DW_OFF + NX * BM * 8,
+        TOTAL = BAR_OFF + 8 * 32
+    };
+    static_assert(TOTAL <= 227 * 1024 - 256, "shared memory budget");
+    static_assert(RAW_STAGE % 128 == 0 && EXTRA % 128 == 0, "tiled copies");
+};
+
+enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_CODE_FULL = 6, BAR_CODE_EMPTY = 10, BAR_X_FULL = 14, BAR_X_EMPTY = 17, BAR_A_FULL = 20,
+       BAR_A_EMPTY = 22, BAR_ACC_FULL = 24, BAR_ACC_EMPTY = 26, BAR_COUNT = 28 };
+static_assert(NCODE == 4 && NX == 3 && NG == 2, "barrier slots above");
+
+constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
+
+// The quantizer of the layout above, per-256 form (the reference's kernel_quant_i8 rule: scale bm/127, round to nearest
+// even, zero below 1e-30).
+__global__ void __launch_bounds__(256)
+quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
+                    int64_t N, uint8_t *__restrict__ out, TileRoute id) {
+    // One block per (tile, super-block); a half-warp per column at a time: its sixteen lanes read the column's 256
+    // floats as one contiguous kilobyte (lane l: elements 16 l .. 16 l + 15, i.e. half l & 1 of block j = l >> 1),
+    // take the maximum by shuffles and store their sixteen codes as two 16-byte pieces. Columns of groups past the tile's
+    // last one are never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
+    pdl_trigger();
+    pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
+    const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
+    const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
+    uint8_t *chunk = out + ((size_t)t * nst + s) * CHUNK;
+    int cnt, first = 0;
+    if (id.tiles) {
+        // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
+        if (t >= __ldg(id.n_tiles)) return;
+        first = __ldg(id.tiles + 4 * t + 1);
+        cnt = __ldg(id.tiles + 4 * t + 2);
+    } else {
+        const int64_t left = N - (int64_t)t * BN;
+        cnt = left < BN ? (int)left : BN;
+    }
+    const int live = ((cnt + 7) >> 3) << 3;
+    for (int col0 = 0; col0 < live; col0 += 16) {
+        // (whole warps stay together for the shuffles: a half-warp past the live columns quantizes zeros and stores nothing)
+        const int col = col0 + hw;
+        const float *x = nullptr;
+        if (col < cnt) {
+            if (id.tiles) {
+                const int p = __ldg(id.pairs + first + col), tok = p / id.n_used, slot = p - tok * id.n_used;
+                x = reinterpret_cast<const float *>(base + (size_t)(slot % id.ne11) * id.nb1 + (size_t)tok * id.nb2);
+            } else {
+                const int64_t n = (int64_t)t * BN + col;
+                const int64_t c1 = n % ne1, c23 = n / ne1, c2 = c23 % ne2, c3 = c23 / ne2;
+                x = reinterpret_cast<const float *>(base + c1 * nb1 + c2 * nb2 + c3 * nb3);
+            }
+            x += (int64_t)s * 256 + 16 * l;
+        }
+        float4 v[4];
+        float amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = x ? __ldg(reinterpret_cast<const float4 *>(x) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+        const float bm = amax;
+        const float iq = bm > 1e-30f ? __fdiv_rn(127.f, bm) : 0.f;
+        int q[16], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            q[4 * i] = __float2int_rn(__fmul_rn(v[i].x, iq));
+            q[4 * i + 1] = __float2int_rn(__fmul_rn(v[i].y, iq));
+            q[4 * i + 2] = __float2int_rn(__fmul_rn(v[i].z, iq));
+            q[4 * i + 3] = __float2int_rn(__fmul_rn(v[i].w, iq));
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum += q[i];                // the integer sum of the block's 32 codes (the mins term)
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+        if (col >= live) continue;
+        const int j = l >> 1;
+        uint8_t *o = chunk + (j >> 2) * CODE_STAGE + (col >> 3) * CODE_GROUP + (j & 3) * CODE_BLOCK + (col & 7) * 16;
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __half2 a = __floats2half2_rn((float)q[4 * i], (float)q[4 * i + 2]), b = __floats2half2_rn((float)q[4 * i + 1], (float)q[4 * i + 3]);
+            w[2 * i] = *reinterpret_cast<const uint32_t *>(&a);
+            w[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&b);
+        }
+        *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * 128) = make_uint4(w[4], w[5], w[6], w[7]);
+        // two exact digits of the sum: bh = round(sum / 256), bl = sum - 256 bh in [-128, 127]
+        const int bh = (sum + 128) >> 8;
+        uint8_t *extra = chunk + 2 * CODE_STAGE;
+        __half *mo = reinterpret_cast<__half *>(extra + EXTRA_MINS + (col >> 3) * MINS_GROUP + (l & 1) * 128 + (col & 7) * 16);
+        mo[j] = __float2half_rn((l & 1) ? (float)(256 * bh) : (float)(sum - 256 * bh));
+        if (l == 0) reinterpret_cast<float *>(extra)[col] = __fdiv_rn(bm, 127.f);
+    }
+}
+
+// two small non-negative integers (one per byte of the low 16 bits) as an f16 pair: 1024 + v is the bit
+// pattern 0x6400 | v, then subtract 1024
+__device__ __forceinline__ uint32_t u8x2_to_h2(uint32_t two_bytes) {
+    const uint32_t bits = 0x64006400u | (two_bytes & 0xFFu) | ((two_bytes & 0xFF00u) << 8);
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&bits), __half2half2(__ushort_as_half((unsigned short)0x6400)));
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, __half2 b, __half2 c) {
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), b, c);
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+// the eight 16-bit pairs of four packed bytes each (32 bytes q; fifth bits hb, bit HB of each byte, for Q5_K) of the low
+// (HI = false) or high nibbles, as halves sc * code: 1024 + code (or 1024 + 16 code) is a bit pattern, one fused
+// multiply-add with exact factors and an exact result takes the 1024 away and multiplies by the scale
+template <bool HI, bool FIFTH>
+__device__ __forceinline__ void nibbles_to_products(const uint32_t (&q)[8], const uint32_t (&hb)[8], int bit, uint32_t sc, uint32_t (&out)[16]) {
+    const __half s = __hsub(__ushort_as_half((unsigned short)(0x6400u | sc)), __ushort_as_half((unsigned short)0x6400));
+    const __half2 mul = __half2half2(HI ? __hmul(s, __float2half_rn(0.0625f)) : s);
+    const __half2 add = __half2half2(__hmul(s, __float2half_rn(HI ? -64.f : -1024.f)));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {                                       // bytes 0 and 2 of the word, then 1 and 3
+            const uint32_t w = o ? q[i] >> 8 : q[i];
+            uint32_t c = (w & (HI ? 0x00F000F0u : 0x000F000Fu)) | 0x64006400u;
+            if (FIFTH) {
+                const uint32_t b = hb[i] >> (bit + 8 * o);
+                c |= (b & 0x00010001u) << (HI ? 8 : 4);
+            }
+            out[2 * i + o] = h2_fma(c, mul, add);
+        }
+    }
+}
+
+// The A blocks of one group (GB = 4 blocks of 32 weights) that this thread decodes, u = 0 or 1, into tensor memory: `blk`
+// points at the row's super-block in the raw stage, `ta` at the group's columns (with the warp's lanes). Rows past the
+// matrix multiply by a zero scale.
+template <int TYPE>
+__device__ __forceinline__ void unpack_group(const uint8_t *blk, const uint4 &hdr, int jg, int u, bool row_ok, uint32_t ta) {
+    // d, dmin | 12 scale bytes | (Q5_K: 32 bytes of fifth bits) | 4 x 32 bytes; bytes 32 G .. + 31 hold sub-block 2 G in
+    // their low nibbles and 2 G + 1 in their high ones. Bit 2 G of fifth-bit byte t goes with the low nibble of byte
+    // t of run G, bit 2 G + 1 with the high one.
+    constexpr bool Q5 = TYPE == B200Q_TYPE_Q5_K;
+    const int G = 2 * jg + u;
+    uint32_t c03, c47;
+    q4k_scales8(hdr.y, hdr.z, hdr.w, &c03, &c47);
+    const uint32_t cw = (row_ok ? (jg ? c47 : c03) : 0u) >> (16 * u);
+    const uint8_t *qp = blk + (Q5 ? 48 : 16) + 32 * G;
+    const uint4 qa = *reinterpret_cast<const uint4 *>(qp), qb = *reinterpret_cast<const uint4 *>(qp + 16);
+    const uint32_t q[8] = { qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w };
+    uint32_t hb[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
+    if (Q5) {
+        const uint4 ha = *reinterpret_cast<const uint4 *>(blk + 16), hc = *reinterpret_cast<const uint4 *>(blk + 32);
+        hb[0] = ha.x; hb[1] = ha.y; hb[2] = ha.z; hb[3] = ha.w; hb[4] = hc.x; hb[5] = hc.y; hb[6] = hc.z; hb[7] = hc.w;
+    }
+    uint32_t v[16];
+    nibbles_to_products<false, Q5>(q, hb, 2 * G, cw & 0xFFu, v);
+    tmem_st16(ta + (2 * u) * A_COLS, v);
+    nibbles_to_products<true, Q5>(q, hb, 2 * G + 1, (cw >> 8) & 0xFFu, v);
+    tmem_st16(ta + (2 * u + 1) * A_COLS, v);
+}
+
+// One unit of work: a 128-row x 128-column output tile over the super-blocks [sb0, sb1). Dense: tile_n-th run of 128
+// tokens; MUL_MAT_ID: route tile tile_n (one expert, up to 128 routed pairs).
+struct Unit {
+    int tile_n, row0, valid_rows, expert, first, ncols, sb0, sb1, part, cw;      // cw: columns of a scale-accumulate warp group
+};
+
+template <int TYPE>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
+               int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
+               int *__restrict__ error_word, TileRoute id) {
+    typedef Smem<TYPE> L;
+    constexpr int SBB = Fmt<TYPE>::SBB, NRAW = L::NRAW;
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler, too)
+    const int nsb = K / 256;                    // super-blocks of a row
+    const uint32_t sbase = smem_u32(smem);
+    const uint32_t bars = sbase + L::BAR_OFF;
+    auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+    // The block is persistent: it walks the units blockIdx.x, blockIdx.x + gridDim.x, ... and every role
+    // keeps running counters for its rings, so the pipeline never drains between units (the loads,
+    // the unpacking and the MMAs of the next tile run while the last tile's results are stored).
+    // Units of one row tile are neighbours, so blocks running together share weight rows in L2 (MUL_MAT_ID: the
+    // tiles of one expert). A contiguous run of units per block measured slower on the 512-expert configuration (+18 %:
+    // the full tiles of busy experts pile up on a few blocks). A dense product with few tiles is cut along K: a unit is
+    // then one part of a tile and writes part `part` of a scratch buffer.
+    // Launched with programmatic dependence: before pdl_wait() a block may only read the weights. The producer waits before
+    // its first activation load, the scaling warps before they store; a route's tile list is read by everybody.
+    if (id.tiles) pdl_wait();
+    const int tiles_m = (M + BM - 1) / BM;
+    const int tiles_n = id.tiles ? __ldg(id.n_tiles) : n_tiles_dense;
+    const int n_units = tiles_m * tiles_n * ksplit;
+    auto unit_of = [&](int u) {
+        Unit U;
+        U.part = u % ksplit;
+        U.sb0 = U.part * nsb / ksplit;
+        U.sb1 = (U.part + 1) * nsb / ksplit;
+        u /= ksplit;
+        U.tile_n = u % tiles_n;
+        U.row0 = (u / tiles_n) * BM;
+        U.valid_rows = min(BM, M - U.row0);
+        U.expert = 0;
+        U.first = 0;
+        U.ncols = min(BN, N - U.tile_n * BN);
+        if (id.tiles) {
+            U.expert = __ldg(id.tiles + 4 * U.tile_n);
+            U.first = __ldg(id.tiles + 4 * U.tile_n + 1);
+            U.ncols = __ldg(id.tiles + 4 * U.tile_n + 2);
+        }
+        // 64 columns for a full tile; for a short one (the ragged end, a route tile of a small expert) half of what
+        // there is, in steps of 16
+        U.cw = U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
+        return U;
+    };
+    if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < NRAW; ++i) {
+            mbar_init(bar(BAR_RAW_FULL + i), 1);
+            mbar_init(bar(BAR_RAW_EMPTY + i), 8);                  // unpack warps
+        }
+        for (int i = 0; i < NCODE; ++i) {
+            mbar_init(bar(BAR_CODE_FULL + i), 1);
+            mbar_init(bar(BAR_CODE_EMPTY + i), 1);                 // MMA commit
+        }
+        for (int i = 0; i < NX; ++i) {
+            mbar_init(bar(BAR_X_FULL + i), 1);
+            mbar_init(bar(BAR_X_EMPTY + i), 1 + 8);                // MMA commit (mins) + scaling warps
+        }
+        for (int i = 0; i < NG; ++i) {
+            mbar_init(bar(BAR_A_FULL + i), 8);                     // unpack warps
+            mbar_init(bar(BAR_A_EMPTY + i), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar(BAR_ACC_FULL + i), 1);
+            mbar_init(bar(BAR_ACC_EMPTY + i), 8);                  // scaling warps
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_slot, 0);
+    volatile int *abortp = &abort_flag;
+    PROF_DECL
+
+    if (warp == 0) {
+        // ---- producer ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
+        if (lane == 0) tma_prefetch_desc(&wmap);
+        int s_run = 0;                                    // super-blocks fetched so far
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * CHUNK;
+            const uint32_t groups = (uint32_t)(U.ncols + 7) >> 3;          // live column groups
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int st = s_run % NRAW, xt = s_run % NX;
+                if (!WAITP(1, bar(BAR_RAW_EMPTY + st), ((s_run / NRAW) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    // the [128 rows x super-block] box in one tiled copy; rows past M arrive as zeros
+                    mbar_expect_tx(bar(BAR_RAW_FULL + st), L::RAW_STAGE);
+                    tma_load_3d(sbase + L::RAW_OFF + st * L::RAW_STAGE, &wmap, s * (SBB / 4), U.row0, U.expert, bar(BAR_RAW_FULL + st));
+                }
+                if (s_run == 0) pdl_wait();
+                const uint8_t *chunk = act_tile + (size_t)s * CHUNK;
+                for (int h = 0; h < 2; ++h) {
+                    // only the column groups the tile has; the MMA still reads a multiple of sixteen columns, the rest of the
+                    // stage holds older codes whose products land in accumulator columns nobody stores
+                    const int c_run = 2 * s_run + h, ct = c_run % NCODE;
+                    if (!WAITP(3, bar(BAR_CODE_EMPTY + ct), ((c_run / NCODE) & 1) ^ 1)) { ok = false; break; }
+                    if (lane == 0) {
+                        mbar_expect_tx(bar(BAR_CODE_FULL + ct), groups * CODE_GROUP);
+                        bulk_g2s(sbase + L::CODE_OFF + ct * CODE_STAGE, chunk + h * CODE_STAGE, groups * CODE_GROUP, bar(BAR_CODE_FULL + ct));
+                    }
+                    __syncwarp();
+                }
+                if (!ok || !WAITP(3, bar(BAR_X_EMPTY + xt), ((s_run / NX) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    const uint32_t bytes = EXTRA_MINS + groups * MINS_GROUP;
+                    mbar_expect_tx(bar(BAR_X_FULL + xt), bytes);
+                    bulk_g2s(sbase + L::EXTRA_OFF + xt * EXTRA, chunk + 2 * CODE_STAGE, bytes, bar(BAR_X_FULL + xt));
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
+        int s_run = 0;
+        const uint32_t leader = elect_one();
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            const uint32_t idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);       // N: the live columns, in sixteens
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int buf = s_run & 1, xt = s_run % NX;
+                const uint32_t acc = tmem_base + (uint32_t)buf * BN;
+                if (!WAITP(7, bar(BAR_ACC_EMPTY + buf), ((s_run >> 1) & 1) ^ 1)) { ok = false; break; }
+                for (int jg = 0; jg < SB / GB; ++jg) {
+                    const int g = 2 * s_run + jg, gs = g % NG, ct = g % NCODE;
+                    if (!WAITP(2, bar(BAR_CODE_FULL + ct), (g / NCODE) & 1)) { ok = false; break; }
+                    if (!WAITP(4, bar(BAR_A_FULL + gs), (g / NG) & 1)) { ok = false; break; }
+                    tc_fence_after();
+#pragma unroll
+                    for (int jj = 0; jj < GB; ++jj) {
+                        const uint32_t a = tmem_base + A_BASE + (uint32_t)((gs * GB + jj) * A_COLS);
+                        const uint32_t b = sbase + L::CODE_OFF + ct * CODE_STAGE + jj * CODE_BLOCK;
+                        // K = 16 per MMA: eight columns of A, two pieces of B
+                        umma_ts<true>(leader, acc, a, umma_desc2(b, 128, CODE_GROUP), idesc, (uint32_t)(jg + jj > 0));
+                        umma_ts<true>(leader, acc, a + 8, umma_desc2(b + 256, 128, CODE_GROUP), idesc, 1u);
+                    }
+                    tc_commit_one(leader, bar(BAR_A_EMPTY + gs));
+                    tc_commit_one(leader, bar(BAR_CODE_EMPTY + ct));
+                }
+                if (!ok) break;
+                // the mins term, into the one Y accumulator: the scaling warps have read the last super-block's with its X
+                if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
+                if (s_run > 0 && !WAITP(7, bar(BAR_ACC_EMPTY + (buf ^ 1)), ((s_run - 1) >> 1) & 1)) { ok = false; break; }
+                tc_fence_after();
+                umma_ss<true>(leader, tmem_base + Y_BASE, umma_desc2(sbase + L::MINS_OFF + buf * 4096, 2048, 128),
+                            umma_desc2(sbase + L::EXTRA_OFF + xt * EXTRA + EXTRA_MINS, 128, MINS_GROUP), idesc, 0u);
+                tc_commit_one(leader, bar(BAR_ACC_FULL + buf));
+                tc_commit_one(leader, bar(BAR_X_EMPTY + xt));
+            }
+        }
+    } else if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
+    } else if (warp < 12) {
+        // ---- unpack: two threads per weight row ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;" ::: "memory");
+        // warp w writes the tensor-memory lanes of its quadrant w & 3; two warps share a quadrant and the blocks of a group
+        const int r = (warp & 3) * 32 + lane, uu = (warp - 4) >> 2;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + A_BASE;
+        int s_run = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            const bool row_ok = r < U.valid_rows;
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int st = s_run % NRAW, xt = s_run % NX;
+                if (!WAITP(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1)) { ok = false; break; }
+                const uint8_t *blk = smem + L::RAW_OFF + st * L::RAW_STAGE + r * SBB;
+                const uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
+                // the place of the row's scales: every scaling warp is done with the super-block NX back
+                if (!WAITP(5, bar(BAR_X_EMPTY + xt), ((s_run / NX) & 1) ^ 1)) { ok = false; break; }
+                if (uu == 0)
+                    *reinterpret_cast<float2 *>(smem + L::DW_OFF + (xt * BM + r) * 8) =
+                        make_float2(half_bits_to_float((uint16_t)(hdr.x & 0xFFFFu)), -half_bits_to_float((uint16_t)(hdr.x >> 16)));
+#pragma unroll
+                for (int jg = 0; jg < SB / GB; ++jg) {
+                    const int g = 2 * s_run + jg, gs = g % NG;
+                    if (!WAITP(5, bar(BAR_A_EMPTY + gs), ((g / NG) & 1) ^ 1)) { ok = false; break; }
+                    tc_fence_after();
+                    if (jg == 0) {
+                        // the mins as an A operand. The MMA that read this place two super-blocks ago was issued before the
+                        // MMAs whose completion the wait above saw.
+                        uint32_t m03, m47;
+                        q4k_mins8(hdr.y, hdr.z, hdr.w, &m03, &m47);
+                        *reinterpret_cast<uint4 *>(smem + L::MINS_OFF + (s_run & 1) * 4096 + uu * 2048 + r * 16) =
+                            make_uint4(u8x2_to_h2(m03 & 0xFFFFu), u8x2_to_h2(m03 >> 16), u8x2_to_h2(m47 & 0xFFFFu), u8x2_to_h2(m47 >> 16));
+                        fence_async_smem();
+                    }
+                    unpack_group<TYPE>(blk, hdr, jg, uu, row_ok, ta + gs * (GB * A_COLS));
+                    if (jg == SB / GB - 1) mbar_arrive_warp(bar(BAR_RAW_EMPTY + st), lane);      // the row's bytes are in registers
+                    tmem_st_wait();
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(BAR_A_FULL + gs), lane);
+                }
+            }
+        }
+    } else {
+        // ---- scale-accumulate, once per super-block: a warp group per half of the tile's columns ----
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 160;" ::: "memory");
+        // 16x256b loads give a thread, of every eight columns, columns 2 c and 2 c + 1 of rows g and g + 8
+        const int q4 = warp & 3, half = (warp - 12) >> 2, g = lane >> 2, c = lane & 3;
+        int s_run = 0;
+        pdl_wait();
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            const int cbase = half * U.cw, ncol = min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
+            const bool live = ncol > 0, two = ncol > 32;
+            f32x2 acc2[4][8];                                  // rows g, g + 8, g + 16, g + 24; column pairs 8 i + 2 c
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc2[k][i] = 0ull;
+            const uint32_t tq = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)cbase;
+            for (int s = U.sb0; s < U.sb1; ++s, ++s_run) {
+                const int buf = s_run & 1, xt = s_run % NX;
+                if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
+                if (!WAITP(6, bar(BAR_ACC_FULL + buf), (s_run >> 1) & 1)) { ok = false; break; }
+                tc_fence_after();
+                if (live) {
+                    // rows 16 rh .. + 15 of the quarter at a time: X and Y, all columns, in flight together
+                    uint32_t vx[2][16], vy[2][16];
+                    auto load = [&](int rh) {
+                        const uint32_t a = tq + ((uint32_t)(rh * 16) << 16);
+                        tmem_ld_16x256_x4(a + (uint32_t)buf * BN, vx[0]);
+                        tmem_ld_16x256_x4(a + Y_BASE, vy[0]);
+                        if (two) {
+                            tmem_ld_16x256_x4(a + (uint32_t)buf * BN + 32, vx[1]);
+                            tmem_ld_16x256_x4(a + Y_BASE + 32, vy[1]);
+                        }
+                    };
+                    load(0);
+                    const uint32_t xa = sbase + L::EXTRA_OFF + xt * EXTRA + (cbase + 2 * c) * 4;
+                    f32x2 dx[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) dx[i] = lds64_f2(xa + 32 * i);
+                    const float2 *dp = reinterpret_cast<const float2 *>(smem + L::DW_OFF + (xt * BM + q4 * 32 + g) * 8);
+#pragma unroll
+                    for (int rh = 0; rh < 2; ++rh) {
+                        const float2 w0 = dp[16 * rh], w1 = dp[16 * rh + 8];
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int hc = 0; hc < 2; ++hc) {
+                            if (hc == 0 || two) {
+#pragma unroll
+                                for (int k = 0; k < 2; ++k) {
+                                    const f32x2 d2 = k ? f2_pack(w1.x, w1.x) : f2_pack(w0.x, w0.x), m2 = k ? f2_pack(w1.y, w1.y) : f2_pack(w0.y, w0.y);
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        const f32x2 x = f2_pack(__uint_as_float(vx[hc][4 * i + 2 * k]), __uint_as_float(vx[hc][4 * i + 2 * k + 1]));
+                                        const f32x2 y = f2_pack(__uint_as_float(vy[hc][4 * i + 2 * k]), __uint_as_float(vy[hc][4 * i + 2 * k + 1]));
+                                        // (d sum(sc q x) - dmin sum(m x)) d_x
+                                        acc2[2 * rh + k][4 * hc + i] = f2_fma(f2_fma(x, d2, f2_mul(y, m2)), dx[4 * hc + i], acc2[2 * rh + k][4 * hc + i]);
+                                    }
+                                }
+                            }
+                        }
+                        if (rh == 0) load(1);
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive_warp(bar(BAR_ACC_EMPTY + buf), lane);
+                mbar_arrive_warp(bar(BAR_X_EMPTY + xt), lane);
+            }
+            if (ok && live) {
+                const int r0 = q4 * 32 + g;
+                if (id.tiles) {
+                    // where the half's columns go: every lane looks up two of them (loads in flight together), the
+                    // store loop takes them by shuffle
+                    long long off[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        off[h] = 0;
+                        if (lane + 32 * h < ncol) {
+                            const int p = __ldg(id.pairs + U.first + cbase + lane + 32 * h), tok = p / id.n_used, slot = p - tok * id.n_used;
+                            off[h] = tok * id.ld2 + slot * id.ld1;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int d = 0; d < 2; ++d) {
+                            const int col = 8 * i + 2 * c + d;
+                            const long long o = __shfl_sync(0xFFFFFFFFu, off[i >> 2], col & 31);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                float a[2];
+                                f2_unpack(acc2[k][i], a[0], a[1]);
+                                if (col < ncol && r0 + 8 * k < U.valid_rows) dst[o + U.row0 + r0 + 8 * k] = a[d];
+                            }
+                        }
+                } else {
+                    float *o = dst + (int64_t)U.part * part_stride + (int64_t)(U.tile_n * BN + cbase + 2 * c) * ldd + U.row0 + r0;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            float a0, a1;
+                            f2_unpack(acc2[k][i], a0, a1);
+                            if (r0 + 8 * k < U.valid_rows) {
+                                if (8 * i + 2 * c < ncol) o[8 * k] = a0;
+                                if (8 * i + 2 * c + 1 < ncol) o[ldd + 8 * k] = a1;
+                            }
+                        }
+                        o += 8 * ldd;
+                    }
+                }
+            }
+        }
+    }
+
+    PROF_DUMP(warp == 0 ? "prod" : warp == 1 ? "mma " : warp < 4 ? "idle" : warp < 12 ? "unpk" : "epi ")
+    tc_fence_before();
+    __syncthreads();
+    pdl_trigger();
+    if (abort_flag) {
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        if (threadIdx.x == 0) atomicExch(error_word, 2);
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
+}  // namespace kf
+
+static const TileRoute NO_ROUTE_KF = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0 };
+
+size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + kf::BN - 1) / kf::BN) * (K / 256)) * kf::CHUNK; }
+size_t gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles) { return gemm_kf_act_bytes(K, max_tiles * kf::BN); }
+
+bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride) {
+    if (type != B200Q_TYPE_Q4_K && type != B200Q_TYPE_Q5_K) return false;
+    if (K <= 0 || K % 256 || M <= 0 || N <= 0) return false;
+    if ((uintptr_t)w % 16 || row_stride % 16) return false;           // raw stages are tiled copies
+    return M <= (1 << 30) && N <= (1 << 30) && K <= (1 << 30);
+}
+
+static b200q_status quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
+    const int64_t K = src1->ne[0];
+    dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kf::quantize_f16_kernel, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
+                               src1->nb[1], src1->nb[2], src1->nb[3], K, src1->ne[1] * src1->ne[2] * src1->ne[3], out, tr));
+    B200Q_CUDA(ctx, cudaGetLastError());
+    count(ctx, ST_GEMM_TC_QUANT);
+    return B200Q_OK;
+}
+
+b200q_status launch_quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out) {
+    const int64_t N = src1->ne[1] * src1->ne[2] * src1->ne[3];
+    return quantize_f16(ctx, src1, out, (N + kf::BN - 1) / kf::BN, NO_ROUTE_KF);
+}
+
+// n_tiles: the column tiles (dense: of N; MUL_MAT_ID: the upper bound of the route's tile count, blocks past the
+// device-side count leave at once)
+template <int TYPE>
+static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
+                                int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
+                                const TileRoute &tr) {
+    typedef kf::Smem<TYPE> L;
+    auto kern = kf::gemm_kf_kernel<TYPE>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES];
+    if (!attr_set) {
+        B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
+        attr_set = true;
+    }
+    CUtensorMap wmap;
+    b200q_status st = make_weight_tmap3(ctx, &wmap, w, row_stride, M, (K / 256) * kf::Fmt<TYPE>::SBB, kf::Fmt<TYPE>::SBB, n_mat, mat_stride);
+    if (st != B200Q_OK) return st;
+    // persistent blocks, one per SM, walking the (row tile, column tile, part of K) units
+    const int64_t tiles = n_tiles * ((M + kf::BM - 1) / kf::BM), S = ctx->sm_count;
+    const int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, S, K / 256, KF_SB_NS, M * N);
+    float *out = dst;
+    int64_t out_ld = ldd, part_stride = 0;
+    if (ksplit > 1) {
+        // parts write their own scratch and a second kernel adds them in a fixed order
+        part_stride = N * M;
+        if ((st = ws_reserve(ctx, &ctx->moe_ws[9], sizeof(float) * (size_t)part_stride * ksplit)) != B200Q_OK) return st;
+        out = (float *)ctx->moe_ws[9].ptr;
+        out_ld = M;
+    }
+    const int64_t units = tiles * ksplit;
+    const unsigned grid = (unsigned)(units < S ? units : S);
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3(grid), dim3(kf::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr));
+    B200Q_CUDA(ctx, cudaGetLastError());
+    if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
+    count(ctx, ST_GEMM_TC);
+    count(ctx, ST_GEMM_KQ_MINS);
+    return B200Q_OK;
+}
+
+b200q_status launch_gemm_kf(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd) {
+    const int64_t n_tiles = (N + kf::BN - 1) / kf::BN;
+    const size_t ms = row_stride * (size_t)M;
+    if (type == B200Q_TYPE_Q4_K) return launch_kf_t<B200Q_TYPE_Q4_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_KF);
+    if (type == B200Q_TYPE_Q5_K) return launch_kf_t<B200Q_TYPE_Q5_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_KF);
+    return fail(ctx, B200Q_UNSUPPORTED, "gemm_kf: type %d", type);
+}
+
+// MUL_MAT_ID on the tensor cores: the route's 128-pair tiles are the column tiles; the activation of
+// every tile is gathered and quantized into `act` (gemm_kf_id_act_bytes) first.
+b200q_status launch_gemm_kf_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
+                               int64_t max_tiles, uint8_t *act, float *dst, bool act_ready) {
+    const int64_t K = src0->ne[0], M = src0->ne[1];
+    b200q_status st = act_ready ? B200Q_OK : quantize_f16(ctx, src1, act, max_tiles, tr);
+    if (st != B200Q_OK) return st;
+    if (src0->type == B200Q_TYPE_Q4_K)
+        return launch_kf_t<B200Q_TYPE_Q4_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+    if (src0->type == B200Q_TYPE_Q5_K)
+        return launch_kf_t<B200Q_TYPE_Q5_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+    return fail(ctx, B200Q_UNSUPPORTED, "gemm_kf_id: type %d", src0->type);
+}
+
+}  // namespace b200q

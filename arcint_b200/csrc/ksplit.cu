@@ -1,0 +1,62 @@
+// ksplit.cu -- products of the tensor-core GEMMs cut along K: how many parts, and the pass that adds them up.
+#include "common.cuh"
+#include "pdl.cuh"
+
+namespace b200q {
+
+// dst[n][m] = sum over the K parts, part 0 first: V consecutive rows a thread, a column of dst per blockIdx.y
+template <int V>
+__global__ void __launch_bounds__(256)
+ksplit_sum_kernel(const float *__restrict__ parts, int ksplit, int64_t part_stride, int M, float *__restrict__ dst, int64_t ldd) {
+    pdl_trigger();
+    pdl_wait();
+    const int m = ((int)blockIdx.x * 256 + (int)threadIdx.x) * V;
+    if (m >= M) return;
+    const float *p = parts + (int64_t)blockIdx.y * M + m;
+    float *o = dst + (int64_t)blockIdx.y * ldd + m;
+    if (V == 4) {
+        float4 acc = *reinterpret_cast<const float4 *>(p);
+        for (int z = 1; z < ksplit; ++z) {
+            const float4 v = *reinterpret_cast<const float4 *>(p + z * part_stride);
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        *reinterpret_cast<float4 *>(o) = acc;
+    } else {
+        float acc = *p;
+        for (int z = 1; z < ksplit; ++z) acc += p[z * part_stride];
+        *o = acc;
+    }
+}
+
+// Into how many parts to cut K: the schedule's length in nanoseconds, rounds of units over the SMs plus, for more than one
+// part, the pass that adds them. step_ns: a k-step (one raw stage) of the kernel on a full tile; a unit costs some 1.2 us
+// beyond its steps (pipeline fill, drain, stores), the adding pass a launch and its traffic.
+int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_t outputs) {
+    int best_ks = 1;
+    int64_t best = 0;
+    for (int ks = 1; ks <= 8 && (ks == 1 || steps / ks >= 2); ++ks) {
+        const int64_t rounds = (tiles * ks + sms - 1) / sms;
+        const int64_t len = rounds * ((steps + ks - 1) / ks * step_ns + 1200) + (ks > 1 ? 2500 + outputs * (ks + 1) / 1000 : 0);
+        if (ks == 1 || len < best) { best = len; best_ks = ks; }
+    }
+    return best_ks;
+}
+
+b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd) {
+    // four rows a thread where every part's and dst's columns start on 16 bytes
+    const bool vec = M % 4 == 0 && ldd % 4 == 0 && (uintptr_t)dst % 16 == 0;
+    for (int64_t n0 = 0; n0 < N; n0 += 65535) {
+        const unsigned nn = (unsigned)(N - n0 < 65535 ? N - n0 : 65535);
+        const float *p = parts + n0 * M;
+        float *o = dst + n0 * ldd;
+        B200Q_CUDA(ctx, vec ? launch_pdl(!ctx->no_pdl, ksplit_sum_kernel<4>, dim3((unsigned)((M / 4 + 255) / 256), nn), dim3(256), 0, ctx->stream, p, ksplit,
+                                         part_stride, (int)M, o, ldd)
+                            : launch_pdl(!ctx->no_pdl, ksplit_sum_kernel<1>, dim3((unsigned)((M + 255) / 256), nn), dim3(256), 0, ctx->stream, p, ksplit,
+                                         part_stride, (int)M, o, ldd));
+        B200Q_CUDA(ctx, cudaGetLastError());
+    }
+    count(ctx, ST_GEMM_KSPLIT);
+    return B200Q_OK;
+}
+
+}  // namespace b200q
