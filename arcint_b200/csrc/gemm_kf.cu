@@ -241,7 +241,8 @@ struct Unit {
     int tile_n, row0, valid_rows, expert, first, ncols, sb0, sb1, part, cw;      // cw: columns of a scale-accumulate warp group
 };
 
-template <int TYPE>
+// FULL: every column tile has BN columns (and there is no route): the build without a branch on the columns that are live
+template <int TYPE, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
@@ -288,7 +289,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         }
         // 64 columns for a full tile; for a short one (the ragged end, a route tile of a small expert) half of what
         // there is, in steps of 16
-        U.cw = U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
+        U.cw = FULL || U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
         return U;
     };
     if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
@@ -464,8 +465,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
-            const int cbase = half * U.cw, ncol = min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
-            const bool live = ncol > 0, two = ncol > 32;
+            const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
+            const bool live = FULL || ncol > 0, two = FULL || ncol > 32;
             f32x2 acc2[4][8];                                  // rows g, g + 8, g + 16, g + 24; column pairs 8 i + 2 c
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -524,7 +525,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             }
             if (ok && live) {
                 const int r0 = q4 * 32 + g;
-                if (id.tiles) {
+                if (!FULL && id.tiles) {
                     // where the half's columns go: every lane looks up two of them (loads in flight together), the
                     // store loop takes them by shuffle
                     long long off[2];
@@ -558,8 +559,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                             float a0, a1;
                             f2_unpack(acc2[k][i], a0, a1);
                             if (r0 + 8 * k < U.valid_rows) {
-                                if (8 * i + 2 * c < ncol) o[8 * k] = a0;
-                                if (8 * i + 2 * c + 1 < ncol) o[ldd + 8 * k] = a1;
+                                if (FULL || 8 * i + 2 * c < ncol) o[8 * k] = a0;
+                                if (FULL || 8 * i + 2 * c + 1 < ncol) o[ldd + 8 * k] = a1;
                             }
                         }
                         o += 8 * ldd;
@@ -619,9 +620,10 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
                                 int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
                                 const TileRoute &tr) {
     typedef kf::Smem<TYPE> L;
-    auto kern = kf::gemm_kf_kernel<TYPE>;
-    static bool attr_set_dev[B200Q_MAX_DEVICES] = {};
-    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES];
+    const bool full = !tr.tiles && N % kf::BN == 0;
+    auto kern = full ? kf::gemm_kf_kernel<TYPE, true> : kf::gemm_kf_kernel<TYPE, false>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES][2] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][full];
     if (!attr_set) {
         B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
         attr_set = true;

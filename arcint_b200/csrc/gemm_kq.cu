@@ -228,7 +228,8 @@ struct Unit {
     int tile_n, row0, valid_rows, expert, first, ncols, sb0, nsu, part;      // sb0, nsu: first super-block and how many (split K)
 };
 
-template <int TYPE, int FV = TYPE>
+// FULL: every column tile has BN columns (and there is no route): the build without a branch on the columns that are live
+template <int TYPE, int FV, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word,
@@ -468,7 +469,7 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             // The tile's columns are shared out between the two warps of a row quadrant: 64 each for a full tile, and
             // for a short one (the ragged end, a route tile of a small expert) half of what there is, in steps of 16.
             const int row_shift = rowcopy ? (int)(((uintptr_t)wraw + (size_t)U.expert * mat_stride + (size_t)(U.row0 + r) * row_stride) & 15) : 0;
-            const int cw_eff = U.ncols > CW ? CW : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
+            const int cw_eff = FULL || U.ncols > CW ? CW : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
             const int cbase = u4 * cw_eff;
             f32x2 acc2[CW / 2];
 #pragma unroll
@@ -488,10 +489,10 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 const f32x2 dw2 = f2_pack(dwb, dwb);
                 const uint32_t dxa = sbase + L::ACT_OFF + at * ACT_CHUNK + (cbase / 8) * ACT_GROUP + ACT_SCALES;   // scales of this thread's first group
                 const uint32_t taddr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)buf * (2 * BN) + (uint32_t)cbase;
-                const int ncol = min(cw_eff, U.ncols - cbase);   // this thread's columns inside the tile (warp-uniform)
+                const int ncol = FULL ? CW : min(cw_eff, U.ncols - cbase);   // this thread's columns inside the tile (warp-uniform)
 #pragma unroll
                 for (int q = 0; q < CW / 16; ++q) {
-                    if (q * 16 >= ncol) {                    // a short tile (the ragged end, a small expert): nothing to scale
+                    if (!FULL && q * 16 >= ncol) {                    // a short tile (the ragged end, a small expert): nothing to scale
                         if (q == CW / 16 - 1) {
                             tc_fence_before();
                             mbar_arrive_warp(bar(BAR_ACC_EMPTY + buf), lane);
@@ -524,8 +525,8 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             }
             ++rs_run;                                    // past the unit's last raw stage
             if (ok) {
-                const int ncol = min(cw_eff, U.ncols - cbase);   // this thread's columns inside the tile
-                if (id.tiles) {
+                const int ncol = FULL ? CW : min(cw_eff, U.ncols - cbase);   // this thread's columns inside the tile
+                if (!FULL && id.tiles) {
                     // where the warp's 64 columns go: every lane looks up two of them (loads in flight
                     // together), the store loop takes them by shuffle -- a load and a division per column
                     // inside that loop would serialize 64 memory latencies
@@ -554,8 +555,8 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                     for (int c = 0; c < CW; c += 2) {
                         float a0, a1;
                         f2_unpack(acc2[c / 2], a0, a1);
-                        if (c < ncol) *o = a0;
-                        if (c + 1 < ncol) o[ldd] = a1;
+                        if (FULL || c < ncol) *o = a0;
+                        if (FULL || c + 1 < ncol) o[ldd] = a1;
                         o += 2 * ldd;
                     }
                 }
@@ -622,9 +623,10 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
                                 int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
                                 const TileRoute &tr) {
     typedef kq::Smem<FV> L;
-    auto kern = kq::gemm_kq_kernel<TYPE, FV>;
-    static bool attr_set_dev[B200Q_MAX_DEVICES] = {};
-    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES];
+    const bool full = !tr.tiles && N % kq::BN == 0;
+    auto kern = full ? kq::gemm_kq_kernel<TYPE, FV, true> : kq::gemm_kq_kernel<TYPE, FV, false>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES][2] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][full];
     if (!attr_set) {
         B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
         attr_set = true;

@@ -24,7 +24,10 @@
 //               block accumulator out of tensor memory (tcgen05.ld), free it, convert, scale by
 //               d_w * d_x and accumulate into f32 registers (thread = row x 128/NW columns).
 // Four 128-column accumulators fill the 512 tensor-memory columns, so the MMA of block b+1..
-// b+3 runs while block b is being scaled. The scaling is the bound, not the tensor pipe:
+// b+3 runs while block b is being scaled. Whole column tiles have a build of their own (FULL) without a branch on which
+// columns are live: with such branches in the scaling loop, never taken, Q8_0 12288x3072 x 2048 measured 684 us against 563.
+// Putting the weight operand into tensor memory (tcgen05.st, three accumulators left) and reading the accumulators in the 16x256b
+// shape (a quarter of the scale loads) were built and measured 2 to 10 % slower. The scaling is the bound, not the tensor pipe:
 // every output element needs a convert, a multiply and a fused multiply-add per 32 of K,
 // 16K elements per block against 128 FP32 lanes per SM and clock.
 //
@@ -35,6 +38,7 @@
 
 #include "formats.cuh"
 #include "common.cuh"
+#include "pdl.cuh"
 #include "tc_common.cuh"
 
 namespace b200q {
@@ -85,11 +89,11 @@ template <int TYPE, bool F16> struct Smem {
 };
 static_assert(Smem<B200Q_TYPE_Q4_0, true>::TOTAL <= 227 * 1024 && Smem<B200Q_TYPE_Q8_0, true>::TOTAL <= 227 * 1024, "shared memory");
 
-constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);          // without the N field
 // fp16 operands, f32 accumulator: integer-valued halves (|v| <= 255) multiply and add exactly (every
 // partial sum of a 32-block stays far below 2^24), so the accumulator holds float(I_b) with the bits the
 // int8 MMA's result would convert to -- without the conversion
-constexpr uint32_t IDESC_F16 = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+constexpr uint32_t IDESC_F16 = (1u << 4) | ((uint32_t)(BM >> 4) << 24);
 
 // barrier slots inside the shared block
 enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_ACT_FULL = 6, BAR_ACT_EMPTY = 9, BAR_A_FULL = 12, BAR_A_EMPTY = 20,
@@ -108,6 +112,8 @@ quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1,
     // floats as one contiguous kilobyte (lane l: k = 16 l .. 16 l + 15, i.e. half l & 1 of block j = l >> 1), the two
     // lanes of a block share their maximum by one shuffle, and every lane stores its 16 codes as one piece (int8) or
     // two (fp16). Columns past the tile's last one are written as zeros.
+    pdl_trigger();
+    pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
     constexpr int OPER_BYTES = Oper<F16>::BYTES, ACT_CHUNK = Oper<F16>::ACT_CHUNK;
@@ -173,18 +179,6 @@ quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1,
     }
 }
 
-// dst[n][m] = sum over the K parts, part 0 first
-__global__ void __launch_bounds__(256)
-ksplit_sum_kernel(const float *__restrict__ parts, int ksplit, int64_t part_stride, int M, int64_t N, float *__restrict__ dst, int64_t ldd) {
-    const int64_t total = N * M;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        float acc = parts[i];
-        for (int z = 1; z < ksplit; ++z) acc += parts[(int64_t)z * part_stride + i];
-        const int64_t n = i / M, m = i - n * M;
-        dst[n * ldd + m] = acc;
-    }
-}
-
 template <int N> __device__ __forceinline__ uint32_t word_at(const uint32_t (&w)[N], int byte_off) {
     // 32-bit word at a compile-time even byte offset of a register array
     const int i = byte_off >> 2, sh = (byte_off & 3) * 8;
@@ -201,13 +195,8 @@ __device__ __forceinline__ void bytes_to_halves(uint32_t b4, uint32_t bias2, uin
     h23 = *reinterpret_cast<const uint32_t *>(&rb);
 }
 
-__device__ __forceinline__ void umma_f16_acc(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-template <int TYPE, bool F16>
+// FULL: every column tile has BN columns (and there is no route)
+template <int TYPE, bool F16, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word, TileRoute id) {
@@ -219,14 +208,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler, too)
     const int tile_n = blockIdx.x, tile_m = blockIdx.y;
     const int row0 = tile_m * BM;
     // gridDim.z > 1: the product is cut along K (few tiles on many SMs); this block takes nst of the K / 256
     // stages, from s_off, and writes its partial result to part blockIdx.z of a scratch buffer
     const int nst_all = K / (SB * KB);
-    const int nst = nst_all / (int)gridDim.z;   // k-stages of this block
-    const int s_off = (int)blockIdx.z * nst;
+    const int s_off = (int)blockIdx.z * nst_all / (int)gridDim.z;
+    const int nst = ((int)blockIdx.z + 1) * nst_all / (int)gridDim.z - s_off;   // k-stages of this block
     const int nblk = nst * SB;
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bars = sbase + L::BAR_OFF;
@@ -235,7 +224,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // the tile's matrix and columns: dense, tile_n-th run of 128 tokens; MUL_MAT_ID, a route tile (one
     // expert, up to 128 routed pairs)
     int expert = 0, first = 0, ncols = min(BN, N - tile_n * BN);
+    // Launched with programmatic dependence: before pdl_wait() a block may only read the weights. The producer waits before
+    // its first activation load, the scaling warps before they store; a route's tile list is read by everybody.
     if (id.tiles) {
+        pdl_wait();
         if (tile_n >= __ldg(id.n_tiles)) return;          // the whole block: nothing is set up yet
         expert = __ldg(id.tiles + 4 * tile_n);
         first = __ldg(id.tiles + 4 * tile_n + 1);
@@ -268,7 +260,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_slot, 0);
     volatile int *abortp = &abort_flag;
     PROF_DECL
 
@@ -289,6 +281,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 mbar_expect_tx(bar(BAR_RAW_FULL + st), L::RAW_STAGE);
                 tma_load_3d(sbase + L::RAW_OFF + st * L::RAW_STAGE, &wmap, (s_off + s) * (ROWB / 4), row0, expert, bar(BAR_RAW_FULL + st));
             }
+            if (s == 0) pdl_wait();
             if (!WAITP(3, bar(BAR_ACT_EMPTY + st), par)) break;
             if (lane == 0) {
                 mbar_expect_tx(bar(BAR_ACT_FULL + st), ACT_CHUNK);
@@ -300,26 +293,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     } else if (warp == 1) {
         // ---- MMA issuer ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 " B200Q_STR(64) ";" ::: "memory");   // REGS_CTRL
+        const uint32_t leader = elect_one();
+        const uint32_t n16 = (uint32_t)((ncols + 15) >> 4) << 18;             // N: the live columns, in sixteens
         for (int b = 0; b < nblk; ++b) {
             const int s = b / SB, j = b % SB, st = s % NSTAGE, acc = b % NACC, slot = b % A_SLOTS;
             if (j == 0 && !WAITP(2, bar(BAR_ACT_FULL + st), (s / NSTAGE) & 1)) break;
             if (!WAITP(4, bar(BAR_A_FULL + slot), (b / A_SLOTS) & 1)) break;
             if (!WAITP(7, bar(BAR_ACC_EMPTY + acc), ((b / NACC) & 1) ^ 1)) break;
             tc_fence_after();
-            if (lane == 0) {
-                const uint32_t a_addr = sbase + L::A_OFF + slot * OPER_BYTES, b_addr = sbase + L::ACT_OFF + st * ACT_CHUNK + j * OPER_BYTES;
-                if (F16) {
-                    // K = 16 per fp16 MMA: the block's first two 16-byte K pieces, then the other two
-                    umma_f16_acc(tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_F16, 0u);
-                    umma_f16_acc(tmem_base + (uint32_t)acc * BN, umma_desc(a_addr + 2 * LBO), umma_desc(b_addr + 2 * LBO), IDESC_F16, 1u);
-                } else {
-                    umma_i8(tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_I8);
-                }
-                tc_commit(bar(BAR_ACC_FULL + acc));
-                tc_commit(bar(BAR_A_EMPTY + slot));
-                if (j == SB - 1) tc_commit(bar(BAR_ACT_EMPTY + st));
+            const uint32_t a_addr = sbase + L::A_OFF + slot * OPER_BYTES, b_addr = sbase + L::ACT_OFF + st * ACT_CHUNK + j * OPER_BYTES;
+            if (F16) {
+                // K = 16 per fp16 MMA: the block's first two 16-byte K pieces, then the other two
+                umma_ss<true>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_F16 | n16, 0u);
+                umma_ss<true>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr + 2 * LBO), umma_desc(b_addr + 2 * LBO), IDESC_F16 | n16, 1u);
+            } else {
+                umma_ss<false>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_I8 | n16, 0u);
             }
-            __syncwarp();
+            tc_commit_one(leader, bar(BAR_ACC_FULL + acc));
+            tc_commit_one(leader, bar(BAR_A_EMPTY + slot));
+            if (j == SB - 1) tc_commit_one(leader, bar(BAR_ACT_EMPTY + st));
         }
     } else if (warp < 4) {
         // idle warps of the first warp group
@@ -413,6 +405,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         const int q4 = warp & 3, u = (warp - 8) >> 2;      // lane quarter (fixed by warp id % 4), column part
         const int r = q4 * 32 + lane;
         const bool row_ok = r < valid_rows;
+        // the columns are shared out between the two warps of a lane quarter: 64 each for a full tile, for a short one half of
+        // what there is, in steps of 16
+        const int cw = FULL || ncols > CW ? CW : max(16, (((ncols + 1) >> 1) + 15) & ~15);
+        const int cbase = u * cw, ncol = FULL ? CW : min(cw, ncols - cbase);       // this warp's columns (none: <= 0)
+        const bool full = FULL || ncol > CW - 16;                              // every chunk of sixteen is live
+        pdl_wait();
         f32x2 acc2[CW / 2];                                // column pairs
 #pragma unroll
         for (int c = 0; c < CW / 2; ++c) acc2[c] = 0ull;
@@ -425,41 +423,76 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             if (j == 0 && !WAITP(0, bar(BAR_RAW_FULL + st), (s / NSTAGE) & 1)) break;
             if (!WAITP(6, bar(BAR_ACC_FULL + acc), (b / NACC) & 1)) break;
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)acc * BN + (uint32_t)u * CW;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)acc * BN + (uint32_t)cbase;
             // the block's fp16 weight scale, straight from the packed row in the raw stage
             constexpr int BB = TYPE == B200Q_TYPE_Q8_0 ? 34 : 18;
             const float dwb = row_ok ? half_bits_to_float(*reinterpret_cast<const uint16_t *>(
                                            smem + L::RAW_OFF + st * L::RAW_STAGE + r * ROWB + BB * j)) : 0.f;
             const f32x2 dw2 = f2_pack(dwb, dwb), negc2 = f2_pack(-12582912.f, -12582912.f);
-            const uint32_t dxa = sbase + L::ACT_OFF + st * ACT_CHUNK + SB * OPER_BYTES + (j * BN + u * CW) * 4;
-            // the whole accumulator slice in one go: the CW/16 tensor-memory loads are issued back to back and
-            // waited for once (one load latency per block, not one per sixteen columns), then the accumulator
-            // is free for the MMA three blocks ahead while these registers are scaled
-            uint32_t v[CW / 16][16];
+            const uint32_t dxa = sbase + L::ACT_OFF + st * ACT_CHUNK + SB * OPER_BYTES + (j * BN + cbase) * 4;
+            // Sixteen columns at a time, the next sixteen (and their scales) in flight under this chunk's arithmetic; for whole
+            // tiles of the four-bit types the whole slice in one go, which leaves the scheduler of those builds more room:
+            // Q4_0 4096x4096 x 512 80 us in one go, 85 in chunks; Q8_0 12288x3072 x 2048 563 in one go, 532 in chunks; short
+            // tiles are faster in chunks throughout (Q4_0 4096x4096 x 24: 34 and 31).
+            constexpr bool ONE_GO = FULL && TYPE != B200Q_TYPE_Q8_0;
+            uint32_t v[ONE_GO ? CW / 16 : 2][16];
+            f32x2 dxs[2][8];
+            auto fetch_scales = [&](int q, int to) {
 #pragma unroll
-            for (int q = 0; q < CW / 16; ++q) tmem_ld16(taddr + q * 16, v[q]);
-            tmem_ld_wait();
-            tc_fence_before();
-            mbar_arrive_warp(bar(BAR_ACC_EMPTY + acc), lane);
-#pragma unroll
-            for (int q = 0; q < CW / 16; ++q) {
-                f32x2 dx[8];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) lds128_f2(dxa + (q * 16 + 4 * c) * 4, dx[2 * c], dx[2 * c + 1]);
+                for (int c = 0; c < 4; ++c) lds128_f2(dxa + (q * 16 + 4 * c) * 4, dxs[to][2 * c], dxs[to][2 * c + 1]);
+            };
+            auto fetch = [&](int q, int to) {
+                tmem_ld16(taddr + q * 16, v[to]);
+                fetch_scales(q, to);
+            };
+            auto release_acc = [&]() {
+                tc_fence_before();
+                mbar_arrive_warp(bar(BAR_ACC_EMPTY + acc), lane);
+            };
+            auto scale_chunk = [&](int q, int from, int sc) {
 #pragma unroll
                 for (int c = 0; c < 16; c += 4) {
                     const int e = (q * 16 + c) / 2;
                     // int8 arm: exact int -> float without the conversion pipe (|I| < 2^22): add the magic
                     // exponent as an integer, subtract it as a float; the fp16 arm's accumulator already holds floats
-                    const f32x2 x01 = F16 ? f2_pack(__uint_as_float(v[q][c]), __uint_as_float(v[q][c + 1]))
-                                          : f2_add(f2_pack(__int_as_float((int)v[q][c] + 0x4B400000),
-                                                           __int_as_float((int)v[q][c + 1] + 0x4B400000)), negc2);
-                    const f32x2 x23 = F16 ? f2_pack(__uint_as_float(v[q][c + 2]), __uint_as_float(v[q][c + 3]))
-                                          : f2_add(f2_pack(__int_as_float((int)v[q][c + 2] + 0x4B400000),
-                                                           __int_as_float((int)v[q][c + 3] + 0x4B400000)), negc2);
-                    acc2[e]     = f2_fma(x01, f2_mul(dw2, dx[c / 2]), acc2[e]);
-                    acc2[e + 1] = f2_fma(x23, f2_mul(dw2, dx[c / 2 + 1]), acc2[e + 1]);
+                    const f32x2 x01 = F16 ? f2_pack(__uint_as_float(v[from][c]), __uint_as_float(v[from][c + 1]))
+                                          : f2_add(f2_pack(__int_as_float((int)v[from][c] + 0x4B400000),
+                                                           __int_as_float((int)v[from][c + 1] + 0x4B400000)), negc2);
+                    const f32x2 x23 = F16 ? f2_pack(__uint_as_float(v[from][c + 2]), __uint_as_float(v[from][c + 3]))
+                                          : f2_add(f2_pack(__int_as_float((int)v[from][c + 2] + 0x4B400000),
+                                                           __int_as_float((int)v[from][c + 3] + 0x4B400000)), negc2);
+                    acc2[e]     = f2_fma(x01, f2_mul(dw2, dxs[sc][c / 2]), acc2[e]);
+                    acc2[e + 1] = f2_fma(x23, f2_mul(dw2, dxs[sc][c / 2 + 1]), acc2[e + 1]);
                 }
+            };
+            if constexpr (ONE_GO) {
+#pragma unroll
+                for (int q = 0; q < CW / 16; ++q) tmem_ld16(taddr + q * 16, v[q]);
+                tmem_ld_wait();
+                release_acc();
+#pragma unroll
+                for (int q = 0; q < CW / 16; ++q) {
+                    fetch_scales(q, 0);
+                    scale_chunk(q, q, 0);
+                }
+            } else if (full) {
+                fetch(0, 0);
+#pragma unroll
+                for (int q = 0; q < CW / 16; ++q) {
+                    tmem_ld_wait();
+                    if (q + 1 < CW / 16) fetch(q + 1, (q + 1) & 1);
+                    else release_acc();
+                    scale_chunk(q, q & 1, q & 1);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < CW / 16 - 1; ++q)
+                    if (q * 16 < ncol) {
+                        fetch(q, 0);
+                        tmem_ld_wait();
+                        scale_chunk(q, 0, 0);
+                    }
+                release_acc();
             }
             if (j == SB - 1) {                                         // done with this stage's scales
                 mbar_arrive_warp(bar(BAR_ACT_EMPTY + st), lane);
@@ -467,8 +500,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             }
             done = b == nblk - 1;
         }
-        const int ncol = ncols - u * CW;                         // this thread's columns inside the tile
-        if (done && id.tiles) {
+        if (!FULL && done && id.tiles) {
             // where the warp's columns go: every lane looks up some of them (loads in flight together), the
             // store loop takes them by shuffle
             long long off[(CW + 31) / 32];
@@ -476,7 +508,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             for (int h = 0; h < (CW + 31) / 32; ++h) {
                 off[h] = 0;
                 if (lane + 32 * h < ncol) {
-                    const int p = __ldg(id.pairs + first + u * CW + lane + 32 * h), tok = p / id.n_used, slot = p - tok * id.n_used;
+                    const int p = __ldg(id.pairs + first + cbase + lane + 32 * h), tok = p / id.n_used, slot = p - tok * id.n_used;
                     off[h] = tok * id.ld2 + slot * id.ld1;
                 }
             }
@@ -491,15 +523,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 }
             }
         } else if (done && row_ok) {
-            float *o = dst + (int64_t)blockIdx.z * part_stride + (int64_t)(tile_n * BN + u * CW) * ldd + row0 + r;
+            float *o = dst + (int64_t)blockIdx.z * part_stride + (int64_t)(tile_n * BN + cbase) * ldd + row0 + r;
 #pragma unroll
             for (int c = 0; c < CW; c += 2) {
                 float a0, a1;
                 f2_unpack(acc2[c / 2], a0, a1);
                 // (with the product cut along K, dst is this K part's own [N][ldd] scratch: plain stores, added up
                 // afterwards in a fixed order)
-                if (c < ncol) *o = a0;
-                if (c + 1 < ncol) o[ldd] = a1;
+                if (FULL || c < ncol) *o = a0;
+                if (FULL || c + 1 < ncol) o[ldd] = a1;
                 o += 2 * ldd;
             }
         }
@@ -508,6 +540,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     PROF_DUMP(warp == 0 ? "prod" : warp == 1 ? "mma " : warp < 4 ? "idle" : warp < 8 ? "unpk" : "epi ")
     tc_fence_before();
     __syncthreads();
+    pdl_trigger();
     if (abort_flag) {
         // a wait ran out: give copies still in flight time to land before the block's shared
         // memory is released, and tell the host
@@ -541,12 +574,9 @@ static const TileRoute NO_ROUTE_TC = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0,
 static b200q_status quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     dim3 grid((unsigned)(K / (tc::SB * tc::KB)), (unsigned)n_tiles);
-    if (ctx->tc_f16)
-        tc::quantize_tiled_kernel<true><<<grid, 256, 0, ctx->stream>>>((const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
-                                                                      src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr);
-    else
-        tc::quantize_tiled_kernel<false><<<grid, 256, 0, ctx->stream>>>((const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
-                                                                       src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr);
+    auto kern = ctx->tc_f16 ? tc::quantize_tiled_kernel<true> : tc::quantize_tiled_kernel<false>;
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1],
+                               src1->nb[2], src1->nb[3], K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);
     return B200Q_OK;
@@ -564,9 +594,11 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
                               int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
                               const TileRoute &tr) {
     typedef tc::Smem<TYPE, F16> L;
-    auto kern = tc::gemm_tc_kernel<TYPE, F16>;
-    static bool attr_set_dev[B200Q_MAX_DEVICES] = {};
-    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES];
+    // whole column tiles only (and no route): the build without a branch on the columns that are live
+    const bool full = !tr.tiles && N % tc::BN == 0;
+    auto kern = full ? tc::gemm_tc_kernel<TYPE, F16, true> : tc::gemm_tc_kernel<TYPE, F16, false>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES][2] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][full];
     if (!attr_set) {
         B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
         attr_set = true;
@@ -575,22 +607,11 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
     constexpr int BB = TYPE == B200Q_TYPE_Q8_0 ? 34 : 18;
     b200q_status st = make_weight_tmap3(ctx, &wmap, w, row_stride, M, (K / 32) * BB, tc::Raw<TYPE>::ROW, n_mat, mat_stride);
     if (st != B200Q_OK) return st;
-    // Cut K into 2, 4 or 8 parts when the tiles alone leave SMs idle (a 512-row shard of a tensor-parallel product is
-    // 16 tiles on 148 SMs and every tile walks all of K): the schedule's length is rounds of blocks x stages per
-    // block. Parts write their own scratch and a second kernel adds them in a fixed order, so the result does not
-    // depend on which block finishes first.
-    const int64_t units = n_tiles * ((M + tc::BM - 1) / tc::BM), S = ctx->sm_count, nst = K / 256;
-    unsigned ksplit = 1;
-    if (!tr.tiles && !ctx->no_ksplit) {
-        // in stages: a block costs about three stages' time beyond its K walk (set-up, drain, stores), the adding pass one
-        constexpr int64_t FIXED = 3;
-        int64_t best = ((units + S - 1) / S) * (nst + FIXED);
-        for (unsigned ks = 2; ks <= 8; ks *= 2) {
-            if (nst % ks || nst / ks < 2) break;
-            const int64_t len = ((units * ks + S - 1) / S) * (nst / ks + FIXED) + 1;
-            if (len < best) { best = len; ksplit = ks; }
-        }
-    }
+    // Cut K when the tiles alone leave SMs idle (a 512-row shard of a tensor-parallel product is 16 tiles on 148 SMs and
+    // every tile walks all of K). Parts write their own scratch and a second kernel adds them in a fixed order, so the result
+    // does not depend on which block finishes first.
+    const int64_t tiles = n_tiles * ((M + tc::BM - 1) / tc::BM);
+    const int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, ctx->sm_count, K / 256, TC_SB_NS, M * N);
     float *out = dst;
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
@@ -599,17 +620,11 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
         out = (float *)ctx->moe_ws[9].ptr;
         out_ld = M;
     }
-    dim3 grid((unsigned)n_tiles, (unsigned)((M + tc::BM - 1) / tc::BM), ksplit);
-    kern<<<grid, tc::THREADS, L::TOTAL, ctx->stream>>>(wmap, (int)M, (int)K, act, (int)N, out, out_ld, part_stride, ctx->error_word, tr);
+    dim3 grid((unsigned)n_tiles, (unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)ksplit);
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(tc::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N, out, out_ld,
+                               part_stride, ctx->error_word, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
-    if (ksplit > 1) {
-        const int64_t total = N * M;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > (int64_t)S * 8) blocks = (int64_t)S * 8;
-        tc::ksplit_sum_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(out, (int)ksplit, part_stride, (int)M, N, dst, ldd);
-        B200Q_CUDA(ctx, cudaGetLastError());
-        count(ctx, ST_GEMM_KSPLIT);
-    }
+    if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);
     if (F16) count(ctx, ST_GEMM_TC_F16);
     return B200Q_OK;
