@@ -154,12 +154,13 @@ static b200q_status check_ids(b200q_ctx *ctx, const b200q_tensor *src0, const b2
 }
 
 // Quantize src1 once per graph: q/k/v and gate/up share their input (P01:670-688).
-static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor *src1, ActView *out) {
+static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor *src1, ActView *out, int64_t gate = 0) {
     ActKey key;
     key.data = src1->data;
     key.id = src1->id;
     key.form = form;
     key.gen = ctx->generation;
+    key.gate = gate;
     for (int i = 0; i < 4; ++i) { key.ne[i] = src1->ne[i]; key.nb[i] = src1->nb[i]; }
     ActEntry *hit = nullptr;
     for (auto &e : ctx->act_cache)
@@ -202,7 +203,7 @@ static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor 
         if (form == ACT_Q8_256 && (st = ws_reserve(ctx, &e.sums16, sizeof(int16_t) * (size_t)(N * (K / 16)) + 64)) != B200Q_OK)
             return st;
         if ((st = launch_quantize_act(ctx, form, src1, (int8_t *)e.codes.ptr, e.scales.ptr, (int16_t *)e.sums.ptr,
-                                      (int16_t *)e.sums16.ptr)) != B200Q_OK)
+                                      (int16_t *)e.sums16.ptr, gate)) != B200Q_OK)
             return st;
         e.key = key;
         e.valid = true;
@@ -423,7 +424,13 @@ b200q_status b200q_mul_mat(b200q_ctx *ctx, const b200q_tensor *src0, const b200q
 
 b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1,
                               const b200q_tensor *ids, b200q_tensor *dst) {
-    if (!ctx) return B200Q_INVALID;
+    return ctx ? mul_mat_id(ctx, src0, src1, ids, dst, 0) : B200Q_INVALID;
+}
+
+}  // extern "C"
+
+b200q_status b200q::mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const b200q_tensor *ids,
+                               b200q_tensor *dst, int64_t gate) {
     b200q_status st = check_mul_mat(ctx, src0, src1, dst, true);
     if (st != B200Q_OK) return st;
     st = check_ids(ctx, src0, src1, ids, dst);
@@ -451,11 +458,11 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
         const void *before = ctx->moe_ws[7].ptr;
         if ((st = ws_reserve(ctx, &ctx->moe_ws[7], bytes)) != B200Q_OK) return st;
         const bool grew = ctx->moe_ws[7].ptr != before;
-        TileRoute tr = { rv.tiles128, rv.n_tiles + 4, rv.pairs, n_used, ne11, src1->nb[1], src1->nb[2], ld1, ld2 };
+        TileRoute tr = { rv.tiles128, rv.n_tiles + 4, rv.pairs, n_used, ne11, src1->nb[1], src1->nb[2], ld1, ld2, gate };
         count(ctx, ST_MOE_GEMM);
         // the scratch may already hold this very activation, gathered for these ids in this graph
         auto &ma = ctx->moe_act;
-        bool ready = !grew && ma.src1 == src1->data && ma.ids == ids->data && ma.src1_id == src1->id && ma.ids_id == ids->id && ma.gen == ctx->generation && ma.form == form &&
+        bool ready = !grew && ma.src1 == src1->data && ma.ids == ids->data && ma.src1_id == src1->id && ma.ids_id == ids->id && ma.gen == ctx->generation && ma.form == form && ma.gate == gate &&
                      ma.n_expert == n_expert;
         for (int i = 0; i < 4 && ready; ++i) ready = ma.ne[i] == src1->ne[i] && ma.nb[i] == src1->nb[i];
         if (ready) count(ctx, ST_ACT_CACHE_HIT);
@@ -465,6 +472,7 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
         ma.ids_id = ids->id;
         ma.gen = ctx->generation;
         ma.form = form;
+        ma.gate = gate;
         ma.n_expert = n_expert;
         for (int i = 0; i < 4; ++i) { ma.ne[i] = src1->ne[i]; ma.nb[i] = src1->nb[i]; }
         return per32 ? launch_gemm_tc_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
@@ -472,7 +480,7 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
                      : launch_gemm_kq_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready);
     }
     ActView act;
-    if ((st = get_activation(ctx, ti.act_form, src1, &act)) != B200Q_OK) return st;
+    if ((st = get_activation(ctx, ti.act_form, src1, &act, gate)) != B200Q_OK) return st;
     // a handful of tokens: one unit per pair, its expert read on the device (the reference's
     // per-pair GEMV below GGML_OPENCL_KQ_MM_ID_MIN_TOK); more: route once per ids tensor
     // and graph, then one launch per tile size class
@@ -489,6 +497,8 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
     }
     return B200Q_OK;
 }
+
+extern "C" {
 
 static b200q_status join_copy_stream(b200q_ctx *ctx);
 

@@ -76,8 +76,9 @@ struct ActKey {
     size_t  nb[4];
     int     form;
     uint64_t gen;
+    int64_t gate;            // SwiGLU in the quantizer (see TileRoute), 0: the values as they are
     bool operator==(const ActKey &o) const {
-        if (data != o.data || id != o.id || form != o.form || gen != o.gen) return false;
+        if (data != o.data || id != o.id || form != o.form || gen != o.gen || gate != o.gate) return false;
         for (int i = 0; i < 4; ++i) if (ne[i] != o.ne[i] || nb[i] != o.nb[i]) return false;
         return true;
     }
@@ -118,7 +119,7 @@ struct b200q_ctx {
     uint64_t     generation = 1;
     // what the gathered, tiled activation scratch of the tensor-core MUL_MAT_ID holds (gate and up of a layer
     // read the same src1 through the same ids: the second call finds it ready)
-    struct { const void *src1 = nullptr, *ids = nullptr, *src1_id = nullptr, *ids_id = nullptr; int64_t ne[4] = {0, 0, 0, 0}; size_t nb[4] = {0, 0, 0, 0}; uint64_t gen = 0; int form = -1, n_expert = 0; } moe_act;
+    struct { const void *src1 = nullptr, *ids = nullptr, *src1_id = nullptr, *ids_id = nullptr; int64_t ne[4] = {0, 0, 0, 0}; size_t nb[4] = {0, 0, 0, 0}; uint64_t gen = 0; int64_t gate = 0; int form = -1, n_expert = 0; } moe_act;
     bool         route_skip_negative = false;   // expert-parallel local product: negative ids are empty slots
     int          route_pinned = -1;       // a route entry in use across a nested call: not a victim
     uint64_t     private_generation = 0;  // expert-parallel calls: generations of their internal products
@@ -175,7 +176,7 @@ inline void  count(b200q_ctx *ctx, int stat) { ++ctx->counters[stat]; }
 
 // quantize.cu
 b200q_status launch_quantize_act(b200q_ctx *ctx, int form, const b200q_tensor *src1, int8_t *codes, void *scales,
-                                 int16_t *sums32, int16_t *sums16);
+                                 int16_t *sums32, int16_t *sums16, int64_t gate = 0);
 b200q_status launch_dequantize(b200q_ctx *ctx, int type, const void *w, int64_t M, int64_t K, size_t row_stride,
                                float *out);
 
@@ -200,6 +201,15 @@ b200q_status launch_gemv_allreduce(b200q_ctx *ctx, int type, const void *w, size
                                    const b200q_tensor *src1, int ncols, float *dst, int64_t ldd, uint64_t *const *peers, uint32_t *state,
                                    int rank, int nranks);
 bool gemv_ar_shape_ok(int type, const void *w, size_t row_stride, int64_t M, int64_t K, int ncols, int64_t ldd);
+// api.cu: MUL_MAT_ID; gate != 0: src1 is the up projection of a SwiGLU whose gate values lie `gate` floats from it, and what is
+// quantized and multiplied is silu(gate) * src1
+b200q_status mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const b200q_tensor *ids, b200q_tensor *dst,
+                        int64_t gate);
+// silu(g) * u, as every quantizer that takes the gate along computes it
+__device__ __forceinline__ float swiglu(float g, float u) { return g / (1.f + expf(-g)) * u; }
+__device__ __forceinline__ float4 swiglu4(float4 g, float4 u) {
+    return make_float4(swiglu(g.x, u.x), swiglu(g.y, u.y), swiglu(g.z, u.z), swiglu(g.w, u.w));
+}
 // api.cu: the quantized activation of src1 in the decode layout of the weight type's form (cached per graph)
 b200q_status get_decode_activation(b200q_ctx *ctx, int weight_type, const b200q_tensor *src1, ActView *out);
 // moe.cu: route (pairs sorted by expert, tile lists by size class)
@@ -226,6 +236,7 @@ struct TileRoute {
     int            n_used, ne11;
     size_t         nb1, nb2;   // src1: bytes between slot rows and between tokens
     int64_t        ld1, ld2;   // dst: floats between slots and between tokens
+    int64_t        gate;       // SwiGLU in the quantizer: floats from an element of src1 to the gate value of the same place (0: none)
 };
 b200q_status make_weight_tmap3(b200q_ctx *ctx, void *tmap_out, const void *w, size_t row_stride, int64_t M, int64_t row_bytes,
                                int box_bytes, int64_t n_mat, size_t mat_stride);

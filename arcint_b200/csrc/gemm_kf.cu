@@ -92,6 +92,7 @@ constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 
 
 // The quantizer of the layout above, per-256 form (the reference's kernel_quant_i8 rule: scale bm/127, round to nearest
 // even, zero below 1e-30).
+template <bool GATE>
 __global__ void __launch_bounds__(256)
 quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
                     int64_t N, uint8_t *__restrict__ out, TileRoute id) {
@@ -135,6 +136,7 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             v[i] = x ? __ldg(reinterpret_cast<const float4 *>(x) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (GATE && x) v[i] = swiglu4(__ldg(reinterpret_cast<const float4 *>(x + id.gate) + i), v[i]);
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
         }
 #pragma unroll
@@ -586,7 +588,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 
 }  // namespace kf
 
-static const TileRoute NO_ROUTE_KF = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0 };
+static const TileRoute NO_ROUTE_KF = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
 size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + kf::BN - 1) / kf::BN) * (K / 256)) * kf::CHUNK; }
 size_t gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles) { return gemm_kf_act_bytes(K, max_tiles * kf::BN); }
@@ -601,7 +603,7 @@ bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 static b200q_status quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0];
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kf::quantize_f16_kernel, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kf::quantize_f16_kernel<true> : kf::quantize_f16_kernel<false>, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
                                src1->nb[1], src1->nb[2], src1->nb[3], K, src1->ne[1] * src1->ne[2] * src1->ne[3], out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);

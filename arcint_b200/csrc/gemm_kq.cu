@@ -100,6 +100,7 @@ static_assert(NG == 2 && NACT == 2 && NBUF == 2, "barrier slots above");
 
 // Activation chunk (128-token tile t, super-block s), per-256 form (the reference's
 // kernel_quant_i8 rule: scale bm/127, round to nearest even, zero below 1e-30), in the group layout above.
+template <bool GATE>
 __global__ void __launch_bounds__(256)
 quantize_tiled256_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
                          int64_t N, uint8_t *__restrict__ out, TileRoute id) {
@@ -141,6 +142,7 @@ quantize_tiled256_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t n
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             v[i] = x ? __ldg(reinterpret_cast<const float4 *>(x) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (GATE && x) v[i] = swiglu4(__ldg(reinterpret_cast<const float4 *>(x + id.gate) + i), v[i]);
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
         }
 #pragma unroll
@@ -581,7 +583,7 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 }  // namespace kq
 
 static size_t kq_chunks(int64_t K, int64_t N) { return (size_t)(((N + kq::BN - 1) / kq::BN) * (K / 256)); }
-static const TileRoute NO_ROUTE = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0 };
+static const TileRoute NO_ROUTE = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
 size_t gemm_kq_act_bytes(int64_t K, int64_t N) {
     return kq_chunks(K, N) * kq::ACT_CHUNK;
@@ -604,7 +606,7 @@ bool gemm_kq_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 static b200q_status quantize256(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0];
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kq::quantize_tiled256_kernel, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kq::quantize_tiled256_kernel<true> : kq::quantize_tiled256_kernel<false>, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
                                src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, src1->ne[1] * src1->ne[2] * src1->ne[3], out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);

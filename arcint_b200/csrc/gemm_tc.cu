@@ -104,7 +104,7 @@ static_assert(BAR_COUNT <= 64, "the shared block reserves 64 mbarrier slots");
 //   codes  [block j < 8][piece c][group g < 16][column r < 8][16 bytes]   column 8g + r; int8: two pieces of 16 k
 //          (k = 32j + 16c + byte), fp16: four pieces of 8 k (k = 32j + 8c + half), the codes as exact halves
 //   scales [block j < 8][column < 128] f32 (the fp16-rounded block scale)
-template <bool F16>
+template <bool F16, bool GATE>
 __global__ void __launch_bounds__(256)
 quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
                       int64_t N, uint8_t *__restrict__ out, TileRoute id) {
@@ -129,6 +129,7 @@ quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1,
         cnt = left < BN ? (int)left : BN;
     }
     const int j = l >> 1;
+    const int64_t gate = id.gate;                        // (the block scale below is called id)
 #pragma unroll 1
     for (int col = hw; col < BN; col += 16) {
         const float *x = nullptr;
@@ -147,7 +148,8 @@ quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1,
         float amax = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float4 f = x ? *reinterpret_cast<const float4 *>(x + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 f = x ? *reinterpret_cast<const float4 *>(x + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (GATE && x) f = swiglu4(*reinterpret_cast<const float4 *>(x + gate + 4 * i), f);
             v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
         }
@@ -569,12 +571,13 @@ bool gemm_tc_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
     return true;
 }
 
-static const TileRoute NO_ROUTE_TC = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0 };
+static const TileRoute NO_ROUTE_TC = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
 static b200q_status quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     dim3 grid((unsigned)(K / (tc::SB * tc::KB)), (unsigned)n_tiles);
-    auto kern = ctx->tc_f16 ? tc::quantize_tiled_kernel<true> : tc::quantize_tiled_kernel<false>;
+    auto kern = tr.gate ? (ctx->tc_f16 ? tc::quantize_tiled_kernel<true, true> : tc::quantize_tiled_kernel<false, true>)
+                        : (ctx->tc_f16 ? tc::quantize_tiled_kernel<true, false> : tc::quantize_tiled_kernel<false, false>);
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1],
                                src1->nb[2], src1->nb[3], K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());

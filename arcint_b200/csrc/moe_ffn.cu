@@ -9,7 +9,7 @@
 //            w_j /= clamp(sum_j w_j, cmin, cmax);
 //   gate/up  two MUL_MAT_ID over the token's activation (they share the route, the gathered activation and,
 //            under expert parallelism, the dispatch);
-//   SwiGLU   h = silu(gate) * up, elementwise;
+//   SwiGLU   h = silu(gate) * up, in the quantizer of the down projection's activation;
 //   down     MUL_MAT_ID over h;
 //   combine  y[:, t] = sum_i w[i, t] * down[:, i, t].
 //
@@ -18,6 +18,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace b200q {
 
@@ -27,6 +28,8 @@ template <int NPER>
 __global__ void __launch_bounds__(128)
 moe_router_kernel(const uint8_t *__restrict__ logits, size_t nb1, int n_expert, int n_used, int n_tok, float cmin, float cmax,
                   uint8_t *__restrict__ ids, size_t ids_nb1, uint8_t *__restrict__ wts, size_t wts_nb1) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31, t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= n_tok) return;                                    // whole warps leave together
     const float *x = reinterpret_cast<const float *>(logits + (size_t)t * nb1);
@@ -79,24 +82,12 @@ moe_router_kernel(const uint8_t *__restrict__ logits, size_t nb1, int n_expert, 
     if (lane < n_used) wo[lane] = wsel / denom;
 }
 
-// h = silu(g) * u over n elements; g, u, h may be the same buffers (h may overwrite g)
-__global__ void __launch_bounds__(256)
-swiglu_kernel(const float *__restrict__ g, const float *__restrict__ u, float *__restrict__ h, int64_t n4) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 a = reinterpret_cast<const float4 *>(g)[i], b = reinterpret_cast<const float4 *>(u)[i];
-        float4 r;
-        r.x = a.x / (1.f + expf(-a.x)) * b.x;
-        r.y = a.y / (1.f + expf(-a.y)) * b.y;
-        r.z = a.z / (1.f + expf(-a.z)) * b.z;
-        r.w = a.w / (1.f + expf(-a.w)) * b.w;
-        reinterpret_cast<float4 *>(h)[i] = r;
-    }
-}
-
 // y[m, t] = sum_i w[i, t] * d[m, i, t]; d is [M][n_used][n_tok] packed, y has column stride ldy, added in slot order
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float *__restrict__ d, const uint8_t *__restrict__ wts, size_t wts_nb1, int M, int n_used, int n_tok,
                    float *__restrict__ y, int64_t ldy) {
+    pdl_trigger();
+    pdl_wait();
     const int t = blockIdx.y;
     const float *w = reinterpret_cast<const float *>(wts + (size_t)t * wts_nb1);
     const float *dt = d + (size_t)t * n_used * M;
@@ -113,8 +104,8 @@ static b200q_status launch_router(b200q_ctx *ctx, const b200q_tensor *logits, in
     if (n_tok == 0) return B200Q_OK;
     const dim3 grid((unsigned)((n_tok + 3) / 4));
 #define B200Q_ROUTER(NPER)                                                                                                   \
-    moe_router_kernel<NPER><<<grid, 128, 0, ctx->stream>>>((const uint8_t *)logits->data, logits->nb[1], n_expert, n_used, n_tok, \
-                                                           cmin, cmax, (uint8_t *)ids->data, ids->nb[1], (uint8_t *)wts->data, wts->nb[1])
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, moe_router_kernel<NPER>, grid, dim3(128), 0, ctx->stream, (const uint8_t *)logits->data, logits->nb[1], \
+                               n_expert, n_used, n_tok, cmin, cmax, (uint8_t *)ids->data, ids->nb[1], (uint8_t *)wts->data, wts->nb[1]))
     if (n_expert <= 64) B200Q_ROUTER(2);
     else if (n_expert <= 128) B200Q_ROUTER(4);
     else if (n_expert <= 256) B200Q_ROUTER(8);
@@ -193,19 +184,13 @@ b200q_status b200q_moe_ffn(b200q_ctx *ctx, const b200q_tensor *gate_w, const b20
     b200q_tensor d = tensor(B200Q_TYPE_F32, ws + o_d, d_model, n_used, n_tok, ws + o_d);
     st = b200q_mul_mat_id(ctx, gate_w, &x3, &ids, &g);
     if (st == B200Q_OK) st = b200q_mul_mat_id(ctx, up_w, &x3, &ids, &u);
-    if (st == B200Q_OK) {
-        const int64_t n4 = (int64_t)(pairs * d_ff / 4);
-        const int64_t blocks = (n4 + 255) / 256;
-        swiglu_kernel<<<(unsigned)(blocks > 148 * 8 ? 148 * 8 : blocks), 256, 0, ctx->stream>>>((const float *)g.data, (const float *)u.data,
-                                                                                                (float *)u.data, n4);
-        if (cudaGetLastError() != cudaSuccess) st = fail(ctx, B200Q_CUDA_ERROR, "swiglu launch");
-    }
-    if (st == B200Q_OK) st = b200q_mul_mat_id(ctx, down_w, &u, &ids, &d);
+    // the activation of the down projection is silu(gate) * up, computed where it is quantized
+    if (st == B200Q_OK) st = mul_mat_id(ctx, down_w, &u, &ids, &d, (const float *)g.data - (const float *)u.data);
     if (st == B200Q_OK) {
         const dim3 grid((unsigned)((d_model + 255) / 256), (unsigned)n_tok);
-        moe_combine_kernel<<<grid, 256, 0, ctx->stream>>>((const float *)d.data, (const uint8_t *)wts.data, wts.nb[1], (int)d_model, n_used,
-                                                          (int)n_tok, (float *)y->data, (int64_t)(y->nb[1] / 4));
-        if (cudaGetLastError() != cudaSuccess) st = fail(ctx, B200Q_CUDA_ERROR, "combine launch");
+        const cudaError_t e = launch_pdl(!ctx->no_pdl, moe_combine_kernel, grid, dim3(256), 0, ctx->stream, (const float *)d.data, (const uint8_t *)wts.data,
+                                         wts.nb[1], (int)d_model, n_used, (int)n_tok, (float *)y->data, (int64_t)(y->nb[1] / 4));
+        if (e != cudaSuccess) st = fail(ctx, B200Q_CUDA_ERROR, "combine launch: %s", cudaGetErrorString(e));
     }
     ctx->generation = caller_gen;
     if (st == B200Q_OK) count(ctx, ST_MOE_FFN);

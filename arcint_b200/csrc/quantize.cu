@@ -29,10 +29,11 @@ __device__ __forceinline__ const float *col_ptr(const ColAddr &a, int64_t c) {
     return reinterpret_cast<const float *>(a.base + c1 * a.nb1 + c2 * a.nb2 + c3 * a.nb3);
 }
 
-// 8 lanes per 32-block, 4 values per lane
+// 8 lanes per 32-block, 4 values per lane. GATE: the values are silu(gate) * src, the gate values `gate` floats from src
+template <bool GATE>
 __global__ void __launch_bounds__(256)
 quantize_q8_0_kernel(ColAddr src, int64_t K, int64_t ncols, int8_t *__restrict__ codes, uint16_t *__restrict__ d16,
-                     int16_t *__restrict__ sums32) {
+                     int16_t *__restrict__ sums32, int64_t gate) {
     pdl_trigger();
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -40,7 +41,11 @@ quantize_q8_0_kernel(ColAddr src, int64_t K, int64_t ncols, int8_t *__restrict__
     const int64_t c = gid / per_col, i4 = gid % per_col;
     const bool live = c < ncols;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) v = *reinterpret_cast<const float4 *>(col_ptr(src, c) + 4 * i4);
+    if (live) {
+        const float *x = col_ptr(src, c) + 4 * i4;
+        v = *reinterpret_cast<const float4 *>(x);
+        if (GATE) v = swiglu4(*reinterpret_cast<const float4 *>(x + gate), v);
+    }
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
@@ -64,9 +69,10 @@ quantize_q8_0_kernel(ColAddr src, int64_t K, int64_t ncols, int8_t *__restrict__
 }
 
 // one warp per 256-block, 8 values per lane
+template <bool GATE>
 __global__ void __launch_bounds__(256)
 quantize_q8_256_kernel(ColAddr src, int64_t K, int64_t ncols, int8_t *__restrict__ codes, float *__restrict__ d32,
-                       int16_t *__restrict__ bsums, int16_t *__restrict__ bsums16) {
+                       int16_t *__restrict__ bsums, int16_t *__restrict__ bsums16, int64_t gate) {
     pdl_trigger();
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -75,7 +81,11 @@ quantize_q8_256_kernel(ColAddr src, int64_t K, int64_t ncols, int8_t *__restrict
     const int64_t c = wid / per_col, b = wid % per_col;
     if (c >= ncols) return;                       // whole warps leave together
     const float *x = col_ptr(src, c) + 256 * b + 8 * lane;
-    const float4 v0 = *reinterpret_cast<const float4 *>(x), v1 = *reinterpret_cast<const float4 *>(x + 4);
+    float4 v0 = *reinterpret_cast<const float4 *>(x), v1 = *reinterpret_cast<const float4 *>(x + 4);
+    if (GATE) {
+        v0 = swiglu4(*reinterpret_cast<const float4 *>(x + gate), v0);
+        v1 = swiglu4(*reinterpret_cast<const float4 *>(x + gate + 4), v1);
+    }
     float bm = fmaxf(fmaxf(fmaxf(fabsf(v0.x), fabsf(v0.y)), fmaxf(fabsf(v0.z), fabsf(v0.w))),
                      fmaxf(fmaxf(fabsf(v1.x), fabsf(v1.y)), fmaxf(fabsf(v1.z), fabsf(v1.w))));
 #pragma unroll
@@ -103,7 +113,7 @@ quantize_q8_256_kernel(ColAddr src, int64_t K, int64_t ncols, int8_t *__restrict
 }
 
 b200q_status launch_quantize_act(b200q_ctx *ctx, int form, const b200q_tensor *src1, int8_t *codes, void *scales,
-                                 int16_t *bsums, int16_t *bsums16) {
+                                 int16_t *bsums, int16_t *bsums16, int64_t gate) {
     const int64_t K = src1->ne[0];
     const int64_t ncols = src1->ne[1] * src1->ne[2] * src1->ne[3];
     if (ncols == 0) return B200Q_OK;
@@ -116,13 +126,13 @@ b200q_status launch_quantize_act(b200q_ctx *ctx, int form, const b200q_tensor *s
     a.nb3 = src1->nb[3];
     if (form == ACT_Q8_0) {
         const int64_t threads = ncols * (K / 4);
-        B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, quantize_q8_0_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,
-                                   ctx->stream, a, K, ncols, codes, (uint16_t *)scales, bsums));
+        B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, gate ? quantize_q8_0_kernel<true> : quantize_q8_0_kernel<false>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,
+                                   ctx->stream, a, K, ncols, codes, (uint16_t *)scales, bsums, gate));
         count(ctx, ST_QUANT_Q8_0);
     } else {
         const int64_t warps = ncols * (K / 256);
-        B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, quantize_q8_256_kernel, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0,
-                                   ctx->stream, a, K, ncols, codes, (float *)scales, bsums, bsums16));
+        B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, gate ? quantize_q8_256_kernel<true> : quantize_q8_256_kernel<false>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0,
+                                   ctx->stream, a, K, ncols, codes, (float *)scales, bsums, bsums16, gate));
         count(ctx, ST_QUANT_Q8_256);
     }
     B200Q_CUDA(ctx, cudaGetLastError());
