@@ -266,6 +266,7 @@ b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_
 // the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
 
+b200q_status ksplit_scratch(b200q_ctx *ctx, int64_t M, int64_t N, int *ksplit, float **parts);
 // K parts of a product whose tiles fill the SMs badly; the times of a 256-weight step on a full tile that it counts with
 int          choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_t outputs);
 constexpr int TC_SB_NS = 2000, KQ_SB_NS = 2000, KF_SB_NS = 900;

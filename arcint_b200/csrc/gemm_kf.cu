@@ -635,14 +635,13 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     if (st != B200Q_OK) return st;
     // persistent blocks, one per SM, walking the (row tile, column tile, part of K) units
     const int64_t tiles = n_tiles * ((M + kf::BM - 1) / kf::BM), S = ctx->sm_count;
-    const int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, S, K / 256, KF_SB_NS, M * N);
+    int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, S, K / 256, KF_SB_NS, M * N);
     float *out = dst;
     int64_t out_ld = ldd, part_stride = 0;
+    if (ksplit > 1 && (st = ksplit_scratch(ctx, M, N, &ksplit, &out)) != B200Q_OK) return st;
     if (ksplit > 1) {
         // parts write their own scratch and a second kernel adds them in a fixed order
         part_stride = N * M;
-        if ((st = ws_reserve(ctx, &ctx->moe_ws[9], sizeof(float) * (size_t)part_stride * ksplit)) != B200Q_OK) return st;
-        out = (float *)ctx->moe_ws[9].ptr;
         out_ld = M;
     }
     const int64_t units = tiles * ksplit;

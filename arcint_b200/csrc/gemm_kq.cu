@@ -651,10 +651,11 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     float *out = dst;
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
-        b200q_status st = ws_reserve(ctx, &ctx->moe_ws[9], sizeof(float) * (size_t)(N * M) * ksplit);
+        const b200q_status st = ksplit_scratch(ctx, M, N, &ksplit, &out);
         if (st != B200Q_OK) return st;
+    }
+    if (ksplit > 1) {
         part_stride = N * M;
-        out = (float *)ctx->moe_ws[9].ptr;
         out_ld = M;
         units *= ksplit;
     }

@@ -614,13 +614,12 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
     // every tile walks all of K). Parts write their own scratch and a second kernel adds them in a fixed order, so the result
     // does not depend on which block finishes first.
     const int64_t tiles = n_tiles * ((M + tc::BM - 1) / tc::BM);
-    const int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, ctx->sm_count, K / 256, TC_SB_NS, M * N);
+    int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, ctx->sm_count, K / 256, TC_SB_NS, M * N);
     float *out = dst;
     int64_t out_ld = ldd, part_stride = 0;
+    if (ksplit > 1 && (st = ksplit_scratch(ctx, M, N, &ksplit, &out)) != B200Q_OK) return st;
     if (ksplit > 1) {
         part_stride = N * M;
-        if ((st = ws_reserve(ctx, &ctx->moe_ws[9], sizeof(float) * (size_t)part_stride * ksplit)) != B200Q_OK) return st;
-        out = (float *)ctx->moe_ws[9].ptr;
         out_ld = M;
     }
     dim3 grid((unsigned)n_tiles, (unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)ksplit);

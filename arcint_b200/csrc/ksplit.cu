@@ -42,6 +42,18 @@ int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_
     return best_ks;
 }
 
+// Scratch for the parts. Without the memory for it the product is not cut: ksplit becomes 1.
+b200q_status ksplit_scratch(b200q_ctx *ctx, int64_t M, int64_t N, int *ksplit, float **parts) {
+    const b200q_status st = ws_reserve(ctx, &ctx->moe_ws[9], sizeof(float) * (size_t)(N * M) * *ksplit);
+    if (st == B200Q_NO_MEMORY) {
+        (void)cudaGetLastError();
+        *ksplit = 1;
+        return B200Q_OK;
+    }
+    *parts = (float *)ctx->moe_ws[9].ptr;
+    return st;
+}
+
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd) {
     // four rows a thread where every part's and dst's columns start on 16 bytes
     const bool vec = M % 4 == 0 && ldd % 4 == 0 && (uintptr_t)dst % 16 == 0;
