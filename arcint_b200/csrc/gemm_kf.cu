@@ -6,10 +6,20 @@
 // out += d * d_x * sum_sb sc_sb I_sb - dmin * d_x * sum_sb m_sb bsum_sb, with I_sb the exact dot of the weight codes with the
 // int8 activation (per-256 activation scale) and bsum_sb the sum of the activation codes. The integer sub-scale is folded
 // into the weight operand: p = sc * q <= 63 * 31 = 1953 is an integer that a half holds exactly, the activation code too, so
-// one chain of kind::f16 MMAs over the super-block gives sum(p x) in an f32 accumulator: every partial sum below 2^24 is
-// exact, larger ones carry f32 rounding as ggml's own float(sumi) does. The mins term is one more K = 16 MMA per
-// super-block into an accumulator of its own: a row of A is [m_0..m_7, m_0..m_7], a column of B is
-// [bl_0..bl_7, 256 bh_0..256 bh_7] with bsum_j = 256 bh_j + bl_j (all exact in f16).
+// one chain of kind::f16 MMAs over the super-block gives sum(p x) in an f32 accumulator, exactly while every partial sum stays
+// within 2^24. Past it the tensor core cuts bits off at each of the sixteen steps (measured on one-sided activations, sums up to 3.3 x
+// 2^24: 3.2 ulp too small on average, where rounding the integer sum once is off by half an ulp at most). p >= 0, so no partial sum of
+// a column, in any order, exceeds max(p) times the larger of the sums of its positive and of its negative codes. The quantizer
+// writes the largest of these per (column tile, super-block). A column tile where one does not rule 2^24 out takes its super-blocks in
+// two chains of four blocks (Q4_K: 128 * 945 * 127 < 2^24) or four of two (Q5_K: 64 * 1953 * 127), each exact, which the scaling
+// warps add one after the other in f32. Distance from the 64-bit product, activations uniform in 0.6..1, K = 4096: 1.2e-6 (Q4_K), 1.4e-6
+// (Q5_K; 7.4e-6 with one chain; int32 sums with the mins in a second pass: 1.0e-5). The largest sums of a tile are read once a unit,
+// which then has one chain or several throughout: asked per super-block, the answer cost the MMA issuer 4 %, and reading a unit
+// ahead cost registers and 2 % of a 512-expert block. Q4_K 11008x4096 x 512 tokens: 75 us with one chain, 93 with two;
+// Q5_K 85 and 136 with four. N(0, 1) activations take one, their one-sided sums are half of what Q5_K's chain holds; activations of
+// one sign take more from a mean of 0.55 (Q4_K) and 0.26 (Q5_K) of the largest.
+// The mins term is one more K = 16 MMA per super-block into an accumulator of its own: a row of A is [m_0..m_7, m_0..m_7], a column of
+// B is [bl_0..bl_7, 256 bh_0..256 bh_7] with bsum_j = 256 bh_j + bl_j (all exact in f16).
 //
 // The weight operand goes through TENSOR MEMORY: an unpack thread decodes a row's blocks in registers and stores them with
 // tcgen05.st into the lane of its row, and the MMAs take A from there: no operand stores, proxy fences and operand reads
@@ -61,13 +71,19 @@ static_assert(128 * 48 + 256 * 56 + 256 * 160 <= THREADS * LAUNCH_REGS, "registe
 //   codes, twice (blocks 0..3, 4..7): [group g < 16][block j < 4][piece c < 4][column r < 8][8 codes as halves, each run of four
 //          in the order 0 2 1 3, in which the unpack threads mask nibbles out of a word]
 //   extra: 128 f32 scales, then the mins operand [group g < 16][piece c < 2][column r < 8][8 halves: bl_0..7 or 256 bh_0..7]
+// A column tile is its chunks, then an int32 per super-block: the largest one-sided sum of codes of a column, see above.
 constexpr int CODE_BLOCK = 512, CODE_GROUP = GB * CODE_BLOCK, CODE_STAGE = (BN / 8) * CODE_GROUP;
 constexpr int MINS_GROUP = 256, EXTRA_MINS = BN * 4, EXTRA = EXTRA_MINS + (BN / 8) * MINS_GROUP;
 constexpr int CHUNK = 2 * CODE_STAGE + EXTRA;
+__host__ __device__ constexpr size_t tile_bytes(int64_t nsb) { return (size_t)nsb * CHUNK + (size_t)((4 * nsb + 127) / 128 * 128); }
 
 template <int TYPE> struct Fmt;
-template <> struct Fmt<B200Q_TYPE_Q4_K> { enum { SBB = 144, NRAW = 3 }; };
-template <> struct Fmt<B200Q_TYPE_Q5_K> { enum { SBB = 176, NRAW = 2 }; };
+template <> struct Fmt<B200Q_TYPE_Q4_K> { enum { SBB = 144, NRAW = 3, PMAX = 63 * 15, CHAINS = 2 }; };
+template <> struct Fmt<B200Q_TYPE_Q5_K> { enum { SBB = 176, NRAW = 2, PMAX = 63 * 31, CHAINS = 4 }; };
+
+// a super-block with a larger one-sided sum makes its column tile take several chains; a chain of theirs is exact
+template <int TYPE> __host__ __device__ constexpr int one_chain_side() { return (1 << 24) / Fmt<TYPE>::PMAX; }
+static_assert(256 / 2 * 127 * 63 * 15 <= (1 << 24) && 256 / 4 * 127 * 63 * 31 <= (1 << 24), "CHAINS");
 
 template <int TYPE> struct Smem {
     enum {
@@ -84,9 +100,9 @@ template <int TYPE> struct Smem {
     static_assert(RAW_STAGE % 128 == 0 && EXTRA % 128 == 0, "tiled copies");
 };
 
-enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_CODE_FULL = 6, BAR_CODE_EMPTY = 10, BAR_X_FULL = 14, BAR_X_EMPTY = 17, BAR_A_FULL = 20,
-       BAR_A_EMPTY = 22, BAR_ACC_FULL = 24, BAR_ACC_EMPTY = 26, BAR_COUNT = 28 };
-static_assert(NCODE == 4 && NX == 3 && NG == 2, "barrier slots above");
+enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_CODE_FULL = 6, BAR_CODE_EMPTY = 10, BAR_X_FULL = 14, BAR_X_EMPTY = 17, BAR_A_FULL = 22,
+       BAR_A_EMPTY = 24, BAR_ACC_FULL = 26, BAR_ACC_EMPTY = 28, BAR_COUNT = 30 };
+static_assert(NCODE == 4 && NX == 3 && NG == 2 && BAR_COUNT <= 32, "barrier slots above");
 
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
 
@@ -104,7 +120,7 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
-    uint8_t *chunk = out + ((size_t)t * nst + s) * CHUNK;
+    uint8_t *chunk = out + t * tile_bytes(nst) + (size_t)s * CHUNK;
     int cnt, first = 0;
     if (id.tiles) {
         // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
@@ -116,6 +132,8 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
         cnt = left < BN ? (int)left : BN;
     }
     const int live = ((cnt + 7) >> 3) << 3;
+    __shared__ int side_of_warp[8];
+    int side = 0;                        // the largest one-sided sum of codes among this thread's columns
     for (int col0 = 0; col0 < live; col0 += 16) {
         // (whole warps stay together for the shuffles: a half-warp past the live columns quantizes zeros and stores nothing)
         const int col = col0 + hw;
@@ -143,35 +161,46 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
         for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
         const float bm = amax;
         const float iq = bm > 1e-30f ? __fdiv_rn(127.f, bm) : 0.f;
-        int q[16], sum = 0;
+        // the sixteen codes as halves, each run of four in the order 0 2 1 3; their sum and the sum of the positive ones (whole numbers
+        // up to 8 * 127 a half, exact)
+        auto code = [&](float x) { return (float)__float2int_rn(__fmul_rn(x, iq)); };       // (0 for a NaN)
+        __align__(16) __half2 w[8];
+        __half2 all = __float2half2_rn(0.f), pos = all;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            q[4 * i] = __float2int_rn(__fmul_rn(v[i].x, iq));
-            q[4 * i + 1] = __float2int_rn(__fmul_rn(v[i].y, iq));
-            q[4 * i + 2] = __float2int_rn(__fmul_rn(v[i].z, iq));
-            q[4 * i + 3] = __float2int_rn(__fmul_rn(v[i].w, iq));
+            w[2 * i] = __floats2half2_rn(code(v[i].x), code(v[i].z));
+            w[2 * i + 1] = __floats2half2_rn(code(v[i].y), code(v[i].w));
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) sum += q[i];                // the integer sum of the block's 32 codes (the mins term)
-        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+        for (int i = 0; i < 8; ++i) {
+            all = __hadd2(all, w[i]);
+            pos = __hadd2(pos, __hmax2(w[i], __float2half2_rn(0.f)));
+        }
+        // both sums of the sixteen lanes' codes in one word: all above, positive below (at most 256 * 127)
+        int sums = __half2int_rn(__hadd(__low2half(all), __high2half(all))) * 65536 + __half2int_rn(__hadd(__low2half(pos), __high2half(pos)));
+        sums += __shfl_xor_sync(0xFFFFFFFFu, sums, 1);
+        const int sum = sums >> 16;                             // of the block's 32 codes (the mins term)
+#pragma unroll
+        for (int o = 2; o < 16; o *= 2) sums += __shfl_xor_sync(0xFFFFFFFFu, sums, o);
+        side = max(side, (sums & 0xFFFF) - min(sums >> 16, 0));
         if (col >= live) continue;
         const int j = l >> 1;
         uint8_t *o = chunk + (j >> 2) * CODE_STAGE + (col >> 3) * CODE_GROUP + (j & 3) * CODE_BLOCK + (col & 7) * 16;
-        uint32_t w[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __half2 a = __floats2half2_rn((float)q[4 * i], (float)q[4 * i + 2]), b = __floats2half2_rn((float)q[4 * i + 1], (float)q[4 * i + 3]);
-            w[2 * i] = *reinterpret_cast<const uint32_t *>(&a);
-            w[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&b);
-        }
-        *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * 128) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * 128) = make_uint4(w[4], w[5], w[6], w[7]);
+        *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * 128) = *reinterpret_cast<const uint4 *>(w);
+        *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * 128) = *reinterpret_cast<const uint4 *>(w + 4);
         // two exact digits of the sum: bh = round(sum / 256), bl = sum - 256 bh in [-128, 127]
         const int bh = (sum + 128) >> 8;
         uint8_t *extra = chunk + 2 * CODE_STAGE;
         __half *mo = reinterpret_cast<__half *>(extra + EXTRA_MINS + (col >> 3) * MINS_GROUP + (l & 1) * 128 + (col & 7) * 16);
         mo[j] = __float2half_rn((l & 1) ? (float)(256 * bh) : (float)(sum - 256 * bh));
         if (l == 0) reinterpret_cast<float *>(extra)[col] = __fdiv_rn(bm, 127.f);
+    }
+    side = __reduce_max_sync(0xFFFFFFFFu, side);
+    if ((threadIdx.x & 31) == 0) side_of_warp[threadIdx.x >> 5] = side;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) side = max(side, side_of_warp[i]);
+        reinterpret_cast<int *>(out + t * tile_bytes(nst) + (size_t)nst * CHUNK)[s] = side;
     }
 }
 
@@ -294,6 +323,16 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         U.cw = FULL || U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
         return U;
     };
+    // the largest one-sided sum of codes in unit u's column tile, a share per lane, and whether the unit takes more than one chain
+    auto side_of = [&](int u) {
+        int side = 0;
+        if (u < n_units) {
+            const int *p = reinterpret_cast<const int *>(act + (size_t)(u / ksplit % tiles_n) * tile_bytes(nsb) + (size_t)nsb * CHUNK);
+            for (int i = lane; i < nsb; i += 32) side = max(side, __ldg(p + i));
+        }
+        return side;
+    };
+    auto takes_more = [&](int side) { return __any_sync(0xFFFFFFFFu, side > one_chain_side<TYPE>()) != 0; };
     if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
 
     if (threadIdx.x == 0) {
@@ -340,7 +379,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
-            const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * CHUNK;
+            const uint8_t *act_tile = act + (size_t)U.tile_n * tile_bytes(nsb);
             const uint32_t groups = (uint32_t)(U.ncols + 7) >> 3;          // live column groups
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int st = s_run % NRAW, xt = s_run % NX;
@@ -352,6 +391,12 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 }
                 if (s_run == 0) pdl_wait();
                 const uint8_t *chunk = act_tile + (size_t)s * CHUNK;
+                if (!WAITP(3, bar(BAR_X_EMPTY + xt), ((s_run / NX) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    const uint32_t bytes = EXTRA_MINS + groups * MINS_GROUP;
+                    mbar_expect_tx(bar(BAR_X_FULL + xt), bytes);
+                    bulk_g2s(sbase + L::EXTRA_OFF + xt * EXTRA, chunk + 2 * CODE_STAGE, bytes, bar(BAR_X_FULL + xt));
+                }
                 for (int h = 0; h < 2; ++h) {
                     // only the column groups the tile has; the MMA still reads a multiple of sixteen columns, the rest of the
                     // stage holds older codes whose products land in accumulator columns nobody stores
@@ -363,53 +408,85 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                     }
                     __syncwarp();
                 }
-                if (!ok || !WAITP(3, bar(BAR_X_EMPTY + xt), ((s_run / NX) & 1) ^ 1)) { ok = false; break; }
-                if (lane == 0) {
-                    const uint32_t bytes = EXTRA_MINS + groups * MINS_GROUP;
-                    mbar_expect_tx(bar(BAR_X_FULL + xt), bytes);
-                    bulk_g2s(sbase + L::EXTRA_OFF + xt * EXTRA, chunk + 2 * CODE_STAGE, bytes, bar(BAR_X_FULL + xt));
-                }
-                __syncwarp();
             }
         }
     } else if (warp == 1) {
         // ---- MMA issuer ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
-        int s_run = 0;
+        int s_run = 0, v_run = 0;                         // super-blocks, chains so far (a chain fills an accumulator)
         const uint32_t leader = elect_one();
+        uint32_t idesc = 0;
+        // K = 16 per MMA: eight columns of A, two pieces of B
+        auto block = [&](uint32_t acc, int gs, int ct, int jj, uint32_t accumulate) {
+            const uint32_t a = tmem_base + A_BASE + (uint32_t)((gs * GB + jj) * A_COLS);
+            const uint32_t b = sbase + L::CODE_OFF + ct * CODE_STAGE + jj * CODE_BLOCK;
+            umma_ts<true>(leader, acc, a, umma_desc2(b, 128, CODE_GROUP), idesc, accumulate);
+            umma_ts<true>(leader, acc, a + 8, umma_desc2(b + 256, 128, CODE_GROUP), idesc, 1u);
+        };
+        // the mins term, into the one Y accumulator: the scaling warps have read the last chain's X, and the last super-block's Y with
+        // it or before it
+        auto mins = [&](int xt) {
+            if (v_run > 0 && !WAITP(7, bar(BAR_ACC_EMPTY + ((v_run - 1) & 1)), ((v_run - 1) >> 1) & 1)) return false;
+            tc_fence_after();
+            umma_ss<true>(leader, tmem_base + Y_BASE, umma_desc2(sbase + L::MINS_OFF + (s_run & 1) * 4096, 2048, 128),
+                          umma_desc2(sbase + L::EXTRA_OFF + xt * EXTRA + EXTRA_MINS, 128, MINS_GROUP), idesc, 0u);
+            return true;
+        };
+        pdl_wait();
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
-            const uint32_t idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);       // N: the live columns, in sixteens
-            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
-                const int buf = s_run & 1, xt = s_run % NX;
-                const uint32_t acc = tmem_base + (uint32_t)buf * BN;
-                if (!WAITP(7, bar(BAR_ACC_EMPTY + buf), ((s_run >> 1) & 1) ^ 1)) { ok = false; break; }
-                for (int jg = 0; jg < SB / GB; ++jg) {
-                    const int g = 2 * s_run + jg, gs = g % NG, ct = g % NCODE;
-                    if (!WAITP(2, bar(BAR_CODE_FULL + ct), (g / NCODE) & 1)) { ok = false; break; }
-                    if (!WAITP(4, bar(BAR_A_FULL + gs), (g / NG) & 1)) { ok = false; break; }
-                    tc_fence_after();
+            idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);                      // N: the live columns, in sixteens
+            const bool more = takes_more(side_of(u));
+            if (!more) {
+                for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run, ++v_run) {
+                    const int xt = s_run % NX;
+                    const uint32_t acc = tmem_base + (uint32_t)(v_run & 1) * BN;
+                    if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
+                    if (!WAITP(7, bar(BAR_ACC_EMPTY + (v_run & 1)), ((v_run >> 1) & 1) ^ 1)) { ok = false; break; }
+                    for (int jg = 0; jg < SB / GB; ++jg) {
+                        const int g = 2 * s_run + jg, gs = g % NG, ct = g % NCODE;
+                        if (!WAITP(2, bar(BAR_CODE_FULL + ct), (g / NCODE) & 1)) { ok = false; break; }
+                        if (!WAITP(4, bar(BAR_A_FULL + gs), (g / NG) & 1)) { ok = false; break; }
+                        tc_fence_after();
 #pragma unroll
-                    for (int jj = 0; jj < GB; ++jj) {
-                        const uint32_t a = tmem_base + A_BASE + (uint32_t)((gs * GB + jj) * A_COLS);
-                        const uint32_t b = sbase + L::CODE_OFF + ct * CODE_STAGE + jj * CODE_BLOCK;
-                        // K = 16 per MMA: eight columns of A, two pieces of B
-                        umma_ts<true>(leader, acc, a, umma_desc2(b, 128, CODE_GROUP), idesc, (uint32_t)(jg + jj > 0));
-                        umma_ts<true>(leader, acc, a + 8, umma_desc2(b + 256, 128, CODE_GROUP), idesc, 1u);
+                        for (int jj = 0; jj < GB; ++jj) block(acc, gs, ct, jj, (uint32_t)(jg + jj > 0));
+                        tc_commit_one(leader, bar(BAR_A_EMPTY + gs));
+                        tc_commit_one(leader, bar(BAR_CODE_EMPTY + ct));
                     }
-                    tc_commit_one(leader, bar(BAR_A_EMPTY + gs));
-                    tc_commit_one(leader, bar(BAR_CODE_EMPTY + ct));
+                    if (!ok || !mins(xt)) { ok = false; break; }
+                    tc_commit_one(leader, bar(BAR_ACC_FULL + (v_run & 1)));
+                    tc_commit_one(leader, bar(BAR_X_EMPTY + xt));
                 }
-                if (!ok) break;
-                // the mins term, into the one Y accumulator: the scaling warps have read the last super-block's with its X
+                continue;
+            }
+            constexpr int CB = SB / Fmt<TYPE>::CHAINS;                                    // blocks of a chain
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int xt = s_run % NX;
                 if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
-                if (s_run > 0 && !WAITP(7, bar(BAR_ACC_EMPTY + (buf ^ 1)), ((s_run - 1) >> 1) & 1)) { ok = false; break; }
-                tc_fence_after();
-                umma_ss<true>(leader, tmem_base + Y_BASE, umma_desc2(sbase + L::MINS_OFF + buf * 4096, 2048, 128),
-                            umma_desc2(sbase + L::EXTRA_OFF + xt * EXTRA + EXTRA_MINS, 128, MINS_GROUP), idesc, 0u);
-                tc_commit_one(leader, bar(BAR_ACC_FULL + buf));
-                tc_commit_one(leader, bar(BAR_X_EMPTY + xt));
+#pragma unroll 1
+                for (int j = 0; j < SB; ++j) {
+                    const int g = 2 * s_run + j / GB, gs = g % NG, ct = g % NCODE;
+                    if (j % GB == 0) {
+                        if (!WAITP(2, bar(BAR_CODE_FULL + ct), (g / NCODE) & 1)) { ok = false; break; }
+                        if (!WAITP(4, bar(BAR_A_FULL + gs), (g / NG) & 1)) { ok = false; break; }
+                    }
+                    if (j % CB == 0 && !WAITP(7, bar(BAR_ACC_EMPTY + (v_run & 1)), ((v_run >> 1) & 1) ^ 1)) { ok = false; break; }
+                    tc_fence_after();
+                    block(tmem_base + (uint32_t)(v_run & 1) * BN, gs, ct, j % GB, (uint32_t)(j % CB > 0));
+                    if (j % GB == GB - 1) {
+                        tc_commit_one(leader, bar(BAR_A_EMPTY + gs));
+                        tc_commit_one(leader, bar(BAR_CODE_EMPTY + ct));
+                    }
+                    if (j % CB == CB - 1) {
+                        if (j == CB - 1) {                                                // the first chain takes the mins along
+                            if (!mins(xt)) { ok = false; break; }
+                            tc_commit_one(leader, bar(BAR_X_EMPTY + xt));
+                        }
+                        tc_commit_one(leader, bar(BAR_ACC_FULL + (v_run & 1)));
+                        ++v_run;
+                    }
+                }
             }
         }
     } else if (warp < 4) {
@@ -458,15 +535,16 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             }
         }
     } else {
-        // ---- scale-accumulate, once per super-block: a warp group per half of the tile's columns ----
+        // ---- scale-accumulate, once per chain: a warp group per half of the tile's columns ----
         asm volatile("setmaxnreg.inc.sync.aligned.u32 160;" ::: "memory");
         // 16x256b loads give a thread, of every eight columns, columns 2 c and 2 c + 1 of rows g and g + 8
         const int q4 = warp & 3, half = (warp - 12) >> 2, g = lane >> 2, c = lane & 3;
-        int s_run = 0;
+        int s_run = 0, v_run = 0;
         pdl_wait();
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
+            const int chains = takes_more(side_of(u)) ? Fmt<TYPE>::CHAINS : 1;
             const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
             const bool live = FULL || ncol > 0, two = FULL || ncol > 32;
             f32x2 acc2[4][8];                                  // rows g, g + 8, g + 16, g + 24; column pairs 8 i + 2 c
@@ -475,54 +553,59 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc2[k][i] = 0ull;
             const uint32_t tq = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)cbase;
-            for (int s = U.sb0; s < U.sb1; ++s, ++s_run) {
-                const int buf = s_run & 1, xt = s_run % NX;
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int xt = s_run % NX;
                 if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
-                if (!WAITP(6, bar(BAR_ACC_FULL + buf), (s_run >> 1) & 1)) { ok = false; break; }
-                tc_fence_after();
-                if (live) {
-                    // rows 16 rh .. + 15 of the quarter at a time: X and Y, all columns, in flight together
-                    uint32_t vx[2][16], vy[2][16];
-                    auto load = [&](int rh) {
-                        const uint32_t a = tq + ((uint32_t)(rh * 16) << 16);
-                        tmem_ld_16x256_x4(a + (uint32_t)buf * BN, vx[0]);
-                        tmem_ld_16x256_x4(a + Y_BASE, vy[0]);
-                        if (two) {
-                            tmem_ld_16x256_x4(a + (uint32_t)buf * BN + 32, vx[1]);
-                            tmem_ld_16x256_x4(a + Y_BASE + 32, vy[1]);
-                        }
-                    };
-                    load(0);
-                    const uint32_t xa = sbase + L::EXTRA_OFF + xt * EXTRA + (cbase + 2 * c) * 4;
-                    f32x2 dx[8];
+#pragma unroll 1
+                for (int ch = 0; ch < chains; ++ch, ++v_run) {
+                    const int buf = v_run & 1;
+                    if (!WAITP(6, bar(BAR_ACC_FULL + buf), (v_run >> 1) & 1)) { ok = false; break; }
+                    tc_fence_after();
+                    if (live) {
+                        // rows 16 rh .. + 15 of the quarter at a time: X and Y, all columns, in flight together
+                        uint32_t vx[2][16], vy[2][16];
+                        auto load = [&](int rh) {
+                            const uint32_t a = tq + ((uint32_t)(rh * 16) << 16);
+                            tmem_ld_16x256_x4(a + (uint32_t)buf * BN, vx[0]);
+                            tmem_ld_16x256_x4(a + Y_BASE, vy[0]);
+                            if (two) {
+                                tmem_ld_16x256_x4(a + (uint32_t)buf * BN + 32, vx[1]);
+                                tmem_ld_16x256_x4(a + Y_BASE + 32, vy[1]);
+                            }
+                        };
+                        load(0);
+                        const uint32_t xa = sbase + L::EXTRA_OFF + xt * EXTRA + (cbase + 2 * c) * 4;
+                        f32x2 dx[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) dx[i] = lds64_f2(xa + 32 * i);
-                    const float2 *dp = reinterpret_cast<const float2 *>(smem + L::DW_OFF + (xt * BM + q4 * 32 + g) * 8);
+                        for (int i = 0; i < 8; ++i) dx[i] = lds64_f2(xa + 32 * i);
+                        const float2 *dp = reinterpret_cast<const float2 *>(smem + L::DW_OFF + (xt * BM + q4 * 32 + g) * 8);
 #pragma unroll
-                    for (int rh = 0; rh < 2; ++rh) {
-                        const float2 w0 = dp[16 * rh], w1 = dp[16 * rh + 8];
-                        tmem_ld_wait();
+                        for (int rh = 0; rh < 2; ++rh) {
+                            float2 w0 = dp[16 * rh], w1 = dp[16 * rh + 8];
+                            if (ch > 0) w0.y = w1.y = 0.f;           // the mins went with the first chain (Y still holds them, finite)
+                            tmem_ld_wait();
 #pragma unroll
-                        for (int hc = 0; hc < 2; ++hc) {
-                            if (hc == 0 || two) {
+                            for (int hc = 0; hc < 2; ++hc) {
+                                if (hc == 0 || two) {
 #pragma unroll
-                                for (int k = 0; k < 2; ++k) {
-                                    const f32x2 d2 = k ? f2_pack(w1.x, w1.x) : f2_pack(w0.x, w0.x), m2 = k ? f2_pack(w1.y, w1.y) : f2_pack(w0.y, w0.y);
+                                    for (int k = 0; k < 2; ++k) {
+                                        const f32x2 d2 = k ? f2_pack(w1.x, w1.x) : f2_pack(w0.x, w0.x), m2 = k ? f2_pack(w1.y, w1.y) : f2_pack(w0.y, w0.y);
 #pragma unroll
-                                    for (int i = 0; i < 4; ++i) {
-                                        const f32x2 x = f2_pack(__uint_as_float(vx[hc][4 * i + 2 * k]), __uint_as_float(vx[hc][4 * i + 2 * k + 1]));
-                                        const f32x2 y = f2_pack(__uint_as_float(vy[hc][4 * i + 2 * k]), __uint_as_float(vy[hc][4 * i + 2 * k + 1]));
-                                        // (d sum(sc q x) - dmin sum(m x)) d_x
-                                        acc2[2 * rh + k][4 * hc + i] = f2_fma(f2_fma(x, d2, f2_mul(y, m2)), dx[4 * hc + i], acc2[2 * rh + k][4 * hc + i]);
+                                        for (int i = 0; i < 4; ++i) {
+                                            const f32x2 x = f2_pack(__uint_as_float(vx[hc][4 * i + 2 * k]), __uint_as_float(vx[hc][4 * i + 2 * k + 1]));
+                                            const f32x2 y = f2_pack(__uint_as_float(vy[hc][4 * i + 2 * k]), __uint_as_float(vy[hc][4 * i + 2 * k + 1]));
+                                            // (d sum(sc q x) - dmin sum(m x)) d_x
+                                            acc2[2 * rh + k][4 * hc + i] = f2_fma(f2_fma(x, d2, f2_mul(y, m2)), dx[4 * hc + i], acc2[2 * rh + k][4 * hc + i]);
+                                        }
                                     }
                                 }
                             }
+                            if (rh == 0) load(1);
                         }
-                        if (rh == 0) load(1);
                     }
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(BAR_ACC_EMPTY + buf), lane);
                 }
-                tc_fence_before();
-                mbar_arrive_warp(bar(BAR_ACC_EMPTY + buf), lane);
                 mbar_arrive_warp(bar(BAR_X_EMPTY + xt), lane);
             }
             if (ok && live) {
@@ -590,7 +673,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 
 static const TileRoute NO_ROUTE_KF = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
-size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + kf::BN - 1) / kf::BN) * (K / 256)) * kf::CHUNK; }
+size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)((N + kf::BN - 1) / kf::BN) * kf::tile_bytes(K / 256); }
 size_t gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles) { return gemm_kf_act_bytes(K, max_tiles * kf::BN); }
 
 bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride) {

@@ -65,9 +65,103 @@ def test_many_units_per_block(ctx, t):
     check(got, t, w, k, x)
 
 
-def test_sums_beyond_24_bits(ctx):
-    """Constant activations give the largest super-block sums (up to 256 * 1953 * 127): float rounding, not wrap-around."""
-    for t in (A.Q4_K, A.Q5_K):
-        w, _ = data(t, 64, 512, 9, 3)
-        x = np.ones((9, 512), np.float32)
-        check(ctx.run_mul_mat(t, w, 512, x), t, w, 512, x)
+def integer_blocks(t, m, nsb, rng, low):
+    """Packed super-blocks with d = 1, dmin = 0, every sub-scale 63 and codes low .. top, and the weights as integers [m, 256 nsb]"""
+    top = 15 if t == A.Q4_K else 31
+    q = rng.integers(low, top + 1, size=(m, nsb, 8, 32)).astype(np.uint8)
+    w = np.zeros((m, nsb, A.block_bytes(t)), np.uint8)
+    w[:, :, 0:2] = np.frombuffer(np.float16(1).tobytes(), np.uint8)
+    w[:, :, 4:8] = 63 | (3 << 6)                            # sub-scales 0..3 and the two high bits of 4..7
+    w[:, :, 12:16] = 15                                     # their four low bits
+    if t == A.Q5_K:
+        w[:, :, 16:48] = ((q >> 4) << np.arange(8, dtype=np.uint8)[None, None, :, None]).sum(2)
+    w[:, :, -128:] = ((q[:, :, 0::2] & 15) | ((q[:, :, 1::2] & 15) << 4)).reshape(m, nsb, 128)
+    return w.reshape(m, -1), 63.0 * q.reshape(m, -1)
+
+
+def integer_codes(n, nsb, rng, one_sided):
+    """Integer activations whose 8-bit codes are themselves (every super-block holds a 127): [n, 256 nsb]; one_sided[s]: 1 or -1 for codes of
+    that sign only, 100 and more, 0 for codes around zero"""
+    x = np.empty((n, nsb, 256), np.float32)
+    for s in range(nsb):
+        x[:, s] = one_sided[s] * rng.integers(100, 128, (n, 256)) if one_sided[s] else rng.integers(-60, 61, (n, 256))
+        x[np.arange(n), s, rng.integers(0, 256, n)] = 127 * (one_sided[s] or 1)
+    return x.reshape(n, -1)
+
+
+@pytest.mark.parametrize("t", [A.Q4_K, A.Q5_K])
+@pytest.mark.parametrize("n", [9, 40, 128])
+@pytest.mark.parametrize("side", [1, -1])
+def test_sums_beyond_24_bits(ctx, t, n, side):
+    """Integer sums of a super-block past 2^24, with scales of 1. Two exact chains (Q4_K): the sum, rounded once. Four (Q5_K): three
+    additions of one sign, each rounded by half an ulp of at most the sum."""
+    rng = np.random.default_rng(n)
+    w, wi = integer_blocks(t, 130, 1, rng, 12 if t == A.Q4_K else 28)
+    x = integer_codes(n, 1, rng, [side])
+    exact = x.astype(np.float64) @ wi.T
+    assert np.abs(exact).max() > 2 ** 24 and (exact.astype(np.float32) != exact).any()
+    got = ctx.run_mul_mat(t, w, 256, x)
+    if t == A.Q4_K:
+        assert np.array_equal(got, exact.astype(np.float32))
+    assert (np.abs(got - exact) <= 3 * 2.0 ** -24 * np.abs(exact)).all()
+
+
+@pytest.mark.parametrize("t,edge", [(A.Q4_K, 17753), (A.Q5_K, 8590)])
+def test_sums_at_24_bits(ctx, t, edge):
+    """Either side of the one-sided sum of codes up to which one chain is exact, 2^24 over 63 * 15 and over 63 * 31"""
+    rng = np.random.default_rng(5)
+    w, wi = integer_blocks(t, 64, 1, rng, 14 if t == A.Q4_K else 30)
+    wi[0], w[0] = wi.max(), integer_blocks(t, 1, 1, rng, 15 if t == A.Q4_K else 31)[0]
+    for total in (edge - 1, edge, edge + 1):
+        x = np.zeros((12, 256), np.float32)
+        for c in range(12):
+            left = total
+            for i in range(256):
+                x[c, i] = min(127, left) if i < 255 - c else 0
+                left -= int(x[c, i])
+            assert left == 0
+        x[:, 1:] = rng.permuted(x[:, 1:], axis=1)
+        exact = x.astype(np.float64) @ wi.T
+        assert exact.max() == total * wi.max()
+        assert np.array_equal(ctx.run_mul_mat(t, w, 256, x), exact.astype(np.float32))
+
+
+@pytest.mark.parametrize("t", [A.Q4_K, A.Q5_K])
+@pytest.mark.parametrize("m,n", [(300, 24), (128 * 60, 128 * 4 + 20), (128 * 40, 128 * 4)])
+def test_one_and_more_chains_in_turn(ctx, t, m, n):
+    """Super-blocks that need more than one chain between ones that do not, over several units of a block; one rounding of the running
+    sum a chain."""
+    rng = np.random.default_rng(m + n)
+    sides = [0, 1, 1, 0, -1, 0, 0, 1, -1]
+    w, wi = integer_blocks(t, m, len(sides), rng, 10)
+    x = integer_codes(n, len(sides), rng, sides)
+    exact = x.astype(np.float64) @ wi.T
+    terms = sum(np.abs(x[:, 256 * s:256 * s + 256].astype(np.float64) @ wi[:, 256 * s:256 * s + 256].T) for s in range(len(sides)))
+    got = ctx.run_mul_mat(t, w, 256 * len(sides), x)
+    # (the largest running sum is within the sum of the super-blocks' absolute sums)
+    assert (np.abs(got - exact) <= (2 if t == A.Q4_K else 4) * len(sides) * 2.0 ** -24 * terms).all()
+
+
+@pytest.mark.parametrize("t", [A.Q4_K, A.Q5_K])
+def test_more_chains_in_route_tiles(ctx, t):
+    n_exp, n_used, m, nsb, n_tok = 4, 2, 256, 2, 150
+    rng = np.random.default_rng(8)
+    blocks = [integer_blocks(t, m, nsb, rng, 10) for _ in range(n_exp)]
+    w, wi = np.stack([b[0] for b in blocks]), np.stack([b[1] for b in blocks])
+    x = integer_codes(n_tok, nsb, rng, [1, 0])
+    ids = O.route_ids(n_used, n_tok, n_exp, 3)
+    k, rb = 256 * nsb, w.shape[-1]
+    dw, dx, di, dy = ctx.upload(w), ctx.upload(x), ctx.upload(ids), ctx.alloc(n_tok * n_used * m * 4)
+    W = A.Tensor.make(t, [k, m, n_exp, 1], [A.block_bytes(t), rb, rb * m, rb * m * n_exp], dw)
+    ctx.stats_reset()
+    ctx.graph_begin()
+    ctx.mul_mat_id(W, A.Tensor.make(A.F32, [k, 1, n_tok, 1], [4, 4 * k, 4 * k], dx), A.Tensor.make(A.I32, [n_used, n_tok, 1, 1], [4, 4 * n_used], di),
+                   A.Tensor.f32(dy, [m, n_used, n_tok]))
+    got = ctx.download(dy, (n_tok, n_used, m), np.float32)
+    assert ctx.stats().get("moe_gemm", 0) == 1
+    exact = np.einsum("tk,tumk->tum", x.astype(np.float64), wi[ids])
+    assert np.abs(exact).max() > 2 ** 24
+    # the second super-block's sum stays below 2^24: a rounding per chain of the first and one of the total
+    assert (np.abs(got - exact) <= 5 * 2.0 ** -24 * (np.abs(exact) + 2.0 ** 24)).all()
+    for p in (dw, dx, di, dy):
+        ctx.free(p)
