@@ -59,6 +59,32 @@ b200q_status fail(b200q_ctx *ctx, b200q_status st, const char *fmt, ...) {
     return st;
 }
 
+// A block of `bytes` bytes into the empty *ws. *total: what was asked of the device.
+static cudaError_t ws_alloc(b200q_ctx *ctx, Workspace *ws, size_t bytes, size_t *total_out) {
+    // Normally whole megabytes, so that a slowly growing request does not reallocate every time. With guard words the block
+    // has the size asked for (to 256 bytes), so that a write past the request lands in the guard and not in rounding slack.
+    const size_t guard = ctx->canary ? WS_GUARD : 0;
+    const size_t unit = ctx->canary ? 256 : (size_t)1 << 20;
+    const size_t want = (bytes + unit - 1) / unit * unit;
+    // (behind the tail guard another 64 KiB, so that a read past the block -- which no guard can see -- stays inside the allocation)
+    const size_t total = *total_out = want + 2 * guard + (guard ? (size_t)64 << 10 : 0);
+    cudaError_t e = ctx->scratch_limit && total > ctx->scratch_limit ? cudaErrorMemoryAllocation : cudaMalloc(&ws->base, total);
+    if (e != cudaSuccess) {
+        ws->base = nullptr;
+        (void)cudaGetLastError();
+        return e;
+    }
+    ws->ptr = (uint8_t *)ws->base + guard;
+    ws->cap = want;
+    if (guard) {
+        e = cudaMemsetAsync(ws->base, WS_GUARD_BYTE, guard, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync((uint8_t *)ws->ptr + want, WS_GUARD_BYTE, guard, ctx->stream);
+        if (e != cudaSuccess) { ws_release(ws); return e; }
+    }
+    count(ctx, ST_WORKSPACE_GROW);
+    return cudaSuccess;
+}
+
 // grow-only scratch (the reference's prealloc_* buffers never shrink either)
 b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
     if (bytes <= ws->cap) return B200Q_OK;
@@ -71,26 +97,29 @@ b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
         ws->ptr = ws->base = nullptr;
         ws->cap = 0;
     }
-    // Normally whole megabytes, so that a slowly growing request does not reallocate every time. With guard words the block
-    // has the size asked for (to 256 bytes), so that a write past the request lands in the guard and not in rounding slack.
-    const size_t guard = ctx->canary ? WS_GUARD : 0;
-    const size_t unit = ctx->canary ? 256 : (size_t)1 << 20;
-    const size_t want = (bytes + unit - 1) / unit * unit;
-    // (behind the tail guard another 64 KiB, so that a read past the block -- which no guard can see -- stays inside the allocation)
-    const size_t total = want + 2 * guard + (guard ? (size_t)64 << 10 : 0);
-    cudaError_t e = cudaMalloc(&ws->base, total);
-    if (e != cudaSuccess) {
-        ws->base = nullptr;
-        return fail(ctx, B200Q_NO_MEMORY, "cudaMalloc(%zu): %s", total, cudaGetErrorString(e));
-    }
-    ws->ptr = (uint8_t *)ws->base + guard;
-    ws->cap = want;
-    if (guard) {
-        B200Q_CUDA(ctx, cudaMemsetAsync(ws->base, WS_GUARD_BYTE, guard, ctx->stream));
-        B200Q_CUDA(ctx, cudaMemsetAsync((uint8_t *)ws->ptr + want, WS_GUARD_BYTE, guard, ctx->stream));
-    }
-    count(ctx, ST_WORKSPACE_GROW);
+    size_t total = 0;
+    const cudaError_t e = ws_alloc(ctx, ws, bytes, &total);
+    if (e == cudaErrorMemoryAllocation) return fail(ctx, B200Q_NO_MEMORY, "cudaMalloc(%zu): %s", total, cudaGetErrorString(e));
+    B200Q_CUDA(ctx, e);
     return B200Q_OK;
+}
+
+// The same for scratch that a call can do without: true when *ws holds `bytes` bytes. Otherwise (no memory for them, or a capture
+// is open) everything is as before: the block there is stays, with the recorded graphs that use it, and no error is set.
+bool ws_try_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
+    if (bytes <= ws->cap) return true;
+    if (ctx->capturing) return false;
+    Workspace next;
+    size_t total = 0;
+    if (ws_alloc(ctx, &next, bytes, &total) != cudaSuccess) return false;
+    // the old block may still be in use by work already enqueued on the stream
+    if (ws->ptr && cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        ws_release(&next);                                   // (the launch that follows reports the stream's error)
+        return false;
+    }
+    ws_release(ws);
+    *ws = next;
+    return true;
 }
 
 void ws_release(Workspace *ws) {
@@ -718,6 +747,12 @@ b200q_status b200q_debug_wait_timeout(b200q_ctx *ctx, unsigned polls) {
     B200Q_CUDA(ctx, cudaSetDevice(ctx->device));
     debug_wait_timeout_kernel<<<1, 1, 0, ctx->stream>>>(polls, ctx->error_word);
     B200Q_CUDA(ctx, cudaGetLastError());
+    return B200Q_OK;
+}
+
+b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes) {
+    if (!ctx) return B200Q_INVALID;
+    ctx->scratch_limit = bytes;
     return B200Q_OK;
 }
 

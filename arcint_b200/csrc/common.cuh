@@ -142,6 +142,7 @@ struct b200q_ctx {
     int          gemv_mma_slice = 0;      // B200Q_GEMV_MMA_SLICE=2|3|4: super-blocks per warp of the warp-MMA GEMV (0: by row length)
     int          gemv_mma_min = 0;        // B200Q_GEMV_MMA_MIN: fewest columns at which a product takes the warp-MMA GEMV (99: never; 0: Q6_K 3, Q8_0 7, the others 4, measured)
     bool         gemv_no_small = false;   // B200Q_GEMV_NO_SMALL=1: never the 128-thread, 170-register build of the wide Q6_K GEMV
+    size_t       scratch_limit = 0;       // b200q_debug_scratch_limit: a scratch allocation beyond it fails as on a full device (0: none does)
     bool         no_stream = false;       // B200Q_NO_STREAM=1: every GEMV through the per-warp ring kernel (comparisons)
     std::string  last_error;
     std::string  stats_text;
@@ -162,6 +163,7 @@ namespace b200q {
 
 b200q_status fail(b200q_ctx *ctx, b200q_status st, const char *fmt, ...);
 b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
+bool         ws_try_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
 void ws_release(Workspace *ws);
 int moe_route_workspaces(b200q_ctx *ctx, Workspace **out, const char **names);   // the route caches' blocks, for the guard check
 inline void  count(b200q_ctx *ctx, int stat) { ++ctx->counters[stat]; }
@@ -266,9 +268,9 @@ b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_
 // the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
 
-b200q_status ksplit_scratch(b200q_ctx *ctx, int64_t M, int64_t N, int *ksplit, float **parts);
-// K parts of a product whose tiles fill the SMs badly; the times of a 256-weight step on a full tile that it counts with
-int          choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_t outputs);
+// K parts of a product whose tiles fill the SMs badly, and the scratch for their results (ksplit.cu); the times of a 256-weight step on a full
+// tile that it counts with
+int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, int step_ns, int64_t M, int64_t N, float **parts);
 constexpr int TC_SB_NS = 2000, KQ_SB_NS = 2000, KF_SB_NS = 900;
 
 // gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types

@@ -718,11 +718,11 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     if (st != B200Q_OK) return st;
     // persistent blocks, one per SM, walking the (row tile, column tile, part of K) units
     const int64_t tiles = n_tiles * ((M + kf::BM - 1) / kf::BM), S = ctx->sm_count;
-    int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, S, K / 256, KF_SB_NS, M * N);
-    float *out = dst;
+    float *out = dst, *parts = nullptr;
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, KF_SB_NS, M, N, &parts);
     int64_t out_ld = ldd, part_stride = 0;
-    if (ksplit > 1 && (st = ksplit_scratch(ctx, M, N, &ksplit, &out)) != B200Q_OK) return st;
     if (ksplit > 1) {
+        out = parts;
         // parts write their own scratch and a second kernel adds them in a fixed order
         part_stride = N * M;
         out_ld = M;

@@ -645,16 +645,12 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     }
     // persistent blocks, one per SM, walking the (row tile, column tile) units
     int64_t units = n_tiles * ((M + kq::BM - 1) / kq::BM);
-    int ksplit = 1;
     const int64_t S = ctx->sm_count, nst = K / 256 / L::SPS;
-    if (!tr.tiles && !ctx->no_ksplit) ksplit = choose_ksplit(units, S, nst, L::SPS * KQ_SB_NS, M * N);
-    float *out = dst;
+    float *out = dst, *parts = nullptr;
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, units, nst, L::SPS * KQ_SB_NS, M, N, &parts);
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
-        const b200q_status st = ksplit_scratch(ctx, M, N, &ksplit, &out);
-        if (st != B200Q_OK) return st;
-    }
-    if (ksplit > 1) {
+        out = parts;
         part_stride = N * M;
         out_ld = M;
         units *= ksplit;

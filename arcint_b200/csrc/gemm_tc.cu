@@ -614,11 +614,11 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
     // every tile walks all of K). Parts write their own scratch and a second kernel adds them in a fixed order, so the result
     // does not depend on which block finishes first.
     const int64_t tiles = n_tiles * ((M + tc::BM - 1) / tc::BM);
-    int ksplit = tr.tiles || ctx->no_ksplit ? 1 : choose_ksplit(tiles, ctx->sm_count, K / 256, TC_SB_NS, M * N);
-    float *out = dst;
+    float *out = dst, *parts = nullptr;
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, TC_SB_NS, M, N, &parts);
     int64_t out_ld = ldd, part_stride = 0;
-    if (ksplit > 1 && (st = ksplit_scratch(ctx, M, N, &ksplit, &out)) != B200Q_OK) return st;
     if (ksplit > 1) {
+        out = parts;
         part_stride = N * M;
         out_ld = M;
     }

@@ -31,10 +31,10 @@ ksplit_sum_kernel(const float *__restrict__ parts, int ksplit, int64_t part_stri
 // Into how many parts to cut K: the schedule's length in nanoseconds, rounds of units over the SMs plus, for more than one
 // part, the pass that adds them. step_ns: a k-step (one raw stage) of the kernel on a full tile; a unit costs some 1.2 us
 // beyond its steps (pipeline fill, drain, stores), the adding pass a launch and its traffic.
-int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_t outputs) {
+static int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_t outputs, int64_t most) {
     int best_ks = 1;
     int64_t best = 0;
-    for (int ks = 1; ks <= 8 && (ks == 1 || steps / ks >= 2); ++ks) {
+    for (int ks = 1; ks <= most && (ks == 1 || steps / ks >= 2); ++ks) {
         const int64_t rounds = (tiles * ks + sms - 1) / sms;
         const int64_t len = rounds * ((steps + ks - 1) / ks * step_ns + 1200) + (ks > 1 ? 2500 + outputs * (ks + 1) / 1000 : 0);
         if (ks == 1 || len < best) { best = len; best_ks = ks; }
@@ -42,16 +42,19 @@ int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, int step_ns, int64_
     return best_ks;
 }
 
-// Scratch for the parts. Without the memory for it the product is not cut: ksplit becomes 1.
-b200q_status ksplit_scratch(b200q_ctx *ctx, int64_t M, int64_t N, int *ksplit, float **parts) {
-    const b200q_status st = ws_reserve(ctx, &ctx->moe_ws[9], sizeof(float) * (size_t)(N * M) * *ksplit);
-    if (st == B200Q_NO_MEMORY) {
-        (void)cudaGetLastError();
-        *ksplit = 1;
-        return B200Q_OK;
+// The number of parts (1: the product stays whole) and where they go. Where the scratch cannot be had, on a full device or inside a
+// capture that would have to grow it, the product is cut into what the block there is holds.
+int plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, int step_ns, int64_t M, int64_t N, float **parts) {
+    if (ctx->no_ksplit) return 1;
+    Workspace *ws = &ctx->moe_ws[9];
+    const size_t part = sizeof(float) * (size_t)(N * M);
+    int ks = choose_ksplit(tiles, ctx->sm_count, steps, step_ns, M * N, 8);
+    if (ks > 1 && !ws_try_reserve(ctx, ws, part * ks)) {
+        const size_t hold = ws->cap / part;                 // (less than ks)
+        ks = choose_ksplit(tiles, ctx->sm_count, steps, step_ns, M * N, hold < 1 ? 1 : (int64_t)hold);
     }
-    *parts = (float *)ctx->moe_ws[9].ptr;
-    return st;
+    *parts = (float *)ws->ptr;
+    return ks;
 }
 
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd) {

@@ -121,3 +121,69 @@ def test_bounded_wait_runs_out_and_context_survives(ctx):
     w = make_weights(t, m, k, 77)
     x = np.random.default_rng(1).normal(0, 1, size=(2, k)).astype(np.float32)
     assert rel_err(ctx.run_mul_mat(t, w, k, x), O.mul_mat_f64(t, w, k, x, True)) < TOL
+
+
+def prompt(ctx, t, m, k, n, seed):
+    """(weights, activation, tensors, device pointers) of a prompt product"""
+    w, x = make_weights(t, m, k, seed), np.random.default_rng(seed).normal(0, 1, size=(n, k)).astype(np.float32)
+    p = ctx.upload(w), ctx.upload(x), ctx.alloc(n * m * 4)
+    return w, x, (A.Tensor.weights(t, p[0], k, m), A.Tensor.f32(p[1], [k, n]), A.Tensor.f32(p[2], [m, n])), p
+
+
+@pytest.mark.parametrize("t", [A.Q8_0, A.Q4_K, A.Q6_K])
+def test_no_memory_for_the_parts_of_k(t):
+    """Without memory for the parts of a product cut along K it runs whole, without an error text, and can be recorded."""
+    m, k, n = 512, 4096, 512                                # eight parts of 1 MiB; the activation takes at most 4.4 MB
+    with A.Context(0) as ctx:
+        ctx.scratch_limit(6 << 20)
+        w, x, mm, p = prompt(ctx, t, m, k, n, 600 + t)
+        ctx.graph_begin()
+        ctx.mul_mat(*mm)
+        assert rel_err(ctx.download(p[2], (n, m), np.float32), O.mul_mat_f64(t, w, k, x, True)) < TOL
+        assert ctx.stats().get("gemm_ksplit", 0) == 0 and ctx.L.b200q_last_error(ctx.h) == b""
+        g = ctx.capture(lambda: ctx.mul_mat(*mm))
+        ctx.upload(-x, p[1])
+        ctx.graph_launch(g)
+        assert rel_err(ctx.download(p[2], (n, m), np.float32), O.mul_mat_f64(t, w, k, -x, True)) < TOL
+        ctx.graph_free(g)
+        ctx.scratch_limit(0)
+        ctx.graph_begin()
+        ctx.mul_mat(*mm)
+        assert ctx.stats().get("gemm_ksplit", 0) == 1
+        assert rel_err(ctx.download(p[2], (n, m), np.float32), O.mul_mat_f64(t, w, k, -x, True)) < TOL
+
+
+def test_capture_takes_the_parts_that_fit():
+    """A recording whose parts would not fit the scratch is accepted with fewer of them."""
+    t, k, n = A.Q6_K, 4096, 512
+    with A.Context(0) as ctx:
+        _, _, small, _ = prompt(ctx, t, 128, k, n, 1)       # eight parts of 256 KiB, and the activation scratch
+        w, x, big, p = prompt(ctx, t, 512, k, n, 2)         # eight of 1 MiB
+        ctx.graph_begin()
+        ctx.mul_mat(*small)
+        grown = ctx.stats()["workspace_grow"]
+        g = ctx.capture(lambda: ctx.mul_mat(*big))
+        ctx.graph_launch(g)
+        assert rel_err(ctx.download(p[2], (n, 512), np.float32), O.mul_mat_f64(t, w, k, x, True)) < TOL
+        assert ctx.stats()["gemm_ksplit"] == 2 and ctx.stats()["workspace_grow"] == grown
+        ctx.graph_free(g)
+
+
+def test_failed_growth_keeps_the_recorded_block():
+    """A recording that adds up its parts in the scratch stays good when a later, larger product finds no memory for its own."""
+    t, k, n = A.Q6_K, 4096, 512
+    with A.Context(0) as ctx:
+        w, x, small, p = prompt(ctx, t, 128, k, n, 1)
+        _, _, big, _ = prompt(ctx, t, 512, k, n, 2)
+        ctx.graph_begin()
+        ctx.mul_mat(*small)
+        g = ctx.capture(lambda: ctx.mul_mat(*small))
+        grown = ctx.stats()["workspace_grow"]
+        ctx.scratch_limit(4 << 20)
+        ctx.graph_begin()
+        ctx.mul_mat(*big)
+        assert ctx.stats()["workspace_grow"] == grown
+        ctx.upload(2 * x, p[1])
+        ctx.graph_launch(g)
+        assert rel_err(ctx.download(p[2], (n, 128), np.float32), O.mul_mat_f64(t, w, k, 2 * x, True)) < TOL
+        ctx.graph_free(g)
