@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "pdl.cuh"
 #include "tc_common.cuh"
 
 namespace b200q {
@@ -26,6 +27,13 @@ __global__ void debug_wait_timeout_kernel(unsigned polls, int *error_word) {
     bool done = false;
     for (unsigned i = 0; i < polls && !done; ++i) done = tc::mbar_try(b, 0);
     if (!done) atomicExch(error_word, 3);
+}
+
+// A writer that lets the kernels behind it start at once and writes late: what a product must wait for.
+__global__ void debug_late_copy_kernel(uint8_t *dst, const uint8_t *src, size_t bytes, unsigned microseconds) {
+    pdl_trigger();
+    for (unsigned i = 0; i < microseconds; ++i) __nanosleep(1000);          // (sleeps up to twice that long: bounded)
+    for (size_t i = threadIdx.x; i < bytes; i += blockDim.x) dst[i] = src[i];
 }
 
 const char *stat_name(int s) {
@@ -195,6 +203,7 @@ static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor 
     for (auto &e : ctx->act_cache)
         if (e.valid && e.key == key) { hit = &e; break; }
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
+    out->fresh = !hit;
     if (!hit) {
         if (ctx->act_cache.size() < 4) ctx->act_cache.resize(4);
         // victim: an entry of an older graph (its contents are dead), the first one if several,
@@ -414,17 +423,17 @@ b200q_status b200q_mul_mat(b200q_ctx *ctx, const b200q_tensor *src0, const b200q
     if (N > 8 && uniform && !ctx->no_tc && gemm_tc_supported(src0->type, M, K, N, src0->data, src0->nb[1])) {
         if ((st = get_activation(ctx, ACT_Q8_0_TILED, src1, &act)) != B200Q_OK) return st;
         return launch_gemm_tc(ctx, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
-                              (float *)dst->data, ldd);
+                              (float *)dst->data, ldd, act.fresh);
     }
     if (N > 8 && uniform && !ctx->no_tc && gemm_kq_supported(src0->type, M, K, N, src0->data, src0->nb[1])) {
         if ((st = get_activation(ctx, ACT_Q8_256_TILED, src1, &act)) != B200Q_OK) return st;
         return launch_gemm_kq(ctx, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
-                              (float *)dst->data, ldd);
+                              (float *)dst->data, ldd, act.fresh);
     }
     if (N > 8 && uniform && !ctx->no_tc && gemm_kf_supported(src0->type, M, K, N, src0->data, src0->nb[1])) {
         if ((st = get_activation(ctx, ACT_Q8_256_TILED_F16, src1, &act)) != B200Q_OK) return st;
         return launch_gemm_kf(ctx, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
-                              (float *)dst->data, ldd);
+                              (float *)dst->data, ldd, act.fresh);
     }
     if (N > 8) count(ctx, ST_GEMM_FALLBACK_SHAPE);
     // small per-32 products at one or two columns: the GEMV quantizes its own slice of the activation, one launch
@@ -746,6 +755,15 @@ b200q_status b200q_debug_wait_timeout(b200q_ctx *ctx, unsigned polls) {
     if (polls > (1u << 20)) polls = 1u << 20;
     B200Q_CUDA(ctx, cudaSetDevice(ctx->device));
     debug_wait_timeout_kernel<<<1, 1, 0, ctx->stream>>>(polls, ctx->error_word);
+    B200Q_CUDA(ctx, cudaGetLastError());
+    return B200Q_OK;
+}
+
+b200q_status b200q_debug_late_copy(b200q_ctx *ctx, void *dev_dst, const void *dev_src, size_t bytes, unsigned microseconds) {
+    if (!ctx || !dev_dst || !dev_src) return B200Q_INVALID;
+    if (microseconds > 20000) microseconds = 20000;
+    B200Q_CUDA(ctx, cudaSetDevice(ctx->device));
+    debug_late_copy_kernel<<<1, 256, 0, ctx->stream>>>((uint8_t *)dev_dst, (const uint8_t *)dev_src, bytes, microseconds);
     B200Q_CUDA(ctx, cudaGetLastError());
     return B200Q_OK;
 }

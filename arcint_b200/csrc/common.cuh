@@ -56,6 +56,7 @@ struct ActView {
     int             form;
     int64_t         K;
     int64_t         N;
+    bool            fresh = false;      // the quantizer has just been launched (not found in the cache): it is the launch before the product
 };
 
 // ---- context ------------------------------------------------------------------------
@@ -263,7 +264,7 @@ size_t       gemm_tc_id_act_bytes(int64_t K, int64_t max_tiles);
 b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
                                int64_t max_tiles, uint8_t *act, float *dst, bool act_ready);
 b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
-                            const uint8_t *act, int64_t N, float *dst, int64_t ldd);
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early);
 
 // the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
@@ -282,7 +283,7 @@ size_t       gemm_kq_id_act_bytes(int64_t K, int64_t max_tiles);
 b200q_status launch_gemm_kq_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
                                int64_t max_tiles, uint8_t *act, float *dst, bool act_ready);
 b200q_status launch_gemm_kq(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
-                            const uint8_t *act, int64_t N, float *dst, int64_t ldd);
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early);
 bool         gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride);
 size_t       gemm_kf_act_bytes(int64_t K, int64_t N);
 b200q_status launch_quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out);
@@ -290,6 +291,6 @@ size_t       gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles);
 b200q_status launch_gemm_kf_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
                                int64_t max_tiles, uint8_t *act, float *dst, bool act_ready);
 b200q_status launch_gemm_kf(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
-                            const uint8_t *act, int64_t N, float *dst, int64_t ldd);
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early);
 
 }  // namespace b200q

@@ -116,8 +116,8 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
     // floats as one contiguous kilobyte (lane l: elements 16 l .. 16 l + 15, i.e. half l & 1 of block j = l >> 1),
     // take the maximum by shuffles and store their sixteen codes as two 16-byte pieces. Columns of groups past the tile's
     // last one are never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
-    pdl_trigger();
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
+    pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
     uint8_t *chunk = out + t * tile_bytes(nst) + (size_t)s * CHUNK;
@@ -277,7 +277,7 @@ template <int TYPE, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
-               int *__restrict__ error_word, TileRoute id) {
+               int *__restrict__ error_word, int early, TileRoute id) {
     typedef Smem<TYPE> L;
     constexpr int SBB = Fmt<TYPE>::SBB, NRAW = L::NRAW;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -295,9 +295,11 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // tiles of one expert). A contiguous run of units per block measured slower on the 512-expert configuration (+18 %:
     // the full tiles of busy experts pile up on a few blocks). A dense product with few tiles is cut along K: a unit is
     // then one part of a tile and writes part `part` of a scratch buffer.
-    // Launched with programmatic dependence: before pdl_wait() a block may only read the weights. The producer waits before
-    // its first activation load, the scaling warps before they store; a route's tile list is read by everybody.
-    if (id.tiles) pdl_wait();
+    // Launched with programmatic dependence. early: the launch before is this product's quantizer, which has waited for what came
+    // before it; a block may read the weights at once, the producer waits before its first activation load, the scaling warps
+    // before they store. Otherwise (the activation was there already, a route) the launch before may be anybody's, the
+    // weights' writer too, and may run for long: everybody waits before anything else.
+    if (!early) pdl_wait();
     const int tiles_m = (M + BM - 1) / BM;
     const int tiles_n = id.tiles ? __ldg(id.n_tiles) : n_tiles_dense;
     const int n_units = tiles_m * tiles_n * ksplit;
@@ -703,7 +705,7 @@ b200q_status launch_quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8
 template <int TYPE>
 static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
                                 int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
-                                const TileRoute &tr) {
+                                bool early, const TileRoute &tr) {
     typedef kf::Smem<TYPE> L;
     const bool full = !tr.tiles && N % kf::BN == 0;
     auto kern = full ? kf::gemm_kf_kernel<TYPE, true> : kf::gemm_kf_kernel<TYPE, false>;
@@ -730,7 +732,7 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     const int64_t units = tiles * ksplit;
     const unsigned grid = (unsigned)(units < S ? units : S);
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3(grid), dim3(kf::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
-                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr));
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, (int)early, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);
@@ -739,11 +741,11 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
 }
 
 b200q_status launch_gemm_kf(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
-                            const uint8_t *act, int64_t N, float *dst, int64_t ldd) {
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + kf::BN - 1) / kf::BN;
     const size_t ms = row_stride * (size_t)M;
-    if (type == B200Q_TYPE_Q4_K) return launch_kf_t<B200Q_TYPE_Q4_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_KF);
-    if (type == B200Q_TYPE_Q5_K) return launch_kf_t<B200Q_TYPE_Q5_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_KF);
+    if (type == B200Q_TYPE_Q4_K) return launch_kf_t<B200Q_TYPE_Q4_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_KF);
+    if (type == B200Q_TYPE_Q5_K) return launch_kf_t<B200Q_TYPE_Q5_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_KF);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_kf: type %d", type);
 }
 
@@ -755,9 +757,9 @@ b200q_status launch_gemm_kf_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
     b200q_status st = act_ready ? B200Q_OK : quantize_f16(ctx, src1, act, max_tiles, tr);
     if (st != B200Q_OK) return st;
     if (src0->type == B200Q_TYPE_Q4_K)
-        return launch_kf_t<B200Q_TYPE_Q4_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+        return launch_kf_t<B200Q_TYPE_Q4_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     if (src0->type == B200Q_TYPE_Q5_K)
-        return launch_kf_t<B200Q_TYPE_Q5_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+        return launch_kf_t<B200Q_TYPE_Q5_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_kf_id: type %d", src0->type);
 }
 

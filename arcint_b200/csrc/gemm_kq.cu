@@ -108,8 +108,8 @@ quantize_tiled256_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t n
     // floats as one contiguous kilobyte (lane l: elements 16 l .. 16 l + 15, i.e. half c = l & 1 of block j = l >> 1),
     // take the maximum by shuffles and store one 16-byte piece each. Columns of groups past the tile's last one are
     // never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
-    pdl_trigger();
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
+    pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
     uint8_t *chunk = out + ((size_t)t * nst + s) * ACT_CHUNK;
@@ -235,7 +235,7 @@ template <int TYPE, int FV, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word,
-               TileRoute id, const uint8_t *__restrict__ wraw, size_t row_stride, size_t mat_stride, int rowcopy) {
+               int early, TileRoute id, const uint8_t *__restrict__ wraw, size_t row_stride, size_t mat_stride, int rowcopy) {
     typedef Smem<FV> L;                         // FV: the staging variant of the type's format
     constexpr int SBB = L::SBB, SPS = L::SPS, NRAW = L::NRAW, ROWB = L::ROWB;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -256,9 +256,11 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // units per block (+18 %: the full tiles of busy experts pile up on a few blocks), groups of four row tiles of
     // one column tile so that its activation chunks stay in the ring (+10 % at K = 512), and fetching the next
     // unit's description and the column destinations one unit ahead in the scale-accumulate warps (+4 / +10 %).
-    // Launched with programmatic dependence: before pdl_wait() a block may only read the weights. The producer waits before
-    // its first activation load, the scaling warps before they store; a route's tile list is read by everybody.
-    if (id.tiles) pdl_wait();
+    // Launched with programmatic dependence. early: the launch before is this product's quantizer, which has waited for what came
+    // before it; a block may read the weights at once, the producer waits before its first activation load, the scaling warps
+    // before they store. Otherwise (the activation was there already, a route) the launch before may be anybody's, the
+    // weights' writer too, and may run for long: everybody waits before anything else.
+    if (!early) pdl_wait();
     const int tiles_m = (M + BM - 1) / BM;
     const int tiles_n = id.tiles ? __ldg(id.n_tiles) : n_tiles_dense;
     const int n_units = tiles_m * tiles_n * ksplit;
@@ -623,7 +625,7 @@ b200q_status launch_quantize_tiled256(b200q_ctx *ctx, const b200q_tensor *src1, 
 template <int TYPE, int FV = TYPE>
 static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
                                 int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
-                                const TileRoute &tr) {
+                                bool early, const TileRoute &tr) {
     typedef kq::Smem<FV> L;
     const bool full = !tr.tiles && N % kq::BN == 0;
     auto kern = full ? kq::gemm_kq_kernel<TYPE, FV, true> : kq::gemm_kq_kernel<TYPE, FV, false>;
@@ -657,7 +659,7 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     }
     const unsigned grid = (unsigned)(units < S ? units : S);
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3(grid), dim3(kq::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
-                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr, (const uint8_t *)w, row_stride, mat_stride, rowcopy));
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, (int)early, tr, (const uint8_t *)w, row_stride, mat_stride, rowcopy));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC);
     if (ksplit > 1) return launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd);
@@ -669,13 +671,13 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
 static bool iq4_rows(int64_t K, size_t row_stride, size_t mat_stride) { return K % 512 != 0 || row_stride % 16 != 0 || mat_stride % 16 != 0; }
 
 b200q_status launch_gemm_kq(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
-                            const uint8_t *act, int64_t N, float *dst, int64_t ldd) {
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + kq::BN - 1) / kq::BN;
     const size_t ms = row_stride * (size_t)M;
     if (type == B200Q_TYPE_IQ4_XS && iq4_rows(K, row_stride, ms))
-        return launch_kq_t<B200Q_TYPE_IQ4_XS, kq::FMT_IQ4_XS_ROWS>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE);
-    if (type == B200Q_TYPE_IQ4_XS) return launch_kq_t<B200Q_TYPE_IQ4_XS>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE);
-    if (type == B200Q_TYPE_Q6_K) return launch_kq_t<B200Q_TYPE_Q6_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE);
+        return launch_kq_t<B200Q_TYPE_IQ4_XS, kq::FMT_IQ4_XS_ROWS>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE);
+    if (type == B200Q_TYPE_IQ4_XS) return launch_kq_t<B200Q_TYPE_IQ4_XS>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE);
+    if (type == B200Q_TYPE_Q6_K) return launch_kq_t<B200Q_TYPE_Q6_K>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_kq: type %d", type);
 }
 
@@ -689,10 +691,10 @@ b200q_status launch_gemm_kq_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
     if (src0->type == B200Q_TYPE_IQ4_XS)
         return iq4_rows(K, src0->nb[1], src0->nb[2])
                    ? launch_kq_t<B200Q_TYPE_IQ4_XS, kq::FMT_IQ4_XS_ROWS>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0,
-                                                                         max_tiles, dst, 0, tr)
-                   : launch_kq_t<B200Q_TYPE_IQ4_XS>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+                                                                         max_tiles, dst, 0, false, tr)
+                   : launch_kq_t<B200Q_TYPE_IQ4_XS>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     if (src0->type == B200Q_TYPE_Q6_K)
-        return launch_kq_t<B200Q_TYPE_Q6_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+        return launch_kq_t<B200Q_TYPE_Q6_K>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_kq_id: type %d", src0->type);
 }
 

@@ -112,8 +112,8 @@ quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1,
     // floats as one contiguous kilobyte (lane l: k = 16 l .. 16 l + 15, i.e. half l & 1 of block j = l >> 1), the two
     // lanes of a block share their maximum by one shuffle, and every lane stores its 16 codes as one piece (int8) or
     // two (fp16). Columns past the tile's last one are written as zeros.
-    pdl_trigger();
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
+    pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
     constexpr int OPER_BYTES = Oper<F16>::BYTES, ACT_CHUNK = Oper<F16>::ACT_CHUNK;
@@ -201,7 +201,7 @@ __device__ __forceinline__ void bytes_to_halves(uint32_t b4, uint32_t bias2, uin
 template <int TYPE, bool F16, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
-               int N, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word, TileRoute id) {
+               int N, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word, int early, TileRoute id) {
     typedef Smem<TYPE, F16> L;
     constexpr int ROWB = Raw<TYPE>::ROW;
     constexpr int NSTAGE = L::NSTAGE;
@@ -226,10 +226,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // the tile's matrix and columns: dense, tile_n-th run of 128 tokens; MUL_MAT_ID, a route tile (one
     // expert, up to 128 routed pairs)
     int expert = 0, first = 0, ncols = min(BN, N - tile_n * BN);
-    // Launched with programmatic dependence: before pdl_wait() a block may only read the weights. The producer waits before
-    // its first activation load, the scaling warps before they store; a route's tile list is read by everybody.
+    // Launched with programmatic dependence. early: the launch before is this product's quantizer, which has waited for what came
+    // before it; a block may read the weights at once, the producer waits before its first activation load, the scaling warps
+    // before they store. Otherwise (the activation was there already, a route) the launch before may be anybody's, the
+    // weights' writer too, and may run for long: everybody waits before anything else.
+    if (!early) pdl_wait();
     if (id.tiles) {
-        pdl_wait();
         if (tile_n >= __ldg(id.n_tiles)) return;          // the whole block: nothing is set up yet
         expert = __ldg(id.tiles + 4 * tile_n);
         first = __ldg(id.tiles + 4 * tile_n + 1);
@@ -595,7 +597,7 @@ b200q_status launch_quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uin
 template <int TYPE, bool F16>
 static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
                               int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
-                              const TileRoute &tr) {
+                              bool early, const TileRoute &tr) {
     typedef tc::Smem<TYPE, F16> L;
     // whole column tiles only (and no route): the build without a branch on the columns that are live
     const bool full = !tr.tiles && N % tc::BN == 0;
@@ -624,7 +626,7 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
     }
     dim3 grid((unsigned)n_tiles, (unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)ksplit);
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(tc::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N, out, out_ld,
-                               part_stride, ctx->error_word, tr));
+                               part_stride, ctx->error_word, (int)early, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);
@@ -637,18 +639,18 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
 template <int TYPE>
 static b200q_status launch_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
                              int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
-                             const TileRoute &tr) {
-    return ctx->tc_f16 ? launch_tf<TYPE, true>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, tr)
-                       : launch_tf<TYPE, false>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, tr);
+                             bool early, const TileRoute &tr) {
+    return ctx->tc_f16 ? launch_tf<TYPE, true>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, tr)
+                       : launch_tf<TYPE, false>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, tr);
 }
 
 b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
-                            const uint8_t *act, int64_t N, float *dst, int64_t ldd) {
+                            const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + tc::BN - 1) / tc::BN;
     const size_t ms = row_stride * (size_t)M;
-    if (type == B200Q_TYPE_Q4_0) return launch_t<B200Q_TYPE_Q4_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_TC);
-    if (type == B200Q_TYPE_Q8_0) return launch_t<B200Q_TYPE_Q8_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_TC);
-    if (type == B200Q_TYPE_IQ4_NL) return launch_t<B200Q_TYPE_IQ4_NL>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, NO_ROUTE_TC);
+    if (type == B200Q_TYPE_Q4_0) return launch_t<B200Q_TYPE_Q4_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
+    if (type == B200Q_TYPE_Q8_0) return launch_t<B200Q_TYPE_Q8_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
+    if (type == B200Q_TYPE_IQ4_NL) return launch_t<B200Q_TYPE_IQ4_NL>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_tc: type %d", type);
 }
 
@@ -662,11 +664,11 @@ b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
     b200q_status st = act_ready ? B200Q_OK : quantize_tiled(ctx, src1, act, max_tiles, tr);
     if (st != B200Q_OK) return st;
     if (src0->type == B200Q_TYPE_Q4_0)
-        return launch_t<B200Q_TYPE_Q4_0>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+        return launch_t<B200Q_TYPE_Q4_0>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     if (src0->type == B200Q_TYPE_Q8_0)
-        return launch_t<B200Q_TYPE_Q8_0>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+        return launch_t<B200Q_TYPE_Q8_0>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     if (src0->type == B200Q_TYPE_IQ4_NL)
-        return launch_t<B200Q_TYPE_IQ4_NL>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, tr);
+        return launch_t<B200Q_TYPE_IQ4_NL>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_tc_id: type %d", src0->type);
 }
 

@@ -18,6 +18,10 @@
  *     asynchronous to the host unless the call says otherwise;
  *   - tensor storage belongs to the caller; scratch belongs to the context, grows on
  *     demand and is never shrunk (the reference's prealloc_* buffers, P01:66-88);
+ *   - a product of at most 8 columns starts to read its weights while the kernel ahead of it on the stream may still be
+ *     running (programmatic dependent launch). A kernel of the caller's that writes weights must have written them before it
+ *     lets its dependents start (griddepcontrol.launch_dependents, cudaTriggerProgrammaticLaunchCompletion); one that never
+ *     does, and a copy, are waited for to their end. Everything else, wider products among it, waits for all earlier work;
  *   - there is no CPU fallback: a shape the kernels do not take is B200Q_UNSUPPORTED.
  */
 #ifndef B200Q_H

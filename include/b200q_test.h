@@ -35,6 +35,9 @@ B200Q_API b200q_status b200q_debug_wait_timeout(b200q_ctx *ctx, unsigned polls);
  * overwritten (the first one is named in b200q_last_error). Without B200Q_CANARY: B200Q_INVALID. */
 B200Q_API b200q_status b200q_debug_check_guards(b200q_ctx *ctx, int *blocks, int *violated);
 
+/* Enqueues a kernel that lets its dependents start at once (griddepcontrol.launch_dependents), waits for about `microseconds` (at
+ * most 20,000, doubled) and then copies bytes on the device: a writer that a later call must wait for to the end. */
+B200Q_API b200q_status b200q_debug_late_copy(b200q_ctx *ctx, void *dev_dst, const void *dev_src, size_t bytes, unsigned microseconds);
 /* A fake of the failing allocation: from here on the context's scratch allocations of more than `bytes` bytes fail as on a
  * full device (0: none does). */
 B200Q_API b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes);

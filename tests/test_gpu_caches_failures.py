@@ -187,3 +187,27 @@ def test_failed_growth_keeps_the_recorded_block():
         ctx.graph_launch(g)
         assert rel_err(ctx.download(p[2], (n, 128), np.float32), O.mul_mat_f64(t, w, k, 2 * x, True)) < TOL
         ctx.graph_free(g)
+
+
+@pytest.mark.parametrize("t", [A.Q4_0, A.Q8_0, A.Q4_K, A.Q5_K, A.Q6_K, A.IQ4_XS])
+@pytest.mark.parametrize("cached", [False, True])
+def test_prompt_product_waits_for_its_weights(ctx, t, cached):
+    """A kernel that writes the weights late, but lets its dependents start at once: the product behind it uses the new weights, with a
+    quantizer of its own in between and without."""
+    m, k, n = 384, 2048, 40
+    wa, x, (W, X, Y), p = prompt(ctx, t, m, k, n, 700 + t)
+    wb = make_weights(t, m, k, 800 + t)
+    new = ctx.upload(wb)
+    ctx.graph_begin()
+    ctx.mul_mat(W, X, Y)
+    ctx.sync()
+    if not cached:
+        ctx.graph_begin()
+    hits = ctx.stats().get("act_cache_hit", 0)
+    ctx.late_copy(p[0], new, wb.nbytes, 2000)
+    ctx.mul_mat(W, X, Y)
+    got = ctx.download(p[2], (n, m), np.float32)
+    assert ctx.stats().get("act_cache_hit", 0) - hits == cached
+    assert rel_err(got, O.mul_mat_f64(t, wb, k, x, True)) < TOL
+    for q in p + (new,):
+        ctx.free(q)
