@@ -269,10 +269,12 @@ b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_
 // the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
 
-// K parts of a product whose tiles fill the SMs badly, and the scratch for their results (ksplit.cu); the times of a 256-weight step on a full
-// tile that it counts with
-int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, int step_ns, int64_t M, int64_t N, float **parts);
-constexpr int TC_SB_NS = 2000, KQ_SB_NS = 2000, KF_SB_NS = 900;
+// K parts of a product whose tiles fill the SMs badly, and the scratch for their results (ksplit.cu). It counts with a kernel's times
+// on full tiles: a step of 256 weights, and what a unit costs beyond its steps (fill, drain, stores; gemm_tc, one block a unit, sets
+// itself up and allocates tensor memory too). Measured from products of one round, 16 and 43 steps long.
+struct KsplitTimes { int step_ns, unit_ns; };
+constexpr KsplitTimes TC_TIMES = { 3900, 2600 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 };
+int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts);
 
 // gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types
 // (integer sub-scales folded into the weight operand)

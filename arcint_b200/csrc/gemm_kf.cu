@@ -721,7 +721,7 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     // persistent blocks, one per SM, walking the (row tile, column tile, part of K) units
     const int64_t tiles = n_tiles * ((M + kf::BM - 1) / kf::BM), S = ctx->sm_count;
     float *out = dst, *parts = nullptr;
-    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, KF_SB_NS, M, N, &parts);
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, KF_TIMES, M, N, &parts);
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
         out = parts;

@@ -649,7 +649,7 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     int64_t units = n_tiles * ((M + kq::BM - 1) / kq::BM);
     const int64_t S = ctx->sm_count, nst = K / 256 / L::SPS;
     float *out = dst, *parts = nullptr;
-    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, units, nst, L::SPS * KQ_SB_NS, M, N, &parts);
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, units, nst, { L::SPS * KQ_TIMES.step_ns, KQ_TIMES.unit_ns }, M, N, &parts);
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
         out = parts;

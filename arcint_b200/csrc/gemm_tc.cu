@@ -617,7 +617,7 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
     // does not depend on which block finishes first.
     const int64_t tiles = n_tiles * ((M + tc::BM - 1) / tc::BM);
     float *out = dst, *parts = nullptr;
-    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, TC_SB_NS, M, N, &parts);
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, TC_TIMES, M, N, &parts);
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
         out = parts;
