@@ -1,14 +1,11 @@
 """The tensor-core prompt GEMM where its tiles, halves, parts of K and row stagings end, against the
-fp64 product of the same quantized operands.
-
-The bound: block dots are exact integers and what is left are f32 sums over the K / 256 super-blocks (K / 32 blocks) of a
-row, each of at most three roundings of half an ulp (2^-24) of the running sum, so |error| <= 3 n 2^-24 sum|terms|; the sum of the
-absolute terms is taken from the operands."""
+fp64 product of the same quantized operands. (the bound: `gpu_util.check_sums`)"""
 import numpy as np
 import pytest
 
 import arcint_b200 as A
 import oracle as O
+from gpu_util import check_sums as check, normal_data as data
 
 pytestmark = pytest.mark.gpu
 
@@ -22,27 +19,6 @@ def ctx():
     c.close()
 
 
-def check(got, t, w, k, x):
-    ref = O.mul_mat_f64(t, w, k, x, True)
-    block = 32 if t in (A.Q4_0, A.Q8_0, A.IQ4_NL) else 256
-    # a bound of the absolute terms of an output: |w| row by |x| column
-    wa = np.abs(O.dequantize(t, w, k)).reshape(w.shape[0], k).astype(np.float64)
-    if t in (A.Q4_K, A.Q5_K):
-        # the scale and the mins term are rounded apart: d sc q + dmin m <= |w| + 2 dmin m, and dmin m is minus the weight of code 0
-        zero = w.reshape(w.shape[0], k // 256, -1).copy()
-        zero[:, :, 16:] = 0
-        wa = wa + 2 * np.abs(O.dequantize(t, zero.reshape(w.shape), k)).reshape(w.shape[0], k)
-    terms = np.abs(x.astype(np.float64)) @ wa.T
-    bound = 3 * (k // block) * 2.0 ** -24 * terms * 1.02 + 1e-30     # 1.02: the activation's own rounding to 8 bits
-    assert np.isfinite(got).all()
-    assert (np.abs(got - ref) <= bound).all(), float((np.abs(got - ref) / bound).max())
-
-
-def data(t, m, k, n, seed):
-    rng = np.random.default_rng(seed)
-    return O.quantize(t, O.fill_normal(m * k, seed, 0.02).reshape(m, k)), rng.normal(0, 1, size=(n, k)).astype(np.float32)
-
-
 # one super-block; halves of 16, 32, 48 and 64 columns, the second with one column or none; the second column tile with one
 # column; row tiles with one row or all but one; parts of K of unequal length (K = 2816: eleven super-blocks)
 @pytest.mark.parametrize("t", TYPES)
@@ -53,6 +29,17 @@ def test_tile_edges(ctx, t, m, k, n):
     ctx.stats_reset()
     got = ctx.run_mul_mat(t, w, k, x)
     assert ctx.stats().get("gemm_tc", 0) == 1
+    check(got, t, w, k, x)
+
+
+# whole column tiles only, cut along K: parts of equal and of unequal length, one row tile and a ragged second one
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("m,k,n", [(128, 4096, 128), (200, 2816, 256), (129, 11008, 128)])
+def test_whole_tiles_cut_along_k(ctx, t, m, k, n):
+    w, x = data(t, m, k, n, m + n)
+    ctx.stats_reset()
+    got = ctx.run_mul_mat(t, w, k, x)
+    assert ctx.stats().get("gemm_tc", 0) == 1 and ctx.stats().get("gemm_ksplit", 0) == 1
     check(got, t, w, k, x)
 
 

@@ -109,3 +109,14 @@ def test_ffn_block_against_the_fp64_chain_and_the_unfused_sequence(ctx, t, n_exp
     assert nmse(got, seq) < 1e-6, nmse(got, seq)
     for p in (dg, du, dd, dx, dl, dy, di, dwt, dgo, duo, ddo, dh):
         ctx.free(p)
+
+
+@pytest.mark.parametrize("t,d_ff,i8", [(A.Q4_0, 256, ""), (A.Q8_0, 512, ""), (A.IQ4_NL, 256, ""), (A.Q4_0, 512, "1"), (A.Q8_0, 256, "1"), (A.Q5_K, 256, ""),
+                                       (A.Q6_K, 256, "")])
+def test_ffn_block_on_the_tensor_cores(monkeypatch, t, d_ff, i8):
+    """Prompt-sized blocks whose down projection, too, takes route tiles: SwiGLU in every tiled quantizer, both operand forms of the
+    per-32 types, Q6_K rows of 210 bytes."""
+    monkeypatch.setenv("B200Q_TC_I8", i8)
+    with A.Context(0) as c:
+        test_ffn_block_against_the_fp64_chain_and_the_unfused_sequence(c, t, 8, 2, 512, d_ff, 150)
+        assert c.stats()["moe_gemm"] == 6                  # gate, up and down, in the block and in the sequence it is compared with
