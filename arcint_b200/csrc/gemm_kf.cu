@@ -10,14 +10,14 @@
 // within 2^24. Past it the tensor core cuts bits off at each of the sixteen steps (measured on one-sided activations, sums up to 3.3 x
 // 2^24: 3.2 ulp too small on average, where rounding the integer sum once is off by half an ulp at most). p >= 0, so no partial sum of
 // a column, in any order, exceeds max(p) times the larger of the sums of its positive and of its negative codes. The quantizer
-// writes the largest of these per (column tile, super-block). A column tile where one does not rule 2^24 out takes its super-blocks in
-// two chains of four blocks (Q4_K: 128 * 945 * 127 < 2^24) or four of two (Q5_K: 64 * 1953 * 127), each exact, which the scaling
+// writes the largest of these per (column tile, super-block). An activation where one does not rule 2^24 out has its super-blocks taken
+// in two chains of four blocks (Q4_K: 128 * 945 * 127 < 2^24) or four of two (Q5_K: 64 * 1953 * 127), each exact, which the scaling
 // warps add one after the other in f32. Distance from the 64-bit product, activations uniform in 0.6..1, K = 4096: 1.2e-6 (Q4_K), 1.4e-6
-// (Q5_K; 7.4e-6 with one chain; int32 sums with the mins in a second pass: 1.0e-5). The largest sums of a tile are read once a unit,
-// which then has one chain or several throughout: asked per super-block, the answer cost the MMA issuer 4 %, and reading a unit
-// ahead cost registers and 2 % of a 512-expert block. Q4_K 11008x4096 x 512 tokens: 75 us with one chain, 93 with two;
-// Q5_K 85 and 136 with four. N(0, 1) activations take one, their one-sided sums are half of what Q5_K's chain holds; activations of
-// one sign take more from a mean of 0.55 (Q4_K) and 0.26 (Q5_K) of the largest.
+// (Q5_K; 7.4e-6 with one chain; int32 sums with the mins in a second pass: 1.0e-5). One answer for the whole product: who shares
+// a tile of a route is left to the order of its pairs, which is not fixed, and a pair's bits must not depend on it. (Per tile, an expert's
+// results would change from run to run; per super-block, the answer cost the MMA issuer 4 %.) Q4_K 11008x4096 x 512 tokens: 75 us
+// with one chain, 94 with two; Q5_K 88 and 141 with four. N(0, 1) activations take one, their one-sided sums are half of what
+// Q5_K's chain holds; activations of one sign take more from a mean of 0.55 (Q4_K) and 0.26 (Q5_K) of the largest.
 // The mins term is one more K = 16 MMA per super-block into an accumulator of its own: a row of A is [m_0..m_7, m_0..m_7], a column of
 // B is [bl_0..bl_7, 256 bh_0..256 bh_7] with bsum_j = 256 bh_j + bl_j (all exact in f16).
 //
@@ -71,17 +71,16 @@ static_assert(128 * 48 + 256 * 56 + 256 * 160 <= THREADS * LAUNCH_REGS, "registe
 //   codes, twice (blocks 0..3, 4..7): [group g < 16][block j < 4][piece c < 4][column r < 8][8 codes as halves, each run of four
 //          in the order 0 2 1 3, in which the unpack threads mask nibbles out of a word]
 //   extra: 128 f32 scales, then the mins operand [group g < 16][piece c < 2][column r < 8][8 halves: bl_0..7 or 256 bh_0..7]
-// A column tile is its chunks, then an int32 per super-block: the largest one-sided sum of codes of a column, see above.
+// Behind the chunks of all column tiles an int32 for each: the largest one-sided sum of codes of a column, see above.
 constexpr int CODE_BLOCK = 512, CODE_GROUP = GB * CODE_BLOCK, CODE_STAGE = (BN / 8) * CODE_GROUP;
 constexpr int MINS_GROUP = 256, EXTRA_MINS = BN * 4, EXTRA = EXTRA_MINS + (BN / 8) * MINS_GROUP;
 constexpr int CHUNK = 2 * CODE_STAGE + EXTRA;
-__host__ __device__ constexpr size_t tile_bytes(int64_t nsb) { return (size_t)nsb * CHUNK + (size_t)((4 * nsb + 127) / 128 * 128); }
 
 template <int TYPE> struct Fmt;
 template <> struct Fmt<B200Q_TYPE_Q4_K> { enum { SBB = 144, NRAW = 3, PMAX = 63 * 15, CHAINS = 2 }; };
 template <> struct Fmt<B200Q_TYPE_Q5_K> { enum { SBB = 176, NRAW = 2, PMAX = 63 * 31, CHAINS = 4 }; };
 
-// a super-block with a larger one-sided sum makes its column tile take several chains; a chain of theirs is exact
+// a larger one-sided sum makes the product take several chains a super-block; a chain of theirs is exact
 template <int TYPE> __host__ __device__ constexpr int one_chain_side() { return (1 << 24) / Fmt<TYPE>::PMAX; }
 static_assert(256 / 2 * 127 * 63 * 15 <= (1 << 24) && 256 / 4 * 127 * 63 * 31 <= (1 << 24), "CHAINS");
 
@@ -120,7 +119,7 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
     pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
-    uint8_t *chunk = out + t * tile_bytes(nst) + (size_t)s * CHUNK;
+    uint8_t *chunk = out + ((size_t)t * nst + s) * CHUNK;
     int cnt, first = 0;
     if (id.tiles) {
         // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
@@ -200,7 +199,7 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int i = 1; i < 8; ++i) side = max(side, side_of_warp[i]);
-        reinterpret_cast<int *>(out + t * tile_bytes(nst) + (size_t)nst * CHUNK)[s] = side;
+        reinterpret_cast<int *>(out + (size_t)gridDim.y * nst * CHUNK)[(size_t)t * nst + s] = side;
     }
 }
 
@@ -272,17 +271,20 @@ struct Unit {
     int tile_n, row0, valid_rows, expert, first, ncols, sb0, sb1, part, cw;      // cw: columns of a scale-accumulate warp group
 };
 
-// FULL: every column tile has BN columns (and there is no route): the build without a branch on the columns that are live
-template <int TYPE, bool FULL>
+// Builds by what the column tiles are: whole tiles of a dense product (no branch on the columns that are live), tiles of a dense product
+// with a ragged end, tiles of a route
+enum { COLS_FULL = 0, COLS_RAGGED = 1, COLS_ROUTE = 2 };
+template <int TYPE, int COLS>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
                int *__restrict__ error_word, int early, TileRoute id) {
     typedef Smem<TYPE> L;
+    constexpr bool FULL = COLS == COLS_FULL, ROUTE = COLS == COLS_ROUTE;
     constexpr int SBB = Fmt<TYPE>::SBB, NRAW = L::NRAW;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, more_slot;
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler, too)
     const int nsb = K / 256;                    // super-blocks of a row
     const uint32_t sbase = smem_u32(smem);
@@ -301,7 +303,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // weights' writer too, and may run for long: everybody waits before anything else.
     if (!early) pdl_wait();
     const int tiles_m = (M + BM - 1) / BM;
-    const int tiles_n = id.tiles ? __ldg(id.n_tiles) : n_tiles_dense;
+    const int tiles_n = ROUTE ? __ldg(id.n_tiles) : n_tiles_dense;
     const int n_units = tiles_m * tiles_n * ksplit;
     auto unit_of = [&](int u) {
         Unit U;
@@ -315,7 +317,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         U.expert = 0;
         U.first = 0;
         U.ncols = min(BN, N - U.tile_n * BN);
-        if (id.tiles) {
+        if (ROUTE) {
             U.expert = __ldg(id.tiles + 4 * U.tile_n);
             U.first = __ldg(id.tiles + 4 * U.tile_n + 1);
             U.ncols = __ldg(id.tiles + 4 * U.tile_n + 2);
@@ -325,17 +327,23 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         U.cw = FULL || U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
         return U;
     };
-    // the largest one-sided sum of codes in unit u's column tile, a share per lane, and whether the unit takes more than one chain
-    auto side_of = [&](int u) {
-        int side = 0;
-        if (u < n_units) {
-            const int *p = reinterpret_cast<const int *>(act + (size_t)(u / ksplit % tiles_n) * tile_bytes(nsb) + (size_t)nsb * CHUNK);
-            for (int i = lane; i < nsb; i += 32) side = max(side, __ldg(p + i));
-        }
-        return side;
-    };
-    auto takes_more = [&](int side) { return __any_sync(0xFFFFFFFFu, side > one_chain_side<TYPE>()) != 0; };
     if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
+    // whether one of this thread's share of the one-sided sums asks for more than one chain. Every block reads them all: a route's, with its
+    // many tiles, by all threads (a block waits first anyway), a dense product's by the warps that need the answer, once they
+    // have waited, so that weights are fetched and unpacked meanwhile (asking with the whole block costs 2 us a launch).
+    auto asks_for_more = [&](int first, int step) {
+        const int total = tiles_n * nsb;
+        const int *p = reinterpret_cast<const int *>(act + (size_t)n_tiles_dense * nsb * CHUNK);
+        int side = 0;
+#pragma unroll 4
+        for (int i = 4 * first; i + 3 < total; i += 4 * step) {
+            const int4 v = __ldg(reinterpret_cast<const int4 *>(p + i));
+            side = max(side, max(max(v.x, v.y), max(v.z, v.w)));
+        }
+        if (first < total % 4) side = max(side, __ldg(p + total - 1 - first));
+        return side > one_chain_side<TYPE>();
+    };
+    const bool mine = ROUTE && asks_for_more(threadIdx.x, THREADS);
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -367,6 +375,10 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
+    if (ROUTE) {
+        const int any = __syncthreads_or(mine);
+        if (threadIdx.x == 0) more_slot = any;
+    }
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_slot, 0);
@@ -381,7 +393,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
-            const uint8_t *act_tile = act + (size_t)U.tile_n * tile_bytes(nsb);
+            const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * CHUNK;
             const uint32_t groups = (uint32_t)(U.ncols + 7) >> 3;          // live column groups
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int st = s_run % NRAW, xt = s_run % NX;
@@ -435,11 +447,11 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             return true;
         };
         pdl_wait();
+        const bool more = ROUTE ? *(volatile int *)&more_slot != 0 : __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32)) != 0;
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);                      // N: the live columns, in sixteens
-            const bool more = takes_more(side_of(u));
             if (!more) {
                 for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run, ++v_run) {
                     const int xt = s_run % NX;
@@ -543,10 +555,10 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         const int q4 = warp & 3, half = (warp - 12) >> 2, g = lane >> 2, c = lane & 3;
         int s_run = 0, v_run = 0;
         pdl_wait();
+        const int chains = (ROUTE ? *(volatile int *)&more_slot : __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32))) ? Fmt<TYPE>::CHAINS : 1;
         bool ok = true;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
-            const int chains = takes_more(side_of(u)) ? Fmt<TYPE>::CHAINS : 1;
             const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
             const bool live = FULL || ncol > 0, two = FULL || ncol > 32;
             f32x2 acc2[4][8];                                  // rows g, g + 8, g + 16, g + 24; column pairs 8 i + 2 c
@@ -612,7 +624,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             }
             if (ok && live) {
                 const int r0 = q4 * 32 + g;
-                if (!FULL && id.tiles) {
+                if (ROUTE) {
                     // where the half's columns go: every lane looks up two of them (loads in flight together), the
                     // store loop takes them by shuffle
                     long long off[2];
@@ -675,7 +687,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 
 static const TileRoute NO_ROUTE_KF = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
-size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)((N + kf::BN - 1) / kf::BN) * kf::tile_bytes(K / 256); }
+size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + kf::BN - 1) / kf::BN) * (K / 256)) * (kf::CHUNK + 4); }
 size_t gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles) { return gemm_kf_act_bytes(K, max_tiles * kf::BN); }
 
 bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride) {
@@ -707,10 +719,11 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
                                 int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
                                 bool early, const TileRoute &tr) {
     typedef kf::Smem<TYPE> L;
-    const bool full = !tr.tiles && N % kf::BN == 0;
-    auto kern = full ? kf::gemm_kf_kernel<TYPE, true> : kf::gemm_kf_kernel<TYPE, false>;
-    static bool attr_set_dev[B200Q_MAX_DEVICES][2] = {};
-    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][full];
+    const int cols = tr.tiles ? kf::COLS_ROUTE : N % kf::BN == 0 ? kf::COLS_FULL : kf::COLS_RAGGED;
+    auto kern = cols == kf::COLS_ROUTE ? kf::gemm_kf_kernel<TYPE, kf::COLS_ROUTE>
+              : cols == kf::COLS_FULL  ? kf::gemm_kf_kernel<TYPE, kf::COLS_FULL> : kf::gemm_kf_kernel<TYPE, kf::COLS_RAGGED>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES][3] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][cols];
     if (!attr_set) {
         B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
         attr_set = true;

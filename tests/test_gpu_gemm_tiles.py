@@ -116,8 +116,8 @@ def test_sums_at_24_bits(ctx, t, edge):
 @pytest.mark.parametrize("t", [A.Q4_K, A.Q5_K])
 @pytest.mark.parametrize("m,n", [(300, 24), (128 * 60, 128 * 4 + 20), (128 * 40, 128 * 4)])
 def test_one_and_more_chains_in_turn(ctx, t, m, n):
-    """Super-blocks that need more than one chain between ones that do not, over several units of a block; one rounding of the running
-    sum a chain."""
+    """Super-blocks that need more than one chain between ones that do not, over several units of a block; a rounding for each
+    addition of a chain and one of the running sum a super-block."""
     rng = np.random.default_rng(m + n)
     sides = [0, 1, 1, 0, -1, 0, 0, 1, -1]
     w, wi = integer_blocks(t, m, len(sides), rng, 10)
@@ -150,5 +150,38 @@ def test_more_chains_in_route_tiles(ctx, t):
     assert np.abs(exact).max() > 2 ** 24
     # the second super-block's sum stays below 2^24: a rounding per chain of the first and one of the total
     assert (np.abs(got - exact) <= 5 * 2.0 ** -24 * (np.abs(exact) + 2.0 ** 24)).all()
+    for p in (dw, dx, di, dy):
+        ctx.free(p)
+
+
+@pytest.mark.parametrize("t", [A.Q4_K, A.Q5_K])
+def test_pairs_of_an_expert_in_any_order(ctx, t):
+    """Several tiles to an expert, one token that needs more than one chain: no token's bits depend on who shares its tile."""
+    n_exp, m, k, n_tok = 2, 128, 512, 500
+    rng = np.random.default_rng(4)
+    w, x = data(t, m * n_exp, k, n_tok, 21)
+    x[7] = rng.uniform(0.6, 1, k)
+    ids = rng.integers(0, n_exp, (n_tok, 1)).astype(np.int32)
+    dw, dx, di, dy = ctx.upload(w), ctx.upload(x), ctx.upload(ids), ctx.alloc(n_tok * m * 4)
+    ti = A.Tensor.f32(di, [1, n_tok])
+    ti.type = A.I32
+
+    def run(order):
+        ctx.upload(x[order], dx)
+        ctx.upload(ids[order], di)
+        ctx.stats_reset()
+        ctx.graph_begin()
+        ctx.mul_mat_id(A.Tensor.weights(t, dw, k, m, n_exp), A.Tensor.f32(dx, [k, 1, n_tok]), ti, A.Tensor.f32(dy, [m, 1, n_tok]))
+        out = np.empty((n_tok, m), np.float32)
+        out[order] = ctx.download(dy, (n_tok, m), np.float32)
+        assert ctx.stats().get("moe_gemm", 0) == 1
+        return out
+
+    first = run(np.arange(n_tok))
+    for _ in range(3):
+        assert np.array_equal(run(rng.permutation(n_tok)), first)
+    for e in range(n_exp):
+        tok = np.nonzero(ids[:, 0] == e)[0]
+        check(first[tok], t, w[e * m:(e + 1) * m], k, x[tok])
     for p in (dw, dx, di, dy):
         ctx.free(p)
