@@ -15,7 +15,7 @@
 // warps add one after the other in f32. Distance from the 64-bit product, activations uniform in 0.6..1, K = 4096: 1.2e-6 (Q4_K), 1.4e-6
 // (Q5_K; 7.4e-6 with one chain; int32 sums with the mins in a second pass: 1.0e-5). One answer for the whole product: who shares
 // a tile of a route is left to the order of its pairs, which is not fixed, and a pair's bits must not depend on it. (Per tile, an expert's
-// results would change from run to run; per super-block, the answer cost the MMA issuer 4 %.) Q4_K 11008x4096 x 512 tokens: 75 us
+// results would change from run to run; per super-block, the answer cost the MMA issuer 4 %.) Q4_K 11008x4096 x 512 tokens: 76 us
 // with one chain, 94 with two; Q5_K 88 and 141 with four. N(0, 1) activations take one, their one-sided sums are half of what
 // Q5_K's chain holds; activations of one sign take more from a mean of 0.55 (Q4_K) and 0.26 (Q5_K) of the largest.
 // The mins term is one more K = 16 MMA per super-block into an accumulator of its own: a row of A is [m_0..m_7, m_0..m_7], a column of
@@ -26,7 +26,7 @@
 // in shared memory, whose port (128 bytes per clock) the B reads of the MMAs alone fill by half.
 //
 // Tensor memory, 512 columns: two main accumulators of 128 columns, one for the mins term, and the ring of A blocks (two
-// groups of four 32-weight blocks, 16 columns of packed half pairs a block). Warp roles: producer, MMA issuer, two idle,
+// groups of four 32-weight blocks, 16 columns of packed half pairs a block). Warp roles: producer, MMA issuer, two idle (one reads the one-sided sums),
 // eight unpack warps (a thread = a row and half of the blocks of a group), eight scale-accumulate warps (four per half of
 // the columns, a lane quarter each). Persistent blocks walk the units (row tile, column tile, part of K). Every mbarrier
 // wait is bounded.
@@ -100,7 +100,7 @@ template <int TYPE> struct Smem {
 };
 
 enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_CODE_FULL = 6, BAR_CODE_EMPTY = 10, BAR_X_FULL = 14, BAR_X_EMPTY = 17, BAR_A_FULL = 22,
-       BAR_A_EMPTY = 24, BAR_ACC_FULL = 26, BAR_ACC_EMPTY = 28, BAR_COUNT = 30 };
+       BAR_A_EMPTY = 24, BAR_ACC_FULL = 26, BAR_ACC_EMPTY = 28, BAR_MORE = 30, BAR_COUNT = 31 };
 static_assert(NCODE == 4 && NX == 3 && NG == 2 && BAR_COUNT <= 32, "barrier slots above");
 
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
@@ -278,7 +278,7 @@ template <int TYPE, int COLS>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
-               int *__restrict__ error_word, int early, TileRoute id) {
+               int *__restrict__ error_word, TileRoute id) {
     typedef Smem<TYPE> L;
     constexpr bool FULL = COLS == COLS_FULL, ROUTE = COLS == COLS_ROUTE;
     constexpr int SBB = Fmt<TYPE>::SBB, NRAW = L::NRAW;
@@ -297,11 +297,11 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // tiles of one expert). A contiguous run of units per block measured slower on the 512-expert configuration (+18 %:
     // the full tiles of busy experts pile up on a few blocks). A dense product with few tiles is cut along K: a unit is
     // then one part of a tile and writes part `part` of a scratch buffer.
-    // Launched with programmatic dependence. early: the launch before is this product's quantizer, which has waited for what came
-    // before it; a block may read the weights at once, the producer waits before its first activation load, the scaling warps
-    // before they store. Otherwise (the activation was there already, a route) the launch before may be anybody's, the
-    // weights' writer too, and may run for long: everybody waits before anything else.
-    if (!early) pdl_wait();
+    // Launched with programmatic dependence behind this product's own quantizer, which has waited for what came before it: a block may
+    // read the weights at once, the producer waits before its first activation load, the scaling warps before they store. A
+    // route's tile list is read by everybody. (Where the activation was there already the launch before may be anybody's, the
+    // weights' writer too: such a product is launched in plain stream order.)
+    if (ROUTE) pdl_wait();
     const int tiles_m = (M + BM - 1) / BM;
     const int tiles_n = ROUTE ? __ldg(id.n_tiles) : n_tiles_dense;
     const int n_units = tiles_m * tiles_n * ksplit;
@@ -329,8 +329,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     };
     if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
     // whether one of this thread's share of the one-sided sums asks for more than one chain. Every block reads them all: a route's, with its
-    // many tiles, by all threads (a block waits first anyway), a dense product's by the warps that need the answer, once they
-    // have waited, so that weights are fetched and unpacked meanwhile (asking with the whole block costs 2 us a launch).
+    // many tiles, by all threads (a block waits first anyway), a dense product's by an idle warp behind its wait, so that weights
+    // are fetched and unpacked meanwhile (asking with the whole block costs 2 us a launch).
     auto asks_for_more = [&](int first, int step) {
         const int total = tiles_n * nsb;
         const int *p = reinterpret_cast<const int *>(act + (size_t)n_tiles_dense * nsb * CHUNK);
@@ -367,6 +367,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             mbar_init(bar(BAR_ACC_FULL + i), 1);
             mbar_init(bar(BAR_ACC_EMPTY + i), 8);                  // scaling warps
         }
+        mbar_init(bar(BAR_MORE), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -447,8 +448,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             return true;
         };
         pdl_wait();
-        const bool more = ROUTE ? *(volatile int *)&more_slot != 0 : __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32)) != 0;
-        bool ok = true;
+        bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
+        const bool more = *(volatile int *)&more_slot != 0;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);                      // N: the live columns, in sixteens
@@ -505,6 +506,14 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         }
     } else if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
+        if (!ROUTE && warp == 2) {
+            pdl_wait();
+            const int any = __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32));
+            if (lane == 0) {
+                more_slot = any;
+                mbar_arrive(bar(BAR_MORE));
+            }
+        }
     } else if (warp < 12) {
         // ---- unpack: two threads per weight row ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;" ::: "memory");
@@ -555,8 +564,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         const int q4 = warp & 3, half = (warp - 12) >> 2, g = lane >> 2, c = lane & 3;
         int s_run = 0, v_run = 0;
         pdl_wait();
-        const int chains = (ROUTE ? *(volatile int *)&more_slot : __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32))) ? Fmt<TYPE>::CHAINS : 1;
-        bool ok = true;
+        bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
+        const int chains = *(volatile int *)&more_slot ? Fmt<TYPE>::CHAINS : 1;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
@@ -744,8 +753,8 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     }
     const int64_t units = tiles * ksplit;
     const unsigned grid = (unsigned)(units < S ? units : S);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3(grid), dim3(kf::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
-                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, (int)early, tr));
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl && (early || tr.tiles), kern, dim3(grid), dim3(kf::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);

@@ -235,7 +235,7 @@ template <int TYPE, int FV, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word,
-               int early, TileRoute id, const uint8_t *__restrict__ wraw, size_t row_stride, size_t mat_stride, int rowcopy) {
+               TileRoute id, const uint8_t *__restrict__ wraw, size_t row_stride, size_t mat_stride, int rowcopy) {
     typedef Smem<FV> L;                         // FV: the staging variant of the type's format
     constexpr int SBB = L::SBB, SPS = L::SPS, NRAW = L::NRAW, ROWB = L::ROWB;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -256,11 +256,11 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // units per block (+18 %: the full tiles of busy experts pile up on a few blocks), groups of four row tiles of
     // one column tile so that its activation chunks stay in the ring (+10 % at K = 512), and fetching the next
     // unit's description and the column destinations one unit ahead in the scale-accumulate warps (+4 / +10 %).
-    // Launched with programmatic dependence. early: the launch before is this product's quantizer, which has waited for what came
-    // before it; a block may read the weights at once, the producer waits before its first activation load, the scaling warps
-    // before they store. Otherwise (the activation was there already, a route) the launch before may be anybody's, the
-    // weights' writer too, and may run for long: everybody waits before anything else.
-    if (!early) pdl_wait();
+    // Launched with programmatic dependence behind this product's own quantizer, which has waited for what came before it: a block may
+    // read the weights at once, the producer waits before its first activation load, the scaling warps before they store. A
+    // route's tile list is read by everybody. (Where the activation was there already the launch before may be anybody's, the
+    // weights' writer too: such a product is launched in plain stream order.)
+    if (id.tiles) pdl_wait();
     const int tiles_m = (M + BM - 1) / BM;
     const int tiles_n = id.tiles ? __ldg(id.n_tiles) : n_tiles_dense;
     const int n_units = tiles_m * tiles_n * ksplit;
@@ -658,8 +658,8 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
         units *= ksplit;
     }
     const unsigned grid = (unsigned)(units < S ? units : S);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3(grid), dim3(kq::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
-                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, (int)early, tr, (const uint8_t *)w, row_stride, mat_stride, rowcopy));
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl && (early || tr.tiles), kern, dim3(grid), dim3(kq::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr, (const uint8_t *)w, row_stride, mat_stride, rowcopy));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC);
     if (ksplit > 1) return launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd);

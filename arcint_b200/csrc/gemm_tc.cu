@@ -201,7 +201,7 @@ __device__ __forceinline__ void bytes_to_halves(uint32_t b4, uint32_t bias2, uin
 template <int TYPE, bool F16, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
-               int N, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word, int early, TileRoute id) {
+               int N, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word, TileRoute id) {
     typedef Smem<TYPE, F16> L;
     constexpr int ROWB = Raw<TYPE>::ROW;
     constexpr int NSTAGE = L::NSTAGE;
@@ -226,12 +226,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // the tile's matrix and columns: dense, tile_n-th run of 128 tokens; MUL_MAT_ID, a route tile (one
     // expert, up to 128 routed pairs)
     int expert = 0, first = 0, ncols = min(BN, N - tile_n * BN);
-    // Launched with programmatic dependence. early: the launch before is this product's quantizer, which has waited for what came
-    // before it; a block may read the weights at once, the producer waits before its first activation load, the scaling warps
-    // before they store. Otherwise (the activation was there already, a route) the launch before may be anybody's, the
-    // weights' writer too, and may run for long: everybody waits before anything else.
-    if (!early) pdl_wait();
+    // Launched with programmatic dependence behind this product's own quantizer, which has waited for what came before it: a block may
+    // read the weights at once, the producer waits before its first activation load, the scaling warps before they store. A
+    // route's tile list is read by everybody. (Where the activation was there already the launch before may be anybody's, the
+    // weights' writer too: such a product is launched in plain stream order.)
     if (id.tiles) {
+        pdl_wait();
         if (tile_n >= __ldg(id.n_tiles)) return;          // the whole block: nothing is set up yet
         expert = __ldg(id.tiles + 4 * tile_n);
         first = __ldg(id.tiles + 4 * tile_n + 1);
@@ -625,8 +625,8 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
         out_ld = M;
     }
     dim3 grid((unsigned)n_tiles, (unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)ksplit);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(tc::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N, out, out_ld,
-                               part_stride, ctx->error_word, (int)early, tr));
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl && (early || tr.tiles), kern, grid, dim3(tc::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N, out, out_ld,
+                               part_stride, ctx->error_word, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);
