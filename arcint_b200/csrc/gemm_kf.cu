@@ -435,8 +435,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         auto block = [&](uint32_t acc, int gs, int ct, int jj, uint32_t accumulate) {
             const uint32_t a = tmem_base + A_BASE + (uint32_t)((gs * GB + jj) * A_COLS);
             const uint32_t b = sbase + L::CODE_OFF + ct * CODE_STAGE + jj * CODE_BLOCK;
-            umma_ts<true>(leader, acc, a, umma_desc2(b, 128, CODE_GROUP), idesc, accumulate);
-            umma_ts<true>(leader, acc, a + 8, umma_desc2(b + 256, 128, CODE_GROUP), idesc, 1u);
+            umma_ts(leader, acc, a, umma_desc2(b, 128, CODE_GROUP), idesc, accumulate);
+            umma_ts(leader, acc, a + 8, umma_desc2(b + 256, 128, CODE_GROUP), idesc, 1u);
         };
         // the mins term, into the one Y accumulator: the scaling warps have read the last chain's X, and the last super-block's Y with
         // it or before it
@@ -758,7 +758,7 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);
-    count(ctx, ST_GEMM_KQ_MINS);
+    count(ctx, ST_GEMM_KQ_MINS);                            // products with a mins term
     return B200Q_OK;
 }
 

@@ -435,9 +435,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             const f32x2 dw2 = f2_pack(dwb, dwb), negc2 = f2_pack(-12582912.f, -12582912.f);
             const uint32_t dxa = sbase + L::ACT_OFF + st * ACT_CHUNK + SB * OPER_BYTES + (j * BN + cbase) * 4;
             // Sixteen columns at a time, the next sixteen (and their scales) in flight under this chunk's arithmetic; for whole
-            // tiles of the four-bit types the whole slice in one go, which leaves the scheduler of those builds more room:
-            // Q4_0 4096x4096 x 512 80 us in one go, 85 in chunks; Q8_0 12288x3072 x 2048 563 in one go, 532 in chunks; short
-            // tiles are faster in chunks throughout (Q4_0 4096x4096 x 24: 34 and 31).
+            // tiles of the four-bit types the whole slice in one go, which leaves the scheduler of those builds more room. Seven
+            // shapes from 512x1024 x 128 to 12288x3072 x 2048 tokens, one go against chunks: Q4_0 and IQ4_NL 3 to 7 % faster
+            // in all (4096x4096 x 512: 71.9 and 76.0 us, 76.6 and 81.1), Q8_0 3 to 7 % slower in all (75.8 and 71.3). Short
+            // tiles are faster in chunks throughout (Q4_0 4096x4096 x 24: 34 and 31 us).
             constexpr bool ONE_GO = FULL && TYPE != B200Q_TYPE_Q8_0;
             uint32_t v[ONE_GO ? CW / 16 : 2][16];
             f32x2 dxs[2][8];

@@ -1,4 +1,4 @@
-// pdl.cuh -- programmatic dependent launch for the decode chain (quantize -> GEMV -> quantize -> ...).
+// pdl.cuh -- programmatic dependent launch, for the decode chain (quantize -> GEMV -> quantize -> ...) and the prompt products.
 //
 // A decode-width product is a few microseconds of kernel time, so the gap between two kernels in a
 // stream (drain, launch, ramp) is a large part of a token. Launched with the programmatic-serialization
@@ -6,7 +6,8 @@
 // predecessor produces before pdl_wait() (which returns once every prerequisite grid has completed and its
 // writes are visible). The GEMV uses the head start to put its first weight stages in flight -- weights
 // do not depend on the predecessor -- and the quantizer to get its blocks resident. pdl_trigger() lets the
-// next kernel be scheduled: the small quantizers call it first thing, the GEMV when a block has finished its
+// next kernel be scheduled: the small quantizers call it first thing (those of the prompt products after their wait: the GEMM behind
+// them then reads weights that all earlier work has written), the GEMV when a block has finished its
 // rows (triggered at its start, the blocks of later kernels would occupy the places of its own wave: measured
 // 40 % slower). Both calls do nothing in a kernel
 // launched the plain way. Stream capture keeps the edges, so CUDA graphs replay with them.

@@ -153,17 +153,11 @@ __device__ __forceinline__ uint32_t elect_one() {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
     return p;
 }
-// D (+)= A x B^T with A in tensor memory
-template <bool F16>
+// D (+)= A x B^T with A in tensor memory (halves)
 __device__ __forceinline__ void umma_ts(uint32_t leader, uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    if (F16)
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                     "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                     ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
-    else
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                     "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
-                     ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
 // ... and with A in shared memory
 template <bool F16>
