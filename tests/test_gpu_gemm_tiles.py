@@ -115,9 +115,9 @@ def test_sums_at_24_bits(ctx, t, edge):
 
 @pytest.mark.parametrize("t", [A.Q4_K, A.Q5_K])
 @pytest.mark.parametrize("m,n", [(300, 24), (128 * 60, 128 * 4 + 20), (128 * 40, 128 * 4)])
-def test_one_and_more_chains_in_turn(ctx, t, m, n):
-    """Super-blocks that need more than one chain between ones that do not, over several units of a block; a rounding for each
-    addition of a chain and one of the running sum a super-block."""
+def test_more_chains_over_many_units(ctx, t, m, n):
+    """Several chains a super-block over several units of a block, of sums past 2^24 and within it; a rounding of the running sum for
+    each chain."""
     rng = np.random.default_rng(m + n)
     sides = [0, 1, 1, 0, -1, 0, 0, 1, -1]
     w, wi = integer_blocks(t, m, len(sides), rng, 10)
