@@ -32,7 +32,7 @@
 // wait is bounded.
 //
 // B200, quantizer and GEMM together, against two int8 limbs through shared memory and a second kernel for the mins: Q4_K
-// 11008x4096 x 512 tokens 149 -> 80 us, x 24 tokens 53.6 -> 22.4 us, a 512-expert block over 2048 tokens 842 -> 580 us. What is
+// 11008x4096 x 512 tokens 149 -> 79.5 us, x 24 tokens 53.6 -> 22.7 us, a 512-expert block over 2048 tokens 842 -> 573 us. What is
 // left is the chain unpack -> MMA -> scaling (its 1024 clk of MMAs a super-block take some 2700), whose one mins accumulator and
 // two-group operand ring (all of tensor memory) let it overlap only in part. Reading the accumulators in the 32x32b shape, sixteen columns at a
 // time, measured the same on dense products and 2 % slower on the 512-expert block.
