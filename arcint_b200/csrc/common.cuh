@@ -266,6 +266,15 @@ b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
 b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early);
 
+// gemm_t32.cu: its default arm, f16 operands (tr: a route, or null)
+size_t       gemm_t32_act_bytes(int64_t K, int64_t N);
+b200q_status launch_quantize_t32(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute *tr);
+b200q_status launch_gemm_t32(b200q_ctx *ctx, int type, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M, int64_t K,
+                             const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd, bool early, const TileRoute *tr);
+// Threads of a tiled quantizer's block (one column tile, 256 weights; a half-warp a column at a time): enough for two passes over a whole
+// tile. With 256, eight passes of dependent loads, 64 blocks of a 512 x 4096 activation took 12.5 us.
+inline unsigned quantizer_threads(int64_t N, const TileRoute *tr) { return tr && tr->tiles ? 512 : N >= 64 ? 1024 : N >= 32 ? 512 : 256; }
+
 // the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
 
@@ -273,7 +282,7 @@ b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, i
 // on full tiles: a step of 256 weights, and what a unit costs beyond its steps (fill, drain, stores; gemm_tc, one block a unit, sets
 // itself up and allocates tensor memory too). Measured from products of one round, 16 and 43 steps long.
 struct KsplitTimes { int step_ns, unit_ns; };
-constexpr KsplitTimes TC_TIMES = { 3900, 2600 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 };
+constexpr KsplitTimes TC_TIMES = { 1300, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 };
 int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts);
 
 // gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types

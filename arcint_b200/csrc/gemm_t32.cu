@@ -1,0 +1,583 @@
+// gemm_t32.cu -- prefill GEMM for the per-32 types (Q4_0, Q8_0, IQ4_NL) on the tensor cores (tcgen05 kind::f16).
+//
+//   dst[M, N] = W[M, K] (packed GGUF blocks) x X[K, N] (f32), N > 8 tokens
+//
+// ggml's form is kept exactly: the activation is quantized per 32 to int8 with an fp16 scale (block_q8_0), every 32-wide block
+// dot I_b[r, c] is an exact integer, and the result is sum_b I_b * (d_w[r, b] * d_x[c, b]) in f32, b in order. Weight and
+// activation codes are integer-valued halves: every product and partial sum of a block stays far below 2^24, so the f32
+// accumulator of a K = 32 chain of MMAs holds float(I_b). The product of the scales is a matrix of rank one, and it is
+// left to the tensor core, too: one more K = 16 MMA with [d_w, 0 ...] against [d_x, 0 ...] into an accumulator of its own. Both are
+// halves, so the product is exact in f32 (22 bits). What is left per output element and block is one multiply-add of two values
+// that both come out of tensor memory.
+//
+// What bounds it: that multiply-add. 16,384 a block with three register operands each take 192 clk (two 32-bit register reads a
+// clock and lane), with their tensor memory loads 213 when nothing else runs; the MMAs of a block take 192. The form that this one
+// replaced multiplied in the scales from shared memory (two operations and a 16-byte shared load per four elements): 358 clk a block
+// alone, some 950 in the kernel, since the shared-memory port also carried the weight operand. Here the weight operand goes
+// through tensor memory (tcgen05.st into the lanes of its rows).
+//
+// Tensor memory, 512 columns: three buffers of 128 columns (I and S of a 64-column half of the tile), a ring of four operand slots of 32
+// columns (16 of code pairs; d_w with seven zero columns). A JOB is one block and one half of the tile's columns: three MMAs of
+// 64 columns. Three buffers serve the jobs in turn, so one fills while the two scaling warp groups (a half each) drain two.
+// Warp roles: producer, two MMA issuers, one idle; eight unpack warps, one group takes the even and one the odd blocks of a
+// row (a thread = a weight row); eight scaling warps. Persistent blocks walk the units (row tile, column tile, part of K).
+//
+// Every wait on an mbarrier is bounded; a wait that runs out sets an error word, all roles leave their loops, tensor memory is
+// freed and the launch reports B200Q_TIMEOUT at the next synchronize.
+//
+// The reference's int8 GEMM computes the same sum (marfrit/arcint contrib/llama.cpp/patches/
+// 0099-opencl-q4_0-q8_0-int8-gemm.patch:377-455, 583-628: one int8 DPAS per 32 weights, af = fma(float(ir), d_w, af)), with a
+// per-256 activation scale instead of ggml's per-32 one.
+#include <cuda.h>
+
+#include "formats.cuh"
+#include "common.cuh"
+#include "pdl.cuh"
+#include "tc_common.cuh"
+
+namespace b200q {
+
+namespace t32 {
+
+using namespace tc;
+
+constexpr int BM = 128, BN = 128, SB = 8;                 // rows and tokens of a tile, blocks of a raw stage (256 weights a row)
+constexpr int HB = 4;                                     // blocks of an activation stage
+constexpr int NBUF = 3;                                   // accumulator buffers (I and S, 64 columns each)
+constexpr int NSLOT = 4, SLOT_COLS = 32, A_BASE = NBUF * BN;
+static_assert(A_BASE + NSLOT * SLOT_COLS <= 512, "tensor memory");
+constexpr int NRAW = 2;
+constexpr int THREADS = 32 * 20;                          // warp groups: {producer, 2 x MMA, idle}, 2 x unpack, 2 x scale
+// Registers per thread by role (setmaxnreg): a warp group that asks for more waits until others have
+// given theirs back, so the sum must fit the pool the launch allocated (THREADS x LAUNCH_REGS).
+constexpr int LAUNCH_REGS = (65536 / THREADS) / 8 * 8;
+static_assert(128 * 40 + 256 * 72 + 256 * 144 <= THREADS * LAUNCH_REGS, "register pool: 40 control, 72 unpack, 144 scale");
+
+// The activation of a (column tile, 128 weights), by groups of eight columns, so that a tile with few columns (a route tile of a
+// small expert) is a short prefix:
+//   group g < 16: codes [block j < 4][piece c < 4][column r < 8][8 codes as halves, each run of four in the order 0 2 1 3, in which the
+//                 unpack threads mask nibbles out of a word], then [block j < 4][column r < 8][d_x and seven zeros as halves], then
+//                 eight times sixteen zero bytes, the upper half of K of every scale MMA
+constexpr int CODE_BLOCK = 512, GROUP_SCALES = HB * CODE_BLOCK, GROUP_ZERO = GROUP_SCALES + HB * 128;
+constexpr int GROUP = GROUP_ZERO + 128, STAGE = (BN / 8) * GROUP;         // 2688, 43008 bytes
+
+template <int TYPE> struct Fmt;                           // bytes of a block, activation stages in flight
+template <> struct Fmt<B200Q_TYPE_Q4_0>   { enum { BB = 18, NACT = 4 }; };
+template <> struct Fmt<B200Q_TYPE_IQ4_NL> { enum { BB = 18, NACT = 4 }; };
+template <> struct Fmt<B200Q_TYPE_Q8_0>   { enum { BB = 34, NACT = 3 }; };
+
+template <int TYPE> struct Smem {
+    enum {
+        NACT = Fmt<TYPE>::NACT, ROW = SB * Fmt<TYPE>::BB, RAW_STAGE = BM * ROW,
+        RAW_OFF = 0,
+        ACT_OFF = RAW_OFF + NRAW * RAW_STAGE,
+        BAR_OFF = ACT_OFF + NACT * STAGE,
+        TOTAL = BAR_OFF + 8 * 64
+    };
+    static_assert(TOTAL <= 227 * 1024 - 256, "shared memory budget");
+    static_assert(RAW_STAGE % 128 == 0 && STAGE % 128 == 0, "tiled copies");
+};
+
+// BAR_READY, BAR_FULL: a barrier per job of an activation stage (four blocks x two halves). READY: the block's operand is in its slot (four
+// arrivals) and the accumulator buffer's last job, three back, has been read (four arrivals); FULL: the MMAs are done, which
+// also frees the operand's half. Every waiting role sees each phase of each of its barriers.
+enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 2, BAR_ACT_FULL = 4, BAR_ACT_EMPTY = 8, BAR_READY = 12, BAR_FULL = 20, BAR_COUNT = 28 };
+static_assert(NRAW == 2 && NSLOT == HB && BAR_COUNT <= 64, "barrier slots above");
+
+constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
+
+template <bool GATE>
+__global__ void __launch_bounds__(1024)
+quantize_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
+                int64_t N, uint8_t *__restrict__ out, TileRoute id) {
+    // One block per (tile, 256 weights); a half-warp per column at a time: its sixteen lanes read the column's 256
+    // floats as one contiguous kilobyte (lane l: k = 16 l .. 16 l + 15, i.e. half l & 1 of block l >> 1), the two
+    // lanes of a block share their maximum by one shuffle, and every lane stores its 16 codes as two pieces. Columns of groups
+    // past the tile's last one are never fetched by the GEMM and are skipped; the dead columns of the last live group are
+    // written as zeros.
+    pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
+    pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
+    const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
+    const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
+    uint8_t *stage = out + ((size_t)t * nst + s) * (2 * STAGE);
+    int cnt, first = 0;
+    if (id.tiles) {
+        // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
+        if (t >= __ldg(id.n_tiles)) return;
+        first = __ldg(id.tiles + 4 * t + 1);
+        cnt = __ldg(id.tiles + 4 * t + 2);
+    } else {
+        const int64_t left = N - (int64_t)t * BN;
+        cnt = left < BN ? (int)left : BN;
+    }
+    const int live = ((cnt + 7) >> 3) << 3, j = l >> 1;
+    for (int i = threadIdx.x; i < 2 * live; i += blockDim.x)
+        *reinterpret_cast<uint4 *>(stage + (i & 1) * STAGE + (i >> 4) * GROUP + GROUP_ZERO + ((i >> 1) & 7) * 16) = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+    for (int col = hw; col < live; col += blockDim.x >> 4) {
+        const float *x = nullptr;
+        if (col < cnt) {
+            if (id.tiles) {
+                const int p = __ldg(id.pairs + first + col), tok = p / id.n_used, slot = p - tok * id.n_used;
+                x = reinterpret_cast<const float *>(base + (size_t)(slot % id.ne11) * id.nb1 + (size_t)tok * id.nb2);
+            } else {
+                const int64_t n = (int64_t)t * BN + col;
+                const int64_t c1 = n % ne1, c23 = n / ne1, c2 = c23 % ne2, c3 = c23 / ne2;
+                x = reinterpret_cast<const float *>(base + c1 * nb1 + c2 * nb2 + c3 * nb3);
+            }
+            x += (int64_t)s * 256 + 16 * l;
+        }
+        float4 v[4];
+        float amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = x ? *reinterpret_cast<const float4 *>(x + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (GATE && x) v[i] = swiglu4(*reinterpret_cast<const float4 *>(x + id.gate + 4 * i), v[i]);
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+        }
+        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+        const float d = __fdiv_rn(amax, 127.f);
+        const float inv = d != 0.f ? __fdiv_rn(1.f, d) : 0.f;
+        uint8_t *grp = stage + (j >> 2) * STAGE + (col >> 3) * GROUP;
+        __align__(16) __half2 w[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[2 * i] = __floats2half2_rn(roundf(__fmul_rn(v[i].x, inv)), roundf(__fmul_rn(v[i].z, inv)));
+            w[2 * i + 1] = __floats2half2_rn(roundf(__fmul_rn(v[i].y, inv)), roundf(__fmul_rn(v[i].w, inv)));
+        }
+        uint8_t *o = grp + (j & 3) * CODE_BLOCK + (col & 7) * 16;
+        *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * 128) = *reinterpret_cast<const uint4 *>(w);
+        *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * 128) = *reinterpret_cast<const uint4 *>(w + 4);
+        if ((l & 1) == 0)
+            *reinterpret_cast<uint4 *>(grp + GROUP_SCALES + (j & 3) * 128 + (col & 7) * 16) = make_uint4(__half_as_ushort(__float2half_rn(d)), 0, 0, 0);
+    }
+}
+
+__device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
+    const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b), *reinterpret_cast<const __half2 *>(&c));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+// four signed bytes as halves, bytes 0 and 2, then 1 and 3: a byte b ^ 0x80 = b + 128 becomes the half 0x6400 | b = 1024 + b + 128
+__device__ __forceinline__ void signed_bytes_to_halves(uint32_t b, uint32_t &h02, uint32_t &h13) {
+    b ^= 0x80808080u;
+    h02 = h2_sub(__byte_perm(b, 0x64646464u, 0x4240), 0x64806480u);
+    h13 = h2_sub(__byte_perm(b, 0x64646464u, 0x4341), 0x64806480u);
+}
+
+// the 32-bit word at an even compile-time byte offset of a register array
+template <int N> __device__ __forceinline__ uint32_t word_at(const uint32_t (&w)[N], int byte_off) {
+    const int i = byte_off >> 2;
+    return (byte_off & 3) == 0 ? w[i] : __funnelshift_r(w[i], w[i + 1 < N ? i + 1 : i], 16);
+}
+
+// Block J of the row's raw stage as an operand: sixteen pairs of halves in the K order of the activation codes, and the scale.
+// Blocks are 18 or 34 bytes long: block J begins 2 J bytes into the 16-byte unit J or 2 J, and ends in the next or the one after.
+template <int TYPE, int J>
+__device__ __forceinline__ void unpack_block(const uint8_t *row, uint32_t (&h)[16], uint32_t &d) {
+    constexpr bool Q8 = TYPE == B200Q_TYPE_Q8_0;
+    constexpr int UNITS = Q8 ? 3 : 2, FIRST = Q8 ? 2 * J : J, OFF = 2 * J;
+    uint32_t w[4 * UNITS];
+#pragma unroll
+    for (int i = 0; i < UNITS; ++i) {
+        const uint4 t = *reinterpret_cast<const uint4 *>(row + 16 * (FIRST + i));
+        w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
+    }
+    d = (OFF & 2) ? w[OFF >> 2] >> 16 : w[OFF >> 2] & 0xFFFFu;
+    if constexpr (Q8) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) signed_bytes_to_halves(word_at(w, OFF + 2 + 4 * i), h[2 * i], h[2 * i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t q = word_at(w, OFF + 2 + 4 * i);
+            if (TYPE == B200Q_TYPE_IQ4_NL) {
+                // the nibbles index kvalues_iq4nl (signed bytes, |v| <= 127: exact halves)
+                signed_bytes_to_halves(iq4nl_lookup4(q & 0x0F0F0F0Fu), h[2 * i], h[2 * i + 1]);
+                signed_bytes_to_halves(iq4nl_lookup4((q >> 4) & 0x0F0F0F0Fu), h[8 + 2 * i], h[8 + 2 * i + 1]);
+            } else {
+                // 1024 + n or 1024 + 16 n is a bit pattern; n - 8 is exact either way
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {                                       // bytes 0 and 2 of the word, then 1 and 3
+                    const uint32_t b = o ? q >> 8 : q;
+                    h[2 * i + o] = h2_sub((b & 0x000F000Fu) | 0x64006400u, 0x64086408u);
+                    h[8 + 2 * i + o] = h2_fma((b & 0x00F000F0u) | 0x64006400u, 0x2C002C00u, 0xD480D480u);      // x / 16 - 72
+                }
+            }
+        }
+    }
+}
+
+// One unit of work: a 128-row x 128-column output tile over the 256-weight stages [sb0, sb1). Dense: tile_n-th run of 128
+// tokens; MUL_MAT_ID: route tile tile_n (one expert, up to 128 routed pairs).
+struct Unit {
+    int tile_n, row0, valid_rows, expert, first, ncols, sb0, sb1, part, cw;      // cw: columns of a half
+};
+
+// Builds by what the column tiles are: whole tiles of a dense product (no branch on the columns that are live), tiles of a dense product
+// with a ragged end, tiles of a route
+enum { COLS_FULL = 0, COLS_RAGGED = 1, COLS_ROUTE = 2 };
+template <int TYPE, int COLS>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
+                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
+                int *__restrict__ error_word, TileRoute id) {
+    typedef Smem<TYPE> L;
+    constexpr bool FULL = COLS == COLS_FULL, ROUTE = COLS == COLS_ROUTE;
+    constexpr int NACT = L::NACT;
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler, too)
+    const int nsb = K / 256;                    // raw stages of a row
+    const uint32_t sbase = smem_u32(smem);
+    const uint32_t bars = sbase + L::BAR_OFF;
+    auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+    // The block is persistent: it walks the units blockIdx.x, blockIdx.x + gridDim.x, ... and every role
+    // keeps running counters for its rings, so the pipeline never drains between units. Units of one row tile are neighbours, so
+    // blocks running together share weight rows in L2 (MUL_MAT_ID: the tiles of one expert).
+    // Launched with programmatic dependence behind this product's own quantizer, which has waited for what came before it: a block may
+    // read the weights at once, the producer waits before its first activation load, the scaling warps before they store. A
+    // route's tile list is read by everybody. (Where the activation was there already the launch before may be anybody's, the
+    // weights' writer too: such a product is launched in plain stream order.)
+    if (ROUTE) pdl_wait();
+    const int tiles_m = (M + BM - 1) / BM;
+    const int tiles_n = ROUTE ? __ldg(id.n_tiles) : n_tiles_dense;
+    const int n_units = tiles_m * tiles_n * ksplit;
+    auto unit_of = [&](int u) {
+        Unit U;
+        U.part = u % ksplit;
+        U.sb0 = U.part * nsb / ksplit;
+        U.sb1 = (U.part + 1) * nsb / ksplit;
+        u /= ksplit;
+        U.tile_n = u % tiles_n;
+        U.row0 = (u / tiles_n) * BM;
+        U.valid_rows = min(BM, M - U.row0);
+        U.expert = 0;
+        U.first = 0;
+        U.ncols = min(BN, N - U.tile_n * BN);
+        if (ROUTE) {
+            U.expert = __ldg(id.tiles + 4 * U.tile_n);
+            U.first = __ldg(id.tiles + 4 * U.tile_n + 1);
+            U.ncols = __ldg(id.tiles + 4 * U.tile_n + 2);
+        }
+        // 64 columns for a full tile; for a short one (the ragged end, a route tile of a small expert) half of what
+        // there is, in steps of 16
+        U.cw = FULL || U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
+        return U;
+    };
+    if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < NRAW; ++i) {
+            mbar_init(bar(BAR_RAW_FULL + i), 1);
+            mbar_init(bar(BAR_RAW_EMPTY + i), 8);                  // unpack warps
+        }
+        for (int i = 0; i < NACT; ++i) {
+            mbar_init(bar(BAR_ACT_FULL + i), 1);
+            mbar_init(bar(BAR_ACT_EMPTY + i), 2);                  // both MMA issuers' commits
+        }
+        for (int i = 0; i < 2 * HB; ++i) {
+            mbar_init(bar(BAR_READY + i), 4 + 4);                  // the warps of an unpack group and of a scaling group
+            mbar_init(bar(BAR_FULL + i), 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_slot, 0);
+    volatile int *abortp = &abort_flag;
+    PROF_DECL
+
+    if (warp == 0) {
+        // ---- producer ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;" ::: "memory");
+        if (lane == 0) tma_prefetch_desc(&wmap);
+        int s_run = 0;                                    // raw stages fetched so far
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * (2 * STAGE);
+            // only the column groups the tile has; the MMAs still read a multiple of sixteen columns, the rest of the
+            // stage holds older codes whose products land in accumulator columns nobody stores
+            const uint32_t bytes = (uint32_t)((U.ncols + 7) >> 3) * GROUP;
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int st = s_run % NRAW;
+                if (!WAITP(1, bar(BAR_RAW_EMPTY + st), ((s_run / NRAW) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    // the stage's [128 rows x 256 weights] box in one tiled copy; rows past M arrive as zeros
+                    mbar_expect_tx(bar(BAR_RAW_FULL + st), L::RAW_STAGE);
+                    tma_load_3d(sbase + L::RAW_OFF + st * L::RAW_STAGE, &wmap, s * (L::ROW / 4), U.row0, U.expert, bar(BAR_RAW_FULL + st));
+                }
+                if (s_run == 0) pdl_wait();
+                for (int h = 0; h < 2; ++h) {
+                    const int c_run = 2 * s_run + h, at = c_run % NACT;
+                    if (!WAITP(3, bar(BAR_ACT_EMPTY + at), ((c_run / NACT) & 1) ^ 1)) { ok = false; break; }
+                    if (lane == 0) {
+                        mbar_expect_tx(bar(BAR_ACT_FULL + at), bytes);
+                        bulk_g2s(sbase + L::ACT_OFF + at * STAGE, act_tile + (size_t)(2 * s + h) * STAGE, bytes, bar(BAR_ACT_FULL + at));
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp <= 2) {
+        // ---- MMA issuers, one for each half of the columns: the waits and the issue of a job are a serial chain ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;" ::: "memory");
+        const uint32_t leader = elect_one();
+        const int h = warp - 1;
+        int c_run = 0, buf = h;                           // activation stages so far; the job's buffer
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            // N: the half's live columns, in sixteens (a half without any still takes its turn, with sixteen)
+            const uint32_t idesc = IDESC | ((uint32_t)((max(1, min(U.cw, U.ncols - h * U.cw)) + 15) >> 4) << 18);
+            const uint32_t half_off = (uint32_t)(h * (U.cw >> 3)) * GROUP;
+            for (int c = 2 * U.sb0; c < 2 * U.sb1 && ok; ++c, ++c_run) {
+                const int at = c_run % NACT;
+                if (!WAITP(2, bar(BAR_ACT_FULL + at), (c_run / NACT) & 1)) { ok = false; break; }
+                const uint32_t stage = sbase + L::ACT_OFF + at * STAGE + half_off;
+#pragma unroll
+                for (int jj = 0; jj < HB; ++jj) {
+                    const uint32_t a = tmem_base + A_BASE + jj * SLOT_COLS;          // (a block's slot is its place in the stage)
+                    if (!WAITP(4, bar(BAR_READY + 2 * jj + h), c_run & 1)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t acc = tmem_base + (uint32_t)buf * BN, b = stage + jj * CODE_BLOCK, bs = stage + GROUP_SCALES + jj * 128;
+                    // K = 16 per MMA: eight columns of A, two pieces of B
+                    umma_ts(leader, acc, a, umma_desc2(b, 128, GROUP), idesc, 0u);
+                    umma_ts(leader, acc, a + 8, umma_desc2(b + 256, 128, GROUP), idesc, 1u);
+                    umma_ts(leader, acc + 64, a + 16, umma_desc2(bs, GROUP_ZERO - GROUP_SCALES - jj * 128, GROUP), idesc, 0u);
+                    tc_commit_one(leader, bar(BAR_FULL + 2 * jj + h));
+                    buf = buf == 0 ? 2 : buf - 1;                                    // two jobs on, modulo three
+                }
+                if (ok) tc_commit_one(leader, bar(BAR_ACT_EMPTY + at));
+            }
+        }
+    } else if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;" ::: "memory");
+    } else if (warp < 12) {
+        // ---- unpack: a thread per weight row, even blocks by the first group and odd ones by the second ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
+        const int r = (warp & 3) * 32 + lane;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + A_BASE;
+        auto rows = [&](auto parity) {
+            constexpr int P = decltype(parity)::value;
+            // the scale operand's zero columns, once
+            tmem_st16_const(ta + P * SLOT_COLS + 16, 0u);
+            tmem_st16_const(ta + (P + 2) * SLOT_COLS + 16, 0u);
+            int s_run = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+                const Unit U = unit_of(u);
+                for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                    const int st = s_run % NRAW;
+                    if (!WAITP(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1)) { ok = false; break; }
+                    const uint8_t *row = smem + L::RAW_OFF + st * L::RAW_STAGE + r * L::ROW;
+                    auto one = [&](auto jc) {
+                        constexpr int J = decltype(jc)::value, SLOT = J % NSLOT;
+                        uint32_t h[16], d;
+                        unpack_block<TYPE, J>(row, h, d);
+                        // the slot's last block has been multiplied, by both halves
+                        if (!ok || !WAITP(5, bar(BAR_FULL + 2 * SLOT), (J / NSLOT) ^ 1) || !WAITP(5, bar(BAR_FULL + 2 * SLOT + 1), (J / NSLOT) ^ 1)) {
+                            ok = false;
+                            return;
+                        }
+                        tc_fence_after();
+                        tmem_st16(ta + SLOT * SLOT_COLS, h);
+                        tmem_st1(ta + SLOT * SLOT_COLS + 16, d);
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane < 2) mbar_arrive(bar(BAR_READY + 2 * SLOT + lane));
+                    };
+                    one(Int<P>());
+                    one(Int<P + 2>());
+                    one(Int<P + 4>());
+                    one(Int<P + 6>());
+                    if (ok) mbar_arrive_warp(bar(BAR_RAW_EMPTY + st), lane);
+                }
+            }
+        };
+        if (warp < 8) rows(Int<0>());
+        else rows(Int<1>());
+    } else {
+        // ---- scale: a warp group per half of the tile's columns, a thread a row ----
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 144;" ::: "memory");
+        const int q4 = warp & 3, half = (warp - 12) >> 2, r = q4 * 32 + lane;
+        const uint32_t tq = tmem_base + ((uint32_t)(q4 * 32) << 16);
+        // the buffers of jobs 0, 1 and 2 are free: half 1 says so for 0 and 2, half 0 for 1
+        if (lane == 0) mbar_arrive(bar(BAR_READY + 1 - half));
+        if (lane == 0 && half == 1) mbar_arrive(bar(BAR_READY + 2));
+        int buf = half, b_run = 0;                        // (b_run: blocks so far; a unit has a multiple of eight)
+        pdl_wait();
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
+            f32x2 acc2[32];                                    // column pairs
+#pragma unroll
+            for (int c = 0; c < 32; ++c) acc2[c] = 0ull;
+            for (int b = U.sb0 * SB; b < U.sb1 * SB; ++b, ++b_run) {
+                const int job = (2 * b + half) & 7;
+                if (!WAITP(6, bar(BAR_FULL + job), (b_run >> 2) & 1)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t ti = tq + (uint32_t)buf * BN;
+                // sixteen columns at a time, the next sixteen in flight under this chunk's arithmetic
+                uint32_t vi[2][16], vs[2][16];
+                auto fetch = [&](int q) {
+                    tmem_ld16(ti + q * 16, vi[q & 1]);
+                    tmem_ld16(ti + 64 + q * 16, vs[q & 1]);
+                };
+                auto release = [&]() {                             // the buffer is free for the job three on
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(BAR_READY + ((job + 3) & 7)), lane);
+                };
+                if (FULL || ncol > 0) fetch(0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (FULL || q * 16 < ncol) {
+                        tmem_ld_wait();
+                        if (q < 3 && (FULL || q * 16 + 16 < ncol)) fetch(q + 1);
+                        if (FULL && q == 3) release();
+#pragma unroll
+                        for (int c = 0; c < 16; c += 2)
+                            acc2[q * 8 + c / 2] = f2_fma(f2_pack(__uint_as_float(vi[q & 1][c]), __uint_as_float(vi[q & 1][c + 1])),
+                                                         f2_pack(__uint_as_float(vs[q & 1][c]), __uint_as_float(vs[q & 1][c + 1])), acc2[q * 8 + c / 2]);
+                    }
+                }
+                if (!FULL) release();
+                buf = buf == 0 ? 2 : buf - 1;
+            }
+            if (!ok) break;
+            const bool row_ok = r < U.valid_rows;
+            if (ROUTE) {
+                // where the warp's columns go: every lane looks up two of them (loads in flight together), the
+                // store loop takes them by shuffle
+                long long off[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    off[h] = 0;
+                    if (lane + 32 * h < ncol) {
+                        const int p = __ldg(id.pairs + U.first + cbase + lane + 32 * h), tok = p / id.n_used, slot = p - tok * id.n_used;
+                        off[h] = tok * id.ld2 + slot * id.ld1;
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 64; c += 2) {
+                    float a[2];
+                    f2_unpack(acc2[c / 2], a[0], a[1]);
+#pragma unroll
+                    for (int d = 0; d < 2; ++d) {
+                        const long long o = __shfl_sync(0xFFFFFFFFu, off[(c + d) >> 5], (c + d) & 31);
+                        if (row_ok && c + d < ncol) dst[o + U.row0 + r] = a[d];
+                    }
+                }
+            } else if (row_ok) {
+                float *o = dst + (int64_t)U.part * part_stride + (int64_t)(U.tile_n * BN + cbase) * ldd + U.row0 + r;
+#pragma unroll
+                for (int c = 0; c < 64; c += 2) {
+                    float a0, a1;
+                    f2_unpack(acc2[c / 2], a0, a1);
+                    if (FULL || c < ncol) *o = a0;
+                    if (FULL || c + 1 < ncol) o[ldd] = a1;
+                    o += 2 * ldd;
+                }
+            }
+        }
+    }
+
+    PROF_DUMP(warp == 0 ? "prod" : warp <= 2 ? "mma " : warp < 4 ? "idle" : warp < 12 ? "unpk" : "epi ")
+    tc_fence_before();
+    __syncthreads();
+    pdl_trigger();
+    if (abort_flag) {
+        // a wait ran out: give copies still in flight time to land before the block's shared
+        // memory is released, and tell the host
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        if (threadIdx.x == 0) atomicExch(error_word, 1);
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
+}  // namespace t32
+
+static const TileRoute NO_ROUTE_T32 = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
+
+size_t gemm_t32_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + t32::BN - 1) / t32::BN) * (K / 256)) * (2 * t32::STAGE); }
+
+// n_tiles: the column tiles; tr: a route (n_tiles its upper bound), or null
+b200q_status launch_quantize_t32(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute *tr) {
+    const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
+    const TileRoute &id = tr ? *tr : NO_ROUTE_T32;
+    dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, id.gate ? t32::quantize_kernel<true> : t32::quantize_kernel<false>, grid, dim3(quantizer_threads(N, tr)), 0, ctx->stream,
+                               (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, id));
+    B200Q_CUDA(ctx, cudaGetLastError());
+    count(ctx, ST_GEMM_TC_QUANT);
+    return B200Q_OK;
+}
+
+template <int TYPE>
+static b200q_status launch_t32_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
+                                 int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
+                                 bool early, const TileRoute &tr) {
+    typedef t32::Smem<TYPE> L;
+    const int cols = tr.tiles ? t32::COLS_ROUTE : N % t32::BN == 0 ? t32::COLS_FULL : t32::COLS_RAGGED;
+    auto kern = cols == t32::COLS_ROUTE ? t32::gemm_t32_kernel<TYPE, t32::COLS_ROUTE>
+              : cols == t32::COLS_FULL  ? t32::gemm_t32_kernel<TYPE, t32::COLS_FULL> : t32::gemm_t32_kernel<TYPE, t32::COLS_RAGGED>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES][3] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][cols];
+    if (!attr_set) {
+        B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
+        attr_set = true;
+    }
+    CUtensorMap wmap;
+    b200q_status st = make_weight_tmap3(ctx, &wmap, w, row_stride, M, (K / 32) * t32::Fmt<TYPE>::BB, L::ROW, n_mat, mat_stride);
+    if (st != B200Q_OK) return st;
+    // persistent blocks, one per SM, walking the (row tile, column tile, part of K) units; parts write their own scratch and a
+    // second kernel adds them in a fixed order, so the result does not depend on which block finishes first
+    const int64_t tiles = n_tiles * ((M + t32::BM - 1) / t32::BM), S = ctx->sm_count;
+    float *out = dst, *parts = nullptr;
+    const int ksplit = tr.tiles ? 1 : plan_ksplit(ctx, tiles, K / 256, TC_TIMES, M, N, &parts);
+    int64_t out_ld = ldd, part_stride = 0;
+    if (ksplit > 1) {
+        out = parts;
+        part_stride = N * M;
+        out_ld = M;
+    }
+    const int64_t units = tiles * ksplit;
+    const unsigned grid = (unsigned)(units < S ? units : S);
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl && (early || tr.tiles), kern, dim3(grid), dim3(t32::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr));
+    B200Q_CUDA(ctx, cudaGetLastError());
+    if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
+    count(ctx, ST_GEMM_TC);
+    count(ctx, ST_GEMM_TC_F16);
+    return B200Q_OK;
+}
+
+// n_tiles: the column tiles (dense: of N; MUL_MAT_ID: the upper bound of the route's tile count, blocks past the
+// device-side count leave at once)
+b200q_status launch_gemm_t32(b200q_ctx *ctx, int type, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M, int64_t K,
+                             const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd, bool early, const TileRoute *tr) {
+    const TileRoute &id = tr ? *tr : NO_ROUTE_T32;
+    if (type == B200Q_TYPE_Q4_0) return launch_t32_t<B200Q_TYPE_Q4_0>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, id);
+    if (type == B200Q_TYPE_Q8_0) return launch_t32_t<B200Q_TYPE_Q8_0>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, id);
+    if (type == B200Q_TYPE_IQ4_NL) return launch_t32_t<B200Q_TYPE_IQ4_NL>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, id);
+    return fail(ctx, B200Q_UNSUPPORTED, "gemm_t32: type %d", type);
+}
+
+}  // namespace b200q

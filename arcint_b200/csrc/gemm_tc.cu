@@ -1,4 +1,5 @@
-// gemm_tc.cu -- prefill GEMM for the per-32 types (Q4_0, Q8_0, IQ4_NL) on the 5th-generation tensor cores.
+// gemm_tc.cu -- prefill GEMM for the per-32 types (Q4_0, Q8_0, IQ4_NL): the entries, and the int8 arm (B200Q_TC_I8=1); the default arm,
+// on f16 operands, is gemm_t32.cu.
 //
 //   dst[M, N] = W[M, K] (packed GGUF blocks) x X[K, N] (f32), N > 8 tokens
 //
@@ -15,21 +16,18 @@
 //   warp 0      producer: bulk copies (cp.async.bulk + mbarrier complete_tx) of the raw
 //               packed weight rows of a k-stage (256 weights per row) and of the
 //               activation chunk (int8 codes already in the tensor core's K-major core-matrix
-//               order, plus their scales), three stages deep;
+//               order, plus their scales), two or three stages deep;
 //   warp 1      allocates tensor memory, issues the MMAs (one elected thread) and commits
 //               them to mbarriers;
 //   warps 4..7  one thread per weight row: unpack the row's blocks to int8 (code - 8) into
-//               the A-operand ring in core-matrix order and publish the block's fp16 scale;
+//               the A-operand ring in core-matrix order;
 //   warps 8..   scale-accumulate, NW warps per tensor-memory lane quarter: pull the finished
 //               block accumulator out of tensor memory (tcgen05.ld), free it, convert, scale by
 //               d_w * d_x and accumulate into f32 registers (thread = row x 128/NW columns).
 // Four 128-column accumulators fill the 512 tensor-memory columns, so the MMA of block b+1..
 // b+3 runs while block b is being scaled. Whole column tiles have a build of their own (FULL) without a branch on which
-// columns are live: with such branches in the scaling loop, never taken, Q8_0 12288x3072 x 2048 measured 684 us against 563.
-// Putting the weight operand into tensor memory (tcgen05.st, three accumulators left) and reading the accumulators in the 16x256b
-// shape (a quarter of the scale loads) were built and measured 2 to 10 % slower. The scaling is the bound, not the tensor pipe:
-// every output element needs a convert, a multiply and a fused multiply-add per 32 of K,
-// 16K elements per block against 128 FP32 lanes per SM and clock.
+// columns are live. The scaling is the bound, not the tensor pipe: every output element needs a convert, a multiply and a fused
+// multiply-add per 32 of K, and a share of the loads of the scales from shared memory.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets an error word, all roles
 // leave their loops, tensor memory is freed and the launch reports B200Q_TIMEOUT at the
@@ -50,13 +48,9 @@ constexpr int BN = 128;            // tokens per tile (MMA N, tensor-memory colu
 constexpr int KB = 32;             // weights per MMA (one quantization block)
 constexpr int SB = 8;              // blocks per k-stage (256 weights)
 constexpr int NACC = 4;            // accumulators in tensor memory (4 x 128 = 512 columns)
-// One operand block (128 rows or columns x 32 k) is 4096 B as int8 and 8192 B as fp16; both are K-major
-// core matrices (8 rows x 16 bytes) with the 16-byte K pieces LBO apart: two pieces per block as int8,
-// four as fp16 (an fp16 MMA covers K = 16, so a block is two of them).
-template <bool F16> struct Oper {
-    enum { BYTES = BM * KB * (F16 ? 2 : 1),
-           ACT_CHUNK = SB * BYTES + SB * BN * 4 };          // codes + f32 scales of a stage: 36864 / 69632 B
-};
+// One operand block (128 rows or columns x 32 k): K-major core matrices (8 rows x 16 bytes), its two 16-byte K pieces LBO apart.
+constexpr int OPER_BYTES = BM * KB;                       // 4096
+constexpr int ACT_CHUNK = SB * OPER_BYTES + SB * BN * 4;  // codes + f32 scales of a stage: 36864 B
 constexpr int NW = 2;              // scale-accumulate warps per tensor-memory lane quarter (4 measured no faster)
 constexpr int THREADS = 32 * (8 + 4 * NW);   // warp groups: {producer, MMA, 2 idle}, unpack, NW x scale-accumulate
 // Registers per thread by role (setmaxnreg). The launch gives every thread LAUNCH_REGS; a warp group that
@@ -71,52 +65,45 @@ static_assert(REGS_CTRL <= LAUNCH_REGS && REGS_UNPACK <= LAUNCH_REGS && REGS_SCA
 
 
 template <int TYPE> struct Raw;     // packed bytes of one row per stage
-template <> struct Raw<B200Q_TYPE_Q4_0> { enum { ROW = SB * 18, NSTAGE = 3, A_SLOTS_F16 = 4 }; };     // 144 B per row and stage
-template <> struct Raw<B200Q_TYPE_Q8_0> { enum { ROW = SB * 34, NSTAGE = 2, A_SLOTS_F16 = 2 }; };     // 272 B: two stages fit
-template <> struct Raw<B200Q_TYPE_IQ4_NL> { enum { ROW = SB * 18, NSTAGE = 3, A_SLOTS_F16 = 4 }; };   // Q4_0's block
+template <> struct Raw<B200Q_TYPE_Q4_0> { enum { ROW = SB * 18, NSTAGE = 3 }; };     // 144 B per row and stage
+template <> struct Raw<B200Q_TYPE_Q8_0> { enum { ROW = SB * 34, NSTAGE = 2 }; };     // 272 B: two stages fit
+template <> struct Raw<B200Q_TYPE_IQ4_NL> { enum { ROW = SB * 18, NSTAGE = 3 }; };   // Q4_0's block
 
-template <int TYPE, bool F16> struct Smem {
+template <int TYPE> struct Smem {
     enum {
-        NSTAGE = F16 ? 2 : Raw<TYPE>::NSTAGE,     // raw-weight / activation stages in flight
-        A_SLOTS = F16 ? Raw<TYPE>::A_SLOTS_F16 : SB,      // unpacked A operand blocks in flight
+        NSTAGE = Raw<TYPE>::NSTAGE,     // raw-weight / activation stages in flight
+        A_SLOTS = SB,      // unpacked A operand blocks in flight
         RAW_STAGE = BM * Raw<TYPE>::ROW,
         RAW_OFF = 0,
         ACT_OFF = RAW_OFF + NSTAGE * RAW_STAGE,
-        A_OFF = ACT_OFF + NSTAGE * Oper<F16>::ACT_CHUNK,
-        BAR_OFF = A_OFF + A_SLOTS * Oper<F16>::BYTES,
+        A_OFF = ACT_OFF + NSTAGE * ACT_CHUNK,
+        BAR_OFF = A_OFF + A_SLOTS * OPER_BYTES,
         TOTAL = BAR_OFF + 8 * 64             // room for up to 64 mbarriers (BAR_COUNT of them are used)
     };
 };
-static_assert(Smem<B200Q_TYPE_Q4_0, true>::TOTAL <= 227 * 1024 && Smem<B200Q_TYPE_Q8_0, true>::TOTAL <= 227 * 1024, "shared memory");
+static_assert(Smem<B200Q_TYPE_Q4_0>::TOTAL <= 227 * 1024 && Smem<B200Q_TYPE_Q8_0>::TOTAL <= 227 * 1024, "shared memory");
 
 constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);          // without the N field
-// fp16 operands, f32 accumulator: integer-valued halves (|v| <= 255) multiply and add exactly (every
-// partial sum of a 32-block stays far below 2^24), so the accumulator holds float(I_b) with the bits the
-// int8 MMA's result would convert to -- without the conversion
-constexpr uint32_t IDESC_F16 = (1u << 4) | ((uint32_t)(BM >> 4) << 24);
-
 // barrier slots inside the shared block
 enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_ACT_FULL = 6, BAR_ACT_EMPTY = 9, BAR_A_FULL = 12, BAR_A_EMPTY = 20,
        BAR_ACC_FULL = 28, BAR_ACC_EMPTY = 32, BAR_COUNT = 36 };
 static_assert(BAR_COUNT <= 64, "the shared block reserves 64 mbarrier slots");
 
 // Activation chunk (n-tile t, k-stage s) in global memory, written by quantize_tiled_kernel:
-//   codes  [block j < 8][piece c][group g < 16][column r < 8][16 bytes]   column 8g + r; int8: two pieces of 16 k
-//          (k = 32j + 16c + byte), fp16: four pieces of 8 k (k = 32j + 8c + half), the codes as exact halves
+//   codes  [block j < 8][piece c < 2][group g < 16][column r < 8][16 bytes]   column 8g + r, k = 32j + 16c + byte
 //   scales [block j < 8][column < 128] f32 (the fp16-rounded block scale)
-template <bool F16, bool GATE>
+template <bool GATE>
 __global__ void __launch_bounds__(256)
 quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
                       int64_t N, uint8_t *__restrict__ out, TileRoute id) {
     // One block per (tile, k-stage of 256); a half-warp per column at a time: its sixteen lanes read the column's 256
     // floats as one contiguous kilobyte (lane l: k = 16 l .. 16 l + 15, i.e. half l & 1 of block j = l >> 1), the two
-    // lanes of a block share their maximum by one shuffle, and every lane stores its 16 codes as one piece (int8) or
-    // two (fp16). Columns past the tile's last one are written as zeros.
+    // lanes of a block share their maximum by one shuffle, and every lane stores its 16 codes as one piece. Columns past the
+    // tile's last one are written as zeros.
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
     const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
     const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
-    constexpr int OPER_BYTES = Oper<F16>::BYTES, ACT_CHUNK = Oper<F16>::ACT_CHUNK;
     uint8_t *chunk = out + ((size_t)t * nst + s) * ACT_CHUNK;
     int cnt, first = 0;
     if (id.tiles) {
@@ -157,26 +144,15 @@ quantize_tiled_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1,
         const float d = __fdiv_rn(amax, 127.f);
         const float id = d != 0.f ? __fdiv_rn(1.f, d) : 0.f;
         uint8_t *o = chunk + j * OPER_BYTES + (col >> 3) * 128 + (col & 7) * 16;
-        if (F16) {
-            uint32_t w[8];
+        uint32_t w[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const __half2 h = __floats2half2_rn(roundf(__fmul_rn(v[2 * i], id)), roundf(__fmul_rn(v[2 * i + 1], id)));
-                w[i] = *reinterpret_cast<const uint32_t *>(&h);
-            }
-            *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * LBO) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * LBO) = make_uint4(w[4], w[5], w[6], w[7]);
-        } else {
-            uint32_t w[4];
+        for (int i = 0; i < 4; ++i) {
+            uint32_t p = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t p = 0;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) p |= (uint32_t)((int)roundf(__fmul_rn(v[4 * i + b], id)) & 0xFF) << (8 * b);
-                w[i] = p;
-            }
-            *reinterpret_cast<uint4 *>(o + (l & 1) * LBO) = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int b = 0; b < 4; ++b) p |= (uint32_t)((int)roundf(__fmul_rn(v[4 * i + b], id)) & 0xFF) << (8 * b);
+            w[i] = p;
         }
+        *reinterpret_cast<uint4 *>(o + (l & 1) * LBO) = make_uint4(w[0], w[1], w[2], w[3]);
         if ((l & 1) == 0) reinterpret_cast<float *>(chunk + SB * OPER_BYTES)[j * BN + col] = __half2float(__float2half_rn(d));
     }
 }
@@ -187,26 +163,15 @@ template <int N> __device__ __forceinline__ uint32_t word_at(const uint32_t (&w)
     return sh == 0 ? w[i] : __funnelshift_r(w[i], w[i + 1], sh);
 }
 
-// four int8 bytes -> their values as exact fp16 halves: a byte b becomes the half 0x6400 | b = 1024 + b (byte
-// permute with the constant 0x64), and one packed subtraction removes 1024 and the code's own offset
-__device__ __forceinline__ void bytes_to_halves(uint32_t b4, uint32_t bias2, uint32_t &h01, uint32_t &h23) {
-    const uint32_t a = __byte_perm(b4, 0x64646464u, 0x4140), b = __byte_perm(b4, 0x64646464u, 0x4342);
-    const __half2 bias = *reinterpret_cast<const __half2 *>(&bias2);
-    const __half2 ra = __hsub2(*reinterpret_cast<const __half2 *>(&a), bias), rb = __hsub2(*reinterpret_cast<const __half2 *>(&b), bias);
-    h01 = *reinterpret_cast<const uint32_t *>(&ra);
-    h23 = *reinterpret_cast<const uint32_t *>(&rb);
-}
-
 // FULL: every column tile has BN columns (and there is no route)
-template <int TYPE, bool F16, bool FULL>
+template <int TYPE, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word, TileRoute id) {
-    typedef Smem<TYPE, F16> L;
+    typedef Smem<TYPE> L;
     constexpr int ROWB = Raw<TYPE>::ROW;
     constexpr int NSTAGE = L::NSTAGE;
     constexpr int A_SLOTS = L::A_SLOTS;
-    constexpr int OPER_BYTES = Oper<F16>::BYTES, ACT_CHUNK = Oper<F16>::ACT_CHUNK;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
@@ -306,13 +271,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             if (!WAITP(7, bar(BAR_ACC_EMPTY + acc), ((b / NACC) & 1) ^ 1)) break;
             tc_fence_after();
             const uint32_t a_addr = sbase + L::A_OFF + slot * OPER_BYTES, b_addr = sbase + L::ACT_OFF + st * ACT_CHUNK + j * OPER_BYTES;
-            if (F16) {
-                // K = 16 per fp16 MMA: the block's first two 16-byte K pieces, then the other two
-                umma_ss<true>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_F16 | n16, 0u);
-                umma_ss<true>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr + 2 * LBO), umma_desc(b_addr + 2 * LBO), IDESC_F16 | n16, 1u);
-            } else {
-                umma_ss<false>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_I8 | n16, 0u);
-            }
+            umma_ss<false>(leader, tmem_base + (uint32_t)acc * BN, umma_desc(a_addr), umma_desc(b_addr), IDESC_I8 | n16, 0u);
             tc_commit_one(leader, bar(BAR_ACC_FULL + acc));
             tc_commit_one(leader, bar(BAR_A_EMPTY + slot));
             if (j == SB - 1) tc_commit_one(leader, bar(BAR_ACT_EMPTY + st));
@@ -344,36 +303,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 if (!WAITP(5, bar(BAR_A_EMPTY + slot), ((b / A_SLOTS) & 1) ^ 1)) { ok = false; break; }
                 constexpr int BB = TYPE == B200Q_TYPE_Q8_0 ? 34 : 18;
                 uint8_t *a = smem + L::A_OFF + slot * OPER_BYTES + (r >> 3) * 128 + (r & 7) * 16;
-                if (F16) {
-                    // the block's 32 weights as exact fp16 integers, four pieces of eight
-                    uint32_t h[16];
-                    if (TYPE == B200Q_TYPE_Q4_0) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const uint32_t q = word_at(rw, BB * j + 2 + 4 * i);
-                            bytes_to_halves(q & 0x0F0F0F0Fu, 0x64086408u, h[2 * i], h[2 * i + 1]);               // 1024 + n - 1032
-                            bytes_to_halves((q >> 4) & 0x0F0F0F0Fu, 0x64086408u, h[8 + 2 * i], h[8 + 2 * i + 1]);
-                        }
-                    } else if (TYPE == B200Q_TYPE_IQ4_NL) {
-                        // the nibbles index kvalues_iq4nl (signed bytes, |v| <= 127: exact halves), then as for Q8_0
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const uint32_t q = word_at(rw, BB * j + 2 + 4 * i);
-                            bytes_to_halves(iq4nl_lookup4(q & 0x0F0F0F0Fu) ^ 0x80808080u, 0x64806480u, h[2 * i], h[2 * i + 1]);
-                            bytes_to_halves(iq4nl_lookup4((q >> 4) & 0x0F0F0F0Fu) ^ 0x80808080u, 0x64806480u, h[8 + 2 * i], h[8 + 2 * i + 1]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)                                                               // 1024 + (q + 128) - 1152
-                            bytes_to_halves(word_at(rw, BB * j + 2 + 4 * i) ^ 0x80808080u, 0x64806480u, h[2 * i], h[2 * i + 1]);
-                    }
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        *reinterpret_cast<uint4 *>(a + c * LBO) = make_uint4(h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]);
-                    fence_async_smem();
-                    mbar_arrive_warp(bar(BAR_A_FULL + slot), lane);
-                    continue;
-                }
                 uint32_t lo[4], hi[4];
                 if (TYPE == B200Q_TYPE_Q4_0) {
 #pragma unroll
@@ -434,13 +363,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                                            smem + L::RAW_OFF + st * L::RAW_STAGE + r * ROWB + BB * j)) : 0.f;
             const f32x2 dw2 = f2_pack(dwb, dwb), negc2 = f2_pack(-12582912.f, -12582912.f);
             const uint32_t dxa = sbase + L::ACT_OFF + st * ACT_CHUNK + SB * OPER_BYTES + (j * BN + cbase) * 4;
-            // Sixteen columns at a time, the next sixteen (and their scales) in flight under this chunk's arithmetic; for whole
-            // tiles of the four-bit types the whole slice in one go, which leaves the scheduler of those builds more room. Seven
-            // shapes from 512x1024 x 128 to 12288x3072 x 2048 tokens, one go against chunks: Q4_0 and IQ4_NL 3 to 7 % faster
-            // in all (4096x4096 x 512: 71.9 and 76.0 us, 76.6 and 81.1), Q8_0 3 to 7 % slower in all (75.8 and 71.3). Short
-            // tiles are faster in chunks throughout (Q4_0 4096x4096 x 24: 34 and 31 us).
-            constexpr bool ONE_GO = FULL && TYPE != B200Q_TYPE_Q8_0;
-            uint32_t v[ONE_GO ? CW / 16 : 2][16];
+            // sixteen columns at a time, the next sixteen (and their scales) in flight under this chunk's arithmetic
+            uint32_t v[2][16];
             f32x2 dxs[2][8];
             auto fetch_scales = [&](int q, int to) {
 #pragma unroll
@@ -458,29 +382,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 #pragma unroll
                 for (int c = 0; c < 16; c += 4) {
                     const int e = (q * 16 + c) / 2;
-                    // int8 arm: exact int -> float without the conversion pipe (|I| < 2^22): add the magic
-                    // exponent as an integer, subtract it as a float; the fp16 arm's accumulator already holds floats
-                    const f32x2 x01 = F16 ? f2_pack(__uint_as_float(v[from][c]), __uint_as_float(v[from][c + 1]))
-                                          : f2_add(f2_pack(__int_as_float((int)v[from][c] + 0x4B400000),
-                                                           __int_as_float((int)v[from][c + 1] + 0x4B400000)), negc2);
-                    const f32x2 x23 = F16 ? f2_pack(__uint_as_float(v[from][c + 2]), __uint_as_float(v[from][c + 3]))
-                                          : f2_add(f2_pack(__int_as_float((int)v[from][c + 2] + 0x4B400000),
-                                                           __int_as_float((int)v[from][c + 3] + 0x4B400000)), negc2);
+                    // exact int -> float without the conversion pipe (|I| < 2^22): add the magic exponent as an integer, subtract it
+                    // as a float
+                    const f32x2 x01 = f2_add(f2_pack(__int_as_float((int)v[from][c] + 0x4B400000),
+                                                     __int_as_float((int)v[from][c + 1] + 0x4B400000)), negc2);
+                    const f32x2 x23 = f2_add(f2_pack(__int_as_float((int)v[from][c + 2] + 0x4B400000),
+                                                     __int_as_float((int)v[from][c + 3] + 0x4B400000)), negc2);
                     acc2[e]     = f2_fma(x01, f2_mul(dw2, dxs[sc][c / 2]), acc2[e]);
                     acc2[e + 1] = f2_fma(x23, f2_mul(dw2, dxs[sc][c / 2 + 1]), acc2[e + 1]);
                 }
             };
-            if constexpr (ONE_GO) {
-#pragma unroll
-                for (int q = 0; q < CW / 16; ++q) tmem_ld16(taddr + q * 16, v[q]);
-                tmem_ld_wait();
-                release_acc();
-#pragma unroll
-                for (int q = 0; q < CW / 16; ++q) {
-                    fetch_scales(q, 0);
-                    scale_chunk(q, q, 0);
-                }
-            } else if (full) {
+            if (full) {
                 fetch(0, 0);
 #pragma unroll
                 for (int q = 0; q < CW / 16; ++q) {
@@ -560,10 +472,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 
 }  // namespace tc
 
-// sized for the larger (fp16) form, so one scratch serves either arm
+// sized for the larger form, so one scratch serves either arm
 size_t gemm_tc_act_bytes(int64_t K, int64_t N) {
     const int64_t ntile = (N + tc::BN - 1) / tc::BN, nst = K / (tc::SB * tc::KB);
-    return (size_t)(ntile * nst) * tc::Oper<true>::ACT_CHUNK;
+    const size_t i8 = (size_t)(ntile * nst) * tc::ACT_CHUNK, f16 = gemm_t32_act_bytes(K, N);
+    return i8 > f16 ? i8 : f16;
 }
 
 bool gemm_tc_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride) {
@@ -577,10 +490,10 @@ bool gemm_tc_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 static const TileRoute NO_ROUTE_TC = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
 static b200q_status quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
+    if (ctx->tc_f16) return launch_quantize_t32(ctx, src1, out, n_tiles, tr.tiles ? &tr : nullptr);
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     dim3 grid((unsigned)(K / (tc::SB * tc::KB)), (unsigned)n_tiles);
-    auto kern = tr.gate ? (ctx->tc_f16 ? tc::quantize_tiled_kernel<true, true> : tc::quantize_tiled_kernel<false, true>)
-                        : (ctx->tc_f16 ? tc::quantize_tiled_kernel<true, false> : tc::quantize_tiled_kernel<false, false>);
+    auto kern = tr.gate ? tc::quantize_tiled_kernel<true> : tc::quantize_tiled_kernel<false>;
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1],
                                src1->nb[2], src1->nb[3], K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
@@ -595,14 +508,14 @@ b200q_status launch_quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uin
 
 // n_tiles: grid width (dense: the tiles of N; MUL_MAT_ID: the upper bound of the route's tile count,
 // blocks past the device-side count leave at once)
-template <int TYPE, bool F16>
-static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
+template <int TYPE>
+static b200q_status launch_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
                               int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
                               bool early, const TileRoute &tr) {
-    typedef tc::Smem<TYPE, F16> L;
+    typedef tc::Smem<TYPE> L;
     // whole column tiles only (and no route): the build without a branch on the columns that are live
     const bool full = !tr.tiles && N % tc::BN == 0;
-    auto kern = full ? tc::gemm_tc_kernel<TYPE, F16, true> : tc::gemm_tc_kernel<TYPE, F16, false>;
+    auto kern = full ? tc::gemm_tc_kernel<TYPE, true> : tc::gemm_tc_kernel<TYPE, false>;
     static bool attr_set_dev[B200Q_MAX_DEVICES][2] = {};
     bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][full];
     if (!attr_set) {
@@ -631,24 +544,14 @@ static b200q_status launch_tf(b200q_ctx *ctx, const void *w, size_t row_stride, 
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);
-    if (F16) count(ctx, ST_GEMM_TC_F16);
     return B200Q_OK;
-}
-
-// The arm: fp16 operands (integer-valued, exact) by default; B200Q_TC_I8=1 keeps the int8 MMA. Both give the
-// same block dots bit for bit; the fp16 arm's accumulator needs no int -> float conversion.
-template <int TYPE>
-static b200q_status launch_t(b200q_ctx *ctx, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M,
-                             int64_t K, const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd,
-                             bool early, const TileRoute &tr) {
-    return ctx->tc_f16 ? launch_tf<TYPE, true>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, tr)
-                       : launch_tf<TYPE, false>(ctx, w, row_stride, mat_stride, n_mat, M, K, act, N, n_tiles, dst, ldd, early, tr);
 }
 
 b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + tc::BN - 1) / tc::BN;
     const size_t ms = row_stride * (size_t)M;
+    if (ctx->tc_f16) return launch_gemm_t32(ctx, type, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, nullptr);
     if (type == B200Q_TYPE_Q4_0) return launch_t<B200Q_TYPE_Q4_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
     if (type == B200Q_TYPE_Q8_0) return launch_t<B200Q_TYPE_Q8_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
     if (type == B200Q_TYPE_IQ4_NL) return launch_t<B200Q_TYPE_IQ4_NL>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
@@ -664,6 +567,7 @@ b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
     const int64_t K = src0->ne[0], M = src0->ne[1];
     b200q_status st = act_ready ? B200Q_OK : quantize_tiled(ctx, src1, act, max_tiles, tr);
     if (st != B200Q_OK) return st;
+    if (ctx->tc_f16) return launch_gemm_t32(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, &tr);
     if (src0->type == B200Q_TYPE_Q4_0)
         return launch_t<B200Q_TYPE_Q4_0>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     if (src0->type == B200Q_TYPE_Q8_0)

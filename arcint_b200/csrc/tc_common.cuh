@@ -181,6 +181,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]
                  ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
                  "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
+// one register of each lane into one column of the warp's 32 lanes
+__device__ __forceinline__ void tmem_st1(uint32_t addr, uint32_t v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
+}
+// a compile-time number as an argument
+template <int V> struct Int { enum { value = V }; };
 
 // 32 columns of the sixteen lanes at the address: of every eight columns lane l gets columns 2 (l & 3), + 1 of row l / 4 in
 // two registers and of row l / 4 + 8 in the next two
