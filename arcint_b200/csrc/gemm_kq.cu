@@ -101,7 +101,7 @@ static_assert(NG == 2 && NACT == 2 && NBUF == 2, "barrier slots above");
 // Activation chunk (128-token tile t, super-block s), per-256 form (the reference's
 // kernel_quant_i8 rule: scale bm/127, round to nearest even, zero below 1e-30), in the group layout above.
 template <bool GATE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 quantize_tiled256_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
                          int64_t N, uint8_t *__restrict__ out, TileRoute id) {
     // One block per (tile, super-block); a half-warp per column at a time: its sixteen lanes read the column's 256
@@ -124,7 +124,7 @@ quantize_tiled256_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t n
         cnt = left < BN ? (int)left : BN;
     }
     const int live = ((cnt + 7) >> 3) << 3;
-    for (int col = hw; col < live; col += 16) {
+    for (int col = hw; col < live; col += blockDim.x >> 4) {
         const float *x = nullptr;
         if (col < cnt) {
             if (id.tiles) {
@@ -606,10 +606,10 @@ bool gemm_kq_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 }
 
 static b200q_status quantize256(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
-    const int64_t K = src1->ne[0];
+    const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kq::quantize_tiled256_kernel<true> : kq::quantize_tiled256_kernel<false>, grid, dim3(256), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
-                               src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, src1->ne[1] * src1->ne[2] * src1->ne[3], out, tr));
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kq::quantize_tiled256_kernel<true> : kq::quantize_tiled256_kernel<false>, grid, dim3(quantizer_threads(N, &tr)), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
+                               src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);
     return B200Q_OK;
