@@ -392,10 +392,12 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         if (lane == 0) tma_prefetch_desc(&wmap);
         int s_run = 0;                                    // super-blocks fetched so far
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * CHUNK;
             const uint32_t groups = (uint32_t)(U.ncols + 7) >> 3;          // live column groups
+#pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int st = s_run % NRAW, xt = s_run % NX;
                 if (!WAITP(1, bar(BAR_RAW_EMPTY + st), ((s_run / NRAW) & 1) ^ 1)) { ok = false; break; }
@@ -412,6 +414,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                     mbar_expect_tx(bar(BAR_X_FULL + xt), bytes);
                     bulk_g2s(sbase + L::EXTRA_OFF + xt * EXTRA, chunk + 2 * CODE_STAGE, bytes, bar(BAR_X_FULL + xt));
                 }
+#pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
                     // only the column groups the tile has; the MMA still reads a multiple of sixteen columns, the rest of the
                     // stage holds older codes whose products land in accumulator columns nobody stores
@@ -450,15 +453,18 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         pdl_wait();
         bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
         const bool more = *(volatile int *)&more_slot != 0;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);                      // N: the live columns, in sixteens
             if (!more) {
+#pragma unroll 1
                 for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run, ++v_run) {
                     const int xt = s_run % NX;
                     const uint32_t acc = tmem_base + (uint32_t)(v_run & 1) * BN;
                     if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
                     if (!WAITP(7, bar(BAR_ACC_EMPTY + (v_run & 1)), ((v_run >> 1) & 1) ^ 1)) { ok = false; break; }
+#pragma unroll 1
                     for (int jg = 0; jg < SB / GB; ++jg) {
                         const int g = 2 * s_run + jg, gs = g % NG, ct = g % NCODE;
                         if (!WAITP(2, bar(BAR_CODE_FULL + ct), (g / NCODE) & 1)) { ok = false; break; }
@@ -476,6 +482,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 continue;
             }
             constexpr int CB = SB / Fmt<TYPE>::CHAINS;                                    // blocks of a chain
+#pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int xt = s_run % NX;
                 if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
@@ -522,9 +529,11 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + A_BASE;
         int s_run = 0;
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const bool row_ok = r < U.valid_rows;
+#pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int st = s_run % NRAW, xt = s_run % NX;
                 if (!WAITP(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1)) { ok = false; break; }
@@ -566,6 +575,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         pdl_wait();
         bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
         const int chains = *(volatile int *)&more_slot ? Fmt<TYPE>::CHAINS : 1;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
@@ -576,6 +586,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc2[k][i] = 0ull;
             const uint32_t tq = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)cbase;
+#pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int xt = s_run % NX;
                 if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }

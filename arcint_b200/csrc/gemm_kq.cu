@@ -323,9 +323,11 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         if (lane == 0 && !rowcopy) tma_prefetch_desc(&wmap);
         int rs_run = 0, s_run = 0;                        // raw stages and super-blocks fetched so far
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * ACT_CHUNK;
+#pragma unroll 1
             for (int su = 0; su < U.nsu; ++su, ++s_run) {
                 const int s = U.sb0 + su;                 // the super-block inside the row
                 if (s % SPS == 0 && !rowcopy) {               // (row by row: warps 2 and 3 fetch the raw rows, see below)
@@ -358,12 +360,15 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         int s_run = 0;
         const uint32_t leader = elect_one();
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
+#pragma unroll 1
             for (int su = 0; su < U.nsu && ok; ++su, ++s_run) {
                 const int at = s_run % NACT, buf = s_run % NBUF;
                 if (!WAITP(2, bar(BAR_ACT_FULL + at), (s_run / NACT) & 1)) { ok = false; break; }
                 if (!WAITP(7, bar(BAR_ACC_EMPTY + buf), ((s_run / NBUF) & 1) ^ 1)) { ok = false; break; }
+#pragma unroll 1
                 for (int jg = 0; jg < SB / GB; ++jg) {
                     const int g = s_run * (SB / GB) + jg, gs = g % NG;          // group index, its place in the ring
                     if (!WAITP(4, bar(BAR_A_FULL + gs), (g / NG) & 1)) { ok = false; break; }
@@ -397,8 +402,10 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             const int t = (int)threadIdx.x - 64;
             int rs_run = 0;
             bool ok = true;
+#pragma unroll 1
             for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
                 const Unit U = unit_of(u);
+#pragma unroll 1
                 for (int su = 0; su < U.nsu; ++su) {
                     const int s = U.sb0 + su;
                     if (s % SPS != 0) continue;
@@ -431,11 +438,13 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         const int r = (warp - 4) * 16 + (lane >> 4) * 8 + (lane & 7), kh = (lane >> 3) & 1;
         int rs_run = 0, g_run = 0;
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const bool row_ok = r < U.valid_rows;
             // where the row's bytes begin inside a 16-byte unit (0 unless rows are copied one by one, see the producer)
             const int row_shift = rowcopy ? (int)(((uintptr_t)wraw + (size_t)U.expert * mat_stride + (size_t)(U.row0 + r) * row_stride) & 15) : 0;
+#pragma unroll 1
             for (int rsu = 0; rsu < U.nsu / SPS && ok; ++rsu, ++rs_run) {
                 const int rs = U.sb0 / SPS + rsu;         // the raw stage inside the row
                 const int st = rs_run % NRAW;
@@ -467,6 +476,7 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         int rs_run = 0, s_run = 0;
         pdl_wait();
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const bool row_ok = r < U.valid_rows;
@@ -478,6 +488,7 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             f32x2 acc2[CW / 2];
 #pragma unroll
             for (int c = 0; c < CW / 2; ++c) acc2[c] = 0ull;
+#pragma unroll 1
             for (int su = 0; su < U.nsu; ++su, ++s_run) {
                 const int s = U.sb0 + su;
                 if (s % SPS == 0 && su > 0) ++rs_run;

@@ -37,15 +37,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// bounded wait: false when the limit ran out or another role already gave up
+// Bounded wait: false when the limit ran out or another role already gave up. Kept small and not unrolled: there is one at every
+// handoff, and unrolled four times (the compiler's choice) they made up most of a GEMM's 80 KB of code, whose warps then waited
+// for instructions (1.5 warps of five per issue).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    for (uint32_t i = 0; i < SPIN_LIMIT; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if (i > 64) __nanosleep(20);                // after a short hot spin, leave the issue slots to the working warps
-        if ((i & 63) == 63 && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
+    uint32_t i = 0;
+    bool ok;
+#pragma unroll 1
+    do {
+        ok = mbar_try(bar, parity);
+    } while (!ok && ((++i & 63) || (i < SPIN_LIMIT && !*abort_flag)));
+    if (!ok) *abort_flag = 1;
+    return ok;
 }
 // the same for a whole warp: every lane finishes its own bounded wait, then the warp agrees
 // on the outcome, so the warp-synchronous instructions that follow never see a split warp
