@@ -79,9 +79,9 @@ template <int TYPE> struct Smem {
 };
 
 // BAR_READY, BAR_FULL: a barrier per job of an activation stage (four blocks x two halves). READY: the block's operand is in its slot (four
-// arrivals) and the accumulator buffer's last job, three back, has been read (four arrivals); FULL: the MMAs are done, which
-// also frees the operand's half. Every waiting role sees each phase of each of its barriers.
-enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 2, BAR_ACT_FULL = 4, BAR_ACT_EMPTY = 8, BAR_READY = 12, BAR_FULL = 20, BAR_COUNT = 28 };
+// arrivals) and the accumulator buffer's last job, three back, has been read (four arrivals); FULL: the MMAs are done. BAR_FREE, one
+// per operand slot: both halves' MMAs are done. Every waiting role sees each phase of each of its barriers.
+enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 2, BAR_ACT_FULL = 4, BAR_ACT_EMPTY = 8, BAR_READY = 12, BAR_FULL = 20, BAR_FREE = 28, BAR_COUNT = 32 };
 static_assert(NRAW == 2 && NSLOT == HB && BAR_COUNT <= 64, "barrier slots above");
 
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
@@ -168,32 +168,29 @@ __device__ __forceinline__ void signed_bytes_to_halves(uint32_t b, uint32_t &h02
     h13 = h2_sub(__byte_perm(b, 0x64646464u, 0x4341), 0x64806480u);
 }
 
-// the 32-bit word at an even compile-time byte offset of a register array
-template <int N> __device__ __forceinline__ uint32_t word_at(const uint32_t (&w)[N], int byte_off) {
-    const int i = byte_off >> 2;
-    return (byte_off & 3) == 0 ? w[i] : __funnelshift_r(w[i], w[i + 1 < N ? i + 1 : i], 16);
-}
-
-// Block J of the row's raw stage as an operand: sixteen pairs of halves in the K order of the activation codes, and the scale.
-// Blocks are 18 or 34 bytes long: block J begins 2 J bytes into the 16-byte unit J or 2 J, and ends in the next or the one after.
-template <int TYPE, int J>
-__device__ __forceinline__ void unpack_block(const uint8_t *row, uint32_t (&h)[16], uint32_t &d) {
+// Block 2 I + p (p = 0 or 1) of the row's raw stage as an operand: sixteen pairs of halves in the K order of the activation codes, and
+// the scale. Block J is 18 or 34 bytes long and begins 2 J bytes into the 16-byte unit J or 2 J, so that its codes begin 2 p + 2
+// bytes into word I of the two or three units that hold it. p is an argument: both unpack groups run the same code.
+template <int TYPE, int I>
+__device__ __forceinline__ void unpack_block(const uint8_t *row, int p, uint32_t (&h)[16], uint32_t &d) {
     constexpr bool Q8 = TYPE == B200Q_TYPE_Q8_0;
-    constexpr int UNITS = Q8 ? 3 : 2, FIRST = Q8 ? 2 * J : J, OFF = 2 * J;
+    constexpr int UNITS = Q8 ? 3 : 2, PER = Q8 ? 32 : 16;
     uint32_t w[4 * UNITS];
+    row += PER * (2 * I + p);
 #pragma unroll
     for (int i = 0; i < UNITS; ++i) {
-        const uint4 t = *reinterpret_cast<const uint4 *>(row + 16 * (FIRST + i));
+        const uint4 t = *reinterpret_cast<const uint4 *>(row + 16 * i);
         w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
     }
-    d = (OFF & 2) ? w[OFF >> 2] >> 16 : w[OFF >> 2] & 0xFFFFu;
+    d = (w[I] >> (16 * p)) & 0xFFFFu;
+    const uint32_t shift = 16 + 16 * p;                                             // (32: the upper word)
     if constexpr (Q8) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) signed_bytes_to_halves(word_at(w, OFF + 2 + 4 * i), h[2 * i], h[2 * i + 1]);
+        for (int i = 0; i < 8; ++i) signed_bytes_to_halves(__funnelshift_rc(w[I + i], w[I + i + 1], shift), h[2 * i], h[2 * i + 1]);
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t q = word_at(w, OFF + 2 + 4 * i);
+            const uint32_t q = __funnelshift_rc(w[I + i], w[I + i + 1], shift);
             if (TYPE == B200Q_TYPE_IQ4_NL) {
                 // the nibbles index kvalues_iq4nl (signed bytes, |v| <= 127: exact halves)
                 signed_bytes_to_halves(iq4nl_lookup4(q & 0x0F0F0F0Fu), h[2 * i], h[2 * i + 1]);
@@ -285,6 +282,7 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
             mbar_init(bar(BAR_READY + i), 4 + 4);                  // the warps of an unpack group and of a scaling group
             mbar_init(bar(BAR_FULL + i), 1);
         }
+        for (int i = 0; i < NSLOT; ++i) mbar_init(bar(BAR_FREE + i), 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -305,12 +303,14 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
         if (lane == 0) tma_prefetch_desc(&wmap);
         int s_run = 0;                                    // raw stages fetched so far
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * (2 * STAGE);
             // only the column groups the tile has; the MMAs still read a multiple of sixteen columns, the rest of the
             // stage holds older codes whose products land in accumulator columns nobody stores
             const uint32_t bytes = (uint32_t)((U.ncols + 7) >> 3) * GROUP;
+#pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int st = s_run % NRAW;
                 if (!WAITP(1, bar(BAR_RAW_EMPTY + st), ((s_run / NRAW) & 1) ^ 1)) { ok = false; break; }
@@ -320,6 +320,7 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
                     tma_load_3d(sbase + L::RAW_OFF + st * L::RAW_STAGE, &wmap, s * (L::ROW / 4), U.row0, U.expert, bar(BAR_RAW_FULL + st));
                 }
                 if (s_run == 0) pdl_wait();
+#pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
                     const int c_run = 2 * s_run + h, at = c_run % NACT;
                     if (!WAITP(3, bar(BAR_ACT_EMPTY + at), ((c_run / NACT) & 1) ^ 1)) { ok = false; break; }
@@ -338,11 +339,13 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
         const int h = warp - 1;
         int c_run = 0, buf = h;                           // activation stages so far; the job's buffer
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             // N: the half's live columns, in sixteens (a half without any still takes its turn, with sixteen)
             const uint32_t idesc = IDESC | ((uint32_t)((max(1, min(U.cw, U.ncols - h * U.cw)) + 15) >> 4) << 18);
             const uint32_t half_off = (uint32_t)(h * (U.cw >> 3)) * GROUP;
+#pragma unroll 1
             for (int c = 2 * U.sb0; c < 2 * U.sb1 && ok; ++c, ++c_run) {
                 const int at = c_run % NACT;
                 if (!WAITP(2, bar(BAR_ACT_FULL + at), (c_run / NACT) & 1)) { ok = false; break; }
@@ -358,6 +361,7 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
                     umma_ts(leader, acc, a + 8, umma_desc2(b + 256, 128, GROUP), idesc, 1u);
                     umma_ts(leader, acc + 64, a + 16, umma_desc2(bs, GROUP_ZERO - GROUP_SCALES - jj * 128, GROUP), idesc, 0u);
                     tc_commit_one(leader, bar(BAR_FULL + 2 * jj + h));
+                    tc_commit_one(leader, bar(BAR_FREE + jj));
                     buf = buf == 0 ? 2 : buf - 1;                                    // two jobs on, modulo three
                 }
                 if (ok) tc_commit_one(leader, bar(BAR_ACT_EMPTY + at));
@@ -370,46 +374,42 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
         const int r = (warp & 3) * 32 + lane;
         const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + A_BASE;
-        auto rows = [&](auto parity) {
-            constexpr int P = decltype(parity)::value;
-            // the scale operand's zero columns, once
-            tmem_st16_const(ta + P * SLOT_COLS + 16, 0u);
-            tmem_st16_const(ta + (P + 2) * SLOT_COLS + 16, 0u);
-            int s_run = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-                const Unit U = unit_of(u);
-                for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
-                    const int st = s_run % NRAW;
-                    if (!WAITP(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1)) { ok = false; break; }
-                    const uint8_t *row = smem + L::RAW_OFF + st * L::RAW_STAGE + r * L::ROW;
-                    auto one = [&](auto jc) {
-                        constexpr int J = decltype(jc)::value, SLOT = J % NSLOT;
-                        uint32_t h[16], d;
-                        unpack_block<TYPE, J>(row, h, d);
-                        // the slot's last block has been multiplied, by both halves
-                        if (!ok || !WAITP(5, bar(BAR_FULL + 2 * SLOT), (J / NSLOT) ^ 1) || !WAITP(5, bar(BAR_FULL + 2 * SLOT + 1), (J / NSLOT) ^ 1)) {
-                            ok = false;
-                            return;
-                        }
-                        tc_fence_after();
-                        tmem_st16(ta + SLOT * SLOT_COLS, h);
-                        tmem_st1(ta + SLOT * SLOT_COLS + 16, d);
-                        tmem_st_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane < 2) mbar_arrive(bar(BAR_READY + 2 * SLOT + lane));
-                    };
-                    one(Int<P>());
-                    one(Int<P + 2>());
-                    one(Int<P + 4>());
-                    one(Int<P + 6>());
-                    if (ok) mbar_arrive_warp(bar(BAR_RAW_EMPTY + st), lane);
-                }
+        const int p = (warp - 4) >> 2;
+        // the scale operand's zero columns, once
+        tmem_st16_const(ta + p * SLOT_COLS + 16, 0u);
+        tmem_st16_const(ta + (p + 2) * SLOT_COLS + 16, 0u);
+        int s_run = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+#pragma unroll 1
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int st = s_run % NRAW;
+                if (!WAITP(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1)) { ok = false; break; }
+                const uint8_t *row = smem + L::RAW_OFF + st * L::RAW_STAGE + r * L::ROW;
+                auto one = [&](auto ic) {
+                    constexpr int I = decltype(ic)::value;
+                    const int slot = 2 * (I & 1) + p;
+                    uint32_t h[16], d;
+                    unpack_block<TYPE, I>(row, p, h, d);
+                    // the slot's last block has been multiplied
+                    if (!ok || !WAITP(5, bar(BAR_FREE + slot), (I >> 1) ^ 1)) { ok = false; return; }
+                    tc_fence_after();
+                    tmem_st16(ta + slot * SLOT_COLS, h);
+                    tmem_st1(ta + slot * SLOT_COLS + 16, d);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane < 2) mbar_arrive(bar(BAR_READY + 2 * slot + lane));
+                };
+                one(Int<0>());
+                one(Int<1>());
+                one(Int<2>());
+                one(Int<3>());
+                if (ok) mbar_arrive_warp(bar(BAR_RAW_EMPTY + st), lane);
             }
-        };
-        if (warp < 8) rows(Int<0>());
-        else rows(Int<1>());
+        }
     } else {
         // ---- scale: a warp group per half of the tile's columns, a thread a row ----
         asm volatile("setmaxnreg.inc.sync.aligned.u32 144;" ::: "memory");
@@ -421,38 +421,39 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
         int buf = half, b_run = 0;                        // (b_run: blocks so far; a unit has a multiple of eight)
         pdl_wait();
         bool ok = true;
+#pragma unroll 1
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const Unit U = unit_of(u);
             const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
             f32x2 acc2[32];                                    // column pairs
 #pragma unroll
             for (int c = 0; c < 32; ++c) acc2[c] = 0ull;
+#pragma unroll 1
             for (int b = U.sb0 * SB; b < U.sb1 * SB; ++b, ++b_run) {
                 const int job = (2 * b + half) & 7;
                 if (!WAITP(6, bar(BAR_FULL + job), (b_run >> 2) & 1)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t ti = tq + (uint32_t)buf * BN;
-                // sixteen columns at a time, the next sixteen in flight under this chunk's arithmetic
-                uint32_t vi[2][16], vs[2][16];
-                auto fetch = [&](int q) {
-                    tmem_ld16(ti + q * 16, vi[q & 1]);
-                    tmem_ld16(ti + 64 + q * 16, vs[q & 1]);
-                };
                 auto release = [&]() {                             // the buffer is free for the job three on
                     tc_fence_before();
                     mbar_arrive_warp(bar(BAR_READY + ((job + 3) & 7)), lane);
                 };
-                if (FULL || ncol > 0) fetch(0);
+                // 32 columns at a time (sixteen with the next sixteen in flight: 6 % slower)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (FULL || q * 16 < ncol) {
+                for (int q = 0; q < 2; ++q) {
+                    if (FULL || q * 32 < ncol) {
+                        uint32_t vi[2][16], vs[2][16];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            tmem_ld16(ti + q * 32 + i * 16, vi[i]);
+                            tmem_ld16(ti + 64 + q * 32 + i * 16, vs[i]);
+                        }
                         tmem_ld_wait();
-                        if (q < 3 && (FULL || q * 16 + 16 < ncol)) fetch(q + 1);
-                        if (FULL && q == 3) release();
+                        if (FULL && q == 1) release();
 #pragma unroll
-                        for (int c = 0; c < 16; c += 2)
-                            acc2[q * 8 + c / 2] = f2_fma(f2_pack(__uint_as_float(vi[q & 1][c]), __uint_as_float(vi[q & 1][c + 1])),
-                                                         f2_pack(__uint_as_float(vs[q & 1][c]), __uint_as_float(vs[q & 1][c + 1])), acc2[q * 8 + c / 2]);
+                        for (int c = 0; c < 32; c += 2)
+                            acc2[q * 16 + c / 2] = f2_fma(f2_pack(__uint_as_float(vi[c >> 4][c & 15]), __uint_as_float(vi[c >> 4][(c & 15) + 1])),
+                                                          f2_pack(__uint_as_float(vs[c >> 4][c & 15]), __uint_as_float(vs[c >> 4][(c & 15) + 1])), acc2[q * 16 + c / 2]);
                     }
                 }
                 if (!FULL) release();
