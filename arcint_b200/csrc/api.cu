@@ -789,9 +789,9 @@ b200q_status b200q_debug_check_guards(b200q_ctx *ctx, int *blocks, int *violated
         list[n] = &e.sums;   names[n++] = "activation sums";
         list[n] = &e.sums16; names[n++] = "activation sums16";
     }
-    static const char *ws_names[10] = { "moe_ws[0]", "moe_ws[1]", "moe_ws[2]", "moe_ws[3]", "moe_ws[4]",
-                                        "moe_ws[5]", "moe_ws[6]", "moe_ws[7]", "moe_ws[8]", "moe_ws[9]" };
-    for (int i = 0; i < 10; ++i) { list[n] = &ctx->moe_ws[i]; names[n++] = ws_names[i]; }
+    static const char *ws_names[11] = { "moe_ws[0]", "moe_ws[1]", "moe_ws[2]", "moe_ws[3]", "moe_ws[4]",
+                                        "moe_ws[5]", "moe_ws[6]", "moe_ws[7]", "moe_ws[8]", "moe_ws[9]", "moe_ws[10]" };
+    for (int i = 0; i < 11; ++i) { list[n] = &ctx->moe_ws[i]; names[n++] = ws_names[i]; }
     list[n] = &ctx->flush_buf; names[n++] = "flush buffer";
     n += moe_route_workspaces(ctx, list + n, names + n);
     uint8_t host[2 * WS_GUARD];

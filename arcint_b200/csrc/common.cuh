@@ -152,7 +152,7 @@ struct b200q_ctx {
     std::vector<b200q::ActEntry> act_cache;
     size_t       act_next = 0;
     b200q::Workspace flush_buf;
-    b200q::Workspace moe_ws[10];
+    b200q::Workspace moe_ws[11];
     b200q::RouteEntry *routes[2] = { nullptr, nullptr };
     size_t       route_next = 0;
     cudaEvent_t  ev0 = nullptr, ev1 = nullptr;
@@ -282,7 +282,7 @@ b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, i
 // on full tiles: a step of 256 weights, and what a unit costs beyond its steps (fill, drain, stores; gemm_tc, one block a unit, sets
 // itself up and allocates tensor memory too). Measured from products of one round, 16 and 43 steps long.
 struct KsplitTimes { int step_ns, unit_ns; };
-constexpr KsplitTimes TC_TIMES = { 1300, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 };
+constexpr KsplitTimes TC_TIMES = { 1300, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 }, KX_TIMES = { 1000, 1500 };
 int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts);
 
 // gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types

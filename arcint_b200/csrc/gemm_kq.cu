@@ -593,6 +593,251 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     }
 }
 
+// ---- products with many column tiles: the operand expanded once ----
+//
+// gemm_kq_kernel unpacks a row tile's weights again for every column tile, and the integer work of that is what bounds it (unpack
+// warps busy 88 % of the time; some 3,500 clk a 128 x 128 x 256 super-block against 1,024 of its MMAs). With several column tiles it is
+// cheaper to write the limbs out once, in the order the tensor core reads them, to scratch that stays in L2 (a chunk of row
+// tiles at a time), and to run the MMAs straight from there. What bounds that is the shared-memory port: the copies, operand reads and
+// activation of a super-block are 225 KB, 1,760 clk of the 2,440 it takes. IQ4_XS 17408x5120 x 2048 tokens: 532 -> 457 us. From how
+// many tiles: see expand_wanted.
+constexpr int EXP_DW = 2 * NA * OPER_BYTES;               // 65536: per (row tile, super-block) eight blocks' limbs [block][hi, lo], then ...
+constexpr int EXP_CHUNK = EXP_DW + BM * 4;                // ... the rows' d_w as f32
+
+template <int TYPE>
+__global__ void __launch_bounds__(256)
+expand_kernel(const uint8_t *__restrict__ w, size_t row_stride, int M, int row_tile0, uint8_t *__restrict__ out) {
+    pdl_wait();                          // the scratch may still be read by the product before
+    pdl_trigger();
+    const int s = blockIdx.x, nsb = gridDim.x, tm = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint8_t *chunk = out + ((size_t)tm * nsb + s) * EXP_CHUNK;
+    // the unpack warps' mapping: two threads a row, eight rows and both halves in a half-warp, whose 8- or 16-byte stores are contiguous
+    const int r = warp * 16 + (lane >> 4) * 8 + (lane & 7), kh = (lane >> 3) & 1, row = (row_tile0 + tm) * BM + r;
+    const bool row_ok = row < M;
+    // The rows' blocks by way of shared memory, in 16-byte pieces from the boundary below: read in place, each word of a block is a
+    // load of sixteen lines a warp (Q6_K 4096x11008: 25 us). A piece never reaches past the 16-byte unit of the block's last byte.
+    constexpr int SBB = Fmt<TYPE>::SBB, PIECES = TYPE == B200Q_TYPE_Q6_K ? 14 : 9, PITCH = TYPE == B200Q_TYPE_Q6_K ? 240 : 176;
+    __shared__ __align__(16) uint8_t raw[BM * PITCH];
+    const uint8_t *first = w + (size_t)(row_tile0 + tm) * BM * row_stride + (size_t)s * SBB;
+#pragma unroll
+    for (int i = 0; i < BM * PIECES; i += 256) {
+        const int rr = (i + (int)threadIdx.x) / PIECES, pc = (i + (int)threadIdx.x) % PIECES;
+        const uintptr_t src = (uintptr_t)(first + (size_t)rr * row_stride);
+        if (rr < BM && (row_tile0 + tm) * BM + rr < M && 16 * pc < (int)(src & 15) + SBB)
+            *reinterpret_cast<uint4 *>(raw + rr * PITCH + 16 * pc) = __ldg(reinterpret_cast<const uint4 *>((src & ~(uintptr_t)15) + 16 * pc));
+    }
+    __syncthreads();
+    const uint8_t *blk = raw + r * PITCH + ((uintptr_t)(first + (size_t)r * row_stride) & 15);
+#pragma unroll
+    for (int jg = 0; jg < SB / GB; ++jg) unpack_group<TYPE>(blk, jg, kh, row_ok, chunk + jg * GB * A_SLOT + (r >> 3) * 128 + (r & 7) * 16);
+    if (kh == 0)
+        reinterpret_cast<float *>(chunk + EXP_DW)[r] = row_ok ? half_bits_to_float(*reinterpret_cast<const uint16_t *>(blk + Fmt<TYPE>::D_OFF)) : 0.f;
+}
+
+constexpr int XG = 4;                                     // groups of four blocks in the A ring
+constexpr int X_ACT = ACT_CHUNK + BM * 4;                 // an activation stage, and the rows' d_w behind it
+constexpr int X_A_OFF = NACT * X_ACT, X_BAR_OFF = X_A_OFF + XG * GB * A_SLOT, X_TOTAL = X_BAR_OFF + 8 * 16;
+constexpr int X_THREADS = 32 * (4 + 4 * NW);
+static_assert(X_TOTAL <= 227 * 1024 - 256 && X_ACT % 128 == 0, "shared memory budget");
+enum { XB_ACT_FULL = 0, XB_ACT_EMPTY = 2, XB_A_FULL = 4, XB_A_EMPTY = 8, XB_ACC_FULL = 12, XB_ACC_EMPTY = 14 };
+
+// The product from the expanded operand: producer, MMA issuer, two idle warps, 4 NW scale-accumulate warps as in gemm_kq_kernel
+template <bool FULL>
+__global__ void __launch_bounds__(X_THREADS, 1)
+gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__restrict__ act, int N, int tiles_n, int row_tile0, int row_tiles,
+               int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride, int *__restrict__ error_word) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler, too)
+    const int nsb = K / 256;
+    const uint32_t sbase = smem_u32(smem), bars = sbase + X_BAR_OFF;
+    auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+    const int n_units = row_tiles * tiles_n * ksplit;
+    struct UnitX { int tile_n, tm, ncols, sb0, sb1, part; };
+    auto unit_of = [&](int u) {
+        UnitX U;
+        U.part = u % ksplit;
+        U.sb0 = U.part * nsb / ksplit;
+        U.sb1 = (U.part + 1) * nsb / ksplit;
+        u /= ksplit;
+        U.tile_n = u % tiles_n;
+        U.tm = u / tiles_n;
+        U.ncols = min(BN, N - U.tile_n * BN);
+        return U;
+    };
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar(XB_ACT_FULL + i), 1);
+            mbar_init(bar(XB_ACT_EMPTY + i), 1 + 4 * NW);          // MMA commit + scaling warps
+            mbar_init(bar(XB_ACC_FULL + i), 1);
+            mbar_init(bar(XB_ACC_EMPTY + i), 4 * NW);
+        }
+        for (int i = 0; i < XG; ++i) {
+            mbar_init(bar(XB_A_FULL + i), 1);
+            mbar_init(bar(XB_A_EMPTY + i), 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_slot, 0);
+    volatile int *abortp = &abort_flag;
+    PROF_DECL
+
+    if (warp == 0) {
+        // ---- producer ----
+        pdl_wait();
+        int s_run = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const UnitX U = unit_of(u);
+            const uint32_t bytes = (uint32_t)((U.ncols + 7) >> 3) * ACT_GROUP;       // only the column groups the tile has
+#pragma unroll 1
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const uint8_t *chunk = ops + ((size_t)U.tm * nsb + s) * EXP_CHUNK;
+                const int at = s_run % NACT;
+                if (!WAITP(3, bar(XB_ACT_EMPTY + at), ((s_run / NACT) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    mbar_expect_tx(bar(XB_ACT_FULL + at), bytes + BM * 4);
+                    bulk_g2s(sbase + at * X_ACT, act + ((size_t)U.tile_n * nsb + s) * ACT_CHUNK, bytes, bar(XB_ACT_FULL + at));
+                    bulk_g2s(sbase + at * X_ACT + ACT_CHUNK, chunk + EXP_DW, BM * 4, bar(XB_ACT_FULL + at));
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (int jg = 0; jg < SB / GB; ++jg) {
+                    const int g = 2 * s_run + jg, gs = g % XG;
+                    if (!WAITP(1, bar(XB_A_EMPTY + gs), ((g / XG) & 1) ^ 1)) { ok = false; break; }
+                    if (lane == 0) {
+                        mbar_expect_tx(bar(XB_A_FULL + gs), GB * A_SLOT);
+                        bulk_g2s(sbase + X_A_OFF + gs * (GB * A_SLOT), chunk + jg * GB * A_SLOT, GB * A_SLOT, bar(XB_A_FULL + gs));
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer: per block one MMA per limb, accumulating over the super-block ----
+        int s_run = 0;
+        const uint32_t leader = elect_one();
+        bool ok = true;
+#pragma unroll 1
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const UnitX U = unit_of(u);
+#pragma unroll 1
+            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
+                const int at = s_run % NACT, buf = s_run % NBUF;
+                if (!WAITP(2, bar(XB_ACT_FULL + at), (s_run / NACT) & 1)) { ok = false; break; }
+                if (!WAITP(7, bar(XB_ACC_EMPTY + buf), ((s_run / NBUF) & 1) ^ 1)) { ok = false; break; }
+#pragma unroll 1
+                for (int jg = 0; jg < SB / GB; ++jg) {
+                    const int g = 2 * s_run + jg, gs = g % XG;
+                    if (!WAITP(4, bar(XB_A_FULL + gs), (g / XG) & 1)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t d = tmem_base + (uint32_t)buf * (2 * BN), a = sbase + X_A_OFF + gs * (GB * A_SLOT);
+                    const uint32_t b = sbase + at * X_ACT + jg * (GB * 256);
+#pragma unroll
+                    for (int jj = 0; jj < GB; ++jj) {
+                        const uint64_t db = umma_desc2(b + jj * 256, 128, ACT_GROUP);
+                        umma_ss<false>(leader, d, umma_desc(a + jj * A_SLOT), db, IDESC, (uint32_t)(jg + jj > 0));
+                        umma_ss<false>(leader, d + BN, umma_desc(a + jj * A_SLOT + OPER_BYTES), db, IDESC, (uint32_t)(jg + jj > 0));
+                    }
+                    tc_commit_one(leader, bar(XB_A_EMPTY + gs));
+                }
+                if (!ok) break;
+                tc_commit_one(leader, bar(XB_ACC_FULL + buf));
+                tc_commit_one(leader, bar(XB_ACT_EMPTY + at));
+            }
+        }
+    } else if (warp >= 4) {
+        // ---- scale-accumulate, once per super-block ----
+        constexpr int CW = BN / NW;
+        const int q4 = warp & 3, u4 = (warp - 4) >> 2, r = q4 * 32 + lane;
+        int s_run = 0;
+        pdl_wait();
+        bool ok = true;
+#pragma unroll 1
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const UnitX U = unit_of(u);
+            // the tile's columns are shared out between the two warps of a row quadrant: 64 each, or half of what a short tile has,
+            // in steps of 16
+            const int cw = FULL || U.ncols > CW ? CW : max(16, (((U.ncols + 1) >> 1) + 15) & ~15), cbase = u4 * cw;
+            const int ncol = FULL ? CW : min(cw, U.ncols - cbase);          // this warp's columns (none: <= 0)
+            f32x2 acc2[CW / 2];
+#pragma unroll
+            for (int c = 0; c < CW / 2; ++c) acc2[c] = 0ull;
+#pragma unroll 1
+            for (int s = U.sb0; s < U.sb1; ++s, ++s_run) {
+                const int at = s_run % NACT, buf = s_run % NBUF;
+                if (!WAITP(2, bar(XB_ACT_FULL + at), (s_run / NACT) & 1)) { ok = false; break; }
+                const uint32_t stage = sbase + at * X_ACT;
+                const float dwb = *reinterpret_cast<const float *>(smem + at * X_ACT + ACT_CHUNK + r * 4);
+                const f32x2 dw2 = f2_pack(dwb, dwb);
+                const uint32_t dxa = stage + (cbase / 8) * ACT_GROUP + ACT_SCALES;
+                if (!WAITP(6, bar(XB_ACC_FULL + buf), (s_run / NBUF) & 1)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)buf * (2 * BN) + (uint32_t)cbase;
+#pragma unroll
+                for (int q = 0; q < CW / 16; ++q) {
+                    if (FULL || q * 16 < ncol) {
+                        uint32_t vh[16], vl[16];
+                        tmem_ld16(taddr + q * 16, vh);
+                        tmem_ld16(taddr + BN + q * 16, vl);
+                        f32x2 dx[8];                             // sixteen activation scales, in flight under the tensor-memory loads
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) lds128_f2(dxa + (2 * q + (c >> 1)) * ACT_GROUP + (c & 1) * 16, dx[2 * c], dx[2 * c + 1]);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 16; c += 2) {
+                            const int e = (q * 16 + c) / 2;
+                            // 256 hi + lo as an integer, one rounding to float (ggml's float(sumi))
+                            const f32x2 v = f2_pack(__int2float_rn((int)vl[c] + ((int)vh[c] << 8)), __int2float_rn((int)vl[c + 1] + ((int)vh[c + 1] << 8)));
+                            acc2[e] = f2_fma(v, f2_mul(dw2, dx[c / 2]), acc2[e]);
+                        }
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive_warp(bar(XB_ACC_EMPTY + buf), lane);
+                mbar_arrive_warp(bar(XB_ACT_EMPTY + at), lane);
+            }
+            const int row = (row_tile0 + U.tm) * BM + r;
+            if (ok && row < M) {
+                float *o = dst + (int64_t)U.part * part_stride + (int64_t)(U.tile_n * BN + cbase) * ldd + row;
+#pragma unroll
+                for (int c = 0; c < CW; c += 2) {
+                    float a0, a1;
+                    f2_unpack(acc2[c / 2], a0, a1);
+                    if (FULL || c < ncol) *o = a0;
+                    if (FULL || c + 1 < ncol) o[ldd] = a1;
+                    o += 2 * ldd;
+                }
+            }
+        }
+    }
+
+    PROF_DUMP(warp == 0 ? "prod" : warp == 1 ? "mma " : warp < 4 ? "idle" : "epi ")
+    tc_fence_before();
+    __syncthreads();
+    pdl_trigger();
+    if (abort_flag) {
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        if (threadIdx.x == 0) atomicExch(error_word, 2);
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
 }  // namespace kq
 
 static size_t kq_chunks(int64_t K, int64_t N) { return (size_t)(((N + kq::BN - 1) / kq::BN) * (K / 256)); }
@@ -677,6 +922,57 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     return B200Q_OK;
 }
 
+// Whether a dense product takes the expanded operand: it saves a fifth to a third of a column tile's time and costs a pass that writes two
+// bytes a weight. Quantizer included, unpacking and expanded, us, at 2, 3, 4 and 6 column tiles:
+//   Q6_K   4096x11008  64.3 85.2 114.2 158.7   63.9 79.3 88.3 122.4
+//   IQ4_XS 4096x11008  59.2 79.3 104.4 145.6   62.2 77.6 86.6 121.1      11008x4096  53.8 62.1 87.3 114.7   71.5 72.0 90.2 112.7
+// and at sixteen, IQ4_XS 17408x5120, 532 and 457.
+static bool expand_wanted(int type, int64_t n_tiles) { return n_tiles >= (type == B200Q_TYPE_Q6_K ? 4 : 6); }
+
+// The product from the expanded operand, a chunk of row tiles at a time; *took: false when the scratch cannot be had
+template <int TYPE>
+static b200q_status launch_kx_t(b200q_ctx *ctx, const void *w, size_t row_stride, int64_t M, int64_t K, const uint8_t *act, int64_t N,
+                                int64_t n_tiles, float *dst, int64_t ldd, bool *took) {
+    const int64_t nsb = K / 256, tiles_m = (M + kq::BM - 1) / kq::BM;
+    const size_t per_tile = (size_t)nsb * kq::EXP_CHUNK;
+    constexpr size_t MOST = (size_t)96 << 20;                  // of 126 MB of L2
+    int64_t chunk = (int64_t)(MOST / per_tile);
+    chunk = chunk < 1 ? 1 : chunk < tiles_m ? chunk : tiles_m;
+    const int64_t chunks = (tiles_m + chunk - 1) / chunk;
+    chunk = (tiles_m + chunks - 1) / chunks;                   // of about equal size
+    Workspace *ws = &ctx->moe_ws[10];
+    *took = ws_try_reserve(ctx, ws, per_tile * (size_t)chunk);
+    if (!*took) return B200Q_OK;
+    const bool full = N % kq::BN == 0;
+    auto kern = full ? kq::gemm_kx_kernel<true> : kq::gemm_kx_kernel<false>;
+    static bool attr_set_dev[B200Q_MAX_DEVICES][2] = {};
+    bool &attr_set = attr_set_dev[ctx->device % B200Q_MAX_DEVICES][full];
+    if (!attr_set) {
+        B200Q_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kq::X_TOTAL));
+        attr_set = true;
+    }
+    float *out = dst, *parts = nullptr;
+    const int ksplit = plan_ksplit(ctx, chunk * n_tiles, nsb, KX_TIMES, M, N, &parts);
+    int64_t out_ld = ldd, part_stride = 0;
+    if (ksplit > 1) {
+        out = parts;
+        part_stride = N * M;
+        out_ld = M;
+    }
+    for (int64_t t0 = 0; t0 < tiles_m; t0 += chunk) {
+        const int64_t nt = tiles_m - t0 < chunk ? tiles_m - t0 : chunk, units = nt * n_tiles * ksplit;
+        B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl && t0 > 0, kq::expand_kernel<TYPE>, dim3((unsigned)nsb, (unsigned)nt), dim3(256), 0, ctx->stream, (const uint8_t *)w, row_stride,
+                                   (int)M, (int)t0, (uint8_t *)ws->ptr));
+        B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3((unsigned)(units < ctx->sm_count ? units : ctx->sm_count)), dim3(kq::X_THREADS), (size_t)kq::X_TOTAL, ctx->stream,
+                                   (const uint8_t *)ws->ptr, (int)M, (int)K, act, (int)N, (int)n_tiles, (int)t0, (int)nt, ksplit, out, out_ld, part_stride, ctx->error_word));
+        B200Q_CUDA(ctx, cudaGetLastError());
+    }
+    count(ctx, ST_GEMM_TC);
+    if (row_stride % 16 != 0 || K % (TYPE == B200Q_TYPE_Q6_K ? 2048 : 512) != 0) count(ctx, ST_GEMM_KQ_ROWCOPY);     // rows that no tensor map describes
+    if (ksplit > 1) return launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd);
+    return B200Q_OK;
+}
+
 // IQ4_XS shapes the two-super-block tensor-map staging cannot take: an odd super-block count, or strides that are not
 // 16-byte multiples
 static bool iq4_rows(int64_t K, size_t row_stride, size_t mat_stride) { return K % 512 != 0 || row_stride % 16 != 0 || mat_stride % 16 != 0; }
@@ -685,6 +981,12 @@ b200q_status launch_gemm_kq(b200q_ctx *ctx, int type, const void *w, size_t row_
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + kq::BN - 1) / kq::BN;
     const size_t ms = row_stride * (size_t)M;
+    if (expand_wanted(type, n_tiles) && (type == B200Q_TYPE_IQ4_XS || type == B200Q_TYPE_Q6_K)) {
+        bool took = false;
+        const b200q_status st = type == B200Q_TYPE_IQ4_XS ? launch_kx_t<B200Q_TYPE_IQ4_XS>(ctx, w, row_stride, M, K, act, N, n_tiles, dst, ldd, &took)
+                                                          : launch_kx_t<B200Q_TYPE_Q6_K>(ctx, w, row_stride, M, K, act, N, n_tiles, dst, ldd, &took);
+        if (took || st != B200Q_OK) return st;
+    }
     if (type == B200Q_TYPE_IQ4_XS && iq4_rows(K, row_stride, ms))
         return launch_kq_t<B200Q_TYPE_IQ4_XS, kq::FMT_IQ4_XS_ROWS>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE);
     if (type == B200Q_TYPE_IQ4_XS) return launch_kq_t<B200Q_TYPE_IQ4_XS>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE);
