@@ -468,11 +468,12 @@ b200q_status b200q_mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b2
 }  // extern "C"
 
 b200q_status b200q::mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const b200q_tensor *ids,
-                               b200q_tensor *dst, int64_t gate) {
+                               b200q_tensor *dst, int64_t gate, const b200q_tensor *src0b, b200q_tensor *dstb) {
     b200q_status st = check_mul_mat(ctx, src0, src1, dst, true);
     if (st != B200Q_OK) return st;
     st = check_ids(ctx, src0, src1, ids, dst);
     if (st != B200Q_OK) return st;
+    if (src0b && ((st = check_mul_mat(ctx, src0b, src1, dstb, true)) != B200Q_OK || (st = check_ids(ctx, src0b, src1, ids, dstb)) != B200Q_OK)) return st;
     B200Q_CUDA(ctx, cudaSetDevice(ctx->device));
     TypeInfo ti;
     type_info(src0->type, &ti);
@@ -513,27 +514,33 @@ b200q_status b200q::mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
         ma.gate = gate;
         ma.n_expert = n_expert;
         for (int i = 0; i < 4; ++i) { ma.ne[i] = src1->ne[i]; ma.nb[i] = src1->nb[i]; }
-        return per32 ? launch_gemm_tc_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
+        st = per32 ? launch_gemm_tc_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
              : f16   ? launch_gemm_kf_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
                      : launch_gemm_kq_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready);
+        return st == B200Q_OK && src0b ? mul_mat_id(ctx, src0b, src1, ids, dstb, gate) : st;
     }
+    // two products of one form are one launch
+    const bool both = src0b && src0b->type == src0->type && src0b->ne[1] == M && src0b->ne[2] == n_expert && src0b->nb[1] == src0->nb[1] && src0b->nb[2] == src0->nb[2] &&
+                      dstb->nb[1] == dst->nb[1] && dstb->nb[2] == dst->nb[2];
+    const void *w2 = both ? src0b->data : nullptr;
+    float *dst2 = both ? (float *)dstb->data : nullptr;
     ActView act;
     if ((st = get_activation(ctx, ti.act_form, src1, &act, gate)) != B200Q_OK) return st;
     // a handful of tokens: one unit per pair, its expert read on the device (the reference's
     // per-pair GEMV below GGML_OPENCL_KQ_MM_ID_MIN_TOK); more: route once per ids tensor
     // and graph, then one launch per tile size class
-    if (n_tok <= 4)
-        return launch_gemv_id(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], M, K, act, 1, nullptr, nullptr,
-                              (int64_t)n_used * n_tok, nullptr, ids, n_expert, n_used, ne11, (float *)dst->data, ld1, ld2);
-    RouteView rv;
-    if ((st = moe_route(ctx, ids, n_expert, &rv)) != B200Q_OK) return st;
-    static const int widths[4] = { 1, 2, 4, 8 };
-    for (int k = 3; k >= 0; --k) {
-        st = launch_gemv_id(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], M, K, act, widths[k], rv.tiles[k],
-                            rv.n_tiles + k, rv.max_tiles, rv.pairs, ids, n_expert, n_used, ne11, (float *)dst->data, ld1, ld2);
-        if (st != B200Q_OK) return st;
+    if (n_tok <= 4) {
+        st = launch_gemv_id(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], M, K, act, 1, nullptr, nullptr,
+                            (int64_t)n_used * n_tok, nullptr, ids, n_expert, n_used, ne11, (float *)dst->data, ld1, ld2, w2, dst2);
+    } else {
+        RouteView rv;
+        if ((st = moe_route(ctx, ids, n_expert, &rv)) != B200Q_OK) return st;
+        static const int widths[4] = { 1, 2, 4, 8 };
+        for (int k = 3; k >= 0 && st == B200Q_OK; --k)
+            st = launch_gemv_id(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], M, K, act, widths[k], rv.tiles[k],
+                                rv.n_tiles + k, rv.max_tiles, rv.pairs, ids, n_expert, n_used, ne11, (float *)dst->data, ld1, ld2, w2, dst2);
     }
-    return B200Q_OK;
+    return st == B200Q_OK && src0b && !both ? mul_mat_id(ctx, src0b, src1, ids, dstb, gate) : st;
 }
 
 extern "C" {

@@ -196,7 +196,7 @@ b200q_status launch_gemv_fused(b200q_ctx *ctx, int type, const void *w, size_t r
 b200q_status launch_gemv_id(b200q_ctx *ctx, int type, const void *w, size_t row_stride, size_t expert_stride,
                             int64_t M, int64_t K, const ActView &av, int tile_pairs, const int32_t *tiles,
                             const int32_t *n_tiles, int64_t max_tiles, const int32_t *pairs, const b200q_tensor *ids,
-                            int n_expert, int n_used, int ne11, float *dst, int64_t ld1, int64_t ld2);
+                            int n_expert, int n_used, int ne11, float *dst, int64_t ld1, int64_t ld2, const void *w2 = nullptr, float *dst2 = nullptr);
 // the product of a K shard and the all-reduce of the ranks' partial results in one kernel (gemv_stream.cuh); av: the
 // quantized activation, or NULL with src1 to quantize inside the kernel; peers / state: the all-reduce's mapped
 // buffers and device words (tp.cu). B200Q_UNSUPPORTED: the shape does not qualify.
@@ -205,9 +205,10 @@ b200q_status launch_gemv_allreduce(b200q_ctx *ctx, int type, const void *w, size
                                    int rank, int nranks);
 bool gemv_ar_shape_ok(int type, const void *w, size_t row_stride, int64_t M, int64_t K, int ncols, int64_t ldd);
 // api.cu: MUL_MAT_ID; gate != 0: src1 is the up projection of a SwiGLU whose gate values lie `gate` floats from it, and what is
-// quantized and multiplied is silu(gate) * src1
+// quantized and multiplied is silu(gate) * src1; src0b, dstb: a second product over the same src1 and ids (one launch for both where
+// the GEMV takes them and the two are laid out alike)
 b200q_status mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const b200q_tensor *ids, b200q_tensor *dst,
-                        int64_t gate);
+                        int64_t gate, const b200q_tensor *src0b = nullptr, b200q_tensor *dstb = nullptr);
 // silu(g) * u, as every quantizer that takes the gate along computes it
 __device__ __forceinline__ float swiglu(float g, float u) { return g / (1.f + expf(-g)) * u; }
 __device__ __forceinline__ float4 swiglu4(float4 g, float4 u) {
@@ -279,10 +280,10 @@ inline unsigned quantizer_threads(int64_t N, const TileRoute *tr) { return tr &&
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
 
 // K parts of a product whose tiles fill the SMs badly, and the scratch for their results (ksplit.cu). It counts with a kernel's times
-// on full tiles: a step of 256 weights, and what a unit costs beyond its steps (fill, drain, stores; gemm_tc, one block a unit, sets
-// itself up and allocates tensor memory too). Measured from products of one round, 16 and 43 steps long.
+// on full tiles: a step of 256 weights, and what a unit costs beyond its steps (fill, drain, stores). Measured from products of one
+// round, 16 and 43 steps long (TC: gemm_t32; the int8 arm takes the same, so that both cut a product alike).
 struct KsplitTimes { int step_ns, unit_ns; };
-constexpr KsplitTimes TC_TIMES = { 1300, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 }, KX_TIMES = { 1000, 1500 };
+constexpr KsplitTimes TC_TIMES = { 2500, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 }, KX_TIMES = { 1300, 1500 };
 int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts);
 
 // gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types

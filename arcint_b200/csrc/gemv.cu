@@ -46,12 +46,15 @@ static GemvAct make_act(const ActView &av, int64_t col0, int64_t K) {
 b200q_status launch_gemv_id(b200q_ctx *ctx, int type, const void *w, size_t row_stride, size_t expert_stride,
                             int64_t M, int64_t K, const ActView &av, int tile_pairs, const int32_t *tiles,
                             const int32_t *n_tiles, int64_t max_tiles, const int32_t *pairs, const b200q_tensor *ids,
-                            int n_expert, int n_used, int ne11, float *dst, int64_t ld1, int64_t ld2) {
+                            int n_expert, int n_used, int ne11, float *dst, int64_t ld1, int64_t ld2, const void *w2, float *dst2) {
     TypeInfo ti;
     if (!type_info(type, &ti)) return fail(ctx, B200Q_UNSUPPORTED, "gemv_id: type %d", type);
     const size_t row_bytes = (size_t)(K / ti.block) * ti.bytes;
-    const int rows = gemv_row_mode(type, (size_t)(uintptr_t)w | row_stride | expert_stride, row_bytes);
+    const int rows = gemv_row_mode(type, (size_t)(uintptr_t)w | (size_t)(uintptr_t)w2 | row_stride | expert_stride, row_bytes);
     GemvId id;
+    id.n_mat = w2 ? 2 : 1;
+    id.w_off = w2 ? (const uint8_t *)w2 - (const uint8_t *)w : 0;
+    id.dst_off = w2 ? dst2 - dst : 0;
     id.tiles = tiles;
     id.n_tiles = n_tiles;
     id.pairs = pairs;

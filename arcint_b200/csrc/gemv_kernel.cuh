@@ -37,6 +37,10 @@ struct GemvId {
     int            n_used, ne11;
     size_t         expert_stride;   // bytes between expert matrices
     int64_t        ld1, ld2;        // dst strides of slot i and token t, in floats
+    // a second product over the same activation and route in the same launch (gate and up of a feed-forward block): from the first one's
+    // weights and results to its own, in bytes and floats (n_mat = 1: none)
+    int            n_mat;
+    int64_t        w_off, dst_off;
 };
 
 // How a product's rows lie: every row a 16-byte multiple from a 16-byte start; rows whose starts are only a multiple of what
@@ -83,7 +87,7 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
     const int nstages = (nblk + F::STAGE_BLOCKS - 1) / F::STAGE_BLOCKS;
     const int n_bt = (M + B - 1) / B;                     // row batches per matrix
     const bool direct = ID && id.tiles == nullptr;
-    const int n_units = ID ? (direct ? id.n_pairs : __ldg(id.n_tiles)) * n_bt : n_bt;
+    const int n_tiles = ID ? (direct ? id.n_pairs : __ldg(id.n_tiles)) : 1, n_units = n_tiles * n_bt * (ID ? id.n_mat : 1);
     // direct mode: the expert of pair p, read from ids and clamped like the reference's route kernel
     auto pair_expert = [&](int p) {
         const int t = p / id.n_used, i = p - t * id.n_used;
@@ -100,7 +104,10 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
             const int bytes = min((int)S::BYTES, row_bytes - off);
             const int row0 = (ID ? p_u % n_bt : p_u) * B;
             const uint8_t *src = W + (size_t)row0 * row_stride + off;
-            if (ID) src += (size_t)(direct ? pair_expert(p_u / n_bt) : __ldg(id.tiles + 4 * (p_u / n_bt))) * id.expert_stride;
+            if (ID) {
+                const int t = p_u / n_bt, tile = t < n_tiles ? t : t - n_tiles;
+                src += (size_t)(direct ? pair_expert(tile) : __ldg(id.tiles + 4 * tile)) * id.expert_stride + (t < n_tiles ? 0 : id.w_off);
+            }
             uint8_t *d = ring + p_set * (B * SLOT);
 #pragma unroll
             for (int r = 0; r < B; ++r) {
@@ -146,16 +153,16 @@ gemv_kernel(const uint8_t *__restrict__ W, size_t row_stride, int M, int nblk, G
         int ncol = NC;
         uintptr_t wbase = (uintptr_t)W;                    // where the unit's matrix begins (shifted rows)
         if (ID) {
-            const int tile = u / n_bt;
+            const int tile2 = u / n_bt, tile = tile2 < n_tiles ? tile2 : tile2 - n_tiles;
             const int first = direct ? tile : __ldg(id.tiles + 4 * tile + 1);
             ncol = direct ? 1 : __ldg(id.tiles + 4 * tile + 2);
-            if (ROWS == GEMV_ROWS_SHIFTED) wbase += (size_t)(direct ? pair_expert(tile) : __ldg(id.tiles + 4 * tile)) * id.expert_stride;
+            if (ROWS == GEMV_ROWS_SHIFTED) wbase += (size_t)(direct ? pair_expert(tile) : __ldg(id.tiles + 4 * tile)) * id.expert_stride + (tile2 < n_tiles ? 0 : id.w_off);
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const int p = direct ? tile : __ldg(id.pairs + first + min(c, ncol - 1));   // short tiles repeat their last pair
                 const int t = p / id.n_used, i = p - t * id.n_used;
                 cols[c] = (i % id.ne11) + t * id.ne11;
-                outs[c] = t * id.ld2 + i * id.ld1;
+                outs[c] = t * id.ld2 + i * id.ld1 + (tile2 < n_tiles ? 0 : id.dst_off);
             }
         } else {
 #pragma unroll

@@ -35,7 +35,7 @@ static b200q_status launch_one(b200q_ctx *ctx, const void *w, size_t row_stride,
         occ[rows] = n > 0 ? n : 1;
     }
     const int64_t n_bt = (M + B - 1) / B;
-    const int64_t n_units = ID ? n_bt * max_tiles : n_bt;      // ID: an upper bound, the kernel reads the count
+    const int64_t n_units = ID ? n_bt * max_tiles * id.n_mat : n_bt;      // ID: an upper bound, the kernel reads the count
     int64_t blocks = (n_units + WARPS - 1) / WARPS;
     const int64_t cap = (int64_t)ctx->sm_count * occ[rows];
     if (blocks > cap) blocks = cap;

@@ -182,8 +182,8 @@ b200q_status b200q_moe_ffn(b200q_ctx *ctx, const b200q_tensor *gate_w, const b20
     b200q_tensor g = tensor(B200Q_TYPE_F32, ws + o_g, d_ff, n_used, n_tok, ws + o_g);
     b200q_tensor u = tensor(B200Q_TYPE_F32, ws + o_u, d_ff, n_used, n_tok, ws + o_u);
     b200q_tensor d = tensor(B200Q_TYPE_F32, ws + o_d, d_model, n_used, n_tok, ws + o_d);
-    st = b200q_mul_mat_id(ctx, gate_w, &x3, &ids, &g);
-    if (st == B200Q_OK) st = b200q_mul_mat_id(ctx, up_w, &x3, &ids, &u);
+    // gate and up: one launch for both where the GEMV takes them (one token, 512 experts of 2048 x 512: seven launches become six)
+    st = mul_mat_id(ctx, gate_w, &x3, &ids, &g, 0, up_w, &u);
     // the activation of the down projection is silu(gate) * up, computed where it is quantized
     if (st == B200Q_OK) st = mul_mat_id(ctx, down_w, &u, &ids, &d, (const float *)g.data - (const float *)u.data);
     if (st == B200Q_OK) {

@@ -120,3 +120,10 @@ def test_ffn_block_on_the_tensor_cores(monkeypatch, t, d_ff, i8):
     with A.Context(0) as c:
         test_ffn_block_against_the_fp64_chain_and_the_unfused_sequence(c, t, 8, 2, 512, d_ff, 150)
         assert c.stats()["moe_gemm"] == 6                  # gate, up and down, in the block and in the sequence it is compared with
+
+
+@pytest.mark.parametrize("t", [A.Q4_K, A.Q6_K, A.Q8_0])
+@pytest.mark.parametrize("n_tok", [1, 4, 5, 40])
+def test_gate_and_up_in_one_launch(ctx, t, n_tok):
+    """A pair a unit up to four tokens, tiles of 1, 2, 4 and 8 pairs beyond; Q6_K rows of 420 bytes begin anywhere."""
+    test_ffn_block_against_the_fp64_chain_and_the_unfused_sequence(ctx, t, 8, 4, 512, 256, n_tok)
