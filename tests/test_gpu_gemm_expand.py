@@ -18,9 +18,9 @@ def ctx():
 
 
 # the last column tile with one column, or whole; one super-block; row tiles with one row or all but one; rows that are no
-# multiple of 16 bytes, cut along K
+# multiple of 16 bytes, cut along K (a product of three super-blocks an SM and more)
 @pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
-@pytest.mark.parametrize("m,k,n", [(1, 256, 385), (129, 512, 512), (255, 768, 400), (300, 11008, 449), (128 * 40, 512, 520)])
+@pytest.mark.parametrize("m,k,n", [(1, 28672, 385), (129, 14336, 512), (255, 14336, 400), (300, 11008, 449), (128 * 112, 256, 385), (128 * 60, 512, 520)])
 def test_expanded_operand(ctx, t, m, k, n):
     n += MORE[t]
     w, x = data(t, m, k, n, 40 + m + n)
@@ -39,10 +39,10 @@ def test_chunks_of_row_tiles(ctx):
 
 @pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
 def test_without_scratch(t):
-    """The unpacking kernel takes the product where the scratch (2.2 MB) cannot be had."""
-    m, k, n = 1300, 768, 400 + MORE[t]
+    """The unpacking kernel takes the product where the scratch (8.7 MB) cannot be had."""
+    m, k, n = 1300, 3072, 400 + MORE[t]
     w, x = data(t, m, k, n, 9)
     with A.Context(0) as c:
-        c.scratch_limit(1 << 20)
+        c.scratch_limit(4 << 20)
         got = c.run_mul_mat(t, w, k, x)
     check(got, t, w, k, x)
