@@ -922,14 +922,17 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     return B200Q_OK;
 }
 
-// Whether a dense product takes the expanded operand: it saves a fifth to a third of a column tile's time and costs a pass that writes two
-// bytes a weight. Quantizer included, unpacking and expanded, us, at 2, 3, 4 and 6 column tiles:
-//   Q6_K   4096x11008  64.3 85.2 114.2 158.7   63.9 79.3 88.3 122.4
-//   IQ4_XS 4096x11008  59.2 79.3 104.4 145.6   62.2 77.6 86.6 121.1      11008x4096  53.8 62.1 87.3 114.7   71.5 72.0 90.2 112.7
+// Whether a dense product takes the expanded operand: it saves part of a column tile's time and costs a pass that writes two bytes a
+// weight. Quantizer included, unpacking and expanded, us. Rows that no tensor map describes (copied row by row where they are
+// unpacked), at 3, 4 and 6 column tiles:
+//   Q6_K 4096x11008 85.2 114.2 158.7   79.3 88.3 122.4;  IQ4_XS 4096x11008 79.3 104.4 145.6   77.6 86.6 121.1
+// (three tiles, other shapes: 12 to 20 % slower). The others, at 4 and 5 (IQ4_XS 6 and 8) tiles:
+//   Q6_K 32000x4096 224 282   269 285;  2048x5120 37.0 49.1   32.6 39.8;  IQ4_XS 4096x4096 55.1 62.8   56.2 57.0;  11008x4096 118 149   116 140;
+//   32000x4096 318   329
 // and at sixteen, IQ4_XS 17408x5120, 532 and 457. A small product does not earn the launch: Q6_K 512x2048 x 600 tokens, one super-block of
-// a tile an SM, 16.8 and 18.5 us; IQ4_XS 512x5120 x 700, three, 22.6 and 21.5.
-static bool expand_wanted(const b200q_ctx *ctx, int type, int64_t M, int64_t K, int64_t n_tiles) {
-    return n_tiles >= (type == B200Q_TYPE_Q6_K ? 4 : 6) && (M + kq::BM - 1) / kq::BM * n_tiles * (K / 256) >= 3 * ctx->sm_count;
+// a tile an SM, 16.8 and 18.5 us.
+static bool expand_wanted(const b200q_ctx *ctx, bool row_by_row, int64_t M, int64_t K, int64_t n_tiles) {
+    return n_tiles >= (row_by_row ? 4 : 8) && (M + kq::BM - 1) / kq::BM * n_tiles * (K / 256) >= 3 * ctx->sm_count;
 }
 
 // The product from the expanded operand, a chunk of row tiles at a time; *took: false when the scratch cannot be had
@@ -984,7 +987,8 @@ b200q_status launch_gemm_kq(b200q_ctx *ctx, int type, const void *w, size_t row_
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + kq::BN - 1) / kq::BN;
     const size_t ms = row_stride * (size_t)M;
-    if (expand_wanted(ctx, type, M, K, n_tiles) && (type == B200Q_TYPE_IQ4_XS || type == B200Q_TYPE_Q6_K)) {
+    const bool row_by_row = row_stride % 16 != 0 || K % (type == B200Q_TYPE_Q6_K ? 2048 : 512) != 0;
+    if (expand_wanted(ctx, row_by_row, M, K, n_tiles) && (type == B200Q_TYPE_IQ4_XS || type == B200Q_TYPE_Q6_K)) {
         bool took = false;
         const b200q_status st = type == B200Q_TYPE_IQ4_XS ? launch_kx_t<B200Q_TYPE_IQ4_XS>(ctx, w, row_stride, M, K, act, N, n_tiles, dst, ldd, &took)
                                                           : launch_kx_t<B200Q_TYPE_Q6_K>(ctx, w, row_stride, M, K, act, N, n_tiles, dst, ldd, &took);
