@@ -519,9 +519,10 @@ b200q_status b200q::mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
                      : launch_gemm_kq_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready);
         return st == B200Q_OK && src0b ? mul_mat_id(ctx, src0b, src1, ids, dstb, gate) : st;
     }
-    // two products of one form are one launch
+    // Two products of one form are one launch. It reads both matrices in one row mode, so they begin at the same place inside a 16-byte
+    // unit: an aligned one is not dragged to the copy loop of the other, nor away from the tensor cores that the other cannot take.
     const bool both = src0b && src0b->type == src0->type && src0b->ne[1] == M && src0b->ne[2] == n_expert && src0b->nb[1] == src0->nb[1] && src0b->nb[2] == src0->nb[2] &&
-                      dstb->nb[1] == dst->nb[1] && dstb->nb[2] == dst->nb[2];
+                      ((uintptr_t)src0b->data ^ (uintptr_t)src0->data) % 16 == 0 && dstb->nb[1] == dst->nb[1] && dstb->nb[2] == dst->nb[2];
     const void *w2 = both ? src0b->data : nullptr;
     float *dst2 = both ? (float *)dstb->data : nullptr;
     ActView act;

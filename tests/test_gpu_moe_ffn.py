@@ -127,3 +127,49 @@ def test_ffn_block_on_the_tensor_cores(monkeypatch, t, d_ff, i8):
 def test_gate_and_up_in_one_launch(ctx, t, n_tok):
     """A pair a unit up to four tokens, tiles of 1, 2, 4 and 8 pairs beyond; Q6_K rows of 420 bytes begin anywhere."""
     test_ffn_block_against_the_fp64_chain_and_the_unfused_sequence(ctx, t, 8, 4, 512, 256, n_tok)
+
+
+@pytest.mark.parametrize("t,t_up,off_gate,off_up,n_tok,want", [
+    # one launch for both where they begin alike inside a 16-byte unit, the down projection's beside it ...
+    (A.Q4_K, A.Q4_K, 0, 0, 1, (2, 0, 0)), (A.Q4_K, A.Q4_K, 8, 8, 4, (1, 1, 0)), (A.Q4_K, A.Q4_K, 0, 0, 5, (8, 0, 0)),
+    # ... two, each in its own row mode, where they do not, or are of two types
+    (A.Q4_K, A.Q4_K, 0, 8, 1, (2, 1, 0)), (A.Q4_K, A.Q4_K, 8, 0, 5, (8, 4, 0)), (A.IQ4_XS, A.IQ4_XS, 0, 4, 3, (2, 1, 0)),
+    (A.Q4_K, A.Q5_K, 0, 0, 2, (3, 0, 0)), (A.Q4_0, A.Q8_0, 0, 2, 5, (8, 4, 0)),
+    # prompt widths: only the stack that begins off 16 bytes stays with the GEMV
+    (A.Q4_K, A.Q4_K, 8, 0, 150, (0, 4, 2)), (A.Q4_K, A.Q4_K, 0, 8, 150, (0, 4, 2)), (A.Q8_0, A.Q8_0, 2, 0, 150, (0, 4, 2)), (A.Q8_0, A.Q8_0, 2, 2, 150, (0, 4, 1))])
+def test_which_gate_and_up_share_a_launch(ctx, t, t_up, off_gate, off_up, n_tok, want):
+    """(GEMV launches with 16-byte rows, with others, products on the tensor cores) of a block, and its values against the separate calls:
+    the same products of the same codes."""
+    n_exp, n_used, d_model, d_ff = 8, 2, 512, 512
+    rng = np.random.default_rng(n_tok)
+
+    def stack(ty, k, m, seed, off):
+        w = np.stack([make_weights(ty, m, k, seed + e) for e in range(n_exp)])
+        rb = w.shape[-1]
+        dev = ctx.upload(np.concatenate([np.zeros(off, np.uint8), w.reshape(-1)]))
+        return dev, A.Tensor.make(ty, [k, m, n_exp, 1], [A.block_bytes(ty), rb, rb * m, rb * m * n_exp], dev + off)
+
+    (dg, G), (du, U), (dd, D) = stack(t, d_model, d_ff, 800, off_gate), stack(t_up, d_model, d_ff, 900, off_up), stack(t, d_ff, d_model, 1000, 0)
+    x = ctx.upload(rng.normal(0, 1, size=(n_tok, d_model)).astype(np.float32))
+    logits = ctx.upload(rng.normal(0, 1.5, size=(n_tok, n_exp)).astype(np.float32))
+    y, ids, wts = ctx.alloc(n_tok * d_model * 4), ctx.alloc(n_tok * n_used * 4), ctx.alloc(n_tok * n_used * 4)
+    I = A.Tensor.make(A.I32, [n_used, n_tok, 1, 1], [4, 4 * n_used], ids)
+    ctx.graph_begin()
+    ctx.stats_reset()
+    ctx.moe_ffn(G, U, D, A.Tensor.f32(x, [d_model, n_tok]), A.Tensor.f32(logits, [n_exp, n_tok]), n_used, 6.103515625e-5, float("inf"),
+                A.Tensor.f32(y, [d_model, n_tok]), I, A.Tensor.f32(wts, [n_used, n_tok]))
+    got, st = ctx.download(y, (n_tok, d_model), np.float32), ctx.stats()
+    assert (st.get("gemv_id", 0), st.get("gemv_id_unaligned", 0), st.get("moe_gemm", 0)) == want, st
+    h = [ctx.alloc(n_tok * n_used * d_ff * 4) for _ in range(2)]
+    ctx.graph_begin()
+    for W, p in zip((G, U), h):
+        ctx.mul_mat_id(W, A.Tensor.f32(x, [d_model, 1, n_tok]), I, A.Tensor.f32(p, [d_ff, n_used, n_tok]))
+    g, u = (ctx.download(p, (n_tok, n_used, d_ff), np.float32).astype(np.float64) for p in h)
+    hd, od = ctx.upload((g / (1.0 + np.exp(-g)) * u).astype(np.float32)), ctx.alloc(n_tok * n_used * d_model * 4)
+    ctx.graph_begin()
+    ctx.mul_mat_id(D, A.Tensor.f32(hd, [d_ff, n_used, n_tok]), I, A.Tensor.f32(od, [d_model, n_used, n_tok]))
+    each = ctx.download(od, (n_tok, n_used, d_model), np.float32).astype(np.float64)
+    seq = (each * ctx.download(wts, (n_tok, n_used), np.float32)[:, :, None]).sum(axis=1)
+    assert nmse(got, seq) < 1e-6, nmse(got, seq)
+    for p in [dg, du, dd, x, logits, y, ids, wts, hd, od] + h:
+        ctx.free(p)
