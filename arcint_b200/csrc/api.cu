@@ -51,7 +51,7 @@ const char *stat_name(int s) {
     static const char *rest[] = { "gemv_id", "gemv_id_unaligned", "moe_route", "route_cache_hit", "moe_gemm", "moe_pack",
                                   "gemm_tc", "gemm_tc_quantize", "gemm_fallback_shape", "tp_allreduce", "tp_allgather",
                                   "ep_dispatch", "ep_combine", "graph_launch", "no_alloc", "gemm_kq_mins", "gemv_stream", "tp_allreduce_peer", "gemm_tc_f16", "ep_peer", "ep_dispatch_cached", "moe_router", "moe_ffn", "gemv_knob_ignored", "gemm_ksplit", "gemv_fused_quant", "gemv_allreduce_fused",
-                                  "ep_agreed_exit", "gemm_kq_rowcopy", "gemv_mma" };
+                                  "ep_agreed_exit", "gemm_kq_rowcopy", "gemv_mma", "gemm_kx" };
     return rest[s - ST_GEMV_ID];
 }
 
@@ -331,6 +331,8 @@ b200q_status b200q_init(b200q_ctx **out, int device, void *stream) {
     if (const char *v = getenv("B200Q_FUSE_QUANT_BYTES")) ctx->fuse_quant_bytes = atoll(v);
     const char *no_ks = getenv("B200Q_NO_KSPLIT");
     ctx->no_ksplit = no_ks && no_ks[0] == '1';
+    const char *no_ex = getenv("B200Q_NO_EXPAND");
+    ctx->no_expand = no_ex && no_ex[0] == '1';
     const char *no_small = getenv("B200Q_GEMV_NO_SMALL");
     ctx->gemv_no_small = no_small && no_small[0] == '1';
     const char *mma_min = getenv("B200Q_GEMV_MMA_MIN");  // fewest columns for the warp-MMA GEMV (99: never)
@@ -779,6 +781,12 @@ b200q_status b200q_debug_late_copy(b200q_ctx *ctx, void *dev_dst, const void *de
 b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes) {
     if (!ctx) return B200Q_INVALID;
     ctx->scratch_limit = bytes;
+    return B200Q_OK;
+}
+
+b200q_status b200q_debug_expand_limit(b200q_ctx *ctx, size_t bytes) {
+    if (!ctx) return B200Q_INVALID;
+    ctx->expand_most = bytes;
     return B200Q_OK;
 }
 

@@ -102,7 +102,7 @@ enum Stat {
     ST_GEMV_ID = ST_GEMV_UNALIGNED_COL0 + 9, ST_GEMV_ID_UNALIGNED, ST_MOE_ROUTE, ST_ROUTE_CACHE_HIT, ST_MOE_GEMM,
     ST_MOE_PACK, ST_GEMM_TC, ST_GEMM_TC_QUANT, ST_GEMM_FALLBACK_SHAPE, ST_TP_ALLREDUCE, ST_TP_ALLGATHER,
     ST_EP_DISPATCH, ST_EP_COMBINE, ST_GRAPH_LAUNCH, ST_NO_ALLOC, ST_GEMM_KQ_MINS, ST_GEMV_STREAM, ST_TP_ALLREDUCE_PEER, ST_GEMM_TC_F16, ST_EP_PEER, ST_EP_DISPATCH_CACHED, ST_MOE_ROUTER, ST_MOE_FFN, ST_GEMV_KNOB_IGNORED, ST_GEMM_KSPLIT, ST_GEMV_FUSED_QUANT, ST_GEMV_ALLREDUCE_FUSED,
-    ST_EP_AGREED_EXIT, ST_GEMM_KQ_ROWCOPY, ST_GEMV_MMA,
+    ST_EP_AGREED_EXIT, ST_GEMM_KQ_ROWCOPY, ST_GEMV_MMA, ST_GEMM_KX,
     ST_COUNT
 };
 const char *stat_name(int s);
@@ -137,6 +137,8 @@ struct b200q_ctx {
     // dependent launch). Measured on the 7B decode trace: -2 % at two GPUs, +38 % at eight (1.48 against 1.08 ms).
     int64_t      fuse_quant_bytes = 0;
     bool         no_ksplit = false;       // B200Q_NO_KSPLIT=1: never cut a prompt product along K
+    bool         no_expand = false;       // B200Q_NO_EXPAND=1: never expand the operand of a Q6_K / IQ4_XS prompt product (and take no scratch for it)
+    size_t       expand_most = (size_t)96 << 20;   // scratch of the expanded operand, a chunk of row tiles at a time: of 126 MB of L2 (b200q_debug_expand_limit)
     bool         canary = false;          // B200Q_CANARY=1: guard words around every scratch block, exact sizes (b200q_debug_check_guards)
     bool         gemv_mma_sets3 = false;  // B200Q_GEMV_MMA_SETS=3: a three-stage ring for the warp-MMA GEMV even where four stages fit
     int          gemv_mma_groups = 0;     // B200Q_GEMV_MMA_GROUPS=1: blocks of one group (several blocks per SM) instead of one block per SM

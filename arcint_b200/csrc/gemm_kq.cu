@@ -932,7 +932,7 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
 // and at sixteen, IQ4_XS 17408x5120, 532 and 457. A small product does not earn the launch: Q6_K 512x2048 x 600 tokens, one super-block of
 // a tile an SM, 16.8 and 18.5 us.
 static bool expand_wanted(const b200q_ctx *ctx, bool row_by_row, int64_t M, int64_t K, int64_t n_tiles) {
-    return n_tiles >= (row_by_row ? 4 : 8) && (M + kq::BM - 1) / kq::BM * n_tiles * (K / 256) >= 3 * ctx->sm_count;
+    return !ctx->no_expand && n_tiles >= (row_by_row ? 4 : 8) && (M + kq::BM - 1) / kq::BM * n_tiles * (K / 256) >= 3 * ctx->sm_count;
 }
 
 // The product from the expanded operand, a chunk of row tiles at a time; *took: false when the scratch cannot be had
@@ -941,8 +941,7 @@ static b200q_status launch_kx_t(b200q_ctx *ctx, const void *w, size_t row_stride
                                 int64_t n_tiles, float *dst, int64_t ldd, bool *took) {
     const int64_t nsb = K / 256, tiles_m = (M + kq::BM - 1) / kq::BM;
     const size_t per_tile = (size_t)nsb * kq::EXP_CHUNK;
-    constexpr size_t MOST = (size_t)96 << 20;                  // of 126 MB of L2
-    int64_t chunk = (int64_t)(MOST / per_tile);
+    int64_t chunk = (int64_t)(ctx->expand_most / per_tile);
     chunk = chunk < 1 ? 1 : chunk < tiles_m ? chunk : tiles_m;
     const int64_t chunks = (tiles_m + chunk - 1) / chunk;
     chunk = (tiles_m + chunks - 1) / chunks;                   // of about equal size
@@ -972,9 +971,9 @@ static b200q_status launch_kx_t(b200q_ctx *ctx, const void *w, size_t row_stride
         B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, dim3((unsigned)(units < ctx->sm_count ? units : ctx->sm_count)), dim3(kq::X_THREADS), (size_t)kq::X_TOTAL, ctx->stream,
                                    (const uint8_t *)ws->ptr, (int)M, (int)K, act, (int)N, (int)n_tiles, (int)t0, (int)nt, ksplit, out, out_ld, part_stride, ctx->error_word));
         B200Q_CUDA(ctx, cudaGetLastError());
+        count(ctx, ST_GEMM_KX);                                // one a chunk
     }
     count(ctx, ST_GEMM_TC);
-    if (row_stride % 16 != 0 || K % (TYPE == B200Q_TYPE_Q6_K ? 2048 : 512) != 0) count(ctx, ST_GEMM_KQ_ROWCOPY);     // rows that no tensor map describes
     if (ksplit > 1) return launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd);
     return B200Q_OK;
 }

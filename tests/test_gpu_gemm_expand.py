@@ -1,5 +1,6 @@
 """Q6_K and IQ4_XS prompts of eight column tiles and more (four where rows are copied one by one), whose operand is expanded once: tile edges, parts of K, chunks of row tiles
 and the way back to the unpacking kernel, against the fp64 product of the same quantized operands. (the bound: `gpu_util.check_sums`)"""
+import numpy as np
 import pytest
 
 import arcint_b200 as A
@@ -23,15 +24,57 @@ def test_expanded_operand(ctx, t, m, k, n):
     w, x = data(t, m, k, n, 40 + m + n)
     ctx.stats_reset()
     got = ctx.run_mul_mat(t, w, k, x)
-    assert ctx.stats().get("gemm_tc", 0) == 1
+    assert (ctx.stats().get("gemm_tc", 0), ctx.stats().get("gemm_kx", 0), ctx.stats().get("gemm_kq_rowcopy", 0)) == (1, 1, 0)
     check(got, t, w, k, x)
 
 
+@pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
+def test_many_units_per_block(ctx, t):
+    """Whole column tiles, more units than SMs: the rings run over several units of one block."""
+    m, k, n = 128 * 60, 512, 128 * 8
+    w, x = data(t, m, k, n, 5)
+    ctx.stats_reset()
+    got = ctx.run_mul_mat(t, w, k, x)
+    assert ctx.stats().get("gemm_kx", 0) == 1 and ctx.stats().get("gemm_ksplit", 0) == 0
+    check(got, t, w, k, x)
+
+
+# Two row tiles of a chunk's scratch, five in all: three chunks, the last of one tile that has 88 rows. Parts of K or none, the last
+# column tile ragged or whole; called twice in a row, so that the first chunk follows the last, and replayed from a recording.
+@pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
+@pytest.mark.parametrize("n", [1100, 1152])
+@pytest.mark.parametrize("no_ksplit", ["", "1"])
+def test_chunks(monkeypatch, t, n, no_ksplit):
+    m, k = 600, 2560
+    monkeypatch.setenv("B200Q_NO_KSPLIT", no_ksplit)
+    w, x = data(t, m, k, n, 6)
+    with A.Context(0) as c:
+        c.expand_limit(2 * (k // 256) * 66048)
+        p = c.upload(w), c.upload(x), c.alloc(n * m * 4)
+        mm = A.Tensor.weights(t, p[0], k, m), A.Tensor.f32(p[1], [k, n]), A.Tensor.f32(p[2], [m, n])
+        c.graph_begin()
+        c.mul_mat(*mm)
+        c.mul_mat(*mm)
+        check(c.download(p[2], (n, m), np.float32), t, w, k, x)
+        st = c.stats()
+        assert (st["gemm_tc"], st["gemm_kx"], st.get("gemm_ksplit", 0)) == (2, 6, 0 if no_ksplit else 2), st
+        g = c.capture(lambda: [c.mul_mat(*mm) for _ in range(2)])
+        c.upload(-x, p[1])
+        c.upload(np.zeros((n, m), np.float32), p[2])
+        c.graph_launch(g)
+        check(c.download(p[2], (n, m), np.float32), t, w, k, -x)
+        assert c.stats()["gemm_kx"] == 12 and c.stats()["workspace_grow"] == st["workspace_grow"]
+        c.graph_free(g)
+
+
 def test_chunks_of_row_tiles(ctx):
-    """K = 17408: 21 row tiles fill the expanded operand's scratch, the 22nd makes a second chunk."""
-    t, m, k, n = A.Q6_K, 21 * 128 + 60, 17408, 385
+    """K = 17408: a row tile is 68 x 66,048 bytes and 96 MB hold 22 of them, so that 23 are chunks of 12 and 11."""
+    t, m, k, n = A.Q6_K, 22 * 128 + 60, 17408, 385
     w, x = data(t, m, k, n, 3)
-    check(ctx.run_mul_mat(t, w, k, x), t, w, k, x)
+    ctx.stats_reset()
+    got = ctx.run_mul_mat(t, w, k, x)
+    assert ctx.stats().get("gemm_kx", 0) == 2
+    check(got, t, w, k, x)
 
 
 @pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
@@ -42,4 +85,19 @@ def test_without_scratch(t):
     with A.Context(0) as c:
         c.scratch_limit(4 << 20)
         got = c.run_mul_mat(t, w, k, x)
+        assert (c.stats()["gemm_tc"], c.stats().get("gemm_kx", 0)) == (1, 0)
+        c.scratch_limit(0)
+        c.run_mul_mat(t, w, k, x)
+        assert c.stats()["gemm_kx"] == 1
+    check(got, t, w, k, x)
+
+
+def test_switched_off(monkeypatch):
+    """B200Q_NO_EXPAND=1: no scratch, the unpacking kernel."""
+    t, m, k, n = A.Q6_K, 300, 11008, 449
+    monkeypatch.setenv("B200Q_NO_EXPAND", "1")
+    w, x = data(t, m, k, n, 10)
+    with A.Context(0) as c:
+        got = c.run_mul_mat(t, w, k, x)
+        assert c.stats().get("gemm_kx", 0) == 0 and c.stats()["gemm_kq_rowcopy"] == 1
     check(got, t, w, k, x)

@@ -52,6 +52,18 @@ def test_many_units_per_block(ctx, t):
     check(got, t, w, k, x)
 
 
+# (K = 1280: ten activation stages of the per-32 GEMM a unit, in rings of three and four)
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("k", [512, 1280])
+def test_many_units_of_whole_tiles_per_block(ctx, t, k):
+    m, n = 128 * 60, 128 * 4
+    w, x = data(t, m, k, n, 8)
+    ctx.stats_reset()
+    got = ctx.run_mul_mat(t, w, k, x)
+    assert ctx.stats().get("gemm_tc", 0) == 1 and ctx.stats().get("gemm_ksplit", 0) == 0
+    check(got, t, w, k, x)
+
+
 def integer_blocks(t, m, nsb, rng, low):
     """Packed super-blocks with d = 1, dmin = 0, every sub-scale 63 and codes low .. top, and the weights as integers [m, 256 nsb]"""
     top = 15 if t == A.Q4_K else 31
