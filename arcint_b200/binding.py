@@ -376,7 +376,7 @@ class Context:
         self.check(self.L.b200q_debug_scratch_limit(self.h, nbytes))
 
     def expand_limit(self, nbytes):
-        """the scratch of an expanded Q6_K / IQ4_XS operand from here on, at least one row tile at a time"""
+        """every Q6_K / IQ4_XS prompt product from here on: expanded operand, in chunks of at most nbytes or one row tile (0: by the rule)"""
         self.check(self.L.b200q_debug_expand_limit(self.h, nbytes))
 
     # ---- numpy conveniences for tests ----

@@ -786,7 +786,7 @@ b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes) {
 
 b200q_status b200q_debug_expand_limit(b200q_ctx *ctx, size_t bytes) {
     if (!ctx) return B200Q_INVALID;
-    ctx->expand_most = bytes;
+    ctx->expand_limit = bytes;
     return B200Q_OK;
 }
 

@@ -138,7 +138,7 @@ struct b200q_ctx {
     int64_t      fuse_quant_bytes = 0;
     bool         no_ksplit = false;       // B200Q_NO_KSPLIT=1: never cut a prompt product along K
     bool         no_expand = false;       // B200Q_NO_EXPAND=1: never expand the operand of a Q6_K / IQ4_XS prompt product (and take no scratch for it)
-    size_t       expand_most = (size_t)96 << 20;   // scratch of the expanded operand, a chunk of row tiles at a time: of 126 MB of L2 (b200q_debug_expand_limit)
+    size_t       expand_limit = 0;        // b200q_debug_expand_limit: every prompt product of the two types is expanded, in chunks of so many bytes (0: by the rule)
     bool         canary = false;          // B200Q_CANARY=1: guard words around every scratch block, exact sizes (b200q_debug_check_guards)
     bool         gemv_mma_sets3 = false;  // B200Q_GEMV_MMA_SETS=3: a three-stage ring for the warp-MMA GEMV even where four stages fit
     int          gemv_mma_groups = 0;     // B200Q_GEMV_MMA_GROUPS=1: blocks of one group (several blocks per SM) instead of one block per SM
@@ -283,10 +283,18 @@ b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, i
 
 // K parts of a product whose tiles fill the SMs badly, and the scratch for their results (ksplit.cu). It counts with a kernel's times
 // on full tiles: a step of 256 weights, and what a unit costs beyond its steps (fill, drain, stores). Measured from products of one
-// round, 16 and 43 steps long (TC: gemm_t32; the int8 arm takes the same, so that both cut a product alike).
+// round, 16 and 43 steps long (TC: gemm_t32; the int8 arm takes the same, so that both cut a product alike; KX: 172 products of one to
+// eleven chunks). chunks: the product is so many launches of `tiles` tiles each, one after the other.
 struct KsplitTimes { int step_ns, unit_ns; };
-constexpr KsplitTimes TC_TIMES = { 2500, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 }, KX_TIMES = { 1300, 1500 };
-int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts);
+constexpr KsplitTimes TC_TIMES = { 2500, 1500 }, KQ_TIMES = { 1900, 1200 }, KF_TIMES = { 1400, 1200 }, KX_TIMES = { 1050, 1300 };
+constexpr int MOST_PARTS = 8;
+int          choose_ksplit(const b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t outputs, int64_t most, int64_t chunks = 1);
+int          plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts, int64_t chunks = 1);
+// the nanoseconds of `tiles` tiles in ks parts, and of the pass that adds the parts up
+inline int64_t schedule_ns(const b200q_ctx *ctx, int64_t tiles, int64_t steps, int64_t ks, KsplitTimes t) {
+    return (tiles * ks + ctx->sm_count - 1) / ctx->sm_count * ((steps + ks - 1) / ks * t.step_ns + t.unit_ns);
+}
+inline int64_t ksplit_sum_ns(int64_t ks, int64_t outputs) { return ks > 1 ? 2500 + outputs * (ks + 1) / 1000 : 0; }
 
 // gemm_kq.cu (IQ4_XS, Q6_K: two int8 limbs), gemm_kf.cu (Q4_K, Q5_K: f16): tensor-core prefill GEMM of the super-block types
 // (integer sub-scales folded into the weight operand)

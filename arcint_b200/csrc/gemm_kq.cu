@@ -922,17 +922,42 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     return B200Q_OK;
 }
 
+// Row tiles of a chunk: as many as 96 MB (of 126 MB of L2) hold, at least one, in chunks of about equal size
+static int64_t expand_chunk(const b200q_ctx *ctx, int64_t nsb, int64_t tiles_m) {
+    int64_t chunk = (int64_t)((ctx->expand_limit ? ctx->expand_limit : (size_t)96 << 20) / ((size_t)nsb * kq::EXP_CHUNK));
+    chunk = chunk < 1 ? 1 : chunk < tiles_m ? chunk : tiles_m;
+    const int64_t chunks = (tiles_m + chunk - 1) / chunk;
+    return (tiles_m + chunks - 1) / chunks;
+}
+
 // Whether a dense product takes the expanded operand: it saves part of a column tile's time and costs a pass that writes two bytes a
 // weight. Quantizer included, unpacking and expanded, us. Rows that no tensor map describes (copied row by row where they are
 // unpacked), at 3, 4 and 6 column tiles:
 //   Q6_K 4096x11008 85.2 114.2 158.7   79.3 88.3 122.4;  IQ4_XS 4096x11008 79.3 104.4 145.6   77.6 86.6 121.1
-// (three tiles, other shapes: 12 to 20 % slower). The others, at 4 and 5 (IQ4_XS 6 and 8) tiles:
-//   Q6_K 32000x4096 224 282   269 285;  2048x5120 37.0 49.1   32.6 39.8;  IQ4_XS 4096x4096 55.1 62.8   56.2 57.0;  11008x4096 118 149   116 140;
-//   32000x4096 318   329
-// and at sixteen, IQ4_XS 17408x5120, 532 and 457. A small product does not earn the launch: Q6_K 512x2048 x 600 tokens, one super-block of
-// a tile an SM, 16.8 and 18.5 us.
-static bool expand_wanted(const b200q_ctx *ctx, bool row_by_row, int64_t M, int64_t K, int64_t n_tiles) {
-    return !ctx->no_expand && n_tiles >= (row_by_row ? 4 : 8) && (M + kq::BM - 1) / kq::BM * n_tiles * (K / 256) >= 3 * ctx->sm_count;
+// (three tiles, other shapes: 12 to 20 % slower), Q6_K 2048x5120 at 4 and 5: 37.0 49.1   32.6 39.8. The others, at 4 and 5 (IQ4_XS 6 and 8):
+//   Q6_K 32000x4096 224 282   269 285;  IQ4_XS 4096x4096 55.1 62.8   56.2 57.0;  11008x4096 118 149   116 140;  32000x4096 318   329
+// and at sixteen, IQ4_XS 17408x5120, 532 and 457 (Q6_K with a tensor map was not timed at six and seven). A small product does not
+// earn the launch: Q6_K 512x2048 x 600 tokens, one super-block of a tile an SM, 16.8 and 18.5 us.
+// Chunks that end in a badly filled round lose what the expansion saves (IQ4_XS 4736x11008 x 512: 76 and 72 units, 104 us unpacked and
+// 116 expanded), so both schedules are counted out, with the least squares of 172 products timed both ways (off by 2 % on average,
+// by 10 % at most): the unpacking kernel takes the product where it is shorter by a twelfth. Of the 172 none is then more than 3 %
+// slower than the better form.
+static bool expand_wanted(const b200q_ctx *ctx, int type, bool row_by_row, int64_t M, int64_t K, int64_t N, int64_t n_tiles) {
+    const int64_t nsb = K / 256, tiles_m = (M + kq::BM - 1) / kq::BM;
+    if (ctx->expand_limit && !ctx->no_expand) return true;
+    if (ctx->no_expand || n_tiles < (row_by_row ? 4 : 8) || tiles_m * n_tiles * nsb < 3 * ctx->sm_count) return false;
+    const bool q6 = type == B200Q_TYPE_Q6_K;
+    const int sps = !q6 && !row_by_row ? 2 : 1;                // super-blocks of a step, as in launch_kq_t
+    const KsplitTimes measured = row_by_row ? (q6 ? KsplitTimes{ 2370, 1370 } : KsplitTimes{ 2120, 1120 })
+                                            : (q6 ? KsplitTimes{ 1730, 750 } : KsplitTimes{ 2 * 1550, 1350 });
+    const int64_t ks = choose_ksplit(ctx, tiles_m * n_tiles, nsb / sps, { sps * KQ_TIMES.step_ns, KQ_TIMES.unit_ns }, M * N, MOST_PARTS);
+    const int64_t unpacked = schedule_ns(ctx, tiles_m * n_tiles, nsb / sps, ks, measured) + ksplit_sum_ns(ks, M * N);
+    const int64_t chunk = expand_chunk(ctx, nsb, tiles_m), chunks = (tiles_m + chunk - 1) / chunk;
+    const int64_t kx = choose_ksplit(ctx, chunk * n_tiles, nsb, KX_TIMES, M * N, MOST_PARTS, chunks);
+    const int64_t expanded = (chunks - 1) * schedule_ns(ctx, chunk * n_tiles, nsb, kx, KX_TIMES) +
+                             schedule_ns(ctx, (tiles_m - (chunks - 1) * chunk) * n_tiles, nsb, kx, KX_TIMES) + ksplit_sum_ns(kx, M * N) +
+                             chunks * 5300 + 2350 * tiles_m * nsb / ctx->sm_count;       // launches, and the expansion itself
+    return 12 * expanded <= 13 * unpacked;
 }
 
 // The product from the expanded operand, a chunk of row tiles at a time; *took: false when the scratch cannot be had
@@ -941,10 +966,7 @@ static b200q_status launch_kx_t(b200q_ctx *ctx, const void *w, size_t row_stride
                                 int64_t n_tiles, float *dst, int64_t ldd, bool *took) {
     const int64_t nsb = K / 256, tiles_m = (M + kq::BM - 1) / kq::BM;
     const size_t per_tile = (size_t)nsb * kq::EXP_CHUNK;
-    int64_t chunk = (int64_t)(ctx->expand_most / per_tile);
-    chunk = chunk < 1 ? 1 : chunk < tiles_m ? chunk : tiles_m;
-    const int64_t chunks = (tiles_m + chunk - 1) / chunk;
-    chunk = (tiles_m + chunks - 1) / chunks;                   // of about equal size
+    const int64_t chunk = expand_chunk(ctx, nsb, tiles_m);
     Workspace *ws = &ctx->moe_ws[10];
     *took = ws_try_reserve(ctx, ws, per_tile * (size_t)chunk);
     if (!*took) return B200Q_OK;
@@ -957,7 +979,7 @@ static b200q_status launch_kx_t(b200q_ctx *ctx, const void *w, size_t row_stride
         attr_set = true;
     }
     float *out = dst, *parts = nullptr;
-    const int ksplit = plan_ksplit(ctx, chunk * n_tiles, nsb, KX_TIMES, M, N, &parts);
+    const int ksplit = plan_ksplit(ctx, chunk * n_tiles, nsb, KX_TIMES, M, N, &parts, (tiles_m + chunk - 1) / chunk);
     int64_t out_ld = ldd, part_stride = 0;
     if (ksplit > 1) {
         out = parts;
@@ -987,7 +1009,7 @@ b200q_status launch_gemm_kq(b200q_ctx *ctx, int type, const void *w, size_t row_
     const int64_t n_tiles = (N + kq::BN - 1) / kq::BN;
     const size_t ms = row_stride * (size_t)M;
     const bool row_by_row = row_stride % 16 != 0 || K % (type == B200Q_TYPE_Q6_K ? 2048 : 512) != 0;
-    if (expand_wanted(ctx, row_by_row, M, K, n_tiles) && (type == B200Q_TYPE_IQ4_XS || type == B200Q_TYPE_Q6_K)) {
+    if ((type == B200Q_TYPE_IQ4_XS || type == B200Q_TYPE_Q6_K) && expand_wanted(ctx, type, row_by_row, M, K, N, n_tiles)) {
         bool took = false;
         const b200q_status st = type == B200Q_TYPE_IQ4_XS ? launch_kx_t<B200Q_TYPE_IQ4_XS>(ctx, w, row_stride, M, K, act, N, n_tiles, dst, ldd, &took)
                                                           : launch_kx_t<B200Q_TYPE_Q6_K>(ctx, w, row_stride, M, K, act, N, n_tiles, dst, ldd, &took);

@@ -32,12 +32,12 @@ ksplit_sum_kernel(const float *__restrict__ parts, int ksplit, int64_t part_stri
 // part, the pass that adds them (a launch and its traffic). t: a k-step (one raw stage) and a unit of the kernel, see common.cuh.
 // Of 17 shapes (tiles 12 to 768, 4 to 64 steps) in each of the seven types, timed at every number of parts, the choice is 0.6 % from
 // the fastest on average, at most 13 % (Q4_0 11008x4096 x 100 tokens: 75 us in three parts, 67 in five, 79 whole).
-static int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, KsplitTimes t, int64_t outputs, int64_t most) {
+int choose_ksplit(const b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t outputs, int64_t most, int64_t chunks) {
     int best_ks = 1;
     int64_t best = 0;
+    if (ctx->no_ksplit) return 1;
     for (int ks = 1; ks <= most && (ks == 1 || steps / ks >= 2); ++ks) {
-        const int64_t rounds = (tiles * ks + sms - 1) / sms;
-        const int64_t len = rounds * ((steps + ks - 1) / ks * t.step_ns + t.unit_ns) + (ks > 1 ? 2500 + outputs * (ks + 1) / 1000 : 0);
+        const int64_t len = chunks * schedule_ns(ctx, tiles, steps, ks, t) + ksplit_sum_ns(ks, outputs);
         if (ks == 1 || len < best) { best = len; best_ks = ks; }
     }
     return best_ks;
@@ -45,14 +45,13 @@ static int choose_ksplit(int64_t tiles, int64_t sms, int64_t steps, KsplitTimes 
 
 // The number of parts (1: the product stays whole) and where they go. Where the scratch cannot be had, on a full device or inside a
 // capture that would have to grow it, the product is cut into what the block there is holds.
-int plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts) {
-    if (ctx->no_ksplit) return 1;
+int plan_ksplit(b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t M, int64_t N, float **parts, int64_t chunks) {
     Workspace *ws = &ctx->moe_ws[9];
     const size_t part = sizeof(float) * (size_t)(N * M);
-    int ks = choose_ksplit(tiles, ctx->sm_count, steps, t, M * N, 8);
+    int ks = choose_ksplit(ctx, tiles, steps, t, M * N, MOST_PARTS, chunks);
     if (ks > 1 && !ws_try_reserve(ctx, ws, part * ks)) {
         const size_t hold = ws->cap / part;                 // (less than ks)
-        ks = choose_ksplit(tiles, ctx->sm_count, steps, t, M * N, hold < 1 ? 1 : (int64_t)hold);
+        ks = choose_ksplit(ctx, tiles, steps, t, M * N, hold < 1 ? 1 : (int64_t)hold, chunks);
     }
     *parts = (float *)ws->ptr;
     return ks;

@@ -41,8 +41,9 @@ B200Q_API b200q_status b200q_debug_late_copy(b200q_ctx *ctx, void *dev_dst, cons
 /* A fake of the failing allocation: from here on the context's scratch allocations of more than `bytes` bytes fail as on a
  * full device (0: none does). */
 B200Q_API b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes);
-/* The most scratch that the expanded operand of a wide Q6_K / IQ4_XS product takes from here on (96 MB at first): row tiles are
- * expanded and multiplied in chunks of so much, of one tile at least. Every chunk counts one "gemm_kx" in b200q_stats. */
+/* From here on every prompt product of Q6_K and IQ4_XS weights is multiplied from an expanded operand, in chunks of row tiles that take
+ * at most so many bytes of scratch, of one tile at least (0: by the library's own rule and limit again). Every chunk counts one
+ * "gemm_kx" in b200q_stats. */
 B200Q_API b200q_status b200q_debug_expand_limit(b200q_ctx *ctx, size_t bytes);
 
 #ifdef __cplusplus

@@ -1,5 +1,5 @@
-"""Q6_K and IQ4_XS prompts of eight column tiles and more (four where rows are copied one by one), whose operand is expanded once: tile edges, parts of K, chunks of row tiles
-and the way back to the unpacking kernel, against the fp64 product of the same quantized operands. (the bound: `gpu_util.check_sums`)"""
+"""Q6_K and IQ4_XS prompts whose operand is expanded once: tile edges, parts of K, chunks of row tiles, the rule that picks them and the
+way back to the unpacking kernel, against the fp64 product of the same quantized operands. (the bound: `gpu_util.check_sums`)"""
 import numpy as np
 import pytest
 
@@ -11,15 +11,18 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def ctx():
+    """every product of these types from an expanded operand, in chunks of the library's own size"""
     c = A.Context(0)
+    c.expand_limit(96 << 20)
     yield c
     c.close()
 
 
 # the last column tile with one column, or whole; one super-block; row tiles with one row or all but one; rows that are no
-# multiple of 16 bytes, cut along K (a product of three super-blocks an SM and more)
+# multiple of 16 bytes, cut along K; one column tile
 @pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
-@pytest.mark.parametrize("m,k,n", [(1, 28672, 897), (129, 14336, 1024), (255, 14336, 912), (300, 11008, 449), (128 * 56, 256, 897), (128 * 30, 512, 1032)])
+@pytest.mark.parametrize("m,k,n", [(1, 28672, 897), (129, 14336, 1024), (255, 14336, 912), (300, 11008, 449), (128 * 56, 256, 897), (128 * 30, 512, 1032),
+                                   (300, 1280, 9), (130, 512, 128)])
 def test_expanded_operand(ctx, t, m, k, n):
     w, x = data(t, m, k, n, 40 + m + n)
     ctx.stats_reset()
@@ -75,6 +78,24 @@ def test_chunks_of_row_tiles(ctx):
     got = ctx.run_mul_mat(t, w, k, x)
     assert ctx.stats().get("gemm_kx", 0) == 2
     check(got, t, w, k, x)
+
+
+@pytest.mark.parametrize("t,m,k,n,want", [
+    # (chunks, whether it is cut along K); none: the unpacking kernel. Few column tiles, a small product, chunks that end in bad rounds ...
+    (A.IQ4_XS, 4096, 4096, 512, (0, 0)), (A.Q6_K, 512, 2048, 600, (0, 0)), (A.IQ4_XS, 3072, 1280, 512, (0, 0)), (A.IQ4_XS, 4736, 11008, 512, (0, 0)),
+    # ... one chunk, whole and cut; five, whose rounds all count where the parts of K are chosen
+    (A.Q6_K, 4096, 11008, 512, (1, 0)), (A.Q6_K, 1024, 8192, 1024, (1, 1)), (A.Q6_K, 2048, 28672, 1024, (2, 1)), (A.IQ4_XS, 8192, 28672, 1024, (5, 1))])
+def test_the_rule(t, m, k, n, want):
+    with A.Context(0) as c:
+        one, x = data(t, 8, k, n, 12)
+        dw, dx, dy = c.upload(np.tile(one, (m // 8, 1))), c.upload(x), c.alloc(n * m * 4)
+        c.graph_begin()
+        c.mul_mat(A.Tensor.weights(t, dw, k, m), A.Tensor.f32(dx, [k, n]), A.Tensor.f32(dy, [m, n]))
+        got = c.download(dy, (n, m), np.float32)
+        st = c.stats()
+    assert st.get("gemm_kx", 0) == want[0] and (not want[0] or st.get("gemm_ksplit", 0) == want[1]), st
+    check(got[:, :8], t, one, k, x)
+    assert (got.reshape(n, -1, 8) == got[:, None, :8]).all()
 
 
 @pytest.mark.parametrize("t", [A.Q6_K, A.IQ4_XS])
