@@ -157,6 +157,7 @@ def lib():
     L.b200q_debug_dequantize.argtypes = [vp, TP, vp]
     L.b200q_debug_wait_timeout.argtypes = [vp, C.c_uint]
     L.b200q_debug_scratch_limit.argtypes = [vp, C.c_size_t]
+    L.b200q_debug_scratch_total.argtypes = [vp, C.c_size_t, C.POINTER(C.c_size_t)]
     L.b200q_debug_expand_limit.argtypes = [vp, C.c_size_t]
     L.b200q_debug_late_copy.argtypes = [vp, vp, vp, C.c_size_t, C.c_uint]
     L.b200q_debug_check_guards.argtypes = [vp, C.POINTER(C.c_int), C.POINTER(C.c_int)]
@@ -171,7 +172,7 @@ EXPORTS = [
     "b200q_all_gather", "b200q_mul_mat_allreduce", "b200q_all_to_all_v", "b200q_tp_check", "b200q_mul_mat_id_ep", "b200q_ep_reserve", "b200q_moe_router", "b200q_moe_ffn", "b200q_mul_mat_noalloc", "b200q_noalloc_last_error", "b200q_noalloc_device_error", "b200q_buffer_alloc", "b200q_buffer_free", "b200q_tensor_set",
     "b200q_tensor_get", "b200q_tensor_stage", "b200q_tensor_fetch", "b200q_tensor_copy", "b200q_synchronize", "b200q_host_alloc", "b200q_host_free",
     "b200q_stats", "b200q_stats_reset", "b200q_timer_start", "b200q_timer_stop", "b200q_flush_l2",
-    "b200q_debug_quantize_act", "b200q_debug_dequantize", "b200q_debug_wait_timeout", "b200q_debug_check_guards", "b200q_debug_scratch_limit", "b200q_debug_expand_limit", "b200q_debug_late_copy",
+    "b200q_debug_quantize_act", "b200q_debug_dequantize", "b200q_debug_wait_timeout", "b200q_debug_check_guards", "b200q_debug_scratch_limit", "b200q_debug_expand_limit", "b200q_debug_scratch_total", "b200q_debug_late_copy",
 ]
 
 
@@ -374,6 +375,12 @@ class Context:
     def scratch_limit(self, nbytes):
         """scratch allocations beyond nbytes fail from here on, as on a full device (0: none does)"""
         self.check(self.L.b200q_debug_scratch_limit(self.h, nbytes))
+
+    def scratch_total(self, nbytes):
+        """room for nbytes of scratch and one more allocation from here on, as on a full device (0: no limit); returns what it holds now"""
+        held = C.c_size_t(0)
+        self.check(self.L.b200q_debug_scratch_total(self.h, nbytes, C.byref(held)))
+        return held.value
 
     def expand_limit(self, nbytes):
         """every Q6_K / IQ4_XS prompt product from here on: expanded operand, in chunks of at most nbytes or one row tile (0: by the rule)"""

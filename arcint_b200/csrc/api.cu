@@ -67,8 +67,39 @@ b200q_status fail(b200q_ctx *ctx, b200q_status st, const char *fmt, ...) {
     return st;
 }
 
-// A block of `bytes` bytes into the empty *ws. *total: what was asked of the device.
-static cudaError_t ws_alloc(b200q_ctx *ctx, Workspace *ws, size_t bytes, size_t *total_out) {
+// The blocks a product can do without (the parts of K, the expanded operand) go back to the device. Counted as a growth: recorded graphs
+// that use them are stale. False: there are none, or a capture is open, whose nodes may use them.
+static bool ws_release_optional(b200q_ctx *ctx) {
+    Workspace *parts = &ctx->moe_ws[9], *expanded = &ctx->moe_ws[10];
+    if (ctx->capturing || (!parts->base && !expanded->base) || cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
+    ws_release(parts);
+    ws_release(expanded);
+    count(ctx, ST_WORKSPACE_GROW);
+    return true;
+}
+
+static size_t scratch_held(const b200q_ctx *ctx) {
+    size_t held = 0;
+    for (auto &e : ctx->act_cache) held += e.codes.cap + e.scales.cap + e.sums.cap + e.sums16.cap;
+    for (auto &w : ctx->moe_ws) held += w.cap;
+    return held;
+}
+
+static cudaError_t device_alloc_once(b200q_ctx *ctx, void **p, size_t bytes) {
+    if (ctx->scratch_total && scratch_held(ctx) + bytes > ctx->scratch_total) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) { *p = nullptr; (void)cudaGetLastError(); }
+    return e;
+}
+
+// Memory that a call needs: where the device is full, the optional scratch is given back first
+cudaError_t device_alloc(b200q_ctx *ctx, void **p, size_t bytes) {
+    const cudaError_t e = device_alloc_once(ctx, p, bytes);
+    return e == cudaErrorMemoryAllocation && ws_release_optional(ctx) ? device_alloc_once(ctx, p, bytes) : e;
+}
+
+// A block of `bytes` bytes into the empty *ws. *total: what was asked of the device. needed: see device_alloc.
+static cudaError_t ws_alloc(b200q_ctx *ctx, Workspace *ws, size_t bytes, size_t *total_out, bool needed) {
     // Normally whole megabytes, so that a slowly growing request does not reallocate every time. With guard words the block
     // has the size asked for (to 256 bytes), so that a write past the request lands in the guard and not in rounding slack.
     const size_t guard = ctx->canary ? WS_GUARD : 0;
@@ -76,12 +107,9 @@ static cudaError_t ws_alloc(b200q_ctx *ctx, Workspace *ws, size_t bytes, size_t 
     const size_t want = (bytes + unit - 1) / unit * unit;
     // (behind the tail guard another 64 KiB, so that a read past the block -- which no guard can see -- stays inside the allocation)
     const size_t total = *total_out = want + 2 * guard + (guard ? (size_t)64 << 10 : 0);
-    cudaError_t e = ctx->scratch_limit && total > ctx->scratch_limit ? cudaErrorMemoryAllocation : cudaMalloc(&ws->base, total);
-    if (e != cudaSuccess) {
-        ws->base = nullptr;
-        (void)cudaGetLastError();
-        return e;
-    }
+    if (ctx->scratch_limit && total > ctx->scratch_limit) return cudaErrorMemoryAllocation;
+    cudaError_t e = needed ? device_alloc(ctx, &ws->base, total) : device_alloc_once(ctx, &ws->base, total);
+    if (e != cudaSuccess) return e;
     ws->ptr = (uint8_t *)ws->base + guard;
     ws->cap = want;
     if (guard) {
@@ -106,7 +134,7 @@ b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
         ws->cap = 0;
     }
     size_t total = 0;
-    const cudaError_t e = ws_alloc(ctx, ws, bytes, &total);
+    const cudaError_t e = ws_alloc(ctx, ws, bytes, &total, true);
     if (e == cudaErrorMemoryAllocation) return fail(ctx, B200Q_NO_MEMORY, "cudaMalloc(%zu): %s", total, cudaGetErrorString(e));
     B200Q_CUDA(ctx, e);
     return B200Q_OK;
@@ -119,7 +147,7 @@ bool ws_try_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
     if (ctx->capturing) return false;
     Workspace next;
     size_t total = 0;
-    if (ws_alloc(ctx, &next, bytes, &total) != cudaSuccess) return false;
+    if (ws_alloc(ctx, &next, bytes, &total, false) != cudaSuccess) return false;
     // the old block may still be in use by work already enqueued on the stream
     if (ws->ptr && cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         ws_release(&next);                                   // (the launch that follows reports the stream's error)
@@ -616,7 +644,7 @@ b200q_status b200q_buffer_alloc(b200q_ctx *ctx, size_t bytes, void **dev_ptr) {
     if (!ctx || !dev_ptr) return B200Q_INVALID;
     *dev_ptr = nullptr;
     B200Q_CUDA(ctx, cudaSetDevice(ctx->device));
-    cudaError_t e = cudaMalloc(dev_ptr, bytes ? bytes : 1);
+    cudaError_t e = device_alloc(ctx, dev_ptr, bytes ? bytes : 1);
     if (e != cudaSuccess) return fail(ctx, B200Q_NO_MEMORY, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
     return B200Q_OK;
 }
@@ -781,6 +809,13 @@ b200q_status b200q_debug_late_copy(b200q_ctx *ctx, void *dev_dst, const void *de
 b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes) {
     if (!ctx) return B200Q_INVALID;
     ctx->scratch_limit = bytes;
+    return B200Q_OK;
+}
+
+b200q_status b200q_debug_scratch_total(b200q_ctx *ctx, size_t bytes, size_t *held) {
+    if (!ctx || !held) return B200Q_INVALID;
+    ctx->scratch_total = bytes;
+    *held = scratch_held(ctx);
     return B200Q_OK;
 }
 

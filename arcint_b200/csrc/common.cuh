@@ -146,6 +146,7 @@ struct b200q_ctx {
     int          gemv_mma_min = 0;        // B200Q_GEMV_MMA_MIN: fewest columns at which a product takes the warp-MMA GEMV (99: never; 0: Q6_K 3, Q8_0 7, the others 4, measured)
     bool         gemv_no_small = false;   // B200Q_GEMV_NO_SMALL=1: never the 128-thread, 170-register build of the wide Q6_K GEMV
     size_t       scratch_limit = 0;       // b200q_debug_scratch_limit: a scratch allocation beyond it fails as on a full device (0: none does)
+    size_t       scratch_total = 0;       // b200q_debug_scratch_total: so does an allocation that takes the context's activation and product scratch beyond it
     bool         no_stream = false;       // B200Q_NO_STREAM=1: every GEMV through the per-warp ring kernel (comparisons)
     std::string  last_error;
     std::string  stats_text;
@@ -168,6 +169,7 @@ b200q_status fail(b200q_ctx *ctx, b200q_status st, const char *fmt, ...);
 b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
 bool         ws_try_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
 void ws_release(Workspace *ws);
+cudaError_t  device_alloc(b200q_ctx *ctx, void **p, size_t bytes);
 int moe_route_workspaces(b200q_ctx *ctx, Workspace **out, const char **names);   // the route caches' blocks, for the guard check
 inline void  count(b200q_ctx *ctx, int stat) { ++ctx->counters[stat]; }
 

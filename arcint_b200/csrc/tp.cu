@@ -167,9 +167,9 @@ static void peer_ar_setup(b200q_ctx *ctx, TpState *tp, Nccl *api) {
     const char *off = getenv("B200Q_NO_PEER_AR");
     if ((off && off[0] == '1') || tp->nranks < 2 || tp->nranks > PEER_AR_MAX_RANKS) return;
     const int G = tp->nranks;
-    bool mine = cudaMalloc(&tp->ar_local, PEER_AR_BUFFER_BYTES) == cudaSuccess &&
+    bool mine = device_alloc(ctx, (void **)&tp->ar_local, PEER_AR_BUFFER_BYTES) == cudaSuccess &&
                 cudaMemset(tp->ar_local, 0, PEER_AR_BUFFER_BYTES) == cudaSuccess &&
-                cudaMalloc(&tp->ar_state, 2 * sizeof(uint32_t)) == cudaSuccess &&
+                device_alloc(ctx, (void **)&tp->ar_state, 2 * sizeof(uint32_t)) == cudaSuccess &&
                 cudaMemset(tp->ar_state, 0, 2 * sizeof(uint32_t)) == cudaSuccess;
     cudaIpcMemHandle_t h;
     memset(&h, 0, sizeof(h));
@@ -181,7 +181,7 @@ static void peer_ar_setup(b200q_ctx *ctx, TpState *tp, Nccl *api) {
     memcpy(rec.data(), &h, 64);
     rec[64] = mine ? 1 : 0;
     uint8_t *d = nullptr;
-    bool ok = cudaMalloc(&d, REC * (G + 1)) == cudaSuccess;
+    bool ok = device_alloc(ctx, (void **)&d, REC * (G + 1)) == cudaSuccess;
     auto gather = [&]() {
         return ok && cudaMemcpyAsync(d + REC * G, rec.data(), REC, cudaMemcpyHostToDevice, ctx->stream) == cudaSuccess &&
                api->AllGather(d + REC * G, d, REC, ncclInt8, tp->comm, ctx->stream) == ncclSuccess &&
@@ -284,7 +284,7 @@ b200q_status b200q_tp_init(b200q_ctx *ctx, const void *id128, int rank, int nran
         delete tp;
         return fail(ctx, B200Q_NCCL_ERROR, "ncclCommInitRank: %s", api->GetErrorString ? api->GetErrorString(r) : "error");
     }
-    if (cudaMalloc(&tp->agree_dev, sizeof(int32_t) * (size_t)(nranks + 1) * (nranks + 1)) != cudaSuccess) {
+    if (device_alloc(ctx, (void **)&tp->agree_dev, sizeof(int32_t) * (size_t)(nranks + 1) * (nranks + 1)) != cudaSuccess) {
         cudaGetLastError();
         if (api->CommDestroy) api->CommDestroy(tp->comm);
         delete tp;
@@ -442,11 +442,11 @@ b200q_status b200q_ep_reserve(b200q_ctx *ctx, int64_t max_pairs, int64_t max_k, 
     tp->ep_off_y = tp->ep_off_e + up(e_bytes);
     tp->ep_off_flags = tp->ep_off_y + up(y_bytes);
     const size_t total = tp->ep_off_flags + 4 * 2 * EP_MAX_RANKS * 8;
-    bool mine = cudaMalloc(&tp->ep_local, total) == cudaSuccess &&
+    bool mine = device_alloc(ctx, (void **)&tp->ep_local, total) == cudaSuccess &&
                 cudaMemset(tp->ep_local + tp->ep_off_flags, 0, total - tp->ep_off_flags) == cudaSuccess &&
-                cudaMalloc(&tp->ep_out, (size_t)G * cap * max_m * 4) == cudaSuccess &&
-                cudaMalloc(&tp->ep_ids, ((size_t)G * cap + EP_MAX_RANKS) * 4) == cudaSuccess &&
-                cudaMalloc(&tp->ep_state, 4 * sizeof(uint32_t)) == cudaSuccess &&
+                device_alloc(ctx, (void **)&tp->ep_out, (size_t)G * cap * max_m * 4) == cudaSuccess &&
+                device_alloc(ctx, (void **)&tp->ep_ids, ((size_t)G * cap + EP_MAX_RANKS) * 4) == cudaSuccess &&
+                device_alloc(ctx, (void **)&tp->ep_state, 4 * sizeof(uint32_t)) == cudaSuccess &&
                 cudaMemset(tp->ep_state, 0, 4 * sizeof(uint32_t)) == cudaSuccess;
     if (!mine) cudaGetLastError();
     tp->ep_counts = tp->ep_ids ? tp->ep_ids + (size_t)G * cap : nullptr;
@@ -458,7 +458,7 @@ b200q_status b200q_ep_reserve(b200q_ctx *ctx, int64_t max_pairs, int64_t max_k, 
     memcpy(rec.data(), &h, 64);
     rec[64] = mine ? 1 : 0;
     uint8_t *d = nullptr;
-    bool ok = cudaMalloc(&d, REC * (G + 1)) == cudaSuccess;
+    bool ok = device_alloc(ctx, (void **)&d, REC * (G + 1)) == cudaSuccess;
     auto gather = [&]() {
         return ok && cudaMemcpyAsync(d + REC * G, rec.data(), REC, cudaMemcpyHostToDevice, ctx->stream) == cudaSuccess &&
                api->AllGather(d + REC * G, d, REC, ncclInt8, tp->comm, ctx->stream) == ncclSuccess &&

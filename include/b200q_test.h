@@ -41,6 +41,9 @@ B200Q_API b200q_status b200q_debug_late_copy(b200q_ctx *ctx, void *dev_dst, cons
 /* A fake of the failing allocation: from here on the context's scratch allocations of more than `bytes` bytes fail as on a
  * full device (0: none does). */
 B200Q_API b200q_status b200q_debug_scratch_limit(b200q_ctx *ctx, size_t bytes);
+/* Another: from here on the device has room for `bytes` bytes of the context's activation, MoE and product scratch together with one
+ * more allocation, scratch or b200q_buffer_alloc (0: no such limit). *held: what that scratch takes now. */
+B200Q_API b200q_status b200q_debug_scratch_total(b200q_ctx *ctx, size_t bytes, size_t *held);
 /* From here on every prompt product of Q6_K and IQ4_XS weights is multiplied from an expanded operand, in chunks of row tiles that take
  * at most so many bytes of scratch, of one tile at least (0: by the library's own rule and limit again). Every chunk counts one
  * "gemm_kx" in b200q_stats. */

@@ -211,3 +211,36 @@ def test_prompt_product_waits_for_its_weights(ctx, t, cached):
     assert rel_err(got, O.mul_mat_f64(t, wb, k, x, True)) < TOL
     for q in p + (new,):
         ctx.free(q)
+
+
+@pytest.mark.parametrize("what", ["scratch", "buffer"])
+def test_optional_scratch_goes_back_to_a_full_device(what):
+    """A wide Q6_K product holds an expanded operand and parts of K; where the device is full after it, they make room for the activation of
+    another product or a caller's buffer. It counts as a growth, no error text stays, and the wide product runs without them."""
+    t, m, k, n = A.Q6_K, 1100, 3072, 1000
+    with A.Context(0) as ctx:
+        w, x, wide, p = prompt(ctx, t, m, k, n, 1)          # 7.1 MB of operand, 4.4 MB a part, 3.2 MB of activation
+        v, y, other, q = prompt(ctx, A.Q4_0, 64, 2048, 1000, 2)      # 5.5 MB of activation
+        ctx.expand_limit(96 << 20)
+        ctx.graph_begin()
+        ctx.mul_mat(*wide)
+        st = ctx.stats()
+        assert st["gemm_kx"] == 1 and st["gemm_ksplit"] == 1
+        held = ctx.scratch_total(0)
+        ctx.scratch_total(held + (1 << 20))
+        ctx.graph_begin()
+        if what == "scratch":
+            ctx.mul_mat(*other)
+            assert rel_err(ctx.download(q[2], (n, 64), np.float32), O.mul_mat_f64(A.Q4_0, v, 2048, y, True)) < TOL
+        else:
+            ctx.free(ctx.alloc(4 << 20))
+        assert ctx.stats()["workspace_grow"] > st["workspace_grow"] and ctx.L.b200q_last_error(ctx.h) == b""
+        left = ctx.scratch_total(0)
+        assert left < held - (4 << 20)
+        ctx.scratch_total(left + (4 << 20))                 # the wide product finds its own activation's block, but none of the optional ones
+        ctx.stats_reset()
+        ctx.graph_begin()
+        ctx.mul_mat(*wide)
+        assert rel_err(ctx.download(p[2], (n, m), np.float32), O.mul_mat_f64(t, w, k, x, True)) < TOL
+        st = ctx.stats()
+        assert (st["gemm_tc"], st.get("gemm_kx", 0), st.get("gemm_ksplit", 0)) == (1, 0, 0)
