@@ -106,9 +106,9 @@ static_assert(NCODE == 4 && NX == 3 && NG == 2 && BAR_COUNT <= 32, "barrier slot
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
 
 // The quantizer of the layout above, per-256 form (the reference's kernel_quant_i8 rule: scale bm/127, round to nearest
-// even, zero below 1e-30).
-template <bool GATE>
-__global__ void __launch_bounds__(1024)
+// even, zero below 1e-30). NT threads, a build each: see quantizer_threads.
+template <bool GATE, int NT>
+__global__ void __launch_bounds__(NT)
 quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
                     int64_t N, uint8_t *__restrict__ out, TileRoute id) {
     // One block per (tile, super-block); a half-warp per column at a time: its sixteen lanes read the column's 256
@@ -131,9 +131,9 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
         cnt = left < BN ? (int)left : BN;
     }
     const int live = ((cnt + 7) >> 3) << 3;
-    __shared__ int side_of_warp[32];
+    __shared__ int side_of_warp[NT / 32];
     int side = 0;                        // the largest one-sided sum of codes among this thread's columns
-    for (int col0 = 0; col0 < live; col0 += blockDim.x >> 4) {
+    for (int col0 = 0; col0 < live; col0 += NT / 16) {
         // (whole warps stay together for the shuffles: a half-warp past the live columns quantizes zeros and stores nothing)
         const int col = col0 + hw;
         const float *x = nullptr;
@@ -198,7 +198,7 @@ quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, s
     if ((threadIdx.x & 31) == 0) side_of_warp[threadIdx.x >> 5] = side;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int i = 1; i < (int)blockDim.x >> 5; ++i) side = max(side, side_of_warp[i]);
+        for (int i = 1; i < NT / 32; ++i) side = max(side, side_of_warp[i]);
         reinterpret_cast<int *>(out + (size_t)gridDim.y * nst * CHUNK)[(size_t)t * nst + s] = side;
     }
 }
@@ -719,8 +719,12 @@ bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 
 static b200q_status quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
+    const unsigned threads = quantizer_threads(ctx, src1, n_tiles, tr, 148, true);
+    auto kern = threads == 256   ? (tr.gate ? kf::quantize_f16_kernel<true, 256> : kf::quantize_f16_kernel<false, 256>)
+                : threads == 512 ? (tr.gate ? kf::quantize_f16_kernel<true, 512> : kf::quantize_f16_kernel<false, 512>)
+                                 : (tr.gate ? kf::quantize_f16_kernel<true, 1024> : kf::quantize_f16_kernel<false, 1024>);
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kf::quantize_f16_kernel<true> : kf::quantize_f16_kernel<false>, grid, dim3(quantizer_threads(N, &tr)), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(threads), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
                                src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);

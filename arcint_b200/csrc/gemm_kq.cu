@@ -864,7 +864,7 @@ bool gemm_kq_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 static b200q_status quantize256(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kq::quantize_tiled256_kernel<true> : kq::quantize_tiled256_kernel<false>, grid, dim3(quantizer_threads(N, &tr)), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kq::quantize_tiled256_kernel<true> : kq::quantize_tiled256_kernel<false>, grid, dim3(quantizer_threads(ctx, src1, n_tiles, tr, 480)), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
                                src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);

@@ -524,7 +524,7 @@ b200q_status launch_quantize_t32(b200q_ctx *ctx, const b200q_tensor *src1, uint8
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     const TileRoute &id = tr ? *tr : NO_ROUTE_T32;
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, id.gate ? t32::quantize_kernel<true> : t32::quantize_kernel<false>, grid, dim3(quantizer_threads(N, tr)), 0, ctx->stream,
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, id.gate ? t32::quantize_kernel<true> : t32::quantize_kernel<false>, grid, dim3(quantizer_threads(ctx, src1, n_tiles, id, 320)), 0, ctx->stream,
                                (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, id));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);
