@@ -123,7 +123,19 @@ static cudaError_t ws_alloc(b200q_ctx *ctx, Workspace *ws, size_t bytes, size_t 
 
 // grow-only scratch (the reference's prealloc_* buffers never shrink either)
 b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
-    if (bytes <= ws->cap) return B200Q_OK;
+    bool whole;
+    return ws_reserve_either(ctx, ws, bytes, bytes, &whole);
+}
+
+// Scratch for a call that prefers `best` bytes and can do with `least`; *got_best: which of the two *ws holds. A block that holds the
+// least is not given up for the try, so that a recording of its product stays good.
+b200q_status ws_reserve_either(b200q_ctx *ctx, Workspace *ws, size_t best, size_t least, bool *got_best) {
+    *got_best = true;
+    if (best <= ws->cap) return B200Q_OK;
+    if (least <= ws->cap) {
+        *got_best = ws_try_reserve(ctx, ws, best);
+        return B200Q_OK;
+    }
     if (ctx->capturing)
         return fail(ctx, B200Q_INVALID, "scratch would grow inside a capture: run the sequence once before capturing");
     if (ws->ptr) {
@@ -134,7 +146,11 @@ b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
         ws->cap = 0;
     }
     size_t total = 0;
-    const cudaError_t e = ws_alloc(ctx, ws, bytes, &total, true);
+    cudaError_t e = ws_alloc(ctx, ws, best, &total, true);
+    if (e == cudaErrorMemoryAllocation && least < best) {
+        *got_best = false;
+        e = ws_alloc(ctx, ws, least, &total, true);
+    }
     if (e == cudaErrorMemoryAllocation) return fail(ctx, B200Q_NO_MEMORY, "cudaMalloc(%zu): %s", total, cudaGetErrorString(e));
     B200Q_CUDA(ctx, e);
     return B200Q_OK;
@@ -230,6 +246,11 @@ static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor 
     ActEntry *hit = nullptr;
     for (auto &e : ctx->act_cache)
         if (e.valid && e.key == key) { hit = &e; break; }
+    if (!hit && form == ACT_Q8_0_TILED) {                   // or in the int8 arm's form, where there was no room for the other
+        key.form = ACT_Q8_0_TILED_I8;
+        for (auto &e : ctx->act_cache)
+            if (e.valid && e.key == key) { hit = &e; break; }
+    }
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     out->fresh = !hit;
     if (!hit) {
@@ -247,10 +268,14 @@ static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor 
         ActEntry &e = ctx->act_cache[pick];
         e.valid = false;
         b200q_status st;
-        if (form == ACT_Q8_0_TILED || form == ACT_Q8_256_TILED || form == ACT_Q8_256_TILED_F16) {
-            const bool per32 = form == ACT_Q8_0_TILED, f16 = form == ACT_Q8_256_TILED_F16;
-            if ((st = ws_reserve(ctx, &e.codes, per32 ? gemm_tc_act_bytes(K, N) : f16 ? gemm_kf_act_bytes(K, N) : gemm_kq_act_bytes(K, N))) != B200Q_OK) return st;
-            st = per32 ? launch_quantize_tiled(ctx, src1, (uint8_t *)e.codes.ptr)
+        if (form == ACT_Q8_0_TILED || form == ACT_Q8_0_TILED_I8 || form == ACT_Q8_256_TILED || form == ACT_Q8_256_TILED_F16) {
+            const bool per32 = form == ACT_Q8_0_TILED || form == ACT_Q8_0_TILED_I8, f16 = form == ACT_Q8_256_TILED_F16;
+            const size_t bytes = per32 ? gemm_tc_act_bytes(form, K, N) : f16 ? gemm_kf_act_bytes(K, N) : gemm_kq_act_bytes(K, N);
+            bool best;
+            if ((st = ws_reserve_either(ctx, &e.codes, bytes, form == ACT_Q8_0_TILED ? gemm_tc_act_bytes(ACT_Q8_0_TILED_I8, K, N) : bytes, &best)) != B200Q_OK) return st;
+            if (!best) form = ACT_Q8_0_TILED_I8;
+            key.form = form;
+            st = per32 ? launch_quantize_tiled(ctx, form, src1, (uint8_t *)e.codes.ptr)
                : f16   ? launch_quantize_f16(ctx, src1, (uint8_t *)e.codes.ptr)
                        : launch_quantize_tiled256(ctx, src1, (uint8_t *)e.codes.ptr);
             if (st != B200Q_OK) return st;
@@ -282,7 +307,7 @@ static b200q_status get_activation(b200q_ctx *ctx, int form, const b200q_tensor 
     out->d32 = form == ACT_Q8_256 ? (const float *)hit->scales.ptr : nullptr;
     out->s32 = (const int16_t *)hit->sums.ptr;
     out->s16 = form == ACT_Q8_256 ? (const int16_t *)hit->sums16.ptr : nullptr;
-    out->form = form;
+    out->form = hit->key.form;
     out->K = K;
     out->N = N;
     return B200Q_OK;
@@ -451,8 +476,8 @@ b200q_status b200q_mul_mat(b200q_ctx *ctx, const b200q_tensor *src0, const b200q
     const bool uniform = dst_uniform(dst, &ldd);
     // prompt widths of the per-32 types go to the tensor cores
     if (N > 8 && uniform && !ctx->no_tc && gemm_tc_supported(src0->type, M, K, N, src0->data, src0->nb[1])) {
-        if ((st = get_activation(ctx, ACT_Q8_0_TILED, src1, &act)) != B200Q_OK) return st;
-        return launch_gemm_tc(ctx, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
+        if ((st = get_activation(ctx, ctx->tc_f16 ? ACT_Q8_0_TILED : ACT_Q8_0_TILED_I8, src1, &act)) != B200Q_OK) return st;
+        return launch_gemm_tc(ctx, act.form, src0->type, src0->data, src0->nb[1], M, K, (const uint8_t *)act.codes, N,
                               (float *)dst->data, ldd, act.fresh);
     }
     if (N > 8 && uniform && !ctx->no_tc && gemm_kq_supported(src0->type, M, K, N, src0->data, src0->nb[1])) {
@@ -521,11 +546,14 @@ b200q_status b200q::mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
         src0->nb[2] % 16 == 0 && src1->nb[1] % 16 == 0 && src1->nb[2] % 16 == 0 && (uintptr_t)src1->data % 16 == 0) {
         RouteView rv;
         if ((st = moe_route(ctx, ids, n_expert, &rv)) != B200Q_OK) return st;
-        const int form = per32 ? ACT_Q8_0_TILED : f16 ? ACT_Q8_256_TILED_F16 : ACT_Q8_256_TILED;
-        const size_t bytes = per32 ? gemm_tc_id_act_bytes(K, rv.max_tiles128) : f16 ? gemm_kf_id_act_bytes(K, rv.max_tiles128)
+        int form = per32 ? (ctx->tc_f16 ? ACT_Q8_0_TILED : ACT_Q8_0_TILED_I8) : f16 ? ACT_Q8_256_TILED_F16 : ACT_Q8_256_TILED;
+        const size_t bytes = per32 ? gemm_tc_id_act_bytes(form, K, rv.max_tiles128) : f16 ? gemm_kf_id_act_bytes(K, rv.max_tiles128)
                                                                                 : gemm_kq_id_act_bytes(K, rv.max_tiles128);
         const void *before = ctx->moe_ws[7].ptr;
-        if ((st = ws_reserve(ctx, &ctx->moe_ws[7], bytes)) != B200Q_OK) return st;
+        bool best;
+        if ((st = ws_reserve_either(ctx, &ctx->moe_ws[7], bytes, form == ACT_Q8_0_TILED ? gemm_tc_id_act_bytes(ACT_Q8_0_TILED_I8, K, rv.max_tiles128) : bytes, &best)) != B200Q_OK)
+            return st;
+        if (!best) form = ACT_Q8_0_TILED_I8;
         const bool grew = ctx->moe_ws[7].ptr != before;
         TileRoute tr = { rv.tiles128, rv.n_tiles + 4, rv.pairs, n_used, ne11, src1->nb[1], src1->nb[2], ld1, ld2, gate };
         count(ctx, ST_MOE_GEMM);
@@ -544,7 +572,7 @@ b200q_status b200q::mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b
         ma.gate = gate;
         ma.n_expert = n_expert;
         for (int i = 0; i < 4; ++i) { ma.ne[i] = src1->ne[i]; ma.nb[i] = src1->nb[i]; }
-        st = per32 ? launch_gemm_tc_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
+        st = per32 ? launch_gemm_tc_id(ctx, form, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
              : f16   ? launch_gemm_kf_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready)
                      : launch_gemm_kq_id(ctx, src0, src1, tr, rv.max_tiles128, (uint8_t *)ctx->moe_ws[7].ptr, (float *)dst->data, ready);
         return st == B200Q_OK && src0b ? mul_mat_id(ctx, src0b, src1, ids, dstb, gate) : st;

@@ -39,7 +39,8 @@ __host__ __device__ inline bool type_info(int type, TypeInfo *ti) {
     }
 }
 
-enum { ACT_Q8_0 = 0, ACT_Q8_256 = 1, ACT_Q8_0_TILED = 2, ACT_Q8_256_TILED = 3, ACT_Q8_256_TILED_F16 = 4 };   // TILED: the tensor-core GEMM's chunk layout (F16: codes as halves)
+// TILED: the tensor-core GEMMs' chunk layouts (F16: codes as halves, as ACT_Q8_0_TILED has them; I8: the int8 arm of the per-32 types)
+enum { ACT_Q8_0 = 0, ACT_Q8_256 = 1, ACT_Q8_0_TILED = 2, ACT_Q8_256_TILED = 3, ACT_Q8_256_TILED_F16 = 4, ACT_Q8_0_TILED_I8 = 5 };
 
 // Quantized activation as the kernels read it: column c of K values at
 //   codes  + c*K            int8
@@ -167,6 +168,7 @@ namespace b200q {
 
 b200q_status fail(b200q_ctx *ctx, b200q_status st, const char *fmt, ...);
 b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
+b200q_status ws_reserve_either(b200q_ctx *ctx, Workspace *ws, size_t best, size_t least, bool *got_best);
 bool         ws_try_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
 void ws_release(Workspace *ws);
 cudaError_t  device_alloc(b200q_ctx *ctx, void **p, size_t bytes);
@@ -263,12 +265,13 @@ void         tp_free(b200q_ctx *ctx);
 
 // gemm_tc.cu: tensor-core prefill GEMM (Q4_0, Q8_0)
 bool         gemm_tc_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride);
-size_t       gemm_tc_act_bytes(int64_t K, int64_t N);
-b200q_status launch_quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out);
-size_t       gemm_tc_id_act_bytes(int64_t K, int64_t max_tiles);
-b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
+// form: ACT_Q8_0_TILED (f16 operands) or ACT_Q8_0_TILED_I8
+size_t       gemm_tc_act_bytes(int form, int64_t K, int64_t N);
+b200q_status launch_quantize_tiled(b200q_ctx *ctx, int form, const b200q_tensor *src1, uint8_t *out);
+size_t       gemm_tc_id_act_bytes(int form, int64_t K, int64_t max_tiles);
+b200q_status launch_gemm_tc_id(b200q_ctx *ctx, int form, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
                                int64_t max_tiles, uint8_t *act, float *dst, bool act_ready);
-b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
+b200q_status launch_gemm_tc(b200q_ctx *ctx, int form, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early);
 
 // gemm_t32.cu: its default arm, f16 operands (tr: a route, or null)

@@ -1,5 +1,5 @@
-// gemm_tc.cu -- prefill GEMM for the per-32 types (Q4_0, Q8_0, IQ4_NL): the entries, and the int8 arm (B200Q_TC_I8=1); the default arm,
-// on f16 operands, is gemm_t32.cu.
+// gemm_tc.cu -- prefill GEMM for the per-32 types (Q4_0, Q8_0, IQ4_NL): the entries, and the int8 arm (B200Q_TC_I8=1, and where the scratch
+// for the f16 activation, 86,016 bytes a tile and 256 weights against 36,864, cannot be had); the default arm, on f16 operands, is gemm_t32.cu.
 //
 //   dst[M, N] = W[M, K] (packed GGUF blocks) x X[K, N] (f32), N > 8 tokens
 //
@@ -472,11 +472,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 
 }  // namespace tc
 
-// sized for the larger form, so one scratch serves either arm
-size_t gemm_tc_act_bytes(int64_t K, int64_t N) {
+size_t gemm_tc_act_bytes(int form, int64_t K, int64_t N) {
     const int64_t ntile = (N + tc::BN - 1) / tc::BN, nst = K / (tc::SB * tc::KB);
-    const size_t i8 = (size_t)(ntile * nst) * tc::ACT_CHUNK, f16 = gemm_t32_act_bytes(K, N);
-    return i8 > f16 ? i8 : f16;
+    return form == ACT_Q8_0_TILED ? gemm_t32_act_bytes(K, N) : (size_t)(ntile * nst) * tc::ACT_CHUNK;
 }
 
 bool gemm_tc_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride) {
@@ -489,8 +487,8 @@ bool gemm_tc_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 
 static const TileRoute NO_ROUTE_TC = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
-static b200q_status quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
-    if (ctx->tc_f16) return launch_quantize_t32(ctx, src1, out, n_tiles, tr.tiles ? &tr : nullptr);
+static b200q_status quantize_tiled(b200q_ctx *ctx, int form, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
+    if (form == ACT_Q8_0_TILED) return launch_quantize_t32(ctx, src1, out, n_tiles, tr.tiles ? &tr : nullptr);
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     dim3 grid((unsigned)(K / (tc::SB * tc::KB)), (unsigned)n_tiles);
     auto kern = tr.gate ? tc::quantize_tiled_kernel<true> : tc::quantize_tiled_kernel<false>;
@@ -501,9 +499,9 @@ static b200q_status quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uin
     return B200Q_OK;
 }
 
-b200q_status launch_quantize_tiled(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out) {
+b200q_status launch_quantize_tiled(b200q_ctx *ctx, int form, const b200q_tensor *src1, uint8_t *out) {
     const int64_t N = src1->ne[1] * src1->ne[2] * src1->ne[3];
-    return quantize_tiled(ctx, src1, out, (N + tc::BN - 1) / tc::BN, NO_ROUTE_TC);
+    return quantize_tiled(ctx, form, src1, out, (N + tc::BN - 1) / tc::BN, NO_ROUTE_TC);
 }
 
 // n_tiles: grid width (dense: the tiles of N; MUL_MAT_ID: the upper bound of the route's tile count,
@@ -547,27 +545,27 @@ static b200q_status launch_t(b200q_ctx *ctx, const void *w, size_t row_stride, s
     return B200Q_OK;
 }
 
-b200q_status launch_gemm_tc(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
+b200q_status launch_gemm_tc(b200q_ctx *ctx, int form, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                             const uint8_t *act, int64_t N, float *dst, int64_t ldd, bool early) {
     const int64_t n_tiles = (N + tc::BN - 1) / tc::BN;
     const size_t ms = row_stride * (size_t)M;
-    if (ctx->tc_f16) return launch_gemm_t32(ctx, type, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, nullptr);
+    if (form == ACT_Q8_0_TILED) return launch_gemm_t32(ctx, type, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, nullptr);
     if (type == B200Q_TYPE_Q4_0) return launch_t<B200Q_TYPE_Q4_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
     if (type == B200Q_TYPE_Q8_0) return launch_t<B200Q_TYPE_Q8_0>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
     if (type == B200Q_TYPE_IQ4_NL) return launch_t<B200Q_TYPE_IQ4_NL>(ctx, w, row_stride, ms, 1, M, K, act, N, n_tiles, dst, ldd, early, NO_ROUTE_TC);
     return fail(ctx, B200Q_UNSUPPORTED, "gemm_tc: type %d", type);
 }
 
-size_t gemm_tc_id_act_bytes(int64_t K, int64_t max_tiles) { return gemm_tc_act_bytes(K, max_tiles * tc::BN); }
+size_t gemm_tc_id_act_bytes(int form, int64_t K, int64_t max_tiles) { return gemm_tc_act_bytes(form, K, max_tiles * tc::BN); }
 
 // MUL_MAT_ID on the tensor cores: the route's 128-pair tiles are the column tiles; the activation of
 // every tile is gathered and quantized into `act` (gemm_tc_id_act_bytes) first.
-b200q_status launch_gemm_tc_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
+b200q_status launch_gemm_tc_id(b200q_ctx *ctx, int form, const b200q_tensor *src0, const b200q_tensor *src1, const TileRoute &tr,
                                int64_t max_tiles, uint8_t *act, float *dst, bool act_ready) {
     const int64_t K = src0->ne[0], M = src0->ne[1];
-    b200q_status st = act_ready ? B200Q_OK : quantize_tiled(ctx, src1, act, max_tiles, tr);
+    b200q_status st = act_ready ? B200Q_OK : quantize_tiled(ctx, form, src1, act, max_tiles, tr);
     if (st != B200Q_OK) return st;
-    if (ctx->tc_f16) return launch_gemm_t32(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, &tr);
+    if (form == ACT_Q8_0_TILED) return launch_gemm_t32(ctx, src0->type, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, &tr);
     if (src0->type == B200Q_TYPE_Q4_0)
         return launch_t<B200Q_TYPE_Q4_0>(ctx, src0->data, src0->nb[1], src0->nb[2], src0->ne[2], M, K, act, 0, max_tiles, dst, 0, false, tr);
     if (src0->type == B200Q_TYPE_Q8_0)

@@ -220,18 +220,18 @@ def test_optional_scratch_goes_back_to_a_full_device(what):
     t, m, k, n = A.Q6_K, 1100, 3072, 1000
     with A.Context(0) as ctx:
         w, x, wide, p = prompt(ctx, t, m, k, n, 1)          # 7.1 MB of operand, 4.4 MB a part, 3.2 MB of activation
-        v, y, other, q = prompt(ctx, A.Q4_0, 64, 2048, 1000, 2)      # 5.5 MB of activation
+        v, y, other, q = prompt(ctx, A.Q4_K, 64, 2048, 1000, 2)      # 4.5 MB of activation
         ctx.expand_limit(96 << 20)
         ctx.graph_begin()
         ctx.mul_mat(*wide)
         st = ctx.stats()
         assert st["gemm_kx"] == 1 and st["gemm_ksplit"] == 1
         held = ctx.scratch_total(0)
-        ctx.scratch_total(held + (1 << 20))
+        ctx.scratch_total(held)                             # full
         ctx.graph_begin()
         if what == "scratch":
             ctx.mul_mat(*other)
-            assert rel_err(ctx.download(q[2], (n, 64), np.float32), O.mul_mat_f64(A.Q4_0, v, 2048, y, True)) < TOL
+            assert rel_err(ctx.download(q[2], (n, 64), np.float32), O.mul_mat_f64(A.Q4_K, v, 2048, y, True)) < TOL
         else:
             ctx.free(ctx.alloc(4 << 20))
         assert ctx.stats()["workspace_grow"] > st["workspace_grow"] and ctx.L.b200q_last_error(ctx.h) == b""
@@ -244,3 +244,51 @@ def test_optional_scratch_goes_back_to_a_full_device(what):
         assert rel_err(ctx.download(p[2], (n, m), np.float32), O.mul_mat_f64(t, w, k, x, True)) < TOL
         st = ctx.stats()
         assert (st["gemm_tc"], st.get("gemm_kx", 0), st.get("gemm_ksplit", 0)) == (1, 0, 0)
+
+
+@pytest.mark.parametrize("t", [A.Q4_0, A.Q8_0, A.IQ4_NL])
+def test_no_memory_for_the_f16_activation(monkeypatch, t):
+    """Where only the int8 arm's activation fits (2.3 times smaller, the same bits), the product takes that arm: at once, from its cached
+    activation, from a recording, and for route tiles. With room again it is the f16 arm."""
+    m, k, n = 192, 2048, 500                                # 32 tiles of 256 weights: 2.8 MB in halves, 1.2 MB in bytes
+    monkeypatch.setenv("B200Q_NO_KSPLIT", "1")              # (the limit would change the parts of K as well)
+    with A.Context(0) as ctx:
+        w, x, mm, p = prompt(ctx, t, m, k, n, 900 + t)
+        ctx.scratch_limit(2 << 20)
+        ctx.graph_begin()
+        ctx.mul_mat(*mm)
+        small = ctx.download(p[2], (n, m), np.float32)
+        ctx.mul_mat(*mm)
+        st = ctx.stats()
+        assert (st["gemm_tc"], st.get("gemm_tc_f16", 0), st["act_cache_hit"]) == (2, 0, 1) and ctx.L.b200q_last_error(ctx.h) == b""
+        g = ctx.capture(lambda: ctx.mul_mat(*mm))
+        ctx.graph_begin()
+        ctx.mul_mat(*mm)                                    # (finds no room again, and leaves the recording's block alone)
+        assert ctx.stats()["workspace_grow"] == st["workspace_grow"]
+        ctx.upload(-x, p[1])
+        ctx.graph_launch(g)
+        assert rel_err(ctx.download(p[2], (n, m), np.float32), O.mul_mat_f64(t, w, k, -x, True)) < TOL
+        ctx.graph_free(g)
+        ctx.upload(x, p[1])
+        ctx.scratch_limit(0)
+        ctx.graph_begin()
+        ctx.mul_mat(*mm)
+        assert ctx.stats()["gemm_tc_f16"] == 1
+        whole = ctx.download(p[2], (n, m), np.float32)
+        assert rel_err(whole, O.mul_mat_f64(t, w, k, x, True)) < TOL and np.array_equal(small, whole)
+    # four experts of 48 rows, two used of 250 tokens: eight tiles at most
+    ids = O.route_ids(2, 250, 4, 3)
+    got = []
+    for limit in (0, 3 << 20):                              # eight tiles: 5.5 MB in halves, 2.4 MB in bytes
+        with A.Context(0) as ctx:
+            ctx.scratch_limit(limit)
+            dw, dx, di, dy = ctx.upload(w), ctx.upload(x[:250]), ctx.upload(ids), ctx.alloc(500 * 48 * 4)
+            rb = w.shape[-1]
+            ctx.graph_begin()
+            for _ in range(2):
+                ctx.mul_mat_id(A.Tensor.make(t, [k, 48, 4, 1], [A.block_bytes(t), rb, rb * 48, rb * 192], dw), A.Tensor.f32(dx, [k, 1, 250]),
+                               A.Tensor.make(A.I32, [2, 250, 1, 1], [4, 8], di), A.Tensor.f32(dy, [48, 2, 250]))
+            got.append(ctx.download(dy, (500, 48), np.float32))
+            st = ctx.stats()
+            assert (st["moe_gemm"], st["gemm_tc"], st.get("gemm_tc_f16", 0), st["act_cache_hit"]) == (2, 2, 0 if limit else 2, 1), st
+    assert np.isfinite(got[0]).all() and np.array_equal(*got)
