@@ -286,10 +286,11 @@ b200q_status launch_gemm_t32(b200q_ctx *ctx, int type, const void *w, size_t row
 // gemm_kf's 304 30.7 29.8 30.3, 416 36.6 35.7 33.8, 832 63.4 55.5 59.2, 1504 107 94 90, 4096 265 227 216. w1024: up to how many blocks.
 // gemm_kf's has 51 registers a thread, four blocks of 256 an SM: they are the fastest but where their last round is less than
 // half full (a block of 512 is half as long), and for less than eight column tiles (16384 x 768 tokens 37.5 35.6 40.3).
-// Tiles of a route: 512, but 256 where there are many with few columns each (512 experts, 512 tokens, Q4_K block: 550 and 531 us).
+// Tiles of a route: 512. How full they are is known on the device only: a Q4_K block of 512 experts over 2048 tokens takes 738 us with 512
+// and 720 with 256 where the experts are used evenly, and the same to half a percent where some are favoured.
 inline unsigned quantizer_threads(const b200q_ctx *ctx, const b200q_tensor *src1, int64_t n_tiles, const TileRoute &tr, int w1024, bool kf = false) {
     const int64_t N = src1->ne[1] * src1->ne[2] * src1->ne[3], blocks = src1->ne[0] / 256 * n_tiles;
-    if (tr.tiles) return blocks > 1000 && tr.n_used * src1->ne[2] <= 32 * n_tiles ? 256 : 512;
+    if (tr.tiles) return 512;
     if (N < 64) return N >= 32 ? 512 : 256;
     if (blocks <= w1024) return 1024;
     const int64_t last = blocks % (4 * ctx->sm_count);

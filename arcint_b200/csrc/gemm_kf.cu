@@ -720,9 +720,9 @@ bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 static b200q_status quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     const unsigned threads = quantizer_threads(ctx, src1, n_tiles, tr, 148, true);
-    auto kern = threads == 256   ? (tr.gate ? kf::quantize_f16_kernel<true, 256> : kf::quantize_f16_kernel<false, 256>)
-                : threads == 512 ? (tr.gate ? kf::quantize_f16_kernel<true, 512> : kf::quantize_f16_kernel<false, 512>)
-                                 : (tr.gate ? kf::quantize_f16_kernel<true, 1024> : kf::quantize_f16_kernel<false, 1024>);
+    auto kern = tr.gate          ? kf::quantize_f16_kernel<true, 512>                      // (only the tiles of a route have a gate)
+                : threads == 256 ? kf::quantize_f16_kernel<false, 256>
+                : threads == 512 ? kf::quantize_f16_kernel<false, 512> : kf::quantize_f16_kernel<false, 1024>;
     dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(threads), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
                                src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr));

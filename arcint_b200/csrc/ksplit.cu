@@ -30,8 +30,9 @@ ksplit_sum_kernel(const float *__restrict__ parts, int ksplit, int64_t part_stri
 
 // Into how many parts to cut K: the schedule's length in nanoseconds, rounds of units over the SMs plus, for more than one
 // part, the pass that adds them (a launch and its traffic). t: a k-step (one raw stage) and a unit of the kernel, see common.cuh.
-// Of 17 shapes (tiles 12 to 768, 4 to 64 steps) in each of the seven types, timed at every number of parts, the choice is 0.6 % from
-// the fastest on average, at most 13 % (Q4_0 11008x4096 x 100 tokens: 75 us in three parts, 67 in five, 79 whole).
+// Of 20 shapes (tiles 4 to 256, 4 to 74 steps) in each of the seven types, timed at every number of parts with the kernels as they are, the
+// choice is 0.6 % from the fastest on average, at most 14 % (Q6_K 11008x4096 x 100 tokens: 35 us whole, 31 in three parts; the next
+// worst is Q5_K at the same size, 8 %).
 int choose_ksplit(const b200q_ctx *ctx, int64_t tiles, int64_t steps, KsplitTimes t, int64_t outputs, int64_t most, int64_t chunks) {
     int best_ks = 1;
     int64_t best = 0;

@@ -7,6 +7,8 @@
 namespace b200q {
 namespace tc {
 
+// Polls of a bounded wait. A try_wait that fails has the hardware hold the thread for about 4 us (1000, 65,536 and 2^20 of them took 4.1,
+// 259 and 4148 ms on B200), so a wait gives up after some four seconds.
 constexpr uint32_t SPIN_LIMIT = 1u << 20;
 
 // K-major, no swizzle, 128 rows: 8 rows x 16 bytes are one contiguous 128-byte core matrix; the
