@@ -128,12 +128,14 @@ b200q_status ws_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes) {
 }
 
 // Scratch for a call that prefers `best` bytes and can do with `least`; *got_best: which of the two *ws holds. A block that holds the
-// least is not given up for the try, so that a recording of its product stays good.
+// least is not given up for the try, so that a recording of its product stays good. A capture takes the least only where the call
+// before it had to: otherwise it is refused like any other growth.
 b200q_status ws_reserve_either(b200q_ctx *ctx, Workspace *ws, size_t best, size_t least, bool *got_best) {
     *got_best = true;
     if (best <= ws->cap) return B200Q_OK;
-    if (least <= ws->cap) {
+    if (least <= ws->cap && (!ctx->capturing || ws->least_only)) {
         *got_best = ws_try_reserve(ctx, ws, best);
+        if (!*got_best) ws->least_only = true;
         return B200Q_OK;
     }
     if (ctx->capturing)
@@ -151,6 +153,7 @@ b200q_status ws_reserve_either(b200q_ctx *ctx, Workspace *ws, size_t best, size_
         *got_best = false;
         e = ws_alloc(ctx, ws, least, &total, true);
     }
+    ws->least_only = !*got_best;
     if (e == cudaErrorMemoryAllocation) return fail(ctx, B200Q_NO_MEMORY, "cudaMalloc(%zu): %s", total, cudaGetErrorString(e));
     B200Q_CUDA(ctx, e);
     return B200Q_OK;

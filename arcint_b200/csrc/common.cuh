@@ -66,6 +66,7 @@ struct Workspace {
     void  *ptr = nullptr;
     size_t cap = 0;
     void  *base = nullptr;   // start of the allocation: ptr, or WS_GUARD bytes before it when guard words surround the block
+    bool   least_only = false;   // a larger block, which the last call preferred, could not be had (ws_reserve_either)
 };
 
 constexpr size_t WS_GUARD = 256;          // bytes of guard words on each side of a scratch block (B200Q_CANARY=1)

@@ -17,7 +17,8 @@
  *     instance from one thread); work is enqueued on the context's stream and is
  *     asynchronous to the host unless the call says otherwise;
  *   - tensor storage belongs to the caller; scratch belongs to the context, grows on
- *     demand and is never shrunk (the reference's prealloc_* buffers, P01:66-88);
+ *     demand and is not shrunk (the reference's prealloc_* buffers, P01:66-88), but blocks that products can do
+ *     without are given back where a needed allocation finds the device full (counted as a "workspace_grow");
  *   - a product of at most 8 columns starts to read its weights while the kernel ahead of it on the stream may still be
  *     running (programmatic dependent launch). A kernel of the caller's that writes weights must have written them before it
  *     lets its dependents start (griddepcontrol.launch_dependents, cudaTriggerProgrammaticLaunchCompletion); one that never

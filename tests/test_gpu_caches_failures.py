@@ -276,6 +276,16 @@ def test_no_memory_for_the_f16_activation(monkeypatch, t):
         assert ctx.stats()["gemm_tc_f16"] == 1
         whole = ctx.download(p[2], (n, m), np.float32)
         assert rel_err(whole, O.mul_mat_f64(t, w, k, x, True)) < TOL and np.array_equal(small, whole)
+    with A.Context(0) as ctx:                               # a recording that was not run before is refused, although the bytes would fit
+        _, _, few, _ = prompt(ctx, t, m, k, 200, 1)
+        _, _, mm, _ = prompt(ctx, t, m, k, n, 2)
+        ctx.graph_begin()
+        ctx.mul_mat(*few)
+        with pytest.raises(A.B200QError, match="inside a capture"):
+            ctx.capture(lambda: ctx.mul_mat(*mm))
+        ctx.graph_begin()
+        ctx.mul_mat(*mm)
+        assert ctx.stats()["gemm_tc_f16"] == 2
     # four experts of 48 rows, two used of 250 tokens: eight tiles at most
     ids = O.route_ids(2, 250, 4, 3)
     got = []
