@@ -52,6 +52,17 @@ def test_many_units_per_block(ctx, t):
     check(got, t, w, k, x)
 
 
+# activations of 300, 450 and 612 blocks of the tiled quantizers, whose threads follow that number: 512 and 256 for Q4_K and Q5_K, 512 for the
+# per-32 types from the second, for Q6_K and IQ4_XS in the third; short last column tiles
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("k,n", [(12800, 700), (12800, 1030), (17408, 1030)])
+def test_activations_of_many_blocks(ctx, t, k, n):
+    m = 40
+    w, x = data(t, m, k, n, 9)
+    got = ctx.run_mul_mat(t, w, k, x)
+    check(got, t, w, k, x)
+
+
 # (K = 1280: ten activation stages of the per-32 GEMM a unit, in rings of three and four)
 @pytest.mark.parametrize("t", TYPES)
 @pytest.mark.parametrize("k", [512, 1280])
