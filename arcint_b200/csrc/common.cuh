@@ -217,7 +217,8 @@ bool gemv_ar_shape_ok(int type, const void *w, size_t row_stride, int64_t M, int
 b200q_status mul_mat_id(b200q_ctx *ctx, const b200q_tensor *src0, const b200q_tensor *src1, const b200q_tensor *ids, b200q_tensor *dst,
                         int64_t gate, const b200q_tensor *src0b = nullptr, b200q_tensor *dstb = nullptr);
 // silu(g) * u, as every quantizer that takes the gate along computes it
-__device__ __forceinline__ float swiglu(float g, float u) { return g / (1.f + expf(-g)) * u; }
+__device__ __forceinline__ float silu(float g) { return g / (1.f + expf(-g)); }
+__device__ __forceinline__ float swiglu(float g, float u) { return silu(g) * u; }
 __device__ __forceinline__ float4 swiglu4(float4 g, float4 u) {
     return make_float4(swiglu(g.x, u.x), swiglu(g.y, u.y), swiglu(g.z, u.z), swiglu(g.w, u.w));
 }
@@ -280,24 +281,6 @@ size_t       gemm_t32_act_bytes(int64_t K, int64_t N);
 b200q_status launch_quantize_t32(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute *tr);
 b200q_status launch_gemm_t32(b200q_ctx *ctx, int type, const void *w, size_t row_stride, size_t mat_stride, int64_t n_mat, int64_t M, int64_t K,
                              const uint8_t *act, int64_t N, int64_t n_tiles, float *dst, int64_t ldd, bool early, const TileRoute *tr);
-// Threads of a tiled quantizer's block (one column tile, 256 weights; a half-warp a column at a time). Few blocks: enough threads for two
-// passes over a whole tile (with 256, eight passes of dependent loads, 64 blocks of a 512 x 4096 activation took 12.5 us). Many: blocks
-// of 1024 are one or two an SM, and their last round is left to a few. Quantizer and a GEMM of 128 rows, 1024, 512 and 256 threads, us:
-// gemm_t32's 304 blocks 30.0 31.3 31.4, 380 34.9 33.0 32.6, 1024 82.6 72.8 77.4, 4096 279 239 239; gemm_kq's 480 31.0 31.0 31.3, 1024 58.0 55.0 55.0;
-// gemm_kf's 304 30.7 29.8 30.3, 416 36.6 35.7 33.8, 832 63.4 55.5 59.2, 1504 107 94 90, 4096 265 227 216. w1024: up to how many blocks.
-// gemm_kf's has 51 registers a thread, four blocks of 256 an SM: they are the fastest but where their last round is less than
-// half full (a block of 512 is half as long), and for less than eight column tiles (16384 x 768 tokens 37.5 35.6 40.3).
-// Tiles of a route: 512. How full they are is known on the device only: a Q4_K block of 512 experts over 2048 tokens takes 738 us with 512
-// and 720 with 256 where the experts are used evenly, and the same to half a percent where some are favoured.
-inline unsigned quantizer_threads(const b200q_ctx *ctx, const b200q_tensor *src1, int64_t n_tiles, const TileRoute &tr, int w1024, bool kf = false) {
-    const int64_t N = src1->ne[1] * src1->ne[2] * src1->ne[3], blocks = src1->ne[0] / 256 * n_tiles;
-    if (tr.tiles) return 512;
-    if (N < 64) return N >= 32 ? 512 : 256;
-    if (blocks <= w1024) return 1024;
-    const int64_t last = blocks % (4 * ctx->sm_count);
-    return !kf || N <= 1024 - 128 || (blocks < 2000 && last > 64 && last < 320) ? 512 : 256;
-}
-
 // the sum of ksplit partial results (parts[z][n][m], part_stride floats apart, part 0 first) into dst (ksplit.cu)
 b200q_status launch_ksplit_sum(b200q_ctx *ctx, const float *parts, int ksplit, int64_t part_stride, int64_t M, int64_t N, float *dst, int64_t ldd);
 

@@ -45,6 +45,7 @@
 #include "common.cuh"
 #include "pdl.cuh"
 #include "tc_common.cuh"
+#include "tile_quant.cuh"
 
 namespace b200q {
 
@@ -71,7 +72,9 @@ static_assert(128 * 48 + 256 * 56 + 256 * 160 <= THREADS * LAUNCH_REGS, "registe
 //   codes, twice (blocks 0..3, 4..7): [group g < 16][block j < 4][piece c < 4][column r < 8][8 codes as halves, each run of four
 //          in the order 0 2 1 3, in which the unpack threads mask nibbles out of a word]
 //   extra: 128 f32 scales, then the mins operand [group g < 16][piece c < 2][column r < 8][8 halves: bl_0..7 or 256 bh_0..7]
-// Behind the chunks of all column tiles an int32 for each: the largest one-sided sum of codes of a column, see above.
+// Behind the chunks of all column tiles an int32 for each block of the quantizer (each warp, for a route): the largest one-sided sum of
+// codes of its columns, see above. SIDES: at most so many a chunk.
+constexpr int SIDES = 16;
 constexpr int CODE_BLOCK = 512, CODE_GROUP = GB * CODE_BLOCK, CODE_STAGE = (BN / 8) * CODE_GROUP;
 constexpr int MINS_GROUP = 256, EXTRA_MINS = BN * 4, EXTRA = EXTRA_MINS + (BN / 8) * MINS_GROUP;
 constexpr int CHUNK = 2 * CODE_STAGE + EXTRA;
@@ -106,100 +109,75 @@ static_assert(NCODE == 4 && NX == 3 && NG == 2 && BAR_COUNT <= 32, "barrier slot
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
 
 // The quantizer of the layout above, per-256 form (the reference's kernel_quant_i8 rule: scale bm/127, round to nearest
-// even, zero below 1e-30). NT threads, a build each: see quantizer_threads.
-template <bool GATE, int NT>
-__global__ void __launch_bounds__(NT)
-quantize_f16_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
-                    int64_t N, uint8_t *__restrict__ out, TileRoute id) {
-    // One block per (tile, super-block); a half-warp per column at a time: its sixteen lanes read the column's 256
-    // floats as one contiguous kilobyte (lane l: elements 16 l .. 16 l + 15, i.e. half l & 1 of block j = l >> 1),
-    // take the maximum by shuffles and store their sixteen codes as two 16-byte pieces. Columns of groups past the tile's
-    // last one are never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
+// even, zero below 1e-30).
+template <bool GATE, bool STAGED>
+__global__ void __launch_bounds__(TQ_THREADS, STAGED && !GATE ? 5 : 4)
+quantize_f16_kernel(TqSource src, int64_t K, int64_t N, int64_t n_tiles, uint8_t *__restrict__ out, TileRoute id) {
+    // (tile_quant.cuh) Lane (q, r): blocks 2 q and 2 q + 1 of column r. Columns of groups past the tile's last one are
+    // never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
-    const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
-    const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
-    uint8_t *chunk = out + ((size_t)t * nst + s) * CHUNK;
-    int cnt, first = 0;
-    if (id.tiles) {
-        // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
-        if (t >= __ldg(id.n_tiles)) return;
-        first = __ldg(id.tiles + 4 * t + 1);
-        cnt = __ldg(id.tiles + 4 * t + 2);
-    } else {
-        const int64_t left = N - (int64_t)t * BN;
-        cnt = left < BN ? (int)left : BN;
-    }
-    const int live = ((cnt + 7) >> 3) << 3;
-    __shared__ int side_of_warp[NT / 32];
-    int side = 0;                        // the largest one-sided sum of codes among this thread's columns
-    for (int col0 = 0; col0 < live; col0 += NT / 16) {
-        // (whole warps stay together for the shuffles: a half-warp past the live columns quantizes zeros and stores nothing)
-        const int col = col0 + hw;
-        const float *x = nullptr;
-        if (col < cnt) {
-            if (id.tiles) {
-                const int p = __ldg(id.pairs + first + col), tok = p / id.n_used, slot = p - tok * id.n_used;
-                x = reinterpret_cast<const float *>(base + (size_t)(slot % id.ne11) * id.nb1 + (size_t)tok * id.nb2);
-            } else {
-                const int64_t n = (int64_t)t * BN + col;
-                const int64_t c1 = n % ne1, c23 = n / ne1, c2 = c23 % ne2, c3 = c23 / ne2;
-                x = reinterpret_cast<const float *>(base + c1 * nb1 + c2 * nb2 + c3 * nb3);
+    __shared__ int side_of_warp[TQ_WARPS];
+    const int s = blockIdx.x, nst = gridDim.x, q = (threadIdx.x & 31) >> 3, r = threadIdx.x & 7;
+    int *sides = reinterpret_cast<int *>(out + (size_t)n_tiles * nst * CHUNK);
+    int side = 0;                        // the largest one-sided sum of codes among the warp's columns
+    extern __shared__ __align__(16) uint8_t tiles[];
+    TqWalk walk(src, id, N, BN);
+    const float *x;
+#pragma unroll 1
+    while (walk.step(x)) {
+        const int t = walk.t, g = walk.g;
+        float v[64];
+        tq_load<GATE, STAGED>(x ? x + (int64_t)s * 256 : nullptr, src.base, id.gate, tiles, v);
+        const float bm = tq_column_max(v);
+        tq_codes256(v, bm > 1e-30f ? __fdiv_rn(127.f, bm) : 0.f);
+        uint8_t *chunk = out + ((size_t)t * nst + s) * CHUNK;
+        uint8_t *o = chunk + (q >> 1) * CODE_STAGE + g * CODE_GROUP + 2 * (q & 1) * CODE_BLOCK + r * 16;
+        float sum[2], pos[2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            // the codes as halves, each run of four in the order 0 2 1 3; their sum and the sum of the positive ones (whole numbers, exact)
+            sum[b] = pos[b] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                __align__(16) __half2 w[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float *f = v + 32 * b + 8 * c + 4 * i;
+                    w[2 * i] = __floats2half2_rn(f[0], f[2]);
+                    w[2 * i + 1] = __floats2half2_rn(f[1], f[3]);
+                }
+                *reinterpret_cast<uint4 *>(o + b * CODE_BLOCK + c * 128) = *reinterpret_cast<const uint4 *>(w);
+                // (in halves over eight codes: up to 8 * 127)
+                const __half2 a = __hadd2(__hadd2(w[0], w[1]), __hadd2(w[2], w[3])), z = __float2half2_rn(0.f);
+                const __half2 p = __hadd2(__hadd2(__hmax2(w[0], z), __hmax2(w[1], z)), __hadd2(__hmax2(w[2], z), __hmax2(w[3], z)));
+                sum[b] += __low2float(a) + __high2float(a);
+                pos[b] += __low2float(p) + __high2float(p);
             }
-            x += (int64_t)s * 256 + 16 * l;
         }
-        float4 v[4];
-        float amax = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[i] = x ? __ldg(reinterpret_cast<const float4 *>(x) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (GATE && x) v[i] = swiglu4(__ldg(reinterpret_cast<const float4 *>(x + id.gate) + i), v[i]);
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-        }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-        const float bm = amax;
-        const float iq = bm > 1e-30f ? __fdiv_rn(127.f, bm) : 0.f;
-        // the sixteen codes as halves, each run of four in the order 0 2 1 3; their sum and the sum of the positive ones (whole numbers
-        // up to 8 * 127 a half, exact)
-        auto code = [&](float x) { return (float)__float2int_rn(__fmul_rn(x, iq)); };       // (0 for a NaN)
-        __align__(16) __half2 w[8];
-        __half2 all = __float2half2_rn(0.f), pos = all;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            w[2 * i] = __floats2half2_rn(code(v[i].x), code(v[i].z));
-            w[2 * i + 1] = __floats2half2_rn(code(v[i].y), code(v[i].w));
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            all = __hadd2(all, w[i]);
-            pos = __hadd2(pos, __hmax2(w[i], __float2half2_rn(0.f)));
-        }
-        // both sums of the sixteen lanes' codes in one word: all above, positive below (at most 256 * 127)
-        int sums = __half2int_rn(__hadd(__low2half(all), __high2half(all))) * 65536 + __half2int_rn(__hadd(__low2half(pos), __high2half(pos)));
-        sums += __shfl_xor_sync(0xFFFFFFFFu, sums, 1);
-        const int sum = sums >> 16;                             // of the block's 32 codes (the mins term)
-#pragma unroll
-        for (int o = 2; o < 16; o *= 2) sums += __shfl_xor_sync(0xFFFFFFFFu, sums, o);
-        side = max(side, (sums & 0xFFFF) - min(sums >> 16, 0));
-        if (col >= live) continue;
-        const int j = l >> 1;
-        uint8_t *o = chunk + (j >> 2) * CODE_STAGE + (col >> 3) * CODE_GROUP + (j & 3) * CODE_BLOCK + (col & 7) * 16;
-        *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * 128) = *reinterpret_cast<const uint4 *>(w);
-        *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * 128) = *reinterpret_cast<const uint4 *>(w + 4);
-        // two exact digits of the sum: bh = round(sum / 256), bl = sum - 256 bh in [-128, 127]
-        const int bh = (sum + 128) >> 8;
+        // the mins operand of the lane's two blocks, two exact digits of a sum: bh = round(sum / 256), bl = sum - 256 bh in [-128, 127]
         uint8_t *extra = chunk + 2 * CODE_STAGE;
-        __half *mo = reinterpret_cast<__half *>(extra + EXTRA_MINS + (col >> 3) * MINS_GROUP + (l & 1) * 128 + (col & 7) * 16);
-        mo[j] = __float2half_rn((l & 1) ? (float)(256 * bh) : (float)(sum - 256 * bh));
-        if (l == 0) reinterpret_cast<float *>(extra)[col] = __fdiv_rn(bm, 127.f);
+        const float h0 = 256.f * floorf((sum[0] + 128.f) * 0.00390625f), h1 = 256.f * floorf((sum[1] + 128.f) * 0.00390625f);
+        __half2 *mo = reinterpret_cast<__half2 *>(extra + EXTRA_MINS + g * MINS_GROUP + r * 16) + q;
+        mo[0] = __floats2half2_rn(sum[0] - h0, sum[1] - h1);
+        mo[32] = __floats2half2_rn(h0, h1);                                                  // (128 bytes on)
+        if (q == 0) reinterpret_cast<float *>(extra)[8 * g + r] = __fdiv_rn(bm, 127.f);
+        // both sums of the column in one word: all above, positive below (at most 256 * 127)
+        int sums = __float2int_rn(sum[0] + sum[1]) * 65536 + __float2int_rn(pos[0] + pos[1]);
+        sums += __shfl_xor_sync(0xFFFFFFFFu, sums, 8);
+        sums += __shfl_xor_sync(0xFFFFFFFFu, sums, 16);
+        side = max(side, __reduce_max_sync(0xFFFFFFFFu, (sums & 0xFFFF) - min(sums >> 16, 0)));
     }
-    side = __reduce_max_sync(0xFFFFFFFFu, side);
+    if (id.tiles) {
+        if ((threadIdx.x & 31) == 0) sides[tq_block() * TQ_WARPS + (threadIdx.x >> 5)] = side;
+        return;
+    }
     if ((threadIdx.x & 31) == 0) side_of_warp[threadIdx.x >> 5] = side;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int i = 1; i < NT / 32; ++i) side = max(side, side_of_warp[i]);
-        reinterpret_cast<int *>(out + (size_t)gridDim.y * nst * CHUNK)[(size_t)t * nst + s] = side;
+#pragma unroll
+        for (int i = 1; i < TQ_WARPS; ++i) side = max(side, side_of_warp[i]);
+        sides[tq_block()] = side;
     }
 }
 
@@ -278,7 +256,7 @@ template <int TYPE, int COLS>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uint8_t *__restrict__ act,
                int N, int n_tiles_dense, int ksplit, float *__restrict__ dst, int64_t ldd, int64_t part_stride,
-               int *__restrict__ error_word, TileRoute id) {
+               int *__restrict__ error_word, int n_sides, TileRoute id) {
     typedef Smem<TYPE> L;
     constexpr bool FULL = COLS == COLS_FULL, ROUTE = COLS == COLS_ROUTE;
     constexpr int SBB = Fmt<TYPE>::SBB, NRAW = L::NRAW;
@@ -332,7 +310,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // many tiles, by all threads (a block waits first anyway), a dense product's by an idle warp behind its wait, so that weights
     // are fetched and unpacked meanwhile (asking with the whole block costs 2 us a launch).
     auto asks_for_more = [&](int first, int step) {
-        const int total = tiles_n * nsb;
+        const int total = n_sides;
         const int *p = reinterpret_cast<const int *>(act + (size_t)n_tiles_dense * nsb * CHUNK);
         int side = 0;
 #pragma unroll 4
@@ -707,7 +685,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 
 static const TileRoute NO_ROUTE_KF = { nullptr, nullptr, nullptr, 1, 1, 0, 0, 0, 0, 0 };
 
-size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + kf::BN - 1) / kf::BN) * (K / 256)) * (kf::CHUNK + 4); }
+size_t gemm_kf_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + kf::BN - 1) / kf::BN) * (K / 256)) * (kf::CHUNK + 4 * kf::SIDES); }
 size_t gemm_kf_id_act_bytes(int64_t K, int64_t max_tiles) { return gemm_kf_act_bytes(K, max_tiles * kf::BN); }
 
 bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w, size_t row_stride) {
@@ -719,13 +697,11 @@ bool gemm_kf_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 
 static b200q_status quantize_f16(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
-    const unsigned threads = quantizer_threads(ctx, src1, n_tiles, tr, 148, true);
-    auto kern = tr.gate          ? kf::quantize_f16_kernel<true, 512>                      // (only the tiles of a route have a gate)
-                : threads == 256 ? kf::quantize_f16_kernel<false, 256>
-                : threads == 512 ? kf::quantize_f16_kernel<false, 512> : kf::quantize_f16_kernel<false, 1024>;
-    dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, grid, dim3(threads), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1], src1->ne[2],
-                               src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr));
+    const TqSource src = { (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3] };
+    const bool staged = tr.tiles || N >= TQ_STAGED_COLS;
+    auto kern = tr.gate ? kf::quantize_f16_kernel<true, true> : staged ? kf::quantize_f16_kernel<false, true> : kf::quantize_f16_kernel<false, false>;
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, tq_grid(ctx, K, N, n_tiles, kf::BN, tr), dim3(TQ_THREADS), tq_smem(staged),
+                               ctx->stream, src, K, N, n_tiles, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);
     return B200Q_OK;
@@ -768,8 +744,9 @@ static b200q_status launch_kf_t(b200q_ctx *ctx, const void *w, size_t row_stride
     }
     const int64_t units = tiles * ksplit;
     const unsigned grid = (unsigned)(units < S ? units : S);
+    const dim3 q = tq_grid(ctx, K, N, n_tiles, kf::BN, tr);              // the quantizer's blocks, a one-sided sum each
     B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl && (early || tr.tiles), kern, dim3(grid), dim3(kf::THREADS), (size_t)L::TOTAL, ctx->stream, wmap, (int)M, (int)K, act, (int)N,
-                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, tr));
+                               (int)n_tiles, ksplit, out, out_ld, part_stride, ctx->error_word, (int)(q.x * q.y * q.z * (tr.tiles ? TQ_WARPS : 1)), tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     if (ksplit > 1 && (st = launch_ksplit_sum(ctx, out, ksplit, part_stride, M, N, dst, ldd)) != B200Q_OK) return st;
     count(ctx, ST_GEMM_TC);

@@ -36,6 +36,7 @@
 #include "common.cuh"
 #include "pdl.cuh"
 #include "tc_common.cuh"
+#include "tile_quant.cuh"
 
 namespace b200q {
 
@@ -100,66 +101,39 @@ static_assert(NG == 2 && NACT == 2 && NBUF == 2, "barrier slots above");
 
 // Activation chunk (128-token tile t, super-block s), per-256 form (the reference's
 // kernel_quant_i8 rule: scale bm/127, round to nearest even, zero below 1e-30), in the group layout above.
-template <bool GATE>
-__global__ void __launch_bounds__(1024)
-quantize_tiled256_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
-                         int64_t N, uint8_t *__restrict__ out, TileRoute id) {
-    // One block per (tile, super-block); a half-warp per column at a time: its sixteen lanes read the column's 256
-    // floats as one contiguous kilobyte (lane l: elements 16 l .. 16 l + 15, i.e. half c = l & 1 of block j = l >> 1),
-    // take the maximum by shuffles and store one 16-byte piece each. Columns of groups past the tile's last one are
-    // never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
+template <bool GATE, bool STAGED>
+__global__ void __launch_bounds__(TQ_THREADS, STAGED && !GATE ? 5 : 4)
+quantize_tiled256_kernel(TqSource src, int64_t K, int64_t N, uint8_t *__restrict__ out, TileRoute id) {
+    // (tile_quant.cuh) Lane (q, r): blocks 2 q and 2 q + 1 of column r, a 16-byte piece for a half of a block. Columns of groups past the
+    // tile's last one are never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
-    const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
-    const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
-    uint8_t *chunk = out + ((size_t)t * nst + s) * ACT_CHUNK;
-    int cnt, first = 0;
-    if (id.tiles) {
-        // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
-        if (t >= __ldg(id.n_tiles)) return;
-        first = __ldg(id.tiles + 4 * t + 1);
-        cnt = __ldg(id.tiles + 4 * t + 2);
-    } else {
-        const int64_t left = N - (int64_t)t * BN;
-        cnt = left < BN ? (int)left : BN;
-    }
-    const int live = ((cnt + 7) >> 3) << 3;
-    for (int col = hw; col < live; col += blockDim.x >> 4) {
-        const float *x = nullptr;
-        if (col < cnt) {
-            if (id.tiles) {
-                const int p = __ldg(id.pairs + first + col), tok = p / id.n_used, slot = p - tok * id.n_used;
-                x = reinterpret_cast<const float *>(base + (size_t)(slot % id.ne11) * id.nb1 + (size_t)tok * id.nb2);
-            } else {
-                const int64_t n = (int64_t)t * BN + col;
-                const int64_t c1 = n % ne1, c23 = n / ne1, c2 = c23 % ne2, c3 = c23 / ne2;
-                x = reinterpret_cast<const float *>(base + c1 * nb1 + c2 * nb2 + c3 * nb3);
+    const int s = blockIdx.x, nst = gridDim.x, q = (threadIdx.x & 31) >> 3, r = threadIdx.x & 7;
+    extern __shared__ __align__(16) uint8_t tiles[];
+    TqWalk walk(src, id, N, BN);
+    const float *x;
+#pragma unroll 1
+    while (walk.step(x)) {
+        const int t = walk.t, g = walk.g;
+        float v[64];
+        tq_load<GATE, STAGED>(x ? x + (int64_t)s * 256 : nullptr, src.base, id.gate, tiles, v);
+        const float bm = tq_column_max(v);
+        tq_codes256(v, bm > 1e-30f ? __fdiv_rn(127.f, bm) : 0.f);
+        uint8_t *grp = out + ((size_t)t * nst + s) * ACT_CHUNK + g * ACT_GROUP;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                // the low byte of a code's bits after the same 1.5 * 2^23
+                uint32_t c[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) c[k] = __float_as_uint(__fadd_rn(v[16 * e + 4 * i + k], 12582912.f));
+                w[i] = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410);
             }
-            x += (int64_t)s * 256 + 16 * l;
+            *reinterpret_cast<uint4 *>(grp + (4 * q + e) * 128 + r * 16) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        float4 v[4];
-        float amax = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[i] = x ? __ldg(reinterpret_cast<const float4 *>(x) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (GATE && x) v[i] = swiglu4(__ldg(reinterpret_cast<const float4 *>(x + id.gate) + i), v[i]);
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-        }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-        const float bm = amax;
-        const float iq = bm > 1e-30f ? __fdiv_rn(127.f, bm) : 0.f;
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 f = v[i];
-            w[i] = (uint32_t)(__float2int_rn(__fmul_rn(f.x, iq)) & 0xFF) | ((uint32_t)(__float2int_rn(__fmul_rn(f.y, iq)) & 0xFF) << 8) |
-                   ((uint32_t)(__float2int_rn(__fmul_rn(f.z, iq)) & 0xFF) << 16) | ((uint32_t)(__float2int_rn(__fmul_rn(f.w, iq)) & 0xFF) << 24);
-        }
-        uint8_t *grp = chunk + (col >> 3) * ACT_GROUP;
-        const int j = l >> 1;
-        *reinterpret_cast<uint4 *>(grp + j * 256 + (l & 1) * 128 + (col & 7) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-        if (l == 0) reinterpret_cast<float *>(grp + ACT_SCALES)[col & 7] = __fdiv_rn(bm, 127.f);
+        if (q == 0) reinterpret_cast<float *>(grp + ACT_SCALES)[r] = __fdiv_rn(bm, 127.f);
     }
 }
 
@@ -863,9 +837,11 @@ bool gemm_kq_supported(int type, int64_t M, int64_t K, int64_t N, const void *w,
 
 static b200q_status quantize256(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute &tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
-    dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, tr.gate ? kq::quantize_tiled256_kernel<true> : kq::quantize_tiled256_kernel<false>, grid, dim3(quantizer_threads(ctx, src1, n_tiles, tr, 480)), 0, ctx->stream, (const uint8_t *)src1->data, src1->ne[1],
-                               src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, tr));
+    const TqSource src = { (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3] };
+    const bool staged = tr.tiles || N >= TQ_STAGED_COLS;
+    auto kern = tr.gate ? kq::quantize_tiled256_kernel<true, true> : staged ? kq::quantize_tiled256_kernel<false, true> : kq::quantize_tiled256_kernel<false, false>;
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, tq_grid(ctx, K, N, n_tiles, kq::BN, tr), dim3(TQ_THREADS),
+                               tq_smem(staged), ctx->stream, src, K, N, out, tr));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);
     return B200Q_OK;

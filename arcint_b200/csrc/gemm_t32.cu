@@ -34,6 +34,7 @@
 #include "common.cuh"
 #include "pdl.cuh"
 #include "tc_common.cuh"
+#include "tile_quant.cuh"
 
 namespace b200q {
 
@@ -86,70 +87,47 @@ static_assert(NRAW == 2 && NSLOT == HB && BAR_COUNT <= 64, "barrier slots above"
 
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
 
-template <bool GATE>
-__global__ void __launch_bounds__(1024)
-quantize_kernel(const uint8_t *base, int64_t ne1, int64_t ne2, size_t nb1, size_t nb2, size_t nb3, int64_t K,
-                int64_t N, uint8_t *__restrict__ out, TileRoute id) {
-    // One block per (tile, 256 weights); a half-warp per column at a time: its sixteen lanes read the column's 256
-    // floats as one contiguous kilobyte (lane l: k = 16 l .. 16 l + 15, i.e. half l & 1 of block l >> 1), the two
-    // lanes of a block share their maximum by one shuffle, and every lane stores its 16 codes as two pieces. Columns of groups
-    // past the tile's last one are never fetched by the GEMM and are skipped; the dead columns of the last live group are
-    // written as zeros.
+template <bool GATE, bool STAGED>
+__global__ void __launch_bounds__(TQ_THREADS, STAGED && !GATE ? 5 : 4)
+quantize_kernel(TqSource src, int64_t K, int64_t N, uint8_t *__restrict__ out, TileRoute id) {
+    // (tile_quant.cuh) Lane (q, r): blocks 2 q and 2 q + 1 of column r. Columns of groups past the tile's last one are
+    // never fetched by the GEMM and are skipped; the dead columns of the last live group are written as zeros.
     pdl_wait();                          // src1 may be the output of the kernel before, the scratch its input
     pdl_trigger();                       // (after the wait: the GEMM then starts when all that came before is complete, weights among it)
-    const int t = blockIdx.y, s = blockIdx.x, nst = gridDim.x;
-    const int hw = threadIdx.x >> 4, l = threadIdx.x & 15;
-    uint8_t *stage = out + ((size_t)t * nst + s) * (2 * STAGE);
-    int cnt, first = 0;
-    if (id.tiles) {
-        // MUL_MAT_ID: the tile's columns are routed pairs; pair p = (token, slot) reads src1 row slot % ne11
-        if (t >= __ldg(id.n_tiles)) return;
-        first = __ldg(id.tiles + 4 * t + 1);
-        cnt = __ldg(id.tiles + 4 * t + 2);
-    } else {
-        const int64_t left = N - (int64_t)t * BN;
-        cnt = left < BN ? (int)left : BN;
-    }
-    const int live = ((cnt + 7) >> 3) << 3, j = l >> 1;
-    for (int i = threadIdx.x; i < 2 * live; i += blockDim.x)
-        *reinterpret_cast<uint4 *>(stage + (i & 1) * STAGE + (i >> 4) * GROUP + GROUP_ZERO + ((i >> 1) & 7) * 16) = make_uint4(0, 0, 0, 0);
+    const int s = blockIdx.x, nst = gridDim.x, q = (threadIdx.x & 31) >> 3, r = threadIdx.x & 7;
+    extern __shared__ __align__(16) uint8_t tiles[];
+    TqWalk walk(src, id, N, BN);
+    const float *x;
 #pragma unroll 1
-    for (int col = hw; col < live; col += blockDim.x >> 4) {
-        const float *x = nullptr;
-        if (col < cnt) {
-            if (id.tiles) {
-                const int p = __ldg(id.pairs + first + col), tok = p / id.n_used, slot = p - tok * id.n_used;
-                x = reinterpret_cast<const float *>(base + (size_t)(slot % id.ne11) * id.nb1 + (size_t)tok * id.nb2);
-            } else {
-                const int64_t n = (int64_t)t * BN + col;
-                const int64_t c1 = n % ne1, c23 = n / ne1, c2 = c23 % ne2, c3 = c23 / ne2;
-                x = reinterpret_cast<const float *>(base + c1 * nb1 + c2 * nb2 + c3 * nb3);
+    while (walk.step(x)) {
+        const int t = walk.t, g = walk.g;
+        float v[64];
+        tq_load<GATE, STAGED>(x ? x + (int64_t)s * 256 : nullptr, src.base, id.gate, tiles, v);
+        uint8_t *grp = out + (((size_t)t * nst + s) * 2 + (q >> 1)) * STAGE + g * GROUP;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            float m[4] = { 0.f, 0.f, 0.f, 0.f };
+#pragma unroll
+            for (int i = 0; i < 32; ++i) m[i & 3] = fmaxf(m[i & 3], fabsf(v[32 * b + i]));
+            const float amax = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+            const float d = __fdiv_rn(amax, 127.f);
+            const float inv = d != 0.f ? __fdiv_rn(1.f, d) : 0.f;
+            const int j = 2 * (q & 1) + b;
+            uint8_t *o = grp + j * CODE_BLOCK + r * 16;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                __align__(16) __half2 w[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float *f = v + 32 * b + 8 * c + 4 * i;
+                    w[2 * i] = __floats2half2_rn(tq_round_away(__fmul_rn(f[0], inv)), tq_round_away(__fmul_rn(f[2], inv)));
+                    w[2 * i + 1] = __floats2half2_rn(tq_round_away(__fmul_rn(f[1], inv)), tq_round_away(__fmul_rn(f[3], inv)));
+                }
+                *reinterpret_cast<uint4 *>(o + c * 128) = *reinterpret_cast<const uint4 *>(w);
             }
-            x += (int64_t)s * 256 + 16 * l;
+            *reinterpret_cast<uint4 *>(grp + GROUP_SCALES + j * 128 + r * 16) = make_uint4(__half_as_ushort(__float2half_rn(d)), 0, 0, 0);
         }
-        float4 v[4];
-        float amax = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[i] = x ? *reinterpret_cast<const float4 *>(x + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (GATE && x) v[i] = swiglu4(*reinterpret_cast<const float4 *>(x + id.gate + 4 * i), v[i]);
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-        }
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-        const float d = __fdiv_rn(amax, 127.f);
-        const float inv = d != 0.f ? __fdiv_rn(1.f, d) : 0.f;
-        uint8_t *grp = stage + (j >> 2) * STAGE + (col >> 3) * GROUP;
-        __align__(16) __half2 w[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            w[2 * i] = __floats2half2_rn(roundf(__fmul_rn(v[i].x, inv)), roundf(__fmul_rn(v[i].z, inv)));
-            w[2 * i + 1] = __floats2half2_rn(roundf(__fmul_rn(v[i].y, inv)), roundf(__fmul_rn(v[i].w, inv)));
-        }
-        uint8_t *o = grp + (j & 3) * CODE_BLOCK + (col & 7) * 16;
-        *reinterpret_cast<uint4 *>(o + (2 * (l & 1)) * 128) = *reinterpret_cast<const uint4 *>(w);
-        *reinterpret_cast<uint4 *>(o + (2 * (l & 1) + 1) * 128) = *reinterpret_cast<const uint4 *>(w + 4);
-        if ((l & 1) == 0)
-            *reinterpret_cast<uint4 *>(grp + GROUP_SCALES + (j & 3) * 128 + (col & 7) * 16) = make_uint4(__half_as_ushort(__float2half_rn(d)), 0, 0, 0);
+        if ((q & 1) == 0) *reinterpret_cast<uint4 *>(grp + GROUP_ZERO + r * 16) = make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -523,9 +501,11 @@ size_t gemm_t32_act_bytes(int64_t K, int64_t N) { return (size_t)(((N + t32::BN 
 b200q_status launch_quantize_t32(b200q_ctx *ctx, const b200q_tensor *src1, uint8_t *out, int64_t n_tiles, const TileRoute *tr) {
     const int64_t K = src1->ne[0], N = src1->ne[1] * src1->ne[2] * src1->ne[3];
     const TileRoute &id = tr ? *tr : NO_ROUTE_T32;
-    dim3 grid((unsigned)(K / 256), (unsigned)n_tiles);
-    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, id.gate ? t32::quantize_kernel<true> : t32::quantize_kernel<false>, grid, dim3(quantizer_threads(ctx, src1, n_tiles, id, 320)), 0, ctx->stream,
-                               (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3], K, N, out, id));
+    const TqSource src = { (const uint8_t *)src1->data, src1->ne[1], src1->ne[2], src1->nb[1], src1->nb[2], src1->nb[3] };
+    const bool staged = id.tiles || N >= TQ_STAGED_COLS;
+    auto kern = id.gate ? t32::quantize_kernel<true, true> : staged ? t32::quantize_kernel<false, true> : t32::quantize_kernel<false, false>;
+    B200Q_CUDA(ctx, launch_pdl(!ctx->no_pdl, kern, tq_grid(ctx, K, N, n_tiles, t32::BN, id), dim3(TQ_THREADS), tq_smem(staged),
+                               ctx->stream, src, K, N, out, id));
     B200Q_CUDA(ctx, cudaGetLastError());
     count(ctx, ST_GEMM_TC_QUANT);
     return B200Q_OK;

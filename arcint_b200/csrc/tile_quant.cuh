@@ -1,0 +1,189 @@
+// tile_quant.cuh -- what the tiled quantizers of the prompt GEMMs (gemm_t32.cu, gemm_kq.cu, gemm_kf.cu) share: who reads what.
+//
+// A warp takes 256 values (one super-block) of a group of eight columns of a column tile: lane = (quarter q of the 256 values, column r). It
+// has sixteen 16-byte copies in flight and then two whole 32-blocks in registers; what its values become is stored in 16-byte pieces, and the
+// layouts keep the pieces of eight columns together: eight neighbouring lanes write a line of 128 bytes. No barrier, and no shuffle but for
+// the maximum of a column. A block is four warps: 32 columns of a tile.
+// Bound: memory, and for few columns the latency of one pass. Against a block a tile, a half-warp a column at a time, conversions to int and
+// back: Q4_0 4096x4096 x 512 tokens (64 blocks then) 49.0 -> 45.4 us with its GEMM, Q6_K 4096x11008 x 333 82.3 -> 79.4, Q4_K 11008x4096 x
+// 512 75.9 -> 75.0; the activation of 2048 tokens for ten experts each out of 512 66.5 -> 43 us (with a gate, where it is mostly arithmetic, 40 ->
+// 45; less arithmetic a thread and more threads gave 42 to 46 as well).
+#pragma once
+
+#include "common.cuh"
+
+namespace b200q {
+
+constexpr int TQ_THREADS = 128, TQ_WARPS = TQ_THREADS / 32, TQ_COLS = 8 * TQ_WARPS, TQ_SPLIT = 128 / TQ_COLS;
+
+struct TqSource { const uint8_t *base; int64_t ne1, ne2; size_t nb1, nb2, nb3; };
+
+// The groups of eight columns that a warp walks, and where the lane's column r of each begins (null: the column does not exist; then zeros
+// are quantized). A dense product's warp has one group. Of a route nobody knows on the host how many tiles there are and how full: the
+// blocks walk the tiles y, y + gridDim.y, ..., and a warp takes one of the sixteen groups of each, another one from tile to tile, since
+// only full tiles have the last ones (a block for every tile and 32 columns that could exist were 21504 of 128 threads for 2048 tokens of
+// ten experts out of 512, most of them empty: 64 us; all groups of a tile by one block: 50 us, a few blocks had most of the full tiles).
+// A tile's entry is asked for two tiles ahead, its pair one ahead.
+struct TqWalk {
+    const TqSource &src;
+    const TileRoute &id;
+    int64_t N;
+    int bn, n, t, g;
+    int4 cur, next;
+    int pair, pair_next;
+    __device__ __forceinline__ int group_of(int tile) const { return ((int)blockIdx.z * TQ_WARPS + (int)(threadIdx.x >> 5) + 5 * tile) & 15; }
+    __device__ __forceinline__ int4 entry(int tile) const { return tile < n ? __ldg(reinterpret_cast<const int4 *>(id.tiles) + tile) : make_int4(0, 0, 0, 0); }
+    __device__ __forceinline__ int pair_of(const int4 &e, int tile) const {
+        const int col = 8 * group_of(tile) + (threadIdx.x & 7);
+        return col < e.z ? __ldg(id.pairs + e.y + col) : -1;
+    }
+    __device__ __forceinline__ TqWalk(const TqSource &s_, const TileRoute &id_, int64_t N_, int bn_) : src(s_), id(id_), N(N_), bn(bn_), t((int)blockIdx.y - (int)gridDim.y) {
+        n = (int)gridDim.y;
+        if (!id.tiles) return;
+        n = __ldg(id.n_tiles);
+        next = entry(blockIdx.y);
+        pair_next = pair_of(next, blockIdx.y);
+        cur = next;
+        next = entry(blockIdx.y + gridDim.y);
+    }
+    // on to the next group with columns; x: the lane's column
+    __device__ __forceinline__ bool step(const float *&x) {
+        while ((t += gridDim.y) < n) {
+            if (id.tiles) {
+                const int4 e = cur;
+                pair = pair_next;
+                cur = next;
+                next = entry(t + 2 * gridDim.y);
+                pair_next = pair_of(cur, t + gridDim.y);
+                g = group_of(t);
+                if (8 * g >= e.z) continue;
+                // pair p = (token, slot) reads src1 row slot % ne11
+                const int tok = pair / id.n_used, slot = pair - tok * id.n_used;
+                x = pair < 0 ? nullptr : reinterpret_cast<const float *>(src.base + (size_t)(slot % id.ne11) * id.nb1 + (size_t)tok * id.nb2);
+                return true;
+            }
+            g = (int)blockIdx.z * TQ_WARPS + (int)(threadIdx.x >> 5);
+            const int64_t c0 = (int64_t)t * bn + 8 * g, c = c0 + (threadIdx.x & 7);
+            if (c0 >= N) continue;
+            if (c >= N) x = nullptr;
+            else if (c < src.ne1) x = reinterpret_cast<const float *>(src.base + c * src.nb1);                 // (no 64-bit division for plain columns)
+            else {
+                const int64_t c1 = c % src.ne1, c23 = c / src.ne1, c2 = c23 % src.ne2, c3 = c23 / src.ne2;
+                x = reinterpret_cast<const float *>(src.base + c1 * src.nb1 + c2 * src.nb2 + c3 * src.nb3);
+            }
+            return true;
+        }
+        return false;
+    }
+};
+
+// The lane's 64 values (zeros for a column that does not exist), silu(gate) * value with GATE. mine: where the values of column r begin.
+// STAGED: through shared memory: a warp asks for a column's kilobyte as two instructions of four lines each, where its lanes' own quarters
+// lie in 32 lines (the first-level cache looks up a line a clock: 512 clk for eight columns, 42 us of the 64 that the activation of a
+// 512-expert product of 2048 tokens took). A column's place there is 16 bytes longer than the column: the eight lanes of a read meet no
+// bank twice. Not for few columns: a GEMM's block, which takes all of shared memory, could not start beside the quantizer's (Q4_K
+// 11008x4096 x 24 tokens 21.1 us without and 22.5 with).
+constexpr int TQ_COL = 1024 + 16, TQ_TILE = 8 * TQ_COL;
+constexpr int TQ_STAGED_COLS = 128;
+constexpr int tq_smem(bool staged) { return staged ? TQ_WARPS * TQ_TILE : 0; }
+__device__ __forceinline__ void tq_copy16(uint32_t dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// one kilobyte of eight columns, `off` floats from where they begin
+__device__ __forceinline__ void tq_fetch(const float *mine, int64_t off, const void *any, uint8_t *tile) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(tile) + lane * 16;
+    __syncwarp();                                              // (the tile's last values have been read)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float *p = reinterpret_cast<const float *>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(mine), c));
+        const uint32_t n = p ? 16u : 0u;                       // (0: sixteen zeros, nothing is read)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) tq_copy16(dst + c * TQ_COL + h * 512, p ? (const void *)(p + off + 128 * h + 4 * lane) : any, n);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+}
+template <bool GATE, bool STAGED>
+__device__ __forceinline__ void tq_load(const float *mine, const void *any, int64_t gate, uint8_t *smem, float (&v)[64]) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (!STAGED) {
+        static_assert(!GATE, "routes are staged");
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float4 f = mine ? __ldg(reinterpret_cast<const float4 *>(mine + 64 * (lane >> 3)) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
+        }
+    } else {
+        uint8_t *tile = smem + (threadIdx.x >> 5) * TQ_TILE;
+        const float4 *own = reinterpret_cast<const float4 *>(tile + (lane & 7) * TQ_COL + (lane >> 3) * 256);
+        if (GATE) {                                            // silu(gate) first: one tile a warp, so that four blocks fit an SM
+            tq_fetch(mine, gate, any, tile);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float4 f = own[i];
+                v[4 * i] = silu(f.x); v[4 * i + 1] = silu(f.y); v[4 * i + 2] = silu(f.z); v[4 * i + 3] = silu(f.w);
+            }
+        }
+        tq_fetch(mine, 0, any, tile);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float4 f = own[i];
+            v[4 * i] = GATE ? v[4 * i] * f.x : f.x;
+            v[4 * i + 1] = GATE ? v[4 * i + 1] * f.y : f.y;
+            v[4 * i + 2] = GATE ? v[4 * i + 2] * f.z : f.z;
+            v[4 * i + 3] = GATE ? v[4 * i + 3] * f.w : f.w;
+        }
+    }
+}
+
+// the largest magnitude of the column's 256 values (64 in each of four lanes)
+__device__ __forceinline__ float tq_column_max(const float (&v)[64]) {
+    float m[4] = { 0.f, 0.f, 0.f, 0.f };
+#pragma unroll
+    for (int i = 0; i < 64; ++i) m[i & 3] = fmaxf(m[i & 3], fabsf(v[i]));
+    float amax = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 8));
+    return fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 16));
+}
+
+// The per-256 form's codes as floats, in place: x * iq rounded to the nearest integer, halves to even, 0 for a NaN. Adding 1.5 * 2^23 leaves
+// no bits below one (|x * iq| <= 128), which takes a quarter of the time of a conversion to int and back.
+__device__ __forceinline__ void tq_codes256(float (&v)[64], float iq) {
+    constexpr float MAGIC = 12582912.f;
+    float nan[4] = { 0.f, 0.f, 0.f, 0.f };
+#pragma unroll
+    for (int i = 0; i < 64; ++i) {
+        v[i] = __fadd_rn(__fadd_rn(__fmul_rn(v[i], iq), MAGIC), -MAGIC);
+        nan[i & 3] += v[i];
+    }
+    const float any = (nan[0] + nan[1]) + (nan[2] + nan[3]);
+    if (any != any) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) v[i] = v[i] == v[i] ? v[i] : 0.f;
+    }
+}
+
+// roundf (halves away from zero) for |x| < 2^22, NaN for NaN: rounded halves to even, then one up where that went down by a half
+__device__ __forceinline__ float tq_round_away(float x) {
+    constexpr float MAGIC = 12582912.f;
+    const float a = fabsf(x);
+    float r = __fadd_rn(__fadd_rn(a, MAGIC), -MAGIC);
+    if (__fsub_rn(a, r) == 0.5f) r = __fadd_rn(r, 1.f);
+    return copysignf(r, x);
+}
+
+__device__ __forceinline__ int tq_block() { return ((int)blockIdx.z * (int)gridDim.y + (int)blockIdx.y) * (int)gridDim.x + (int)blockIdx.x; }
+// blocks of a quantizer: 256 weights, tiles (of a route: as many as are resident at a time), runs of 32 columns
+inline dim3 tq_grid(const b200q_ctx *ctx, int64_t K, int64_t N, int64_t n_tiles, int bn, const TileRoute &tr) {
+    const int64_t steps = K / 256;
+    if (tr.tiles) {
+        // (with a gate a step is mostly arithmetic and a block's share of full tiles tells: a block a tile. 512 experts, 2048 tokens: 63 us
+        // with as many blocks as are resident)
+        const int64_t room = tr.gate ? n_tiles : (5 * ctx->sm_count + steps * TQ_SPLIT - 1) / (steps * TQ_SPLIT);
+        return dim3((unsigned)steps, (unsigned)(n_tiles < room ? n_tiles : room), TQ_SPLIT);
+    }
+    return dim3((unsigned)steps, (unsigned)n_tiles, (unsigned)(((N < bn ? N : bn) + TQ_COLS - 1) / TQ_COLS));
+}
+
+}  // namespace b200q
