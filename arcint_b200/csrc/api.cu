@@ -494,6 +494,19 @@ b200q_status b200q_mul_mat(b200q_ctx *ctx, const b200q_tensor *src0, const b200q
                               (float *)dst->data, ldd, act.fresh);
     }
     if (N > 8) count(ctx, ST_GEMM_FALLBACK_SHAPE);
+    if (N == 1) {
+        // (the caches' contract: inside a generation a tensor keeps its values)
+        auto &o = ctx->one_act;
+        const bool known = o.data == src1->data && o.id == src1->id && o.K == K && o.gen == ctx->generation;
+        st = launch_gemv_one(ctx, src0->type, src0->data, src0->nb[1], M, K, src1, (float *)dst->data, known);
+        if (st == B200Q_OK) {
+            o.data = src1->data;
+            o.id = src1->id;
+            o.K = K;
+            o.gen = ctx->generation;
+        }
+        if (st != B200Q_UNSUPPORTED) return st;
+    }
     // small per-32 products at one or two columns: the GEMV quantizes its own slice of the activation, one launch
     // instead of two (what matters once a tensor-parallel shard is a microsecond of weights)
     if (N <= 2 && uniform) {

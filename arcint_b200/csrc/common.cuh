@@ -120,6 +120,9 @@ struct b200q_ctx {
     cudaEvent_t  ev_fork = nullptr, ev_join = nullptr;
     bool         copy_pending = false;    // the copy streams hold work the compute stream has not joined
     uint64_t     generation = 1;
+    // The activation of the one-column product before this call (gemv_one.cuh), if nothing else of the library was launched since: the next product
+    // of the same generation may read it without waiting for that product. (Every launch counts something, and counting forgets it.)
+    struct { const void *data = nullptr, *id = nullptr; int64_t K = 0; uint64_t gen = 0; } one_act;
     // what the gathered, tiled activation scratch of the tensor-core MUL_MAT_ID holds (gate and up of a layer
     // read the same src1 through the same ids: the second call finds it ready)
     struct { const void *src1 = nullptr, *ids = nullptr, *src1_id = nullptr, *ids_id = nullptr; int64_t ne[4] = {0, 0, 0, 0}; size_t nb[4] = {0, 0, 0, 0}; uint64_t gen = 0; int64_t gate = 0; int form = -1, n_expert = 0; } moe_act;
@@ -174,7 +177,10 @@ bool         ws_try_reserve(b200q_ctx *ctx, Workspace *ws, size_t bytes);
 void ws_release(Workspace *ws);
 cudaError_t  device_alloc(b200q_ctx *ctx, void **p, size_t bytes);
 int moe_route_workspaces(b200q_ctx *ctx, Workspace **out, const char **names);   // the route caches' blocks, for the guard check
-inline void  count(b200q_ctx *ctx, int stat) { ++ctx->counters[stat]; }
+inline void  count(b200q_ctx *ctx, int stat) {
+    ++ctx->counters[stat];
+    ctx->one_act.data = nullptr;          // (see there)
+}
 
 #define B200Q_CUDA(ctx, expr)                                                                       \
     do {                                                                                            \
@@ -195,6 +201,9 @@ b200q_status launch_gemv(b200q_ctx *ctx, int type, const void *w, size_t row_str
                          const ActView &act, int64_t col0, int ncols, float *dst, int64_t ldd);
 // the same for one or two columns of a small Q4_0 / Q8_0 product, quantizing src1 inside the kernel;
 // B200Q_UNSUPPORTED: not that case, take the quantizer + launch_gemv
+// one column, quantized inside the GEMV (gemv_one.cuh); B200Q_UNSUPPORTED: not that case. known: a product of this generation, launched
+// the same way on this stream, has read the same activation
+b200q_status launch_gemv_one(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K, const b200q_tensor *src1, float *dst, bool known);
 b200q_status launch_gemv_fused(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                                const b200q_tensor *src1, int ncols, float *dst, int64_t ldd);
 

@@ -81,6 +81,38 @@ b200q_status launch_gemv_id(b200q_ctx *ctx, int type, const void *w, size_t row_
     return fail(ctx, B200Q_UNSUPPORTED, "gemv_id: type %d", type);
 }
 
+b200q_status launch_gemv_one(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K, const b200q_tensor *src1, float *dst, bool known) {
+    TypeInfo ti;
+    if (!type_info(type, &ti)) return B200Q_UNSUPPORTED;
+    // the tuner's switches are of the kernels that this one stands before
+    if (ctx->no_stream || ctx->gemv_stream_mask >= 0 || ctx->gemv_rows || ctx->gemv_block_warps || ctx->fuse_quant_bytes > 0) return B200Q_UNSUPPORTED;
+    const size_t row_bytes = (size_t)(K / ti.block) * ti.bytes;
+    // rows one behind the other, where the lane code can read them; the activation as plain f32
+    if (row_stride != row_bytes || ((uintptr_t)w | row_bytes) % (size_t)gemv_row_align(type) || M > INT32_MAX / 2 || K > INT32_MAX / 256) return B200Q_UNSUPPORTED;
+    // (the per-32 types: rows of whole words)
+    if (ti.block == 32 && ((uintptr_t)w | row_bytes) % 4) return B200Q_UNSUPPORTED;
+    if (src1->nb[0] != 4 || (uintptr_t)src1->data % 16) return B200Q_UNSUPPORTED;
+    const float *x = (const float *)src1->data;
+    // every block reads the whole activation, at its own time: results must not land in it (the two-kernel route has its codes by then)
+    if (dst < x + K && x < dst + M) return B200Q_UNSUPPORTED;
+    b200q_status st = B200Q_UNSUPPORTED;
+    switch (type) {
+    case B200Q_TYPE_Q4_0:   st = launch_one_column<B200Q_TYPE_Q4_0>(ctx, w, M, K, x, dst, known); break;
+    case B200Q_TYPE_Q8_0:   st = launch_one_column<B200Q_TYPE_Q8_0>(ctx, w, M, K, x, dst, known); break;
+    case B200Q_TYPE_Q4_K:   st = launch_one_column<B200Q_TYPE_Q4_K>(ctx, w, M, K, x, dst, known); break;
+    case B200Q_TYPE_Q5_K:   st = launch_one_column<B200Q_TYPE_Q5_K>(ctx, w, M, K, x, dst, known); break;
+    case B200Q_TYPE_Q6_K:   st = launch_one_column<B200Q_TYPE_Q6_K>(ctx, w, M, K, x, dst, known); break;
+    case B200Q_TYPE_IQ4_XS: st = launch_one_column<B200Q_TYPE_IQ4_XS>(ctx, w, M, K, x, dst, known); break;
+    case B200Q_TYPE_IQ4_NL: st = launch_one_column<B200Q_TYPE_IQ4_NL>(ctx, w, M, K, x, dst, known); break;
+    }
+    if (st == B200Q_OK) {
+        count(ctx, (gemv_row_mode(type, (size_t)(uintptr_t)w | row_stride, row_bytes) == GEMV_ROWS_ALIGNED ? ST_GEMV_COL0 : ST_GEMV_UNALIGNED_COL0) + 1);
+        count(ctx, ST_GEMV_STREAM);
+        count(ctx, ST_GEMV_FUSED_QUANT);
+    }
+    return st;
+}
+
 b200q_status launch_gemv_fused(b200q_ctx *ctx, int type, const void *w, size_t row_stride, int64_t M, int64_t K,
                                const b200q_tensor *src1, int ncols, float *dst, int64_t ldd) {
     if (type != B200Q_TYPE_Q4_0 && type != B200Q_TYPE_Q8_0) return B200Q_UNSUPPORTED;

@@ -114,6 +114,17 @@ B200Q_HD uint16_t ld_u16(const uint16_t *p) {
     return *p;
 #endif
 }
+// the activation's loads: from global memory (G), or from wherever the pointer leads (shared memory)
+template <bool G> B200Q_HD I4 act16(const void *p) {
+#ifdef __CUDA_ARCH__
+    if (!G) { const int4 v = *reinterpret_cast<const int4 *>(p); return I4{ v.x, v.y, v.z, v.w }; }
+#endif
+    return hd_ld16(p);
+}
+template <bool G> B200Q_HD int act_s16(const int16_t *p) { return G ? ld_s16(p) : (int)*p; }
+template <bool G> B200Q_HD uint32_t act_u32(const void *p) { return G ? ld_u32(p) : *reinterpret_cast<const uint32_t *>(p); }
+template <bool G> B200Q_HD float act_f32(const float *p) { return G ? ld_f32(p) : *p; }
+template <bool G> B200Q_HD uint16_t act_u16(const uint16_t *p) { return G ? ld_u16(p) : *p; }
 B200Q_HD int sext8(uint32_t v) { return (int)(int8_t)(v & 0xFFu); }
 B200Q_HD int sext16(uint32_t v) { return (int)(int16_t)(v & 0xFFFFu); }
 
@@ -129,7 +140,7 @@ template <int NC> struct GemvX {
 
 // cols[c]: which column of the quantized activation buffer column c of this launch is (the
 // identity for a dense product, a routed pair's column for MUL_MAT_ID).
-template <int TYPE, int NC>
+template <int TYPE, int NC, bool G = true>
 B200Q_HD void gemv_load_x(int lane, int s, int nblk, const GemvAct &act, const int (&cols)[NC], GemvX<NC> &X) {
     typedef GemvFmt<TYPE> F;
     const int K = act.K;
@@ -143,24 +154,24 @@ B200Q_HD void gemv_load_x(int lane, int s, int nblk, const GemvAct &act, const i
             const int8_t *xp = act.q + (size_t)cols[c] * K;
             const size_t sc = (size_t)cols[c] * (K / 32);
             if (X.live) {
-                X.x[c][0] = hd_ld16(xp + 32 * b0);
-                X.x[c][1] = hd_ld16(xp + 32 * b0 + 16);
-                X.f0[c] = hd_half_bits(ld_u16(act.d16 + sc + b0));
+                X.x[c][0] = act16<G>(xp + 32 * b0);
+                X.x[c][1] = act16<G>(xp + 32 * b0 + 16);
+                X.f0[c] = hd_half_bits(act_u16<G>(act.d16 + sc + b0));
                 if (TYPE == B200Q_TYPE_Q4_0) {
 #ifdef B200Q_RED_Q40
-                    X.i0[c] = -64 * ld_s16(act.s32 + sc + b0);
+                    X.i0[c] = -64 * act_s16<G>(act.s32 + sc + b0);
 #else
-                    X.i0[c] = -128 * ld_s16(act.s32 + sc + b0);      // -8 * 16 * sum(x)
+                    X.i0[c] = -128 * act_s16<G>(act.s32 + sc + b0);      // -8 * 16 * sum(x)
 #endif
                     X.f0[c] *= 0.0625f;                              // the nibble dot is kept x16
                 }
             }
             if (X.live2) {
-                X.x[c][2] = hd_ld16(xp + 32 * b1);
-                X.x[c][3] = hd_ld16(xp + 32 * b1 + 16);
-                X.f1[c] = hd_half_bits(ld_u16(act.d16 + sc + b1));
+                X.x[c][2] = act16<G>(xp + 32 * b1);
+                X.x[c][3] = act16<G>(xp + 32 * b1 + 16);
+                X.f1[c] = hd_half_bits(act_u16<G>(act.d16 + sc + b1));
                 if (TYPE == B200Q_TYPE_Q4_0) {
-                    X.i1[c] = -128 * ld_s16(act.s32 + sc + b1);
+                    X.i1[c] = -128 * act_s16<G>(act.s32 + sc + b1);
                     X.f1[c] *= 0.0625f;
                 }
             }
@@ -175,10 +186,10 @@ B200Q_HD void gemv_load_x(int lane, int s, int nblk, const GemvAct &act, const i
         for (int c = 0; c < NC; ++c) {
             const int8_t *xp = act.q + (size_t)cols[c] * K + 256 * blk + 64 * g;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) X.x[c][j] = hd_ld16(xp + 16 * j);
-            X.f0[c] = ld_f32(act.d32 + (size_t)cols[c] * (K / 256) + blk);
+            for (int j = 0; j < 4; ++j) X.x[c][j] = act16<G>(xp + 16 * j);
+            X.f0[c] = act_f32<G>(act.d32 + (size_t)cols[c] * (K / 256) + blk);
             // the sums of the lane's two sub-blocks, kept as the pair of 16-bit halves they are stored as
-            X.i0[c] = (int)ld_u32(act.s32 + (size_t)cols[c] * (K / 32) + 8 * blk + 2 * g);
+            X.i0[c] = (int)act_u32<G>(act.s32 + (size_t)cols[c] * (K / 32) + 8 * blk + 2 * g);
         }
     } else if (TYPE == B200Q_TYPE_IQ4_XS) {
         // lane -> block sb and sub-block pair pp: 32 bytes = sub-blocks 2pp and 2pp+1
@@ -189,8 +200,8 @@ B200Q_HD void gemv_load_x(int lane, int s, int nblk, const GemvAct &act, const i
         for (int c = 0; c < NC; ++c) {
             const int8_t *xp = act.q + (size_t)cols[c] * K + 256 * blk + 64 * pp;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) X.x[c][j] = hd_ld16(xp + 16 * j);
-            X.f0[c] = ld_f32(act.d32 + (size_t)cols[c] * (K / 256) + blk);
+            for (int j = 0; j < 4; ++j) X.x[c][j] = act16<G>(xp + 16 * j);
+            X.f0[c] = act_f32<G>(act.d32 + (size_t)cols[c] * (K / 256) + blk);
         }
     } else if (TYPE == B200Q_TYPE_Q6_K) {
         // lane -> block sb, half n, positions t0..t0+15 of the four 32-weight parts of that
@@ -203,10 +214,10 @@ B200Q_HD void gemv_load_x(int lane, int s, int nblk, const GemvAct &act, const i
         for (int c = 0; c < NC; ++c) {
             const int8_t *xp = act.q + (size_t)cols[c] * K + 256 * blk + 128 * n + t0;
 #pragma unroll
-            for (int p = 0; p < 4; ++p) X.x[c][p] = hd_ld16(xp + 32 * p);
-            X.f0[c] = ld_f32(act.d32 + (size_t)cols[c] * (K / 256) + blk);
+            for (int p = 0; p < 4; ++p) X.x[c][p] = act16<G>(xp + 32 * p);
+            X.f0[c] = act_f32<G>(act.d32 + (size_t)cols[c] * (K / 256) + blk);
             // sums of groups 8n + 2p + hi16, p = 0..3: eight int16 from one 16-byte load
-            const I4 sv = hd_ld16(act.s16 + (size_t)cols[c] * (K / 16) + 16 * blk + 8 * n);
+            const I4 sv = act16<G>(act.s16 + (size_t)cols[c] * (K / 16) + 16 * blk + 8 * n);
             X.i0[c] = -32 * sext16((uint32_t)sv.x >> (16 * hi16));     // sum((q-32) x) = sum(q x) - 32 sum(x)
             X.i1[c] = -32 * sext16((uint32_t)sv.y >> (16 * hi16));
             X.i2[c] = -32 * sext16((uint32_t)sv.z >> (16 * hi16));

@@ -1,0 +1,311 @@
+// gemv_one.cuh -- the decode GEMV of one column, which quantizes its activation itself: one launch per product, built to run beside the
+// next one.
+//
+// At one column a product is one to seventeen microseconds of weight stream, and what a chain of products loses is the time in which
+// no weights are on their way: a launch, the activation's quantizer in a kernel of its own, the first loads' latency, the last rows. So:
+//   - a block's warps put their first rows in flight before they wait for the kernel before: weights depend on nobody. The block uses less
+//     than half of an SM (shared memory, registers), and lets the next product's blocks in as soon as it has seen its own predecessor complete;
+//   - the activation is quantized by every block for itself once the kernel before has completed (16 KB out of L2 at K = 4096), by all
+//     its warps, into shared memory, while the first rows arrive. Same arithmetic as quantize.cu, operation for operation;
+//   - a warp owns one slice of 2048 weights of every row of its group, keeps the slice's activation in registers and streams its slices
+//     through a ring of its own, 16 bytes a lane and copy: no barrier but at the ends. (Plain copies: with an L2 eviction hint the Q8_0 build met
+//     an illegal instruction at its first copy, where the same source for the other types ran. cp.async.bulk copies of one warp follow each other at the
+//     latency of the memory, some 1400 clk each whatever their size and however many stages are free: a block with one warp that
+//     copied whole rows for sixteen took 11.5 us at Q4_0 4096x11008, where this form takes 9.3 alone and 6.3 in a chain.)
+//   - a product whose activation the product before has read (q, k and v, gate and up) does not wait for it, but for its results;
+//   - sums of four rows are reduced together; the slices' halves meet in shared memory and are added in a fixed order when the block's rows are done.
+// Bound: the weight stream, and close behind it instruction issue (Q6_K most of all: 5.1 TB/s where Q8_0 has 6.3).
+// B200, us a product in a recorded chain, first the quantizer's kernel and gemv_stream.cuh (Q6_K: gemv_kernel.cuh), then this kernel, then this
+// kernel where the product before has the same activation: Q4_0 4096x4096 5.4, 4.0, 3.2 (the kernel before with its codes known 3.9), 11008x4096 8.6,
+// 7.5, 5.5 (7.4), 4096x11008 9.4, 9.3, 6.3 (8.0); Q4_K 11008x4096 9.1, 7.6, 5.9; Q6_K 32000x4096 25.2, 21.5, 20.1; Q8_0 11008x4096 12.4, 11.5, 8.1.
+//
+// Stands in, at one column, for the reference's kernel_mul_mv_*_q8_1 family and its activation quantizer (marfrit/arcint
+// contrib/llama.cpp/patches/0000-01-kquant-integer-dpas.patch:3882-3915, 1862-1889).
+#pragma once
+
+#include "gemv_core.cuh"
+#include "gemv_kernel.cuh"
+#include "gemv_stream.cuh"
+#include "pdl.cuh"
+#include "tc_common.cuh"
+
+namespace b200q {
+
+constexpr int GEMV_ONE_WARPS = 16;                        // warps of a block, at most
+constexpr size_t GEMV_ONE_SMEM = 113 * 1024;              // two blocks an SM
+
+template <int TYPE> __host__ __device__ constexpr bool gemv_one_per32() { return TYPE == B200Q_TYPE_Q4_0 || TYPE == B200Q_TYPE_Q8_0 || TYPE == B200Q_TYPE_IQ4_NL; }
+// bytes of a slice's place in a ring (it begins up to 15 bytes in, and the lane code reads a word past it), and places of a ring
+template <int TYPE> __host__ __device__ constexpr int gemv_one_slot() { return (GemvStage<TYPE>::BYTES + 15 + 4 + 15) / 16 * 16; }
+// (two blocks an SM. Rings that take most of an SM were no faster for long streams: 32000x4096 in Q4_K 15.7 us with eight places and with
+// five, in Q6_K 23.3 with six and 21.5 with four, and cost the overlap of a chain: Q4_K 13.2 there)
+template <int TYPE> __host__ __device__ constexpr int gemv_one_depth() {
+    constexpr int slot = gemv_one_slot<TYPE>();
+    return slot < 1300 ? 5 : slot < 1800 ? 4 : 3;
+}
+
+// where the parts of a block's shared memory begin
+struct GemvOneLayout {
+    int nsl, groups;                                      // slices of a row, groups of warps
+    int codes, scales, s32, s16, part, total;             // byte offsets (the rings at 0)
+};
+
+// false: the shape does not fit
+template <int TYPE>
+inline bool gemv_one_layout(int64_t M, int nblk, int blocks, GemvOneLayout &L) {
+    typedef GemvFmt<TYPE> F;
+    const int64_t K = (int64_t)nblk * F::BLK_W;
+    auto up = [](int64_t v) { return (v + 15) / 16 * 16; };
+    L.nsl = (nblk + F::STAGE_BLOCKS - 1) / F::STAGE_BLOCKS;
+    if (L.nsl > GEMV_ONE_WARPS) return false;
+    const int64_t rows = (M + blocks - 1) / blocks;
+    L.groups = GEMV_ONE_WARPS / L.nsl;
+    if (L.groups > rows) L.groups = (int)rows;
+    L.codes = L.nsl * L.groups * gemv_one_depth<TYPE>() * gemv_one_slot<TYPE>();
+    L.scales = L.codes + (int)up(K);
+    L.s32 = L.scales + (int)up(gemv_one_per32<TYPE>() ? K / 16 : K / 64);
+    L.s16 = L.s32 + (int)up(K / 16);
+    L.part = L.s16 + (gemv_one_per32<TYPE>() ? 0 : (int)up(K / 8));
+    L.total = L.part + (int)up(rows * L.nsl * 8);
+    return L.total <= 200 * 1024;
+}
+
+// The column's codes, scales and sums into shared memory by `nth` threads (whole warps), eight values a lane. The codes are those of
+// quantize.cu; whole numbers are rounded and packed in floating point (1.5 * 2^23 added leaves the code in the low bits), since every
+// block does this and conversions run at a quarter of the rate.
+__device__ __forceinline__ uint32_t gemv_one_pack4(float a, float b, float c, float d) {
+    return __byte_perm(__byte_perm(__float_as_uint(a), __float_as_uint(b), 0x0040), __byte_perm(__float_as_uint(c), __float_as_uint(d), 0x0040), 0x5410);
+}
+template <bool PER32>
+__device__ __forceinline__ void gemv_one_quantize(const float *__restrict__ x, int K, int tid, int nth, uint8_t *codes, uint8_t *scales, int16_t *s32, int16_t *s16) {
+    constexpr float MAGIC = 12582912.f;
+    const int lane = tid & 31;
+    for (int i0 = tid - lane; i0 < K / 8; i0 += nth) {
+        const int i = i0 + lane;
+        const bool live = i < K / 8;                          // (per 256: a warp is a block, all lanes are live)
+        float v[8];
+        {
+            const float4 a = live ? *reinterpret_cast<const float4 *>(x + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 b = live ? *reinterpret_cast<const float4 *>(x + 8 * i + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        }
+        float m = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))), fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
+#pragma unroll
+        for (int o = 1; o < (PER32 ? 4 : 32); o *= 2) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+        const float d = __fdiv_rn(m, 127.f);
+        float k;
+        if (PER32) k = d != 0.f ? __fdiv_rn(1.f, d) : 0.f;
+        else k = m > 1e-30f ? __fdiv_rn(127.f, m) : 0.f;
+        float any = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float t = __fmul_rn(v[j], k);
+            if (PER32) {
+                // halves away from zero: to even, and one up where that went down by a half
+                const float a = fabsf(t);
+                float r = __fadd_rn(__fadd_rn(a, MAGIC), -MAGIC);
+                if (__fsub_rn(a, r) == 0.5f) r = __fadd_rn(r, 1.f);
+                v[j] = copysignf(r, t);
+            } else v[j] = __fadd_rn(__fadd_rn(t, MAGIC), -MAGIC);
+            any += v[j];
+        }
+        if (!(fabsf(any) <= 1024.f)) {                        // an infinity or a NaN among them (the conversion of either, as in quantize.cu)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = (float)(int8_t)(PER32 ? (int)v[j] : __float2int_rn(v[j]));
+        }
+        uint32_t w0 = gemv_one_pack4(__fadd_rn(v[0], MAGIC), __fadd_rn(v[1], MAGIC), __fadd_rn(v[2], MAGIC), __fadd_rn(v[3], MAGIC));
+        uint32_t w1 = gemv_one_pack4(__fadd_rn(v[4], MAGIC), __fadd_rn(v[5], MAGIC), __fadd_rn(v[6], MAGIC), __fadd_rn(v[7], MAGIC));
+        int s = dp4a_ss(w0, 0x01010101, dp4a_ss(w1, 0x01010101, 0));
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
+        if (!PER32 && live && (lane & 1) == 0) s16[i >> 1] = (int16_t)s;
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
+        if (live) {
+            reinterpret_cast<uint2 *>(codes)[i] = make_uint2(w0, w1);
+            if ((lane & 3) == 0) s32[i >> 2] = (int16_t)s;
+            if (PER32 && (lane & 3) == 0) reinterpret_cast<uint16_t *>(scales)[i >> 2] = __half_as_ushort(__float2half_rn(d));
+            if (!PER32 && lane == 0) reinterpret_cast<float *>(scales)[i >> 5] = d;
+        }
+    }
+}
+
+template <int TYPE> struct gemv_one_act { typedef GemvX<1> type; };
+struct GemvOneX;
+template <> struct gemv_one_act<B200Q_TYPE_Q4_0> { typedef GemvOneX type; };
+template <> struct gemv_one_act<B200Q_TYPE_Q8_0> { typedef GemvOneX type; };
+template <> struct gemv_one_act<B200Q_TYPE_IQ4_NL> { typedef GemvOneX type; };
+// The per-32 types' lane code for rows of whole words (an even number of blocks): lane l has the blocks 2 l and 2 l + 1 of the slice, 9 or 17
+// whole words an odd number apart, so that no two lanes meet in a bank and only the first block's codes have to be shifted. (As in
+// gemv_core.cuh, blocks l and l + 32, it takes 12 and 20 words, two lanes a bank.)
+struct GemvOneX {
+    I4    x[4];
+    float f0, f1;
+    int   i0, i1;
+};
+template <int TYPE>
+__device__ __forceinline__ void gemv_one_load_x(int lane, int slice, int nblk, const uint8_t *codes, const uint8_t *scales, const int16_t *s32, GemvOneX &X) {
+    const int b = slice * 64 + 2 * lane;
+    const bool live = b < nblk;                           // (a row has an even number of blocks)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) X.x[j] = live ? act16<false>(codes + 32 * b + 16 * j) : I4{ 0, 0, 0, 0 };
+    const uint32_t d = live ? *reinterpret_cast<const uint32_t *>(scales + 2 * b) : 0u, m = live ? *reinterpret_cast<const uint32_t *>(s32 + b) : 0u;
+    X.f0 = hd_half_bits((uint16_t)d);
+    X.f1 = hd_half_bits((uint16_t)(d >> 16));
+    X.i0 = X.i1 = 0;
+    if (TYPE == B200Q_TYPE_Q4_0) {
+        X.i0 = -128 * sext16(m);                          // -8 * 16 * sum(x); the nibble dot is kept x16
+        X.i1 = -128 * sext16(m >> 16);
+        X.f0 *= 0.0625f;
+        X.f1 *= 0.0625f;
+    }
+}
+template <int TYPE>
+__device__ __forceinline__ float gemv_one_row(const uint32_t *p, const GemvOneX &X) {
+    constexpr int N = TYPE == B200Q_TYPE_Q8_0 ? 17 : 9;
+    uint32_t w[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = p[i];
+    float acc = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const float d = hd_half_bits((uint16_t)(u ? w[N / 2] >> 16 : w[0]));
+        const I4 xa = X.x[2 * u], xb = X.x[2 * u + 1];
+        uint32_t q[N / 2];
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) q[i] = u ? w[N / 2 + 1 + i] : __funnelshift_r(w[i], w[i + 1], 16);
+        int si;
+        if constexpr (TYPE == B200Q_TYPE_Q8_0) {
+            int s0 = dp4a_ss(q[0], xa.x, 0), s1 = dp4a_ss(q[1], xa.y, 0);
+            s0 = dp4a_ss(q[2], xa.z, s0); s1 = dp4a_ss(q[3], xa.w, s1);
+            s0 = dp4a_ss(q[4], xb.x, s0); s1 = dp4a_ss(q[5], xb.y, s1);
+            s0 = dp4a_ss(q[6], xb.z, s0); s1 = dp4a_ss(q[7], xb.w, s1);
+            si = s0 + s1;
+        } else if constexpr (TYPE == B200Q_TYPE_IQ4_NL) {
+            int s0 = dp4a_ss(iq4nl_lookup4(q[0] & 0x0F0F0F0Fu), xa.x, 0), s1 = dp4a_ss(iq4nl_lookup4(q[1] & 0x0F0F0F0Fu), xa.y, 0);
+            s0 = dp4a_ss(iq4nl_lookup4(q[2] & 0x0F0F0F0Fu), xa.z, s0); s1 = dp4a_ss(iq4nl_lookup4(q[3] & 0x0F0F0F0Fu), xa.w, s1);
+            s0 = dp4a_ss(iq4nl_lookup4((q[0] >> 4) & 0x0F0F0F0Fu), xb.x, s0); s1 = dp4a_ss(iq4nl_lookup4((q[1] >> 4) & 0x0F0F0F0Fu), xb.y, s1);
+            s0 = dp4a_ss(iq4nl_lookup4((q[2] >> 4) & 0x0F0F0F0Fu), xb.z, s0); s1 = dp4a_ss(iq4nl_lookup4((q[3] >> 4) & 0x0F0F0F0Fu), xb.w, s1);
+            si = s0 + s1;
+        } else {
+            // weights 4j..4j+3 in the low nibbles, 16+4j.. in the high ones (left x16)
+            int lo0 = dp4a_ss(q[0] & 0x0F0F0F0Fu, xa.x, 0), lo1 = dp4a_ss(q[1] & 0x0F0F0F0Fu, xa.y, 0);
+            lo0 = dp4a_ss(q[2] & 0x0F0F0F0Fu, xa.z, lo0);   lo1 = dp4a_ss(q[3] & 0x0F0F0F0Fu, xa.w, lo1);
+            int hi0 = dp4a_us(q[0] & 0xF0F0F0F0u, xb.x, u ? X.i1 : X.i0);
+            int hi1 = dp4a_us(q[1] & 0xF0F0F0F0u, xb.y, 0);
+            hi0 = dp4a_us(q[2] & 0xF0F0F0F0u, xb.z, hi0);   hi1 = dp4a_us(q[3] & 0xF0F0F0F0u, xb.w, hi1);
+            si = 16 * (lo0 + lo1) + (hi0 + hi1);                              // 16 * sum((n - 8) x)
+        }
+        acc += (float)si * (d * (u ? X.f1 : X.f0));
+    }
+    return acc;
+}
+
+// dst[m] = sum_k W[m][k] x[k], rows one behind the other; block b takes the rows [M b / gridDim.x, M (b + 1) / gridDim.x)
+template <int TYPE>
+__global__ void __launch_bounds__(GEMV_ONE_WARPS * 32, 2)
+gemv_one_kernel(const uint8_t *__restrict__ W, int64_t M, int nblk, const float *__restrict__ x, float *__restrict__ dst, int known, const __grid_constant__ GemvOneLayout L) {
+    typedef GemvFmt<TYPE> F;
+    typedef GemvStage<TYPE> S;
+    constexpr bool PER32 = gemv_one_per32<TYPE>();
+    constexpr int SLOT = gemv_one_slot<TYPE>(), D = gemv_one_depth<TYPE>(), PIECES = (S::BYTES + 15 + 511) / 512;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
+    const int row_bytes = nblk * F::BLK_B, K = nblk * F::BLK_W;
+    const int64_t r0 = M * blockIdx.x / gridDim.x;
+    const int rows = (int)(M * (blockIdx.x + 1) / gridDim.x - r0);
+    const int group = warp / L.nsl, slice = warp - group * L.nsl;
+    const int mine = (rows - group + L.groups - 1) / L.groups;              // the warp's slices: rows group, + groups, ...
+    const int bytes = min((int)S::BYTES, row_bytes - slice * (int)S::BYTES);
+    uint8_t *ring = smem + warp * (D * SLOT);
+    const size_t step = (size_t)L.groups * row_bytes;
+    // the next slice to ask for, and its place
+    uintptr_t p_at = (uintptr_t)W + (size_t)(r0 + group) * row_bytes + (size_t)slice * S::BYTES;
+    int p_n = 0;
+    uint32_t p_slot = 0;
+    auto issue = [&]() {
+        if (p_n < mine) {
+            const int sh = (int)(p_at & 15), n = sh + bytes;
+#pragma unroll
+            for (int j = 0; j < PIECES; ++j)
+                if (16 * lane + 512 * j < n) cp_async16(ring + p_slot + 16 * lane + 512 * j, (const void *)(p_at - sh + 16 * lane + 512 * j));
+        }
+        cp_async_commit();
+        ++p_n;
+        p_at += step;
+        p_slot = p_slot == (D - 1) * SLOT ? 0 : p_slot + SLOT;
+    };
+    uintptr_t c_at = p_at;                                                  // the next slice to multiply
+#pragma unroll
+    for (int i = 0; i < D - 1; ++i) issue();
+    // The activation is the output of the kernel before, and dst may be in use by it. Known: an earlier product of this graph, which
+    // waited before it let anybody start, has read the same activation; then only the results wait.
+    if (!known) pdl_wait();
+    pdl_trigger();                       // the next product's blocks may come in beside this one's
+    uint8_t *codes = smem + L.codes, *scales = smem + L.scales;
+    int16_t *s32 = reinterpret_cast<int16_t *>(smem + L.s32), *s16 = reinterpret_cast<int16_t *>(smem + L.s16);
+    gemv_one_quantize<PER32>(x, K, tid, blockDim.x, codes, scales, s32, s16);
+    __syncthreads();
+    typename gemv_one_act<TYPE>::type X;
+    if constexpr (PER32) gemv_one_load_x<TYPE>(lane, slice, nblk, codes, scales, s32, X);
+    else {
+        GemvAct act = {};
+        act.q = reinterpret_cast<const int8_t *>(codes);
+        act.d32 = reinterpret_cast<const float *>(scales);
+        act.s32 = s32;
+        act.s16 = s16;
+        act.K = K;
+        const int cols[1] = { 0 };
+        gemv_load_x<TYPE, 1, false>(lane, slice, nblk, act, cols, X);
+    }
+    float *part = reinterpret_cast<float *>(smem + L.part);
+    uint32_t c_slot = 0;
+#pragma unroll 1
+    for (int n0 = 0; n0 < mine; n0 += 4) {
+        float acc[4];
+#pragma unroll
+        for (int u2 = 0; u2 < 4; u2 += 2) {
+            // two slices at a time, so that the one's loads run under the other's arithmetic
+            issue();
+            cp_async_wait<D - 2>();
+            __syncwarp();
+#pragma unroll
+            for (int u = u2; u < u2 + 2; ++u) {
+                // (past the warp's last one: whatever lies there, and nobody takes the sum)
+                const uint32_t sh = (uint32_t)(c_at & 15);
+                const uint8_t *at = ring + c_slot;
+                if constexpr (PER32) {
+                    constexpr int PAIR = 2 * F::BLK_B;
+                    const float a = gemv_one_row<TYPE>(reinterpret_cast<const uint32_t *>(at + sh + lane * PAIR), X);
+                    acc[u] = lane * PAIR < bytes ? a : 0.f;
+                } else {
+                    float a[1] = { 0.f };
+                    gemv_lane_row<TYPE, 1>(reinterpret_cast<const uint32_t *>(at), lane, X, a, gemv_row_align(TYPE) == 16 ? 0u : sh);
+                    acc[u] = a[0];
+                }
+                c_at += step;
+                c_slot = c_slot == (D - 1) * SLOT ? 0 : c_slot + SLOT;
+            }
+            __syncwarp();                                      // every lane is done with the places about to be refilled
+            issue();
+        }
+        // four sums over 32 lanes, down to two lanes each: lane l holds a half of the slice n0 + l / 8
+        const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+        float a0 = (up16 ? acc[2] : acc[0]) + __shfl_xor_sync(0xFFFFFFFFu, up16 ? acc[0] : acc[2], 16);
+        float a1 = (up16 ? acc[3] : acc[1]) + __shfl_xor_sync(0xFFFFFFFFu, up16 ? acc[1] : acc[3], 16);
+        a0 = (up8 ? a1 : a0) + __shfl_xor_sync(0xFFFFFFFFu, up8 ? a0 : a1, 8);
+        a0 += __shfl_xor_sync(0xFFFFFFFFu, a0, 4);
+        a0 += __shfl_xor_sync(0xFFFFFFFFu, a0, 2);
+        const int n = n0 + (lane >> 3);
+        if ((lane & 6) == 0 && n < mine) part[((n * L.groups + group) * L.nsl + slice) * 2 + (lane & 1)] = a0;
+    }
+    __syncthreads();
+    if (known) pdl_wait();
+    // (what is left is few and large: in 64 bits, rounded once. A row cut in slices is then no further from the exact sum than one that was
+    // not, and closer than with the last steps in 32 bits: Q6_K 32000x4096 7.0e-8, 7.6e-8 in 32 bits, 7.3e-8 for the kernel before)
+    for (int r = tid; r < rows; r += blockDim.x) {
+        double t = 0.0;
+        for (int s = 0; s < 2 * L.nsl; ++s) t += (double)part[r * 2 * L.nsl + s];
+        dst[r0 + r] = (float)t;
+    }
+}
+
+}  // namespace b200q

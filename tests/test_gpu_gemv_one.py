@@ -1,0 +1,122 @@
+"""The one-column GEMV that quantizes its activation itself: shapes at its edges (rows shorter than a slice, ragged last slices, sixteen slices,
+rows that begin inside a 16-byte unit, fewer rows than SMs, a block's last group without rows), against the fp64 product of the same
+operands; what leaves it for the two-kernel route; chains in which a product does not wait for the one before."""
+import numpy as np
+import pytest
+
+import arcint_b200 as A
+import oracle as O
+from gpu_util import TOL, check_sums, make_weights, rel_err
+
+pytestmark = pytest.mark.gpu
+TYPES = [A.Q4_0, A.Q8_0, A.IQ4_NL, A.Q4_K, A.Q5_K, A.Q6_K, A.IQ4_XS]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = A.Context(0)
+    yield c
+    c.close()
+
+
+def one(ctx):
+    return ctx.stats().get("gemv_fused_quant", 0)
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("m,k", [(1, 256), (149, 256), (147, 2048), (1000, 2304), (300, 4352), (200, 11008), (40, 32768), (9000, 512)])
+def test_shapes(ctx, t, m, k):
+    w = make_weights(t, m, k, 3 * t + k)
+    x = np.random.default_rng(m + k).normal(0, 1, (1, k)).astype(np.float32)
+    x[0, :32] = 0
+    x[0, 32:64] = np.arange(-16, 16) * 7.5                 # ties of both rounding rules
+    ctx.stats_reset()
+    got = ctx.run_mul_mat(t, w, k, x)
+    assert one(ctx) == 1
+    check_sums(got, t, w, k, x)
+
+
+@pytest.mark.parametrize("t,m,k", [(A.Q4_0, 70, 64), (A.Q8_0, 300, 320), (A.IQ4_NL, 300, 6208)])
+def test_rows_of_32_weight_blocks(ctx, t, m, k):
+    w = make_weights(t, m, k, 5)
+    x = np.random.default_rng(m).normal(0, 1, (1, k)).astype(np.float32)
+    ctx.stats_reset()
+    check_sums(ctx.run_mul_mat(t, w, k, x), t, w, k, x)
+    assert one(ctx) == 1
+
+
+def test_what_takes_the_two_kernel_route(ctx):
+    """An odd number of 18-byte blocks, padded rows, K beyond sixteen slices, results that land in the activation."""
+    x = np.random.default_rng(1).normal(0, 1, (1, 33024)).astype(np.float32)
+    for t, m, k in ((A.Q4_0, 20, 96), (A.Q4_K, 20, 33024)):
+        w = make_weights(t, m, k, 6)
+        ctx.stats_reset()
+        check_sums(ctx.run_mul_mat(t, w, k, x[:, :k]), t, w, k, x[:, :k])
+        assert one(ctx) == 0
+    t, m, k = A.Q4_K, 512, 512
+    w = make_weights(t, m, k, 7)
+    rb = w.shape[1]
+    padded = np.zeros((m, rb + 16), np.uint8)
+    padded[:, :rb] = w
+    dw, dp, dx, dy = ctx.upload(w), ctx.upload(padded), ctx.upload(x[:, :k]), ctx.alloc(4 * m)
+    ref = O.mul_mat_f64(t, w, k, x[:, :k], True)
+    ctx.stats_reset()
+    ctx.graph_begin()
+    ctx.mul_mat(A.Tensor.make(t, [k, m, 1, 1], [A.block_bytes(t), rb + 16], dp), A.Tensor.f32(dx, [k, 1]), A.Tensor.f32(dy, [m, 1]))
+    assert rel_err(ctx.download(dy, (1, m), np.float32), ref) < TOL
+    ctx.graph_begin()
+    ctx.mul_mat(A.Tensor.weights(t, dw, k, m), A.Tensor.f32(dx, [k, 1]), A.Tensor.f32(dx, [m, 1]))
+    assert rel_err(ctx.download(dx, (1, m), np.float32), ref) < TOL
+    assert one(ctx) == 0
+    for p in (dw, dp, dx, dy):
+        ctx.free(p)
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+def test_chains(ctx, recorded):
+    """Products over one activation, each followed by one over its result, and a result that replaces the activation of an
+    earlier product: every product sees what the one before has written, whether it waited for it at its start or at its end."""
+    t, d = A.Q4_0, 2048
+    ws = [make_weights(t, d, d, 20 + i) for i in range(8)]
+    x = np.random.default_rng(9).normal(0, 1, (1, d)).astype(np.float32)
+    dw = [ctx.upload(w) for w in ws]
+    bufs = [ctx.alloc(4 * d) for _ in range(5)]
+
+    def mul(i, a, b):
+        ctx.mul_mat(A.Tensor.weights(t, dw[i], d, d), A.Tensor.f32(bufs[a], [d, 1]), A.Tensor.f32(bufs[b], [d, 1]))
+
+    def calls():
+        for _ in range(6):                                  # (a generation each: buffer 0 has new values in each)
+            ctx.graph_begin()
+            mul(0, 0, 1)
+            mul(1, 0, 2)
+            mul(2, 0, 3)
+            mul(3, 3, 4)
+            mul(4, 3, 1)
+            ctx.graph_begin()
+            mul(5, 4, 0)
+
+    ctx.upload(x, bufs[0])
+    if recorded:
+        calls()
+        ctx.sync()
+        g = ctx.capture(calls)
+        ctx.upload(x, bufs[0])
+        ctx.graph_launch(g)
+    else:
+        calls()
+    got = [ctx.download(b, (1, d), np.float32) for b in bufs]
+    if recorded:
+        ctx.graph_free(g)
+
+    # the same chain, a product and a wait at a time
+    ctx.upload(x, bufs[0])
+    for _ in range(6):
+        for i, a, b in ((0, 0, 1), (1, 0, 2), (2, 0, 3), (3, 3, 4), (4, 3, 1), (5, 4, 0)):
+            ctx.graph_begin()
+            mul(i, a, b)
+            ctx.sync()
+    for b, y in zip(bufs, got):
+        assert np.array_equal(ctx.download(b, (1, d), np.float32), y)
+    for p in dw + bufs:
+        ctx.free(p)
