@@ -573,7 +573,7 @@ gemm_kq_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 // warps busy 88 % of the time; some 3,500 clk a 128 x 128 x 256 super-block against 1,024 of its MMAs). With several column tiles it is
 // cheaper to write the limbs out once, in the order the tensor core reads them, to scratch that stays in L2 (a chunk of row
 // tiles at a time), and to run the MMAs straight from there. What bounds that is the shared-memory port: the copies, operand reads and
-// activation of a super-block are 225 KB, 1,800 clk of the 2,440 it takes by arithmetic. IQ4_XS 17408x5120 x 2048 tokens: 532 -> 457 us. From how
+// activation of a super-block are 225 KB, 1,800 clk of the 2,440 it takes by arithmetic. IQ4_XS 17408x5120 x 2048 tokens: 532 -> 457 us, since 433 (three producers, chunks by rounds). From how
 // many tiles: see expand_wanted.
 constexpr int EXP_DW = 2 * NA * OPER_BYTES;               // 65536: per (row tile, super-block) eight blocks' limbs [block][hi, lo], then ...
 constexpr int EXP_CHUNK = EXP_DW + BM * 4;                // ... the rows' d_w as f32
@@ -611,12 +611,13 @@ expand_kernel(const uint8_t *__restrict__ w, size_t row_stride, int M, int row_t
 
 constexpr int XG = 4;                                     // groups of four blocks in the A ring
 constexpr int X_ACT = ACT_CHUNK + BM * 4;                 // an activation stage, and the rows' d_w behind it
-constexpr int X_A_OFF = NACT * X_ACT, X_BAR_OFF = X_A_OFF + XG * GB * A_SLOT, X_TOTAL = X_BAR_OFF + 8 * 16;
+constexpr int X_A_OFF = NACT * X_ACT, X_DX_OFF = X_A_OFF + XG * GB * A_SLOT;       // (X_DX: a scaling warp's own copy of its columns' d_x)
+constexpr int X_BAR_OFF = X_DX_OFF + 4 * NW * (BN / NW) * 4, X_TOTAL = X_BAR_OFF + 8 * 16;
 constexpr int X_THREADS = 32 * (4 + 4 * NW);
 static_assert(X_TOTAL <= 227 * 1024 - 256 && X_ACT % 128 == 0, "shared memory budget");
 enum { XB_ACT_FULL = 0, XB_ACT_EMPTY = 2, XB_A_FULL = 4, XB_A_EMPTY = 8, XB_ACC_FULL = 12, XB_ACC_EMPTY = 14 };
 
-// The product from the expanded operand: producer, MMA issuer, two idle warps, 4 NW scale-accumulate warps as in gemm_kq_kernel
+// The product from the expanded operand: MMA issuer, three producers, 4 NW scale-accumulate warps as in gemm_kq_kernel
 template <bool FULL>
 __global__ void __launch_bounds__(X_THREADS, 1)
 gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__restrict__ act, int N, int tiles_n, int row_tile0, int row_tiles,
@@ -667,8 +668,32 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
     volatile int *abortp = &abort_flag;
     PROF_DECL
 
-    if (warp == 0) {
-        // ---- producer ----
+    if (warp == 0 || warp == 3) {
+        // ---- producers of the operand, one for each half of a super-block ----
+        // (A wait and a copy take a warp some 500 clk, whatever the copy's size. One warp for both halves and the activation, which asked for the
+        // next super-block's operand only when the scaling warps had left it a stage for the activation: IQ4_XS 17408x5120 x 2048 tokens 466 us, 447 with
+        // three and the scaling warps' own copy of the scales.)
+        const int jg = warp == 3;
+        pdl_wait();
+        int g = jg;
+        bool ok = true;
+#pragma unroll 1
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const UnitX U = unit_of(u);
+            const uint8_t *src = ops + ((size_t)U.tm * nsb + U.sb0) * EXP_CHUNK + jg * GB * A_SLOT;
+#pragma unroll 1
+            for (int s = U.sb0; s < U.sb1; ++s, g += 2, src += EXP_CHUNK) {
+                const int gs = g % XG;
+                if (!WAITP(1, bar(XB_A_EMPTY + gs), ((g / XG) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    mbar_expect_tx(bar(XB_A_FULL + gs), GB * A_SLOT);
+                    bulk_g2s(sbase + X_A_OFF + gs * (GB * A_SLOT), src, GB * A_SLOT, bar(XB_A_FULL + gs));
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 2) {
+        // ---- producer of the activation and the rows' d_w ----
         pdl_wait();
         int s_run = 0;
         bool ok = true;
@@ -677,26 +702,15 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
             const UnitX U = unit_of(u);
             const uint32_t bytes = (uint32_t)((U.ncols + 7) >> 3) * ACT_GROUP;       // only the column groups the tile has
 #pragma unroll 1
-            for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
-                const uint8_t *chunk = ops + ((size_t)U.tm * nsb + s) * EXP_CHUNK;
+            for (int s = U.sb0; s < U.sb1; ++s, ++s_run) {
                 const int at = s_run % NACT;
                 if (!WAITP(3, bar(XB_ACT_EMPTY + at), ((s_run / NACT) & 1) ^ 1)) { ok = false; break; }
                 if (lane == 0) {
                     mbar_expect_tx(bar(XB_ACT_FULL + at), bytes + BM * 4);
                     bulk_g2s(sbase + at * X_ACT, act + ((size_t)U.tile_n * nsb + s) * ACT_CHUNK, bytes, bar(XB_ACT_FULL + at));
-                    bulk_g2s(sbase + at * X_ACT + ACT_CHUNK, chunk + EXP_DW, BM * 4, bar(XB_ACT_FULL + at));
+                    bulk_g2s(sbase + at * X_ACT + ACT_CHUNK, ops + ((size_t)U.tm * nsb + s) * EXP_CHUNK + EXP_DW, BM * 4, bar(XB_ACT_FULL + at));
                 }
                 __syncwarp();
-#pragma unroll 1
-                for (int jg = 0; jg < SB / GB; ++jg) {
-                    const int g = 2 * s_run + jg, gs = g % XG;
-                    if (!WAITP(1, bar(XB_A_EMPTY + gs), ((g / XG) & 1) ^ 1)) { ok = false; break; }
-                    if (lane == 0) {
-                        mbar_expect_tx(bar(XB_A_FULL + gs), GB * A_SLOT);
-                        bulk_g2s(sbase + X_A_OFF + gs * (GB * A_SLOT), chunk + jg * GB * A_SLOT, GB * A_SLOT, bar(XB_A_FULL + gs));
-                    }
-                    __syncwarp();
-                }
             }
         }
     } else if (warp == 1) {
@@ -736,6 +750,7 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
         // ---- scale-accumulate, once per super-block ----
         constexpr int CW = BN / NW;
         const int q4 = warp & 3, u4 = (warp - 4) >> 2, r = q4 * 32 + lane;
+        const uint32_t own_dx = sbase + X_DX_OFF + (warp - 4) * (CW * 4);
         int s_run = 0;
         pdl_wait();
         bool ok = true;
@@ -756,7 +771,10 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
                 const uint32_t stage = sbase + at * X_ACT;
                 const float dwb = *reinterpret_cast<const float *>(smem + at * X_ACT + ACT_CHUNK + r * 4);
                 const f32x2 dw2 = f2_pack(dwb, dwb);
-                const uint32_t dxa = stage + (cbase / 8) * ACT_GROUP + ACT_SCALES;
+                // the scales into the warp's own place, lane l columns 2 l and 2 l + 1: the stage then waits for its MMAs only
+                __syncwarp();
+                sts64_f2(own_dx + lane * 8, lds64_f2(stage + (cbase / 8 + (lane >> 2)) * ACT_GROUP + ACT_SCALES + (lane & 3) * 8));
+                mbar_arrive_warp(bar(XB_ACT_EMPTY + at), lane);
                 if (!WAITP(6, bar(XB_ACC_FULL + buf), (s_run / NBUF) & 1)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)buf * (2 * BN) + (uint32_t)cbase;
@@ -768,7 +786,7 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
                         tmem_ld16(taddr + BN + q * 16, vl);
                         f32x2 dx[8];                             // sixteen activation scales, in flight under the tensor-memory loads
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) lds128_f2(dxa + (2 * q + (c >> 1)) * ACT_GROUP + (c & 1) * 16, dx[2 * c], dx[2 * c + 1]);
+                        for (int c = 0; c < 4; ++c) lds128_f2(own_dx + q * 64 + c * 16, dx[2 * c], dx[2 * c + 1]);
                         tmem_ld_wait();
 #pragma unroll
                         for (int c = 0; c < 16; c += 2) {
@@ -781,7 +799,6 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
                 }
                 tc_fence_before();
                 mbar_arrive_warp(bar(XB_ACC_EMPTY + buf), lane);
-                mbar_arrive_warp(bar(XB_ACT_EMPTY + at), lane);
             }
             const int row = (row_tile0 + U.tm) * BM + r;
             if (ok && row < M) {
@@ -798,7 +815,7 @@ gemm_kx_kernel(const uint8_t *__restrict__ ops, int M, int K, const uint8_t *__r
         }
     }
 
-    PROF_DUMP(warp == 0 ? "prod" : warp == 1 ? "mma " : warp < 4 ? "idle" : "epi ")
+    PROF_DUMP(warp == 1 ? "mma " : warp < 4 ? "prod" : "epi ")
     tc_fence_before();
     __syncthreads();
     pdl_trigger();
@@ -898,12 +915,21 @@ static b200q_status launch_kq_t(b200q_ctx *ctx, const void *w, size_t row_stride
     return B200Q_OK;
 }
 
-// Row tiles of a chunk: as many as 96 MB (of 126 MB of L2) hold, at least one, in chunks of about equal size
-static int64_t expand_chunk(const b200q_ctx *ctx, int64_t nsb, int64_t tiles_m) {
-    int64_t chunk = (int64_t)((ctx->expand_limit ? ctx->expand_limit : (size_t)96 << 20) / ((size_t)nsb * kq::EXP_CHUNK));
-    chunk = chunk < 1 ? 1 : chunk < tiles_m ? chunk : tiles_m;
-    const int64_t chunks = (tiles_m + chunk - 1) / chunk;
-    return (tiles_m + chunks - 1) / chunks;
+// Row tiles of a chunk: as many as 96 MB (of 126 MB of L2) hold, at least one; of the sizes that need no more chunks the one with the fewest rounds
+// of units over the SMs, the most equal chunks first (IQ4_XS 17408x5120 x 2048 tokens: 68 and 68 row tiles of 16 column tiles are 16
+// rounds, 74 and 62 are 15)
+static int64_t expand_chunk(const b200q_ctx *ctx, int64_t nsb, int64_t tiles_m, int64_t n_tiles) {
+    int64_t most = (int64_t)((ctx->expand_limit ? ctx->expand_limit : (size_t)96 << 20) / ((size_t)nsb * kq::EXP_CHUNK));
+    most = most < 1 ? 1 : most < tiles_m ? most : tiles_m;
+    const int64_t chunks = (tiles_m + most - 1) / most, S = ctx->sm_count;
+    int64_t best = 0, best_rounds = 0;
+    for (int64_t c = (tiles_m + chunks - 1) / chunks; c <= most; ++c) {
+        const int64_t last = tiles_m - (chunks - 1) * c;
+        if (last < 1) break;
+        const int64_t rounds = (chunks - 1) * ((c * n_tiles + S - 1) / S) + (last * n_tiles + S - 1) / S;
+        if (!best || rounds < best_rounds) { best = c; best_rounds = rounds; }
+    }
+    return best;
 }
 
 // Whether a dense product takes the expanded operand: it saves part of a column tile's time and costs a pass that writes two bytes a
@@ -928,7 +954,7 @@ static bool expand_wanted(const b200q_ctx *ctx, int type, bool row_by_row, int64
                                             : (q6 ? KsplitTimes{ 1730, 750 } : KsplitTimes{ 2 * 1550, 1350 });
     const int64_t ks = choose_ksplit(ctx, tiles_m * n_tiles, nsb / sps, { sps * KQ_TIMES.step_ns, KQ_TIMES.unit_ns }, M * N, MOST_PARTS);
     const int64_t unpacked = schedule_ns(ctx, tiles_m * n_tiles, nsb / sps, ks, measured) + ksplit_sum_ns(ks, M * N);
-    const int64_t chunk = expand_chunk(ctx, nsb, tiles_m), chunks = (tiles_m + chunk - 1) / chunk;
+    const int64_t chunk = expand_chunk(ctx, nsb, tiles_m, n_tiles), chunks = (tiles_m + chunk - 1) / chunk;
     const int64_t kx = choose_ksplit(ctx, chunk * n_tiles, nsb, KX_TIMES, M * N, MOST_PARTS, chunks);
     const int64_t expanded = (chunks - 1) * schedule_ns(ctx, chunk * n_tiles, nsb, kx, KX_TIMES) +
                              schedule_ns(ctx, (tiles_m - (chunks - 1) * chunk) * n_tiles, nsb, kx, KX_TIMES) + ksplit_sum_ns(kx, M * N) +
@@ -942,7 +968,7 @@ static b200q_status launch_kx_t(b200q_ctx *ctx, const void *w, size_t row_stride
                                 int64_t n_tiles, float *dst, int64_t ldd, bool *took) {
     const int64_t nsb = K / 256, tiles_m = (M + kq::BM - 1) / kq::BM;
     const size_t per_tile = (size_t)nsb * kq::EXP_CHUNK;
-    const int64_t chunk = expand_chunk(ctx, nsb, tiles_m);
+    const int64_t chunk = expand_chunk(ctx, nsb, tiles_m, n_tiles);
     Workspace *ws = &ctx->moe_ws[10];
     *took = ws_try_reserve(ctx, ws, per_tile * (size_t)chunk);
     if (!*took) return B200Q_OK;

@@ -207,6 +207,7 @@ __device__ __forceinline__ f32x2 lds64_f2(uint32_t addr) {
     asm volatile("ld.shared.b64 %0, [%1];" : "=l"(a) : "r"(addr));
     return a;
 }
+__device__ __forceinline__ void sts64_f2(uint32_t addr, f32x2 v) { asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Optional self-profile (compile with -DB200Q_TC_PROF): every role adds up the clocks it spends in
