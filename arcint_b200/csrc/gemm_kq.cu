@@ -933,21 +933,17 @@ static int64_t expand_chunk(const b200q_ctx *ctx, int64_t nsb, int64_t tiles_m, 
 }
 
 // Whether a dense product takes the expanded operand: it saves part of a column tile's time and costs a pass that writes two bytes a
-// weight. Quantizer included, unpacking and expanded, us. Rows that no tensor map describes (copied row by row where they are
-// unpacked), at 3, 4 and 6 column tiles:
-//   Q6_K 4096x11008 85.2 114.2 158.7   79.3 88.3 122.4;  IQ4_XS 4096x11008 79.3 104.4 145.6   77.6 86.6 121.1
-// (three tiles, other shapes: 12 to 20 % slower), Q6_K 2048x5120 at 4 and 5: 37.0 49.1   32.6 39.8. The others, at 4 and 5 (IQ4_XS 6 and 8):
-//   Q6_K 32000x4096 224 282   269 285;  IQ4_XS 4096x4096 55.1 62.8   56.2 57.0;  11008x4096 118 149   116 140;  32000x4096 318   329
-// and at sixteen, IQ4_XS 17408x5120, 532 and 457 (Q6_K with a tensor map was not timed at six and seven). A small product does not
-// earn the launch: Q6_K 512x2048 x 600 tokens, one super-block of a tile an SM, 16.8 and 18.5 us.
-// Chunks that end in a badly filled round lose what the expansion saves (IQ4_XS 4736x11008 x 512: 76 and 72 units, 104 us unpacked and
-// 116 expanded), so both schedules are counted out, with the least squares of 172 products timed both ways (off by 2 % on average,
-// by 10 % at most): the unpacking kernel takes the product where it is shorter by a twelfth. Of the 172 none is then more than 3 %
-// slower than the better form.
+// weight. Both schedules are counted out, with all chunks and their rounds (a chunk that ends in a badly filled round loses what the
+// expansion saves: IQ4_XS 4736x11008 x 512, 148 whole tiles unpacked), and the unpacking kernel keeps what it does in a 25th less. Fitted to 101
+// products of 2048 to 11008 rows, K 2048 to 17408, 128 to 1024 tokens, timed both ways (off by 5 % on average): the choice is 0.6 % from the
+// better one on average, at most 7 %. From two column tiles: unpacked and expanded, us, Q6_K 4096x11008 (rows that no tensor map describes) x 128, 256,
+// 333, 512 tokens 37.3 63.3 81.0 111.7   45.8 57.1 67.0 77.3; IQ4_XS 11008x4096 x 256, 512, 768 54.2 87.9 114.8   63.3 80.7 97.5. (Before the three
+// producers it took four tiles and eight.) A small product, less than four super-blocks of a tile an SM, has to gain a tenth: it hardly
+// earns the launch (Q6_K 512x2048 x 600 tokens 16.8 and 18.5).
 static bool expand_wanted(const b200q_ctx *ctx, int type, bool row_by_row, int64_t M, int64_t K, int64_t N, int64_t n_tiles) {
     const int64_t nsb = K / 256, tiles_m = (M + kq::BM - 1) / kq::BM;
     if (ctx->expand_limit && !ctx->no_expand) return true;
-    if (ctx->no_expand || n_tiles < (row_by_row ? 4 : 8) || tiles_m * n_tiles * nsb < 3 * ctx->sm_count) return false;
+    if (ctx->no_expand || n_tiles < 2 || tiles_m * n_tiles * nsb < 3 * ctx->sm_count) return false;
     const bool q6 = type == B200Q_TYPE_Q6_K;
     const int sps = !q6 && !row_by_row ? 2 : 1;                // super-blocks of a step, as in launch_kq_t
     const KsplitTimes measured = row_by_row ? (q6 ? KsplitTimes{ 2370, 1370 } : KsplitTimes{ 2120, 1120 })
@@ -958,8 +954,8 @@ static bool expand_wanted(const b200q_ctx *ctx, int type, bool row_by_row, int64
     const int64_t kx = choose_ksplit(ctx, chunk * n_tiles, nsb, KX_TIMES, M * N, MOST_PARTS, chunks);
     const int64_t expanded = (chunks - 1) * schedule_ns(ctx, chunk * n_tiles, nsb, kx, KX_TIMES) +
                              schedule_ns(ctx, (tiles_m - (chunks - 1) * chunk) * n_tiles, nsb, kx, KX_TIMES) + ksplit_sum_ns(kx, M * N) +
-                             chunks * 5300 + 2350 * tiles_m * nsb / ctx->sm_count;       // launches, and the expansion itself
-    return 12 * expanded <= 13 * unpacked;
+                             chunks * 3000 + 2000 * tiles_m * nsb / ctx->sm_count;       // launches, and the expansion itself
+    return tiles_m * n_tiles * nsb < 4 * ctx->sm_count ? 10 * expanded <= 9 * unpacked : 24 * expanded <= 25 * unpacked;
 }
 
 // The product from the expanded operand, a chunk of row tiles at a time; *took: false when the scratch cannot be had
