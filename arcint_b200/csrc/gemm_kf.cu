@@ -26,7 +26,7 @@
 // in shared memory, whose port (128 bytes per clock) the B reads of the MMAs alone fill by half.
 //
 // Tensor memory, 512 columns: two main accumulators of 128 columns, one for the mins term, and the ring of A blocks (two
-// groups of four 32-weight blocks, 16 columns of packed half pairs a block). Warp roles: producer, MMA issuer, two idle (one reads the one-sided sums),
+// groups of four 32-weight blocks, 16 columns of packed half pairs a block). Warp roles: producer, MMA issuer, two producers of codes,
 // eight unpack warps (a thread = a row and half of the blocks of a group), eight scale-accumulate warps (four per half of
 // the columns, a lane quarter each). Persistent blocks walk the units (row tile, column tile, part of K). Every mbarrier
 // wait is bounded.
@@ -61,7 +61,7 @@ constexpr int Y_BASE = 2 * BN, A_BASE = 3 * BN;           // tensor memory: X0, 
 static_assert(A_BASE + NG * GB * A_COLS <= 512, "tensor memory");
 constexpr int NCODE = 4;                                  // stages of activation codes (half a super-block each) in flight
 constexpr int NX = 3;                                     // super-blocks of activation scales, mins operands and row scales in flight
-constexpr int THREADS = 32 * 20;                          // warp groups: {producer, MMA, 2 idle}, 2 x unpack, 2 x scale-accumulate
+constexpr int THREADS = 32 * 20;                          // warp groups: {producer, MMA, 2 producers of codes}, 2 x unpack, 2 x scale-accumulate
 // Registers per thread by role (setmaxnreg): a warp group that asks for more waits until others have
 // given theirs back, so the sum must fit the pool the launch allocated (THREADS x LAUNCH_REGS).
 constexpr int LAUNCH_REGS = (65536 / THREADS) / 8 * 8;
@@ -307,7 +307,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     };
     if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
     // whether one of this thread's share of the one-sided sums asks for more than one chain. Every block reads them all: a route's, with its
-    // many tiles, by all threads (a block waits first anyway), a dense product's by an idle warp behind its wait, so that weights
+    // many tiles, by all threads (a block waits first anyway), a dense product's by one scaling warp behind its wait, so that weights
     // are fetched and unpacked meanwhile (asking with the whole block costs 2 us a launch).
     auto asks_for_more = [&](int first, int step) {
         const int total = n_sides;
@@ -392,18 +392,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                     mbar_expect_tx(bar(BAR_X_FULL + xt), bytes);
                     bulk_g2s(sbase + L::EXTRA_OFF + xt * EXTRA, chunk + 2 * CODE_STAGE, bytes, bar(BAR_X_FULL + xt));
                 }
-#pragma unroll 1
-                for (int h = 0; h < 2; ++h) {
-                    // only the column groups the tile has; the MMA still reads a multiple of sixteen columns, the rest of the
-                    // stage holds older codes whose products land in accumulator columns nobody stores
-                    const int c_run = 2 * s_run + h, ct = c_run % NCODE;
-                    if (!WAITP(3, bar(BAR_CODE_EMPTY + ct), ((c_run / NCODE) & 1) ^ 1)) { ok = false; break; }
-                    if (lane == 0) {
-                        mbar_expect_tx(bar(BAR_CODE_FULL + ct), groups * CODE_GROUP);
-                        bulk_g2s(sbase + L::CODE_OFF + ct * CODE_STAGE, chunk + h * CODE_STAGE, groups * CODE_GROUP, bar(BAR_CODE_FULL + ct));
-                    }
-                    __syncwarp();
-                }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
@@ -490,13 +479,29 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             }
         }
     } else if (warp < 4) {
+        // ---- producers of the activation codes, one for each half of a super-block (a wait and a copy take a warp some 500 clk, whatever
+        // the copy's size: one warp for all four copies of a super-block took 1400 to 2000; Q4_K 11008x4096 x 512 75.0 -> 72.8 us) ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
-        if (!ROUTE && warp == 2) {
-            pdl_wait();
-            const int any = __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32));
-            if (lane == 0) {
-                more_slot = any;
-                mbar_arrive(bar(BAR_MORE));
+        const int h = warp - 2;
+        int c_run = h;                                    // half super-blocks so far
+        bool ok = true;
+        pdl_wait();
+#pragma unroll 1
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit U = unit_of(u);
+            // only the column groups the tile has; the MMA still reads a multiple of sixteen columns, the rest of the
+            // stage holds older codes whose products land in accumulator columns nobody stores
+            const uint32_t bytes = ((uint32_t)(U.ncols + 7) >> 3) * CODE_GROUP;
+            const uint8_t *src = act + ((size_t)U.tile_n * nsb + U.sb0) * CHUNK + h * CODE_STAGE;
+#pragma unroll 1
+            for (int s = U.sb0; s < U.sb1; ++s, c_run += 2, src += CHUNK) {
+                const int ct = c_run % NCODE;
+                if (!WAITP(3, bar(BAR_CODE_EMPTY + ct), ((c_run / NCODE) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    mbar_expect_tx(bar(BAR_CODE_FULL + ct), bytes);
+                    bulk_g2s(sbase + L::CODE_OFF + ct * CODE_STAGE, src, bytes, bar(BAR_CODE_FULL + ct));
+                }
+                __syncwarp();
             }
         }
     } else if (warp < 12) {
@@ -551,6 +556,13 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         const int q4 = warp & 3, half = (warp - 12) >> 2, g = lane >> 2, c = lane & 3;
         int s_run = 0, v_run = 0;
         pdl_wait();
+        if (!ROUTE && warp == 12) {
+            const int any = __any_sync(0xFFFFFFFFu, asks_for_more(lane, 32));
+            if (lane == 0) {
+                more_slot = any;
+                mbar_arrive(bar(BAR_MORE));
+            }
+        }
         bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
         const int chains = *(volatile int *)&more_slot ? Fmt<TYPE>::CHAINS : 1;
 #pragma unroll 1
@@ -667,7 +679,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         }
     }
 
-    PROF_DUMP(warp == 0 ? "prod" : warp == 1 ? "mma " : warp < 4 ? "idle" : warp < 12 ? "unpk" : "epi ")
+    PROF_DUMP(warp == 1 ? "mma " : warp < 4 ? "prod" : warp < 12 ? "unpk" : "epi ")
     tc_fence_before();
     __syncthreads();
     pdl_trigger();
