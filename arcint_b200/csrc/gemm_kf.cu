@@ -25,7 +25,7 @@
 // tcgen05.st into the lane of its row, and the MMAs take A from there: no operand stores, proxy fences and operand reads
 // in shared memory, whose port (128 bytes per clock) the B reads of the MMAs alone fill by half.
 //
-// Tensor memory, 512 columns: two main accumulators of 128 columns, one for the mins term, and the ring of A blocks (two
+// Tensor memory, 512 columns: two main accumulators of 128 columns, one for the mins term (two of 64 for a short tile), and the ring of A blocks (two
 // groups of four 32-weight blocks, 16 columns of packed half pairs a block). Warp roles: producer, MMA issuer, two producers of codes,
 // eight unpack warps (a thread = a row and half of the blocks of a group), eight scale-accumulate warps (four per half of
 // the columns, a lane quarter each). Persistent blocks walk the units (row tile, column tile, part of K). Every mbarrier
@@ -33,8 +33,11 @@
 //
 // B200, quantizer and GEMM together, against two int8 limbs through shared memory and a second kernel for the mins: Q4_K
 // 11008x4096 x 512 tokens 149 -> 79.5 us, x 24 tokens 53.6 -> 22.7 us, a 512-expert block over 2048 tokens 842 -> 573 us. What is
-// left is the chain unpack -> MMA -> scaling (its 1024 clk of MMAs a super-block take some 2700), whose one mins accumulator and
-// two-group operand ring (all of tensor memory) let it overlap only in part. Reading the accumulators in the 32x32b shape, sixteen columns at a
+// left is the chain unpack -> MMA -> scaling (its 1024 clk of MMAs a super-block take some 2500), whose one mins accumulator and
+// two-group operand ring (all of tensor memory) let it overlap only in part. The MMA issuer, one warp, is a part of that chain: with places and
+// descriptors computed in front of each MMA and a wait for each barrier it spent 1000 clk a super-block on a tile of 48 columns beside its waits'
+// 700; with constant places, one look at all the barriers of a group, a fourth stage of scales and two mins accumulators for tiles of up to 64
+// columns: Q4_K 11008x4096 x 512 72.9 -> 68.2 us, x 24 21.1 -> 20.4, the 512-expert block 498 -> 489. Reading the accumulators in the 32x32b shape, sixteen columns at a
 // time, measured the same on dense products and 2 % slower on the 512-expert block.
 //
 // The reference's mins correction is a DPAS of its own, too (marfrit/arcint contrib/llama.cpp/patches/
@@ -60,7 +63,7 @@ constexpr int A_COLS = 16;                                // tensor-memory colum
 constexpr int Y_BASE = 2 * BN, A_BASE = 3 * BN;           // tensor memory: X0, X1, Y, A ring
 static_assert(A_BASE + NG * GB * A_COLS <= 512, "tensor memory");
 constexpr int NCODE = 4;                                  // stages of activation codes (half a super-block each) in flight
-constexpr int NX = 3;                                     // super-blocks of activation scales, mins operands and row scales in flight
+constexpr int NX = 4;                                     // super-blocks of activation scales, mins operands and row scales in flight
 constexpr int THREADS = 32 * 20;                          // warp groups: {producer, MMA, 2 producers of codes}, 2 x unpack, 2 x scale-accumulate
 // Registers per thread by role (setmaxnreg): a warp group that asks for more waits until others have
 // given theirs back, so the sum must fit the pool the launch allocated (THREADS x LAUNCH_REGS).
@@ -102,9 +105,9 @@ template <int TYPE> struct Smem {
     static_assert(RAW_STAGE % 128 == 0 && EXTRA % 128 == 0, "tiled copies");
 };
 
-enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_CODE_FULL = 6, BAR_CODE_EMPTY = 10, BAR_X_FULL = 14, BAR_X_EMPTY = 17, BAR_A_FULL = 22,
+enum { BAR_RAW_FULL = 0, BAR_RAW_EMPTY = 3, BAR_CODE_FULL = 6, BAR_CODE_EMPTY = 10, BAR_X_FULL = 14, BAR_X_EMPTY = 18, BAR_A_FULL = 22,
        BAR_A_EMPTY = 24, BAR_ACC_FULL = 26, BAR_ACC_EMPTY = 28, BAR_MORE = 30, BAR_COUNT = 31 };
-static_assert(NCODE == 4 && NX == 3 && NG == 2 && BAR_COUNT <= 32, "barrier slots above");
+static_assert(NCODE == 4 && NX == 4 && NG == 2 && BAR_COUNT <= 32, "barrier slots above");
 
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BM >> 4) << 24);      // f16 x f16 -> f32, without the N field
 
@@ -362,6 +365,9 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_slot, 0);
     volatile int *abortp = &abort_flag;
+    // A tile of up to 64 columns has two Y accumulators, the halves of the one of a wider tile (chains of a whole super-block only).
+    auto short_tile = [](const Unit &U) { return !FULL && U.ncols <= 64; };
+    auto y_of = [&](const Unit &U, int chain) { return (uint32_t)(Y_BASE + (short_tile(U) ? (chain & 1) * 64 : 0)); };
     PROF_DECL
 
     if (warp == 0) {
@@ -399,8 +405,10 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         // ---- MMA issuer ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
         int s_run = 0, v_run = 0;                         // super-blocks, chains so far (a chain fills an accumulator)
+        bool was_short = false;
         const uint32_t leader = elect_one();
         uint32_t idesc = 0;
+        const uint64_t code_desc = umma_desc2(sbase + L::CODE_OFF, 128, CODE_GROUP);
         // K = 16 per MMA: eight columns of A, two pieces of B
         auto block = [&](uint32_t acc, int gs, int ct, int jj, uint32_t accumulate) {
             const uint32_t a = tmem_base + A_BASE + (uint32_t)((gs * GB + jj) * A_COLS);
@@ -408,12 +416,14 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             umma_ts(leader, acc, a, umma_desc2(b, 128, CODE_GROUP), idesc, accumulate);
             umma_ts(leader, acc, a + 8, umma_desc2(b + 256, 128, CODE_GROUP), idesc, 1u);
         };
-        // the mins term, into the one Y accumulator: the scaling warps have read the last chain's X, and the last super-block's Y with
-        // it or before it
-        auto mins = [&](int xt) {
-            if (v_run > 0 && !WAITP(7, bar(BAR_ACC_EMPTY + ((v_run - 1) & 1)), ((v_run - 1) >> 1) & 1)) return false;
+        // the mins term, into the Y accumulator: the scaling warps have read the last chain's X, and the last super-block's Y with
+        // it or before it. A short tile after a short tile takes the Y accumulators in turn: the one of two chains back has been read
+        // with that chain's X, which the issuer has waited for.
+        auto mins = [&](int xt, uint32_t y, bool in_turn) {
+            const uint32_t bx = bar(BAR_X_FULL + xt), px = (s_run / NX) & 1, be = bar(BAR_ACC_EMPTY + ((v_run - 1) & 1)), pe = ((v_run - 1) >> 1) & 1;
+            if (!(in_turn || v_run == 0 ? WAITP(2, bx, px) : WAITP2(2, bx, px, 7, be, pe))) return false;
             tc_fence_after();
-            umma_ss<true>(leader, tmem_base + Y_BASE, umma_desc2(sbase + L::MINS_OFF + (s_run & 1) * 4096, 2048, 128),
+            umma_ss<true>(leader, tmem_base + y, umma_desc2(sbase + L::MINS_OFF + (s_run & 1) * 4096, 2048, 128),
                           umma_desc2(sbase + L::EXTRA_OFF + xt * EXTRA + EXTRA_MINS, 128, MINS_GROUP), idesc, 0u);
             return true;
         };
@@ -426,23 +436,33 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);                      // N: the live columns, in sixteens
             if (!more) {
 #pragma unroll 1
-                for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run, ++v_run) {
-                    const int xt = s_run % NX;
+                for (int s = U.sb0; s < U.sb1; ++s, ++s_run, ++v_run) {
+                    const int xt = s_run % NX, odd = s_run & 1;
                     const uint32_t acc = tmem_base + (uint32_t)(v_run & 1) * BN;
-                    if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
-                    if (!WAITP(7, bar(BAR_ACC_EMPTY + (v_run & 1)), ((v_run >> 1) & 1) ^ 1)) { ok = false; break; }
-#pragma unroll 1
-                    for (int jg = 0; jg < SB / GB; ++jg) {
-                        const int g = 2 * s_run + jg, gs = g % NG, ct = g % NCODE;
-                        if (!WAITP(2, bar(BAR_CODE_FULL + ct), (g / NCODE) & 1)) { ok = false; break; }
-                        if (!WAITP(4, bar(BAR_A_FULL + gs), (g / NG) & 1)) { ok = false; break; }
+                    const uint64_t db = umma_desc_on(code_desc, odd * (2 * CODE_STAGE));
+                    // (group 2 s_run + jg has place jg of the A ring and place 2 odd + jg of the codes')
+                    static_assert(NG == 2 && NCODE == 4 && SB == 2 * GB, "places");
+#pragma unroll
+                    for (int jg = 0; jg < 2 && ok; ++jg) {
+                        const uint32_t bc = bar(BAR_CODE_FULL + jg) + 16u * odd, ba = bar(BAR_A_FULL + jg), be = bar(BAR_ACC_EMPTY) + 8u * (v_run & 1);
+                        const uint32_t pc = (s_run >> 1) & 1, pe = ((v_run >> 1) & 1) ^ 1;
+                        // one look at all of them costs the issuer what a wait for one of them does, some 100 clk
+                        const bool ready = mbar_try(bc, pc) & mbar_try(ba, odd) & (jg > 0 || mbar_try(be, pe));
+                        if (!__all_sync(0xFFFFFFFFu, ready)) ok = WAITP(2, bc, pc) && WAITP(4, ba, odd) && (jg > 0 || WAITP(7, be, pe));
+                        if (!ok) break;
                         tc_fence_after();
 #pragma unroll
-                        for (int jj = 0; jj < GB; ++jj) block(acc, gs, ct, jj, (uint32_t)(jg + jj > 0));
-                        tc_commit_one(leader, bar(BAR_A_EMPTY + gs));
-                        tc_commit_one(leader, bar(BAR_CODE_EMPTY + ct));
+                        for (int jj = 0; jj < GB; ++jj) {
+                            const uint32_t a = tmem_base + A_BASE + (uint32_t)((jg * GB + jj) * A_COLS);
+                            const uint64_t d = umma_desc_on(db, jg * CODE_STAGE + jj * CODE_BLOCK);
+                            umma_ts(leader, acc, a, d, idesc, (uint32_t)(jg + jj > 0));
+                            umma_ts(leader, acc, a + 8, umma_desc_on(d, 256), idesc, 1u);
+                        }
+                        tc_commit_one(leader, bar(BAR_A_EMPTY + jg));
+                        tc_commit_one(leader, bar(BAR_CODE_EMPTY + jg) + 16u * odd);
                     }
-                    if (!ok || !mins(xt)) { ok = false; break; }
+                    if (!ok || !mins(xt, y_of(U, v_run), was_short && short_tile(U))) { ok = false; break; }
+                    was_short = short_tile(U);
                     tc_commit_one(leader, bar(BAR_ACC_FULL + (v_run & 1)));
                     tc_commit_one(leader, bar(BAR_X_EMPTY + xt));
                 }
@@ -452,7 +472,6 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 #pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int xt = s_run % NX;
-                if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
 #pragma unroll 1
                 for (int j = 0; j < SB; ++j) {
                     const int g = 2 * s_run + j / GB, gs = g % NG, ct = g % NCODE;
@@ -469,7 +488,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                     }
                     if (j % CB == CB - 1) {
                         if (j == CB - 1) {                                                // the first chain takes the mins along
-                            if (!mins(xt)) { ok = false; break; }
+                            if (!mins(xt, Y_BASE, false)) { ok = false; break; }
                             tc_commit_one(leader, bar(BAR_X_EMPTY + xt));
                         }
                         tc_commit_one(leader, bar(BAR_ACC_FULL + (v_run & 1)));
@@ -519,11 +538,10 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 #pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int st = s_run % NRAW, xt = s_run % NX;
-                if (!WAITP(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1)) { ok = false; break; }
+                // the row's bytes, and the place of its scales: every scaling warp is done with the super-block NX back
+                if (!WAITP2(0, bar(BAR_RAW_FULL + st), (s_run / NRAW) & 1, 5, bar(BAR_X_EMPTY + xt), ((s_run / NX) & 1) ^ 1)) { ok = false; break; }
                 const uint8_t *blk = smem + L::RAW_OFF + st * L::RAW_STAGE + r * SBB;
                 const uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
-                // the place of the row's scales: every scaling warp is done with the super-block NX back
-                if (!WAITP(5, bar(BAR_X_EMPTY + xt), ((s_run / NX) & 1) ^ 1)) { ok = false; break; }
                 if (uu == 0)
                     *reinterpret_cast<float2 *>(smem + L::DW_OFF + (xt * BM + r) * 8) =
                         make_float2(half_bits_to_float((uint16_t)(hdr.x & 0xFFFFu)), -half_bits_to_float((uint16_t)(hdr.x >> 16)));
@@ -579,22 +597,22 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
 #pragma unroll 1
             for (int s = U.sb0; s < U.sb1 && ok; ++s, ++s_run) {
                 const int xt = s_run % NX;
-                if (!WAITP(2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
 #pragma unroll 1
                 for (int ch = 0; ch < chains; ++ch, ++v_run) {
                     const int buf = v_run & 1;
-                    if (!WAITP(6, bar(BAR_ACC_FULL + buf), (v_run >> 1) & 1)) { ok = false; break; }
+                    if (!WAITP2(6, bar(BAR_ACC_FULL + buf), (v_run >> 1) & 1, 2, bar(BAR_X_FULL + xt), (s_run / NX) & 1)) { ok = false; break; }
                     tc_fence_after();
                     if (live) {
                         // rows 16 rh .. + 15 of the quarter at a time: X and Y, all columns, in flight together
+                        const uint32_t y_base = chains == 1 ? y_of(U, v_run) : (uint32_t)Y_BASE;
                         uint32_t vx[2][16], vy[2][16];
                         auto load = [&](int rh) {
                             const uint32_t a = tq + ((uint32_t)(rh * 16) << 16);
                             tmem_ld_16x256_x4(a + (uint32_t)buf * BN, vx[0]);
-                            tmem_ld_16x256_x4(a + Y_BASE, vy[0]);
+                            tmem_ld_16x256_x4(a + y_base, vy[0]);
                             if (two) {
                                 tmem_ld_16x256_x4(a + (uint32_t)buf * BN + 32, vx[1]);
-                                tmem_ld_16x256_x4(a + Y_BASE + 32, vy[1]);
+                                tmem_ld_16x256_x4(a + y_base + 32, vy[1]);
                             }
                         };
                         load(0);
@@ -647,7 +665,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
+                    for (int i = 0; i < 8; ++i) {
+                        if (i >= 4 && !two) break;
 #pragma unroll
                         for (int d = 0; d < 2; ++d) {
                             const int col = 8 * i + 2 * c + d;
@@ -659,6 +678,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                                 if (col < ncol && r0 + 8 * k < U.valid_rows) dst[o + U.row0 + r0 + 8 * k] = a[d];
                             }
                         }
+                    }
                 } else {
                     float *o = dst + (int64_t)U.part * part_stride + (int64_t)(U.tile_n * BN + cbase + 2 * c) * ldd + U.row0 + r0;
 #pragma unroll

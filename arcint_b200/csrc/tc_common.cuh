@@ -57,6 +57,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag) ? 1 : 0) != 0;
 }
+// Two barriers, usually both ready: one look and one vote cost a warp what a wait for one of them does, some 100 clk.
+__device__ __forceinline__ bool mbar_ready_warp(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+    const bool a = mbar_try(bar0, parity0), b = mbar_try(bar1, parity1);
+    return __all_sync(0xFFFFFFFFu, a && b ? 1 : 0) != 0;
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -86,6 +91,10 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t addr) {
 // the same with the two strides given: lbo between the 16-byte halves of K, sbo between 8-row groups
 __device__ __forceinline__ uint64_t umma_desc2(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
+}
+// the descriptor of an address `bytes` on (shared-memory addresses stay below 2^18, so the sum carries nowhere)
+__device__ __forceinline__ uint64_t umma_desc_on(uint64_t desc, uint32_t bytes) {
+    return (desc & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)desc + (bytes >> 4));
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -221,6 +230,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 #define WAITP(slot, b, par) mbar_wait_warp(b, par, abortp)
 #define PROF_DUMP(role)
 #endif
+#define WAITP2(slot0, b0, par0, slot1, b1, par1) (mbar_ready_warp(b0, par0, b1, par1) || (WAITP(slot0, b0, par0) && WAITP(slot1, b1, par1)))
 
 }  // namespace tc
 }  // namespace b200q
