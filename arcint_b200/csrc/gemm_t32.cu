@@ -314,6 +314,8 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
         // ---- MMA issuers, one for each half of the columns: the waits and the issue of a job are a serial chain ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;" ::: "memory");
         const uint32_t leader = elect_one();
+        const uint64_t code_desc = umma_desc2(sbase + L::ACT_OFF, 128, GROUP);
+        const uint64_t scale_desc = umma_desc2(sbase + L::ACT_OFF + GROUP_SCALES, GROUP_ZERO - GROUP_SCALES, GROUP);
         const int h = warp - 1;
         int c_run = 0, buf = h;                           // activation stages so far; the job's buffer
         bool ok = true;
@@ -327,17 +329,19 @@ gemm_t32_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const ui
             for (int c = 2 * U.sb0; c < 2 * U.sb1 && ok; ++c, ++c_run) {
                 const int at = c_run % NACT;
                 if (!WAITP(2, bar(BAR_ACT_FULL + at), (c_run / NACT) & 1)) { ok = false; break; }
-                const uint32_t stage = sbase + L::ACT_OFF + at * STAGE + half_off;
+                const uint64_t codes = umma_desc_on(code_desc, at * STAGE + half_off), scales = umma_desc_on(scale_desc, at * STAGE + half_off);
 #pragma unroll
                 for (int jj = 0; jj < HB; ++jj) {
                     const uint32_t a = tmem_base + A_BASE + jj * SLOT_COLS;          // (a block's slot is its place in the stage)
+                    const uint32_t acc = tmem_base + (uint32_t)buf * BN;
+                    // (the scales' second piece is the block of zeros, so much nearer the further on the block)
+                    const uint64_t b = umma_desc_on(codes, jj * CODE_BLOCK), bs = umma_desc_on(scales, jj * 128) - ((uint64_t)(jj * 128 >> 4) << 16);
                     if (!WAITP(4, bar(BAR_READY + 2 * jj + h), c_run & 1)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t acc = tmem_base + (uint32_t)buf * BN, b = stage + jj * CODE_BLOCK, bs = stage + GROUP_SCALES + jj * 128;
                     // K = 16 per MMA: eight columns of A, two pieces of B
-                    umma_ts(leader, acc, a, umma_desc2(b, 128, GROUP), idesc, 0u);
-                    umma_ts(leader, acc, a + 8, umma_desc2(b + 256, 128, GROUP), idesc, 1u);
-                    umma_ts(leader, acc + 64, a + 16, umma_desc2(bs, GROUP_ZERO - GROUP_SCALES - jj * 128, GROUP), idesc, 0u);
+                    umma_ts(leader, acc, a, b, idesc, 0u);
+                    umma_ts(leader, acc, a + 8, umma_desc_on(b, 256), idesc, 1u);
+                    umma_ts(leader, acc + 64, a + 16, bs, idesc, 0u);
                     tc_commit_one(leader, bar(BAR_FULL + 2 * jj + h));
                     tc_commit_one(leader, bar(BAR_FREE + jj));
                     buf = buf == 0 ? 2 : buf - 1;                                    // two jobs on, modulo three
