@@ -369,7 +369,7 @@ b200q_status b200q_init(b200q_ctx **out, int device, void *stream) {
         b200q_free(ctx);
         return B200Q_CUDA_ERROR;
     }
-    if (cudaMalloc(&ctx->error_word, sizeof(int)) != cudaSuccess || cudaMemset(ctx->error_word, 0, sizeof(int)) != cudaSuccess) {
+    if (cudaMalloc(&ctx->error_word, 4 * sizeof(int)) != cudaSuccess || cudaMemset(ctx->error_word, 0, 4 * sizeof(int)) != cudaSuccess) {
         b200q_free(ctx);
         return B200Q_NO_MEMORY;
     }

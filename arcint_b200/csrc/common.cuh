@@ -165,7 +165,9 @@ struct b200q_ctx {
     size_t       route_next = 0;
     cudaEvent_t  ev0 = nullptr, ev1 = nullptr;
     void        *tp = nullptr;   // tensor/expert-parallel state (tp.cu)
-    int         *error_word = nullptr;   // device word a kernel sets when a bounded wait runs out
+    // device words: one a kernel sets when a bounded wait runs out, a spare one, and the units that a route's product has dealt out and the blocks
+    // that are through with it (gemm_kf.cu: zero between launches)
+    int         *error_word = nullptr;
 };
 
 namespace b200q {

@@ -63,6 +63,7 @@ constexpr int A_COLS = 16;                                // tensor-memory colum
 constexpr int Y_BASE = 2 * BN, A_BASE = 3 * BN;           // tensor memory: X0, X1, Y, A ring
 static_assert(A_BASE + NG * GB * A_COLS <= 512, "tensor memory");
 constexpr int NCODE = 4;                                  // stages of activation codes (half a super-block each) in flight
+constexpr int DEALT = 4;                                  // units of a route on their way from the raw producer to the other warps
 constexpr int NX = 4;                                     // super-blocks of activation scales, mins operands and row scales in flight
 constexpr int THREADS = 32 * 20;                          // warp groups: {producer, MMA, 2 producers of codes}, 2 x unpack, 2 x scale-accumulate
 // Registers per thread by role (setmaxnreg): a warp group that asks for more waits until others have
@@ -265,7 +266,8 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     constexpr int SBB = Fmt<TYPE>::SBB, NRAW = L::NRAW;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag, more_slot;
+    __shared__ int abort_flag, more_slot, dealt[DEALT];
+    __shared__ __align__(8) uint64_t dealt_bar[2 * DEALT];
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler, too)
     const int nsb = K / 256;                    // super-blocks of a row
     const uint32_t sbase = smem_u32(smem);
@@ -276,8 +278,10 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     // the unpacking and the MMAs of the next tile run while the last tile's results are stored).
     // Units of one row tile are neighbours, so blocks running together share weight rows in L2 (MUL_MAT_ID: the
     // tiles of one expert). A contiguous run of units per block measured slower on the 512-expert configuration (+18 %:
-    // the full tiles of busy experts pile up on a few blocks). A dense product with few tiles is cut along K: a unit is
-    // then one part of a tile and writes part `part` of a scratch buffer.
+    // the full tiles of busy experts pile up on a few blocks). A route's units differ in width: after the first, a block takes the next that nobody
+    // has, one ahead (the raw producer asks for it and hands it to the other roles): with every 148th unit a block's share
+    // the slowest block took 174k clk of a mean 149k; the 512-expert block over 2048 tokens 494 -> 480 us. A dense product with
+    // few tiles is cut along K: a unit is then one part of a tile and writes part `part` of a scratch buffer.
     // Launched with programmatic dependence behind this product's own quantizer, which has waited for what came before it: a block may
     // read the weights at once, the producer waits before its first activation load, the scaling warps before they store. A
     // route's tile list is read by everybody. (Where the activation was there already the launch before may be anybody's, the
@@ -308,7 +312,20 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         U.cw = FULL || U.ncols > 64 ? 64 : max(16, (((U.ncols + 1) >> 1) + 15) & ~15);
         return U;
     };
-    if ((int)blockIdx.x >= n_units) return;               // the whole block: nothing is set up yet
+    // error_word[2]: units dealt out beyond each block's first; [3]: blocks that are through, the last of which sets both back to zero. A route's
+    // product has waited for everything before it, so no two launches use them at once.
+    auto through = [&]() {
+        __threadfence();
+        if (ROUTE && atomicAdd(error_word + 3, 1) == (int)gridDim.x - 1) {
+            error_word[2] = error_word[3] = 0;
+            __threadfence();
+        }
+    };
+    if ((int)blockIdx.x >= n_units) {                     // the whole block: nothing is set up yet
+        if (threadIdx.x == 0) through();
+        return;
+    }
+    const uint32_t dealt_full = smem_u32(dealt_bar), dealt_empty = dealt_full + 8 * DEALT;
     // whether one of this thread's share of the one-sided sums asks for more than one chain. Every block reads them all: a route's, with its
     // many tiles, by all threads (a block waits first anyway), a dense product's by one scaling warp behind its wait, so that weights
     // are fetched and unpacked meanwhile (asking with the whole block costs 2 us a launch).
@@ -349,6 +366,10 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
             mbar_init(bar(BAR_ACC_EMPTY + i), 8);                  // scaling warps
         }
         mbar_init(bar(BAR_MORE), 1);
+        for (int i = 0; i < DEALT; ++i) {
+            mbar_init(dealt_full + 8 * i, 1);
+            mbar_init(dealt_empty + 8 * i, THREADS / 32 - 1);      // all warps but the raw producer
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -369,6 +390,17 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     auto short_tile = [](const Unit &U) { return !FULL && U.ncols <= 64; };
     auto y_of = [&](const Unit &U, int chain) { return (uint32_t)(Y_BASE + (short_tile(U) ? (chain & 1) * 64 : 0)); };
     PROF_DECL
+    // a route's unit after this role's k-th (counted from 0), from the raw producer
+    auto unit_after = [&](int k, bool &ok) {
+        const int slot = k % DEALT;
+        if (!WAITP(0, dealt_full + 8 * slot, (k / DEALT) & 1)) {
+            ok = false;
+            return n_units;
+        }
+        const int next = *(volatile int *)&dealt[slot];
+        mbar_arrive_warp(dealt_empty + 8 * slot, lane);
+        return next;
+    };
 
     if (warp == 0) {
         // ---- producer ----
@@ -377,7 +409,9 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         int s_run = 0;                                    // super-blocks fetched so far
         bool ok = true;
 #pragma unroll 1
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        for (int u = blockIdx.x, k = 0; u < n_units && ok; ++k) {
+            int next = u + (int)gridDim.x;
+            if (ROUTE && lane == 0) next = atomicAdd(error_word + 2, 1) + (int)gridDim.x;          // (back before it is needed)
             const Unit U = unit_of(u);
             const uint8_t *act_tile = act + (size_t)U.tile_n * nsb * CHUNK;
             const uint32_t groups = (uint32_t)(U.ncols + 7) >> 3;          // live column groups
@@ -400,6 +434,16 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
                 }
                 __syncwarp();
             }
+            if (ROUTE && ok) {
+                const int slot = k % DEALT;
+                if (!WAITP(0, dealt_empty + 8 * slot, ((k / DEALT) & 1) ^ 1)) { ok = false; break; }
+                if (lane == 0) {
+                    *(volatile int *)&dealt[slot] = next;
+                    mbar_arrive(dealt_full + 8 * slot);
+                }
+                next = __shfl_sync(0xFFFFFFFFu, next, 0);
+            }
+            u = next;
         }
     } else if (warp == 1) {
         // ---- MMA issuer ----
@@ -431,7 +475,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
         const bool more = *(volatile int *)&more_slot != 0;
 #pragma unroll 1
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        for (int u = blockIdx.x, k = 0; u < n_units && ok; u = ROUTE ? unit_after(k++, ok) : u + (int)gridDim.x) {
             const Unit U = unit_of(u);
             idesc = IDESC | ((uint32_t)((U.ncols + 15) >> 4) << 18);                      // N: the live columns, in sixteens
             if (!more) {
@@ -506,7 +550,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         bool ok = true;
         pdl_wait();
 #pragma unroll 1
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        for (int u = blockIdx.x, k = 0; u < n_units && ok; u = ROUTE ? unit_after(k++, ok) : u + (int)gridDim.x) {
             const Unit U = unit_of(u);
             // only the column groups the tile has; the MMA still reads a multiple of sixteen columns, the rest of the
             // stage holds older codes whose products land in accumulator columns nobody stores
@@ -532,7 +576,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         int s_run = 0;
         bool ok = true;
 #pragma unroll 1
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        for (int u = blockIdx.x, k = 0; u < n_units && ok; u = ROUTE ? unit_after(k++, ok) : u + (int)gridDim.x) {
             const Unit U = unit_of(u);
             const bool row_ok = r < U.valid_rows;
 #pragma unroll 1
@@ -584,7 +628,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
         bool ok = ROUTE || WAITP(2, bar(BAR_MORE), 0);
         const int chains = *(volatile int *)&more_slot ? Fmt<TYPE>::CHAINS : 1;
 #pragma unroll 1
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        for (int u = blockIdx.x, k = 0; u < n_units && ok; u = ROUTE ? unit_after(k++, ok) : u + (int)gridDim.x) {
             const Unit U = unit_of(u);
             const int cbase = half * U.cw, ncol = FULL ? 64 : min(U.cw, U.ncols - cbase);     // this half's columns inside the tile (none: <= 0)
             const bool live = FULL || ncol > 0, two = FULL || ncol > 32;
@@ -702,6 +746,7 @@ gemm_kf_kernel(const __grid_constant__ CUtensorMap wmap, int M, int K, const uin
     PROF_DUMP(warp == 1 ? "mma " : warp < 4 ? "prod" : warp < 12 ? "unpk" : "epi ")
     tc_fence_before();
     __syncthreads();
+    if (ROUTE && threadIdx.x == 0) through();
     pdl_trigger();
     if (abort_flag) {
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
