@@ -348,7 +348,8 @@ b200q_status launch_one_column(b200q_ctx *ctx, const void *w, int64_t M, int64_t
 #define B200Q_GEMV_TYPE(EXTERN, TYPE)                                                                                          \
     EXTERN template b200q_status launch_type<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, float *, int64_t, int); \
     EXTERN template b200q_status launch_id_type<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, float *, int, \
-                                                      const GemvId &, int64_t);                                              \
+                                                      const GemvId &, int64_t);
+#define B200Q_GEMV_TYPE_ONE(EXTERN, TYPE)                                                                                      \
     EXTERN template b200q_status launch_one_column<TYPE>(b200q_ctx *, const void *, int64_t, int64_t, const float *, float *, bool);
 #define B200Q_GEMV_TYPE_AR(EXTERN, TYPE)                                                                                       \
     EXTERN template b200q_status launch_ar_type<TYPE>(b200q_ctx *, const void *, size_t, int64_t, int64_t, const GemvAct &, int, bool, float *, \

@@ -34,7 +34,7 @@ namespace b200q {
 constexpr int GEMV_ONE_WARPS = 16;                        // warps of a block, at most
 constexpr size_t GEMV_ONE_SMEM = 113 * 1024;              // two blocks an SM
 
-template <int TYPE> __host__ __device__ constexpr bool gemv_one_per32() { return TYPE == B200Q_TYPE_Q4_0 || TYPE == B200Q_TYPE_Q8_0 || TYPE == B200Q_TYPE_IQ4_NL; }
+template <int TYPE> __host__ __device__ constexpr bool gemv_one_per32() { return TYPE == B200Q_TYPE_Q4_0 || TYPE == B200Q_TYPE_Q8_0; }
 // bytes of a slice's place in a ring (it begins up to 15 bytes in, and the lane code reads a word past it), and places of a ring
 template <int TYPE> __host__ __device__ constexpr int gemv_one_slot() { return (GemvStage<TYPE>::BYTES + 15 + 4 + 15) / 16 * 16; }
 // (two blocks an SM. Rings that take most of an SM were no faster for long streams: 32000x4096 in Q4_K 15.7 us with eight places and with
@@ -132,7 +132,6 @@ template <int TYPE> struct gemv_one_act { typedef GemvX<1> type; };
 struct GemvOneX;
 template <> struct gemv_one_act<B200Q_TYPE_Q4_0> { typedef GemvOneX type; };
 template <> struct gemv_one_act<B200Q_TYPE_Q8_0> { typedef GemvOneX type; };
-template <> struct gemv_one_act<B200Q_TYPE_IQ4_NL> { typedef GemvOneX type; };
 // The per-32 types' lane code for rows of whole words (an even number of blocks): lane l has the blocks 2 l and 2 l + 1 of the slice, 9 or 17
 // whole words an odd number apart, so that no two lanes meet in a bank and only the first block's codes have to be shifted. (As in
 // gemv_core.cuh, blocks l and l + 32, it takes 12 and 20 words, two lanes a bank.)
@@ -178,12 +177,6 @@ __device__ __forceinline__ float gemv_one_row(const uint32_t *p, const GemvOneX 
             s0 = dp4a_ss(q[2], xa.z, s0); s1 = dp4a_ss(q[3], xa.w, s1);
             s0 = dp4a_ss(q[4], xb.x, s0); s1 = dp4a_ss(q[5], xb.y, s1);
             s0 = dp4a_ss(q[6], xb.z, s0); s1 = dp4a_ss(q[7], xb.w, s1);
-            si = s0 + s1;
-        } else if constexpr (TYPE == B200Q_TYPE_IQ4_NL) {
-            int s0 = dp4a_ss(iq4nl_lookup4(q[0] & 0x0F0F0F0Fu), xa.x, 0), s1 = dp4a_ss(iq4nl_lookup4(q[1] & 0x0F0F0F0Fu), xa.y, 0);
-            s0 = dp4a_ss(iq4nl_lookup4(q[2] & 0x0F0F0F0Fu), xa.z, s0); s1 = dp4a_ss(iq4nl_lookup4(q[3] & 0x0F0F0F0Fu), xa.w, s1);
-            s0 = dp4a_ss(iq4nl_lookup4((q[0] >> 4) & 0x0F0F0F0Fu), xb.x, s0); s1 = dp4a_ss(iq4nl_lookup4((q[1] >> 4) & 0x0F0F0F0Fu), xb.y, s1);
-            s0 = dp4a_ss(iq4nl_lookup4((q[2] >> 4) & 0x0F0F0F0Fu), xb.z, s0); s1 = dp4a_ss(iq4nl_lookup4((q[3] >> 4) & 0x0F0F0F0Fu), xb.w, s1);
             si = s0 + s1;
         } else {
             // weights 4j..4j+3 in the low nibbles, 16+4j.. in the high ones (left x16)

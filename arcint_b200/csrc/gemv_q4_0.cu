@@ -4,6 +4,7 @@
 namespace b200q {
 
 B200Q_GEMV_TYPE(, B200Q_TYPE_Q4_0)
+B200Q_GEMV_TYPE_ONE(, B200Q_TYPE_Q4_0)
 B200Q_GEMV_TYPE_AR(, B200Q_TYPE_Q4_0)
 B200Q_GEMV_TYPE_FUSED(, B200Q_TYPE_Q4_0)
 

@@ -4,5 +4,6 @@
 namespace b200q {
 
 B200Q_GEMV_TYPE(, B200Q_TYPE_Q5_K)
+B200Q_GEMV_TYPE_ONE(, B200Q_TYPE_Q5_K)
 
 }  // namespace b200q

@@ -9,7 +9,8 @@ import oracle as O
 from gpu_util import TOL, check_sums, make_weights, rel_err
 
 pytestmark = pytest.mark.gpu
-TYPES = [A.Q4_0, A.Q8_0, A.IQ4_NL, A.Q4_K, A.Q5_K, A.Q6_K, A.IQ4_XS]
+# (the super-block types take it from 8 or 12 MB of weights)
+LEAST = {A.Q4_K: 8 << 20, A.Q5_K: 8 << 20, A.Q6_K: 12 << 20}
 
 
 @pytest.fixture(scope="module")
@@ -23,7 +24,23 @@ def one(ctx):
     return ctx.stats().get("gemv_fused_quant", 0)
 
 
-@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("t", list(LEAST))
+@pytest.mark.parametrize("k", [256, 2048, 2304, 4352, 11008])
+def test_super_block_types(ctx, t, k):
+    m = max(1 if t == A.Q6_K else 2048, -(-LEAST[t] // A.row_bytes(t, k)))     # the fewest rows, and one less
+    w = make_weights(t, m, k, 3 * t + k)
+    x = np.random.default_rng(m + k).normal(0, 1, (1, k)).astype(np.float32)
+    x[0, :32] = 0
+    ctx.stats_reset()
+    got = ctx.run_mul_mat(t, w, k, x)
+    assert one(ctx) == 1
+    check_sums(got, t, w, k, x)
+    less = ctx.run_mul_mat(t, w[:-1], k, x)
+    assert one(ctx) == 1
+    check_sums(less, t, w[:-1], k, x)
+
+
+@pytest.mark.parametrize("t", [A.Q4_0, A.Q8_0])
 @pytest.mark.parametrize("m,k", [(1, 256), (149, 256), (147, 2048), (1000, 2304), (300, 4352), (200, 11008), (40, 32768), (9000, 512)])
 def test_shapes(ctx, t, m, k):
     w = make_weights(t, m, k, 3 * t + k)
@@ -36,7 +53,7 @@ def test_shapes(ctx, t, m, k):
     check_sums(got, t, w, k, x)
 
 
-@pytest.mark.parametrize("t,m,k", [(A.Q4_0, 70, 64), (A.Q8_0, 300, 320), (A.IQ4_NL, 300, 6208)])
+@pytest.mark.parametrize("t,m,k", [(A.Q4_0, 70, 64), (A.Q8_0, 300, 320), (A.Q4_0, 300, 6208)])
 def test_rows_of_32_weight_blocks(ctx, t, m, k):
     w = make_weights(t, m, k, 5)
     x = np.random.default_rng(m).normal(0, 1, (1, k)).astype(np.float32)
@@ -48,12 +65,12 @@ def test_rows_of_32_weight_blocks(ctx, t, m, k):
 def test_what_takes_the_two_kernel_route(ctx):
     """An odd number of 18-byte blocks, padded rows, K beyond sixteen slices, results that land in the activation."""
     x = np.random.default_rng(1).normal(0, 1, (1, 33024)).astype(np.float32)
-    for t, m, k in ((A.Q4_0, 20, 96), (A.Q4_K, 20, 33024)):
+    for t, m, k in ((A.Q4_0, 20, 96), (A.Q8_0, 20, 33024), (A.IQ4_NL, 300, 512), (A.IQ4_XS, 300, 512)):
         w = make_weights(t, m, k, 6)
         ctx.stats_reset()
         check_sums(ctx.run_mul_mat(t, w, k, x[:, :k]), t, w, k, x[:, :k])
         assert one(ctx) == 0
-    t, m, k = A.Q4_K, 512, 512
+    t, m, k = A.Q8_0, 512, 512
     w = make_weights(t, m, k, 7)
     rb = w.shape[1]
     padded = np.zeros((m, rb + 16), np.uint8)
