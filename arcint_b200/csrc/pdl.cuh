@@ -9,8 +9,8 @@
 // next kernel be scheduled: the small quantizers call it first thing (those of the prompt products after their wait: the GEMM behind
 // them then reads weights that all earlier work has written), the GEMV when a block has finished its
 // rows (triggered at its start, the blocks of later kernels would occupy the places of its own wave: measured
-// 40 % slower). Both calls do nothing in a kernel
-// launched the plain way. Stream capture keeps the edges, so CUDA graphs replay with them.
+// 40 % slower); gemv_one.cuh, whose blocks leave room beside them, right behind its wait, or at once where it
+// waits only to store. Both calls do nothing in a kernel launched the plain way. Stream capture keeps the edges, so CUDA graphs replay with them.
 #pragma once
 
 #include <cuda_runtime.h>
